@@ -187,6 +187,7 @@ def prepare(case, seed):
     elif kind == "md":
         st["md"] = DeviceRigidWaterMD(_box(case, seed), precision=case["precision"], dt=DT, temperature=TEMPERATURE,
                                       seed=seed, ewald=case["ewald"])
+        st["turn"] = 20
     elif kind == "clusters":
         b = ClusterBatch(_cluster_list(case, seed), precision=case["precision"])
         b.setStream(stream)
@@ -226,7 +227,11 @@ def run(st):
                                         A.F32 if dtype == torch.float32 else A.F64)
         return {"energy": e, "forces": st["frc"]}
     if kind == "md":
+        # The force has no repulsion: left alone, molecules run into one another within some hundred steps.  Velocities
+        # turn round every 20 steps, which leads back along the same path, so a long run stays at the liquid's spacing.
         md = st["md"]
+        if md.steps and md.steps % st["turn"] == 0:
+            md.vel.neg_()
         e = md.step(1)
         # the frame that goes to a trajectory: single precision from the mixed form
         return {"energy": e, "forces": md.frc.to(dtype), "positions": md.pos.to(dtype), "velocities": md.vel.to(dtype)}
