@@ -1582,7 +1582,8 @@ int tdp_get_potential(tdp_handle* h, const void* positions, int32_t pos_dtype, i
         double* dgrid = nullptr;
         double* dout = nullptr;
         TDP_CUDA(cudaMallocAsync((void**)&dgrid, sizeof(double) * 3 * num_points, st));
-        TDP_CUDA(cudaMallocAsync((void**)&dout, sizeof(double) * num_points, st));
+        TDP_CUDA(cudaMallocAsync((void**)&dout,
+                                 sizeof(double) * (size_t)num_points * potential_chunks(h->n, num_points), st));
         TDP_CUDA(cudaMemcpyAsync(dgrid, grid, sizeof(double) * 3 * num_points, cudaMemcpyHostToDevice, st));
         launch_potential(h->d, dgrid, num_points, dout, st);
         TDP_CUDA(cudaMemcpyAsync(out, dout, sizeof(double) * num_points, cudaMemcpyDeviceToHost, st));

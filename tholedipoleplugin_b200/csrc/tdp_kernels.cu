@@ -14,6 +14,8 @@
 
 #include <math.h>
 
+#include <algorithm>
+
 namespace tdp {
 
 // ---------------------------------------------------------------------------
@@ -560,30 +562,65 @@ __global__ void k_forces_out_fixed(int n, const double* __restrict__ f, const in
 }
 
 // Electrostatic potential at grid points, calculateElectrostaticPotential-
-// ForParticleGridPoint (RTDF.cpp:1348-1372), FP64.
-__global__ void k_potential(int n, int ng, PairParams P, const double* __restrict__ pos,
-                            const double* __restrict__ charge, const double* __restrict__ lab,
-                            const double* __restrict__ mu, const double* __restrict__ grid, double* __restrict__ out) {
-    int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= ng) return;
-    d3 gp = ld3(grid + 3 * g);
+// ForParticleGridPoint (RTDF.cpp:1348-1372), FP64.  Bound by the FP64 pipe:
+// about 26 operations a pair.  One thread per point alone left small grids on
+// a few warps per SM, every one stalled on a chain of divide and square root
+// and on its loads (32,768 points x 12,288 atoms: 6.04 ms, now 0.91 ms), so
+// blocks take (128 points, a chunk of atoms) with the atoms staged in shared
+// memory and the chunks' sums are added in order by k_potential_sum.  The minimum image
+// is evaluated only where a component reaches half a box: below that the
+// reference's floor(d/L + 0.5) is 0 and the displacement stays as it is.
+constexpr int kPotPoints = 128;   // points (threads) per block
+constexpr int kPotAtoms = 128;    // atoms staged per step
+
+__global__ void __launch_bounds__(kPotPoints) k_potential(int n, int ng, int chunk, PairParams P,
+                                                          const double* __restrict__ pos,
+                                                          const double* __restrict__ charge,
+                                                          const double* __restrict__ lab,
+                                                          const double* __restrict__ mu,
+                                                          const double* __restrict__ grid, double* __restrict__ part) {
+    __shared__ double2 s_a[kPotAtoms][4];   // (x, y) (z, q) (dx, dy) (dz, -)
+    const int g = blockIdx.x * kPotPoints + threadIdx.x;
+    const int a0 = blockIdx.y * chunk, a1 = min(a0 + chunk, n);
+    const d3 gp = g < ng ? ld3(grid + 3 * g) : d3{0.0, 0.0, 0.0};
+    double half[3];
+    for (int c = 0; c < 3; c++) half[c] = P.periodic && P.box[c] > 0.0 ? 0.4999999 * P.box[c] : INFINITY;
     double pot = 0.0;
-    for (int i = 0; i < n; i++) {
-        d3 dr = ld3(pos + 3 * i) - gp;
-        if (P.periodic) {
-            dr.x = fold_d(dr.x, P.box[0], P.inv_box[0]);
-            dr.y = fold_d(dr.y, P.box[1], P.inv_box[1]);
-            dr.z = fold_d(dr.z, P.box[2], P.inv_box[2]);
+    for (int base = a0; base < a1; base += kPotAtoms) {
+        __syncthreads();
+        const int k = threadIdx.x, i = base + k;
+        if (i < a1) {
+            const d3 p = ld3(pos + 3 * i), m = ld3(lab + 3 * i) + ld3(mu + 3 * i);
+            s_a[k][0] = make_double2(p.x, p.y);
+            s_a[k][1] = make_double2(p.z, charge[i]);
+            s_a[k][2] = make_double2(m.x, m.y);
+            s_a[k][3] = make_double2(m.z, 0.0);
         }
-        double r = sqrt(dot(dr, dr));
-        double rr1 = 1.0 / r, rr2 = rr1 * rr1, rr3 = rr1 * rr2;
-        double p = charge[i] * rr1;
-        double scd = dot(ld3(lab + 3 * i), dr);
-        double scu = dot(ld3(mu + 3 * i), dr);
-        p -= (scd + scu) * rr3;
-        pot += p;
+        __syncthreads();
+        const int cnt = min(kPotAtoms, a1 - base);
+#pragma unroll 4
+        for (int j = 0; j < cnt; j++) {
+            const double2 u = s_a[j][0], v = s_a[j][1], w = s_a[j][2];
+            double dx = u.x - gp.x, dy = u.y - gp.y, dz = v.x - gp.z;
+            if (fabs(dx) >= half[0]) dx = fold_d(dx, P.box[0], P.inv_box[0]);
+            if (fabs(dy) >= half[1]) dy = fold_d(dy, P.box[1], P.inv_box[1]);
+            if (fabs(dz) >= half[2]) dz = fold_d(dz, P.box[2], P.inv_box[2]);
+            const double rr1 = rsqrt(dx * dx + dy * dy + dz * dz);
+            const double rr3 = rr1 * rr1 * rr1;
+            pot += v.y * rr1 - (w.x * dx + w.y * dy + s_a[j][3].x * dz) * rr3;
+        }
     }
-    out[g] = pot;
+    if (g < ng) part[(size_t)blockIdx.y * ng + g] = pot;
+}
+
+// Potential of the chunks, in chunk order; the result goes to chunk 0's row.
+__global__ void k_potential_sum(int ng, int nchunk, double* __restrict__ part) {
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g >= ng) return;
+    double s = 0.0;
+#pragma unroll 8
+    for (int k = 0; k < nchunk; k++) s += part[(size_t)k * ng + g];
+    part[g] = s;
 }
 
 // Block partial sums for the system multipole moments
@@ -794,8 +831,19 @@ void launch_forces_out_fixed(const Dev& d, const int* atom_index, int padded, lo
     k_forces_out_fixed<<<nblk(d.n, kVecThreads), kVecThreads, 0, st>>>(d.n, d.ftotal, atom_index, padded,
                                                                         (unsigned long long*)acc);
 }
-void launch_potential(const Dev& d, const double* grid, int ng, double* out, cudaStream_t st) {
-    k_potential<<<nblk(ng, 128), 128, 0, st>>>(d.n, ng, d.pp, d.pos, d.charge, d.lab, d.mu, grid, out);
+// Chunks of atoms for ng points: enough blocks for 16 resident per SM (the
+// register limit) in whole rounds, no chunk below one staged step.
+int potential_chunks(int n, int ng) {
+    const long gb = nblk(ng, kPotPoints);
+    const long want = (16L * 148 + gb - 1) / gb;
+    return (int)std::max(1L, std::min(want, (long)nblk(n, kPotAtoms)));
+}
+void launch_potential(const Dev& d, const double* grid, int ng, double* part, cudaStream_t st) {
+    const int want = potential_chunks(d.n, ng);
+    const int chunk = nblk(d.n, want), m = nblk(d.n, chunk);
+    k_potential<<<dim3(nblk(ng, kPotPoints), m), kPotPoints, 0, st>>>(d.n, ng, chunk, d.pp, d.pos, d.charge, d.lab,
+                                                                      d.mu, grid, part);
+    if (m > 1) k_potential_sum<<<nblk(ng, 256), 256, 0, st>>>(ng, m, part);
 }
 void launch_moments(const Dev& d, const double* mass, double* scratch, double* out13, cudaStream_t st) {
     int nb = d.nvb;

@@ -121,7 +121,9 @@ void launch_add_forces(const Dev& d, void* acc, int is_f32, cudaStream_t st);
 void launch_positions_in(const Dev& d, const void* src, int is_f32, cudaStream_t st);
 void launch_posq_in(const Dev& d, const void* posq, int is_double, const int* atom_index, cudaStream_t st);
 void launch_forces_out_fixed(const Dev& d, const int* atom_index, int padded, long long* acc, cudaStream_t st);
-void launch_potential(const Dev& d, const double* grid, int ng, double* out, cudaStream_t st);
+// part: potential_chunks(n, ng) * ng doubles of scratch; the result is its first ng.
+int potential_chunks(int n, int ng);
+void launch_potential(const Dev& d, const double* grid, int ng, double* part, cudaStream_t st);
 void launch_moments(const Dev& d, const double* mass, double* scratch, double* out13, cudaStream_t st);
 
 // Adjoint (tdp_adjoint.cu).
