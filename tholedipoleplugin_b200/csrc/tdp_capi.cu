@@ -1116,7 +1116,8 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
         d.nvb = std::max(1, (n + kVecThreads - 1) / kVecThreads);
         d.pp.band_tiles = band;
         d.pp.n_bands = (nt + band - 1) / band;
-        d.nsplit = d.pp.n_bands;
+        d.nslot = d.pp.n_bands;
+        d.nsplit = 1;
         d.n_eblk = d.pp.n_bands * (d.pp.n_bands + 1) / 2;
         const bool variational = (h->flags & TDP_FLAG_VARIATIONAL) != 0;
         // Both gradient modes rest on an energy functional that is stationary
@@ -1134,7 +1135,7 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
             if (h->flags & TDP_FLAG_EWALD)
                 throw TdpError{TDP_ERR_INVALID_ARGUMENT, "TDP_FLAG_VARIATIONAL and TDP_FLAG_EWALD exclude each other"};
             // Real space only: one partial slot.
-            d.nsplit = 1;
+            d.nslot = d.nsplit = 1;
             d.n_eblk = 1;
         }
         const bool ewald = (h->flags & TDP_FLAG_EWALD) != 0;
@@ -1158,14 +1159,14 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
                                "Ewald mode: the Thole damping at the cutoff exceeds 1e-12 (cutoff too short for the "
                                "largest Thole factor)"};
             // Real space in partial slot 0, reciprocal space + self in slot 1.
-            d.nsplit = 2;
+            d.nslot = d.nsplit = 2;
             d.n_eblk = 1;
         } else if (h->precision == TDP_PRECISION_MIXED && !variational) {
             // Mixed all-pairs form: the band sums go into the fixed-point
             // accumulator and one flushed slot.  Each atom's word receives at
             // most 2 n_bands adds of magnitude < 2^23, so with 2^bits units
             // per e/nm^2 the sum stays below 2^61.
-            d.nsplit = 1;
+            d.nslot = 1;
             int lg = 0;
             while ((1L << lg) < 2L * std::max(1, d.pp.n_bands)) lg++;
             const int bits = std::min(32, 38 - lg);
@@ -1232,7 +1233,7 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
         d.p = dalloc<double>(n3, o);
         d.q = dalloc<double>(n3, o);
         d.hist = dalloc<double>(n3 * h->extrap.size(), o);
-        d.partial = dalloc<double>((size_t)d.nsplit * 6 * d.n_pad, o);
+        d.partial = dalloc<double>((size_t)d.nslot * 6 * d.n_pad, o);
         if (d.fix_scale > 0.0) {
             d.fixacc = dalloc<unsigned long long>(6 * (size_t)d.n_pad, o);
             d.fix_err = dalloc<int>(1, o);

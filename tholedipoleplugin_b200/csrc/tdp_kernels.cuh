@@ -7,13 +7,14 @@
 namespace tdp {
 
 // All device buffers of one system (sizes: n atoms, n_pad = n rounded up to a
-// whole number of bands, nsplit partial-sum slots of the pair kernels = one per
-// band, n_eblk energy partials = one per band pair, nvb blocks of the O(N)
-// kernels).
+// whole number of bands, nslot partial-sum slots that the pair kernels write
+// (plain all-pairs form: one per band, added into slot 0 before anything reads
+// them), nsplit slots that their consumers add, n_eblk energy partials = one
+// per band pair, nvb blocks of the O(N) kernels).
 constexpr int kMuHist = 4;
 
 struct Dev {
-    int n = 0, n_pad = 0, nsplit = 1, nvb = 1, n_eblk = 1;
+    int n = 0, n_pad = 0, nsplit = 1, nslot = 1, nvb = 1, n_eblk = 1;
     PairParams pp{};
     // Inputs.
     double* pos = nullptr;       // n_pad*3 (FP64 working copy of the positions)
@@ -67,7 +68,7 @@ struct Dev {
     double* p = nullptr;
     double* q = nullptr;
     double* hist = nullptr;      // extrapolation orders, korder*n*3
-    double* partial = nullptr;   // nsplit*6*n_pad pair-kernel partial sums (scratch)
+    double* partial = nullptr;   // nslot*6*n_pad pair-kernel partial sums (scratch)
     // Mixed all-pairs form: the field and energy kernels add their per-band
     // sums into one 64-bit fixed-point accumulator (6*n_pad, units of
     // 1/fix_scale; integer addition makes the result independent of the order)
