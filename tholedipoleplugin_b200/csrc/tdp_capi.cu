@@ -1164,12 +1164,30 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
         } else if (h->precision == TDP_PRECISION_MIXED && !variational) {
             // Mixed all-pairs form: the band sums go into the fixed-point
             // accumulator and one flushed slot.  Each atom's word receives at
-            // most 2 n_bands adds of magnitude < 2^23, so with 2^bits units
-            // per e/nm^2 the sum stays below 2^61.
+            // most `adds` adds of magnitude < 2^23, so with 2^bits units per
+            // e/nm^2 the sum stays below 2^63.
             d.nslot = 1;
+            // Items of the field kernel: J chunks as long as seven rounds of
+            // resident warps (16 an SM) allow (matvec with L = 1, 2, 4, 8, 16:
+            // 183, 175, 181, 195, 218 us at 12,288 atoms, 619, 569, 554, 557,
+            // 575 at 24,000, 8397, 7562, 7184, 6998, 6912 at 98,304).  Where
+            // the walks are far fewer than the warps, each is split over up
+            // to eight (1, 2, 4, 8 parts: 26, 20, 17, 16 us at 648 atoms, 25,
+            // 20, 17, 19 at 1,029, 43, 43, 49, 66 at 3,993).
+            const long groups = (nt + kFieldNS - 1) / kFieldNS, visits = groups * (nt + kFieldNS) / 2;
+            const long resident = 16L * 148;
+            d.field_L = 1;
+            for (int L : {16, 8, 4, 2})
+                if (visits >= 7 * L * resident) {
+                    d.field_L = L;
+                    break;
+                }
+            d.field_parts = 1;
+            while (d.field_parts < 8 && 2 * d.field_parts * visits <= 9L * 148) d.field_parts *= 2;
+            const long adds = std::max(2L * d.pp.n_bands, d.field_parts * (groups + (nt + d.field_L - 1) / d.field_L));
             int lg = 0;
-            while ((1L << lg) < 2L * std::max(1, d.pp.n_bands)) lg++;
-            const int bits = std::min(32, 38 - lg);
+            while ((1L << lg) < adds) lg++;
+            const int bits = std::min(32, 40 - lg);
             d.fix_scale = std::ldexp(1.0, bits);
             d.fix_limit = std::ldexp(1.0, 23);
         }

@@ -573,6 +573,14 @@ __global__ void k_forces_out_fixed(int n, const double* __restrict__ f, const in
 constexpr int kPotPoints = 128;   // points (threads) per block
 constexpr int kPotAtoms = 128;    // atoms staged per step
 
+// fold_d, with the reference's own quotient where the reciprocal's rounding
+// could decide: points at a lattice distance of half a box are common on grids.
+__device__ __forceinline__ double fold_tie(double d, double L, double invL) {
+    double t = d * invL + 0.5;
+    if (fabs(t - rint(t)) < 1e-12) t = d / L + 0.5;
+    return d - L * floor(t);
+}
+
 __global__ void __launch_bounds__(kPotPoints) k_potential(int n, int ng, int chunk, PairParams P,
                                                           const double* __restrict__ pos,
                                                           const double* __restrict__ charge,
@@ -602,9 +610,9 @@ __global__ void __launch_bounds__(kPotPoints) k_potential(int n, int ng, int chu
         for (int j = 0; j < cnt; j++) {
             const double2 u = s_a[j][0], v = s_a[j][1], w = s_a[j][2];
             double dx = u.x - gp.x, dy = u.y - gp.y, dz = v.x - gp.z;
-            if (fabs(dx) >= half[0]) dx = fold_d(dx, P.box[0], P.inv_box[0]);
-            if (fabs(dy) >= half[1]) dy = fold_d(dy, P.box[1], P.inv_box[1]);
-            if (fabs(dz) >= half[2]) dz = fold_d(dz, P.box[2], P.inv_box[2]);
+            if (fabs(dx) >= half[0]) dx = fold_tie(dx, P.box[0], P.inv_box[0]);
+            if (fabs(dy) >= half[1]) dy = fold_tie(dy, P.box[1], P.inv_box[1]);
+            if (fabs(dz) >= half[2]) dz = fold_tie(dz, P.box[2], P.inv_box[2]);
             const double rr1 = rsqrt(dx * dx + dy * dy + dz * dz);
             const double rr3 = rr1 * rr1 * rr1;
             pot += v.y * rr1 - (w.x * dx + w.y * dy + s_a[j][3].x * dz) * rr3;

@@ -77,6 +77,9 @@ struct Dev {
     unsigned long long* fixacc = nullptr;
     int* fix_err = nullptr;
     double fix_scale = 0.0, fix_limit = 0.0;
+    // Mixed all-pairs field kernel: J tiles per item and parts of each walk
+    // (field_items).
+    int field_L = 1, field_parts = 1;
     double* energy_partial = nullptr;
     double* fpair = nullptr;
     double* torque = nullptr;
@@ -93,7 +96,11 @@ struct Dev {
 
 template <class R> void launch_pack(const Dev& d, cudaStream_t st);
 template <class R> void launch_rotate(const Dev& d, cudaStream_t st);
+// I tiles per item of the mixed field kernel.
+constexpr int kFieldNS = 2;
 template <class R> void launch_field(const Dev& d, int kind, cudaStream_t st);
+template <> void launch_field<float>(const Dev& d, int kind, cudaStream_t st);
+template <> void launch_field<double>(const Dev& d, int kind, cudaStream_t st);
 template <class R> void launch_energy(const Dev& d, cudaStream_t st);
 template <class R> void launch_fixed_done(const Dev& d, cudaStream_t st);
 template <class R> void launch_warm_start(const Dev& d, cudaStream_t st);

@@ -2,7 +2,8 @@
 // mutual-field matvec, energy/force/torque), each unordered pair evaluated
 // once with both of its sides.
 //
-// Work decomposition.  Atoms form 32-atom tiles and tiles form bands of
+// Work decomposition.  The mixed form's field kernel takes warp-sized items
+// (k_field_items).  For the others atoms form 32-atom tiles and tiles form bands of
 // band_tiles tiles.  One CTA (4 warps) owns a band pair (p, q), p <= q, and
 // evaluates every tile pair (I in band p, J in band q, I <= J).  A warp holds
 // the atoms of its I tile(s) in registers (lane = atom) and walks the atoms of
@@ -40,6 +41,8 @@
 #include "tdp_pairs.cuh"
 
 #include <math.h>
+
+#include <algorithm>
 
 namespace tdp {
 
@@ -321,9 +324,10 @@ __device__ __forceinline__ XSlot xslot(int i, float ox, float oy, float oz, floa
 // One I atom against J atoms (m, m + 16): I-side sums into F*, J-side into G*,
 // both with the opposite sign of the field (the walk's caller flips them), so
 // that every term is a plain product-sum with -rr5.
-template <int KIND, bool FOLD, bool DAMP>
+// MASK: bit m of mk (bit m + 16 for the second half) says whether the pair counts.
+template <int KIND, bool FOLD, bool DAMP, bool MASK = false>
 __device__ __forceinline__ void xslot_pairs(const PairParams& P, const double* __restrict__ pos, const XSlot& x,
-                                            int ja, f2 PX, f2 PY, f2 PZ, f2 QJ, f2 VJX, f2 VJY, f2 VJZ, float tja,
+                                            unsigned mk, int m, int ja, f2 PX, f2 PY, f2 PZ, f2 QJ, f2 VJX, f2 VJY, f2 VJZ, float tja,
                                             float tjb, unsigned fm, f2 Lx, f2 Ly, f2 Lz, f2 Ix, f2 Iy, f2 Iz,
                                             f2 NTx, f2 NTy, f2 NTz, float damp_r2, f2& FX, f2& FY, f2& FZ,
                                             f2& GX, f2& GY, f2& GZ) {
@@ -374,6 +378,11 @@ __device__ __forceinline__ void xslot_pairs(const PairParams& P, const double* _
     const f2 R2 = fma2(DX, DX, fma2(DY, DY, mul2(DZ, DZ)));
     float r2a, r2b;
     un2(R2, r2a, r2b);
+    if (MASK) {
+        // A pair that does not count gets an infinite distance: every term is 0.
+        r2a = (mk >> m) & 1u ? r2a : INFINITY;
+        r2b = (mk >> (m + 16)) & 1u ? r2b : INFINITY;
+    }
     const f2 RINV = pk2(rsqrt_r(r2a), rsqrt_r(r2b));
     const f2 RINV2 = mul2(RINV, RINV);
     f2 RR3 = mul2(RINV, RINV2);
@@ -417,11 +426,14 @@ __device__ __forceinline__ void xslot_pairs(const PairParams& P, const double* _
     }
 }
 
-template <int KIND, bool FOLD, bool DAMP>
-__device__ __forceinline__ void field_walk_x4(const PairParams& P, const double* __restrict__ pos,
-                                              const FPackedTile& T, int lane, int jbase, const XSlot& xa,
-                                              const XSlot& xb, bool two, unsigned fm, float damp_r2, float* fa,
-                                              float* fb, float* g) {
+// Steps [s0, s1) of the walk of NS I tiles (lane = atom of each) over one J
+// tile.  g: the J-side sums of atom ((lane + s1) & 15) | (lane & 16).
+template <int KIND, int NS, bool FOLD, bool DAMP, bool MASK>
+__device__ __forceinline__ void field_walk_ns(const PairParams& P, const double* __restrict__ pos,
+                                              const FPackedTile& T, int lane, int jbase, const XSlot (&x)[NS],
+                                              const unsigned (&mk)[NS], const unsigned (&fm)[NS], float damp_r2,
+                                              int s0, int s1,
+                                              float (&f)[NS][3], float (&g)[3]) {
     const int nxt = (lane + 1) & 31;
     f2 Lx = 0, Ly = 0, Lz = 0, Ix = 0, Iy = 0, Iz = 0, NTx = 0, NTy = 0, NTz = 0;
     if (FOLD) {
@@ -435,49 +447,249 @@ __device__ __forceinline__ void field_walk_x4(const PairParams& P, const double*
         NTy = bc2(-(float)(P.half_box_tol[1] * P.half_box_tol[1]));
         NTz = bc2(-(float)(P.half_box_tol[2] * P.half_box_tol[2]));
     }
-    f2 FXA = 0, FYA = 0, FZA = 0, FXB = 0, FYB = 0, FZB = 0;   // I side, packed over (m, m + 16)
-    f2 GX = 0, GY = 0, GZ = 0;                                 // J side (packed atoms m, m + 16)
-    // One step is already four independent pairs: no unrolling (the walk's
+    f2 F[NS][3];               // I side, packed over (m, m + 16)
+#pragma unroll
+    for (int k = 0; k < NS; k++) F[k][0] = F[k][1] = F[k][2] = 0;
+    f2 GX = 0, GY = 0, GZ = 0;   // J side (packed atoms m, m + 16)
+    // One step is already 2 NS independent pairs: no unrolling (the walk's
     // variants must stay small enough for the instruction cache).
 #pragma unroll 1
-    for (int s = 0; s < 16; s++) {
+    for (int s = s0; s < s1; s++) {
         const int m = (lane + s) & 15;
         const float4 a = T.p0[m], b = T.p1[m], c = T.v0[m], d = T.v1[m];
         const f2 PX = pk2(a.x, a.y), PY = pk2(a.z, a.w), PZ = pk2(b.x, b.y), QJ = pk2(b.z, b.w);
         const f2 VJX = pk2(c.x, c.y), VJY = pk2(c.z, c.w), VJZ = pk2(d.x, d.y);
-        xslot_pairs<KIND, FOLD, DAMP>(P, pos, xa, jbase + m, PX, PY, PZ, QJ, VJX, VJY, VJZ, d.z, d.w, fm, Lx, Ly,
-                                      Lz, Ix, Iy, Iz, NTx, NTy, NTz, damp_r2, FXA, FYA, FZA, GX, GY, GZ);
-        if (two)
-            xslot_pairs<KIND, FOLD, DAMP>(P, pos, xb, jbase + m, PX, PY, PZ, QJ, VJX, VJY, VJZ, d.z, d.w, fm, Lx, Ly,
-                                          Lz, Ix, Iy, Iz, NTx, NTy, NTz, damp_r2, FXB, FYB, FZB, GX, GY, GZ);
+#pragma unroll
+        for (int k = 0; k < NS; k++)
+            xslot_pairs<KIND, FOLD, DAMP, MASK>(P, pos, x[k], mk[k], m, jbase + m, PX, PY, PZ, QJ, VJX, VJY, VJZ, d.z,
+                                                d.w, fm[k], Lx, Ly, Lz, Ix, Iy, Iz, NTx, NTy, NTz, damp_r2, F[k][0],
+                                                F[k][1], F[k][2], GX, GY, GZ);
         GX = __shfl_sync(kFull, GX, nxt);
         GY = __shfl_sync(kFull, GY, nxt);
         GZ = __shfl_sync(kFull, GZ, nxt);
     }
     // F and G hold the negated sums (xslot_pairs).
     float lo, hi;
-    un2(FXA, lo, hi);
-    fa[0] -= lo + hi;
-    un2(FYA, lo, hi);
-    fa[1] -= lo + hi;
-    un2(FZA, lo, hi);
-    fa[2] -= lo + hi;
-    if (two) {
-        un2(FXB, lo, hi);
-        fb[0] -= lo + hi;
-        un2(FYB, lo, hi);
-        fb[1] -= lo + hi;
-        un2(FZB, lo, hi);
-        fb[2] -= lo + hi;
-    }
-    // Lane l now holds (atom l & 15, atom (l & 15) + 16); lane l ^ 16 the other copy.
+#pragma unroll
+    for (int k = 0; k < NS; k++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            un2(F[k][c], lo, hi);
+            f[k][c] = -(lo + hi);
+        }
+    // Lanes l and l ^ 16 hold the two copies of atoms (m, m + 16), m = (l + s1) & 15.
     const f2 Js[3] = {GX, GY, GZ};
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-        un2(Js[k], lo, hi);
+    for (int c = 0; c < 3; c++) {
+        un2(Js[c], lo, hi);
         const float olo = __shfl_xor_sync(kFull, lo, 16), ohi = __shfl_xor_sync(kFull, hi, 16);
-        g[k] -= lane < 16 ? lo + olo : hi + ohi;
+        g[c] = -(lane < 16 ? lo + olo : hi + ohi);
     }
+}
+
+// A float sum into the accumulator: v 2^k is exact, so the only rounding is
+// that of the accumulator's unit.
+__device__ __forceinline__ void fix_add(const FixAcc& F, size_t k, float v) {
+    if (v == 0.0f) return;
+    if (!(fabsf(v) < (float)F.limit)) {
+        atomicExch(F.err, 1);
+        return;
+    }
+    atomicAdd(F.acc + k, (unsigned long long)__float2ll_rn(v * (float)F.scale));
+}
+
+// Mixed-form field kernel: KIND 0 = permanent field (operand: lab dipoles, or
+// m + mu0 in the fused start), KIND 1 = mutual-field matvec.  One warp is one
+// item: NS I tiles in registers against J tiles [c L, c L + L), and of each
+// walk the steps of its part (gridDim.y parts).  Items are independent: the J
+// records come from L2 into the warp's own packed tile, the J-side sums of a
+// tile pair go straight into the fixed-point accumulator, so no block waits at
+// a barrier and any number of tiles splits evenly.  Pairs that do not count
+// (self, padding, the second visit on a diagonal tile, partners whose scale is
+// not 1) are masked out; k_field_done adds the scaled partners.
+//
+// Bound by the FP32 pipe and issue (61 FMA-pipe instructions of about 90 a
+// step of four pairs).  The kernel before it owned a band pair per 4-warp
+// block, summed the J side in shared memory and flushed 2 x 3 x 512 sums; its
+// bands had to shrink with the system, which left warps with one I tile (half
+// the work per J load and shuffle) or none.  Matvec, before -> now: 19.7 ->
+// 12 us at 648 atoms (with k_field_done), 94 -> 43 at 3,993, 242 -> 175 at
+// 12,288, 8730 -> 6950 at 98,304.  NS = 4 is slower (7126 us there, 321 at
+// 12,288): the tiles of an item share the fold and damping variant of a walk.
+template <int KIND, int NS>
+__global__ void __launch_bounds__(32, 16) k_field_items(
+    PairParams P, int L, const float4* __restrict__ posq, const float4* __restrict__ jvec,
+    const double4* __restrict__ tctr, const double4* __restrict__ text, const double* __restrict__ pos,
+    const int* __restrict__ exc_off, const int* __restrict__ exc_j, const double* __restrict__ exc_scale,
+    const int2* __restrict__ exc_tiles, int n_pad, FixAcc fix) {
+    __shared__ FPackedTile T;
+    __shared__ double s_my[3 * NS][32];   // I-side sums
+    const int lane = threadIdx.x;
+    // Item -> (I group a, J chunk c): square blocks of B = max(L, NS) tiles, p <= q.
+    int p, q, a, c;
+    if (L >= NS) {
+        const int r = L / NS;
+        band_pair(blockIdx.x / r, p, q);
+        a = p * r + blockIdx.x % r;
+        c = q;
+    } else {
+        const int r = NS / L;
+        band_pair(blockIdx.x / r, p, q);
+        a = p;
+        c = q * r + blockIdx.x % r;
+    }
+    const int I0 = a * NS, J0 = c * L, J1 = min(J0 + L, P.n_tiles);
+    if (I0 >= P.n_tiles || J1 <= max(J0, I0)) return;
+    const int s0 = 16 * blockIdx.y / gridDim.y, s1 = 16 * (blockIdx.y + 1) / gridDim.y;
+    const float damp_r2 = P.damp_r2;
+
+    float4 pi[NS], vi[NS];
+    int2 et[NS];
+    int e0[NS], e1[NS];
+    unsigned own[NS];
+#pragma unroll
+    for (int k = 0; k < NS; k++) {
+        const int I = I0 + k, i = I * 32 + lane;
+        pi[k] = vi[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        et[k] = make_int2(1 << 30, -1);
+        e0[k] = e1[k] = 0;
+        own[k] = 0u;
+        if (I < P.n_tiles) {
+            pi[k] = posq[i];
+            vi[k] = jvec[i];
+            et[k] = exc_tiles[I];
+            if (i < P.n) {
+                own[k] = ~0u;
+                e0[k] = exc_off[i];
+                e1[k] = exc_off[i + 1];
+            }
+        }
+    }
+    // The item's NS x L tile-pair geometries (FP64), one per lane, read by shuffles.
+    float gdx = 0.f, gdy = 0.f, gdz = 0.f;
+    unsigned gfl = 0u;
+    {
+        const int k = lane / L, I = I0 + k, J = J0 + lane % L;
+        if (k < NS && I < P.n_tiles && J < P.n_tiles) {
+            const TileGeom g = tile_geom(P, tctr[I], text[I], tctr[J], text[J]);
+            gdx = (float)g.dcx;
+            gdy = (float)g.dcy;
+            gdz = (float)g.dcz;
+            gfl = g.fmask | (g.fold ? 8u : 0u) | (g.near ? 16u : 0u);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 3 * NS; k++) s_my[k][lane] = 0.0;
+    int J = max(J0, I0);
+    float4 pj = posq[J * 32 + lane], vj = jvec[J * 32 + lane];
+    for (; J < J1; J++) {
+        __syncwarp();
+        stage_fpacked(T, lane, pj, vj);
+        __syncwarp();
+        if (J + 1 < J1) {   // the next tile's records arrive during the walk
+            pj = posq[(J + 1) * 32 + lane];
+            vj = jvec[(J + 1) * 32 + lane];
+        }
+        const int jbase = J * 32;
+        XSlot x[NS];
+        unsigned mk[NS], fm[NS], fl = 0u;
+        bool masked = false;
+        const unsigned real = J == P.n_tiles - 1 && (P.n & 31) ? (1u << (P.n & 31)) - 1u : ~0u;
+#pragma unroll
+        for (int k = 0; k < NS; k++) {
+            const int I = I0 + k, src = k * L + (J - J0);
+            const float dx = __shfl_sync(kFull, gdx, src), dy = __shfl_sync(kFull, gdy, src),
+                        dz = __shfl_sync(kFull, gdz, src);
+            const unsigned fk = __shfl_sync(kFull, gfl, src);
+            mk[k] = own[k] & real;
+            if (I > J) mk[k] = 0u;
+            if (I == J) mk[k] &= ~((2u << lane) - 1u);   // each pair of a diagonal tile once: j > i
+            if (J >= et[k].x && J <= et[k].y)
+                for (int e = e0[k]; e < e1[k]; e++) {
+                    const unsigned off = (unsigned)(exc_j[e] - jbase);
+                    if (off < 32u && exc_scale[e] != 1.0) mk[k] &= ~(1u << off);
+                }
+            masked = masked || mk[k] != ~0u;
+            fl |= fk;
+            fm[k] = fk & 7u;
+            x[k] = xslot(I * 32 + lane, pi[k].x - dx, pi[k].y - dy, pi[k].z - dz, pi[k].w, vi[k]);
+        }
+        float f[NS][3], g[3];
+        if (__any_sync(kFull, masked))
+            field_walk_ns<KIND, NS, true, true, true>(P, pos, T, lane, jbase, x, mk, fm, damp_r2, s0, s1, f, g);
+        else if (fl & 8u) {
+            if (fl & 16u)
+                field_walk_ns<KIND, NS, true, true, false>(P, pos, T, lane, jbase, x, mk, fm, damp_r2, s0, s1, f, g);
+            else
+                field_walk_ns<KIND, NS, true, false, false>(P, pos, T, lane, jbase, x, mk, fm, damp_r2, s0, s1, f, g);
+        } else if (fl & 16u) {
+            field_walk_ns<KIND, NS, false, true, false>(P, pos, T, lane, jbase, x, mk, fm, damp_r2, s0, s1, f, g);
+        } else {
+            field_walk_ns<KIND, NS, false, false, false>(P, pos, T, lane, jbase, x, mk, fm, damp_r2, s0, s1, f, g);
+        }
+        const int jl = ((lane + s1) & 15) | (lane & 16);
+#pragma unroll
+        for (int k = 0; k < 3; k++) fix_add(fix, (size_t)k * n_pad + jbase + jl, g[k]);
+#pragma unroll
+        for (int k = 0; k < NS; k++)
+#pragma unroll
+            for (int d = 0; d < 3; d++) s_my[3 * k + d][lane] += (double)f[k][d];
+    }
+#pragma unroll
+    for (int k = 0; k < NS; k++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) fix_add(fix, (size_t)d * n_pad + (I0 + k) * 32 + lane, s_my[3 * k + d][lane]);
+}
+
+// Fixed-point sums -> partial slot 0, clearing them, plus the covalent
+// partners that k_field_items masked out, one-sided with their scales (FP64
+// displacement and arithmetic on the pair records).  kind 0: M scale; 1: I
+// scale; 2 (fused start, operand P = m + mu0): M field(q, P) + (I - M) T mu0
+// with mu0 = P - m, the second term also where M = 1.
+template <int KIND>
+__global__ void k_field_done(PairParams P, int fused, const float4* __restrict__ posq, const float4* __restrict__ jvec,
+                             const float4* __restrict__ lab, const double* __restrict__ pos,
+                             const int* __restrict__ exc_off, const int* __restrict__ exc_j,
+                             const double* __restrict__ exc_m, const double* __restrict__ exc_s, int n_pad,
+                             unsigned long long* __restrict__ acc, double inv_scale, double* __restrict__ out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n_pad) return;
+    double f[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+        f[c] = (double)(long long)acc[(size_t)c * n_pad + k] * inv_scale;
+        acc[(size_t)c * n_pad + k] = 0ull;
+    }
+    if (k < P.n) {
+        const double ti = (double)jvec[k].w;
+        for (int e = exc_off[k]; e < exc_off[k + 1]; e++) {
+            const double sc = KIND == 0 ? exc_m[e] : exc_s[e], ds = fused ? exc_s[e] - sc : 0.0;
+            if ((sc == 0.0 || sc == 1.0) && ds == 0.0) continue;
+            const int j = exc_j[e];
+            const d3 d = exact_delta(P, pos, k, j);
+            const double r2 = dot(d, d);
+            const float4 vj = jvec[j];
+            double t[3] = {0.0, 0.0, 0.0};
+            if (KIND == 0)
+                pair_fixed<double, true>(d.x, d.y, d.z, r2, (double)posq[j].w, (double)vj.x, (double)vj.y,
+                                         (double)vj.z, ti, (double)vj.w, (double)P.damp_r2, t[0], t[1], t[2]);
+            else
+                pair_matvec<double, true>(d.x, d.y, d.z, r2, (double)vj.x, (double)vj.y, (double)vj.z, ti,
+                                          (double)vj.w, (double)P.damp_r2, t[0], t[1], t[2]);
+            if (sc != 1.0)
+                for (int c = 0; c < 3; c++) f[c] += sc * t[c];
+            if (ds != 0.0) {
+                const float4 mj = lab[j];
+                double u[3] = {0.0, 0.0, 0.0};
+                pair_matvec<double, true>(d.x, d.y, d.z, r2, (double)vj.x - (double)mj.x, (double)vj.y - (double)mj.y,
+                                          (double)vj.z - (double)mj.z, ti, (double)vj.w, (double)P.damp_r2, u[0],
+                                          u[1], u[2]);
+                for (int c = 0; c < 3; c++) f[c] += ds * u[c];
+            }
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; c++) out[(size_t)c * n_pad + k] = f[c];
 }
 
 // Partner pairs of a SLOW tile pair, each side once with its scale (M for
@@ -618,34 +830,15 @@ __device__ __forceinline__ void slot_against(ISlot<R>& a, const PairParams& P, b
     a.partners = a.slow ? partner_bits(exc_j, a.e0, a.e1, J * 32) : 0u;
 }
 
-// The same from the tile pair's geometry computed beforehand (FP32 form):
-// centre displacement dc in FP32 and flags fmask | fold << 3 | near << 4.
-template <class R>
-__device__ __forceinline__ void slot_against_pre(ISlot<R>& a, const PairParams& P, bool same_band, int J, int Jl,
-                                                 float dcx, float dcy, float dcz, unsigned fl,
-                                                 const int* __restrict__ exc_j) {
-    a.valid = a.act && J < P.n_tiles && (!same_band || Jl >= a.Il);
-    if (!a.valid) return;
-    a.ox = a.pi.x - (R)dcx;
-    a.oy = a.pi.y - (R)dcy;
-    a.oz = a.pi.z - (R)dcz;
-    a.fmask = fl & 7u;
-    a.fold = (fl >> 3) & 1u;
-    a.near = (fl >> 4) & 1u;
-    a.diag = a.I == J;
-    a.slow = a.diag || (J == P.n_tiles - 1 && (P.n & 31)) || (J >= a.et.x && J <= a.et.y);
-    a.partners = a.slow ? partner_bits(exc_j, a.e0, a.e1, J * 32) : 0u;
-}
-
-// FP32: 4 CTAs per SM at 128 registers; FP64: 3 CTAs per SM (168 registers),
-// which halves the FP64 walks' register spills (measured 2-4 % faster).
+// Plain form.  3 CTAs per SM (168 registers), which halves the walks' register
+// spills (measured 2-4 % faster than 4).
 template <class R, int KIND>
-__global__ void __launch_bounds__(kSymThreads, sizeof(R) == 4 ? 4 : 3) k_field_sym(
+__global__ void __launch_bounds__(kSymThreads, 3) k_field_sym(
     PairParams P, const typename Vec4T<R>::type* __restrict__ posq, const typename Vec4T<R>::type* __restrict__ jvec,
     const double4* __restrict__ tctr, const double4* __restrict__ text, const double* __restrict__ pos,
     const int* __restrict__ exc_off, const int* __restrict__ exc_j, const double* __restrict__ exc_m,
     const double* __restrict__ exc_s, const int2* __restrict__ exc_tiles, int n_pad, double* __restrict__ partial,
-    FixAcc fix, const typename Vec4T<R>::type* __restrict__ lab) {
+    const typename Vec4T<R>::type* __restrict__ lab) {
     typedef typename Vec4T<R>::type V4;
     extern __shared__ __align__(16) unsigned char smem[];
     const int BT = P.band_tiles, NA = BT * 32;
@@ -657,7 +850,6 @@ __global__ void __launch_bounds__(kSymThreads, sizeof(R) == 4 ? 4 : 3) k_field_s
     V4* s_pos = reinterpret_cast<V4*>(s_ie + 2 * kSymWarps);       // NA
     V4* s_vec = s_pos + NA;                                        // NA
     R* s_acc = reinterpret_cast<R*>(s_vec + NA);                   // kSymWarps * 3 * NA: J-side sums per warp
-    FPackedTile* s_fpt = reinterpret_cast<FPackedTile*>(s_acc + kSymWarps * 3 * NA);  // kSymWarps (FP32 only)
 
     int p, q;
     band_pair(blockIdx.x, p, q);
@@ -693,80 +885,19 @@ __global__ void __launch_bounds__(kSymThreads, sizeof(R) == 4 ? 4 : 3) k_field_s
             s_ie[2 * warp + lane] = s1.act ? text[s1.I] : make_double4(0, 0, 0, 0);
         }
         __syncwarp();
-        // FP32 form: the round's 2 x BT tile-pair geometries (FP64 arithmetic),
-        // one per lane, instead of every lane repeating each of them.
-        float gdx = 0.f, gdy = 0.f, gdz = 0.f;
-        unsigned gfl = 0u;
-        if constexpr (sizeof(R) == 4) {
-            if (lane < 2 * BT) {
-                const int k = lane / BT, Jl = lane - k * BT;
-                const TileGeom g = tile_geom(P, s_ic[2 * warp + k], s_ie[2 * warp + k], s_ctr[Jl], s_ext[Jl]);
-                gdx = (float)g.dcx;
-                gdy = (float)g.dcy;
-                gdz = (float)g.dcz;
-                gfl = g.fmask | (g.fold ? 8u : 0u) | (g.near ? 16u : 0u);
-            }
-        }
         for (int c = 0; c < 6; c++) my[c] = 0.0;
         for (int t = 0; t < BT; t++) {
             const int Jl = (t + warp * stride) % BT;
             const int J = q * BT + Jl;
             const double4 cB = s_ctr[Jl], eB = s_ext[Jl];
-            if constexpr (sizeof(R) == 4) {
-                const int la = Jl, lb = BT + Jl;
-                const float ax = __shfl_sync(kFull, gdx, la), ay = __shfl_sync(kFull, gdy, la),
-                            az = __shfl_sync(kFull, gdz, la);
-                const float bx = __shfl_sync(kFull, gdx, lb), by = __shfl_sync(kFull, gdy, lb),
-                            bz = __shfl_sync(kFull, gdz, lb);
-                const unsigned af = __shfl_sync(kFull, gfl, la), bf = __shfl_sync(kFull, gfl, lb);
-                slot_against_pre<R>(a, P, p == q, J, Jl, ax, ay, az, af, exc_j);
-                slot_against_pre<R>(b, P, p == q, J, Jl, bx, by, bz, bf, exc_j);
-            } else {
-                slot_against<R>(a, P, p == q, J, Jl, s_ic[2 * warp], s_ie[2 * warp], cB, eB, exc_j);
-                slot_against<R>(b, P, p == q, J, Jl, s_ic[2 * warp + 1], s_ie[2 * warp + 1], cB, eB, exc_j);
-            }
+            slot_against<R>(a, P, p == q, J, Jl, s_ic[2 * warp], s_ie[2 * warp], cB, eB, exc_j);
+            slot_against<R>(b, P, p == q, J, Jl, s_ic[2 * warp + 1], s_ie[2 * warp + 1], cB, eB, exc_j);
             if (!(a.valid || b.valid)) continue;
             const int jbase = J * 32;
             const V4* sp = s_pos + Jl * 32;
             const V4* sv = s_vec + Jl * 32;
             R fa[3] = {0, 0, 0}, fb[3] = {0, 0, 0}, g[3] = {0, 0, 0};
-            bool packed = false;
-            if constexpr (sizeof(R) == 4) {
-                // Non-SLOW tile pairs: the packed walk over J-atom pairs, one or both slots.
-                const bool two = a.valid && b.valid;
-                if (two ? !(a.slow || b.slow) : !(a.valid ? a.slow : b.slow)) {
-                    packed = true;
-                    __syncwarp();
-                    stage_fpacked(s_fpt[warp], lane, sp[lane], sv[lane]);
-                    __syncwarp();
-                    const ISlot<R>& s1 = a.valid ? a : b;
-                    const ISlot<R>& s2 = two ? b : s1;
-                    float* f1 = a.valid ? fa : fb;
-                    const XSlot x1 = xslot(s1.i, s1.ox, s1.oy, s1.oz, s1.pi.w, s1.vi);
-                    const XSlot x2 = xslot(s2.i, s2.ox, s2.oy, s2.oz, s2.pi.w, s2.vi);
-                    const unsigned fm = s1.fmask | s2.fmask;
-                    const bool fold = s1.fold || s2.fold, near = s1.near || s2.near;
-// One inlined copy per slot count (the count is a constant inside each).
-#define TDP_FWALKX4(F, D)                                                                                        \
-    do {                                                                                                         \
-        if (two)                                                                                                 \
-            field_walk_x4<KIND, F, D>(P, pos, s_fpt[warp], lane, jbase, x1, x2, true, fm, damp_r2, f1, fb, g);  \
-        else                                                                                                     \
-            field_walk_x4<KIND, F, D>(P, pos, s_fpt[warp], lane, jbase, x1, x2, false, fm, damp_r2, f1, fb, g); \
-    } while (0)
-                    if (fold) {
-                        if (near) TDP_FWALKX4(true, true);
-                        else TDP_FWALKX4(true, false);
-                    } else if (near) {
-                        TDP_FWALKX4(false, true);
-                    } else {
-                        TDP_FWALKX4(false, false);
-                    }
-#undef TDP_FWALKX4
-                }
-            }
-            if (packed) {
-            } else if (a.valid && b.valid) {
+            if (a.valid && b.valid) {
                 const bool slow = a.slow || b.slow, fold = a.fold || b.fold;
                 const bool near = a.near || b.near;
 #define TDP_FWALK2(F, S, D)                                                                                        \
@@ -831,16 +962,11 @@ __global__ void __launch_bounds__(kSymThreads, sizeof(R) == 4 ? 4 : 3) k_field_s
         }
         // I-side sums: slot q of band p; on the diagonal band, slot p, where
         // the J-side sums of the same atoms are added below.
-        // (Mixed form: added into the fixed-point accumulator instead.)
         for (int k = 0; k < 2; k++) {
             const ISlot<R>& s1 = k == 0 ? a : b;
             if (!s1.act) continue;
-            if (sizeof(R) == 4) {
-                for (int c = 0; c < 3; c++) fix_add(fix, (size_t)c * n_pad + s1.i, my[3 * k + c]);
-            } else {
-                const size_t base = (size_t)q * 3 * n_pad;
-                for (int c = 0; c < 3; c++) partial[base + (size_t)c * n_pad + s1.i] = my[3 * k + c];
-            }
+            const size_t base = (size_t)q * 3 * n_pad;
+            for (int c = 0; c < 3; c++) partial[base + (size_t)c * n_pad + s1.i] = my[3 * k + c];
         }
     }
     __syncthreads();
@@ -851,12 +977,8 @@ __global__ void __launch_bounds__(kSymThreads, sizeof(R) == 4 ? 4 : 3) k_field_s
         for (int c = 0; c < 3; c++) {
             double v = 0.0;
             for (int w = 0; w < kSymWarps; w++) v += (double)s_acc[w * 3 * NA + 3 * k + c];
-            if (sizeof(R) == 4) {
-                fix_add(fix, (size_t)c * n_pad + a, v);
-            } else {
-                if (own) v += partial[base + (size_t)c * n_pad + a];
-                partial[base + (size_t)c * n_pad + a] = v;
-            }
+            if (own) v += partial[base + (size_t)c * n_pad + a];
+            partial[base + (size_t)c * n_pad + a] = v;
         }
     }
 }
@@ -1774,8 +1896,7 @@ template <class R>
 size_t field_smem(int BT) {
     const int NA = 32 * BT;
     return sizeof(double) * 6 * kSymThreads + sizeof(double4) * (2 * BT + 4 * kSymWarps) +
-           sizeof(typename Vec4T<R>::type) * 2 * NA + sizeof(R) * kSymWarps * 3 * NA +
-           (sizeof(R) == 4 ? sizeof(FPackedTile) * kSymWarps : 0);
+           sizeof(typename Vec4T<R>::type) * 2 * NA + sizeof(R) * kSymWarps * 3 * NA;
 }
 
 template <class R>
@@ -1832,25 +1953,43 @@ void slot_sum(const Dev& d, int ncomp, cudaStream_t st) {
 // matvec (operand: vec); kind 2: the start of a warm-started solve, the
 // permanent field plus T mu0 in one walk (operand vec = m + mu0, see
 // field_partners).
-template <class R>
-void launch_field(const Dev& d, int kind, cudaStream_t st) {
-    typedef typename Vec4T<R>::type V4;
-    const size_t smem = field_smem<R>(d.pp.band_tiles);
+template <>
+void launch_field<float>(const Dev& d, int kind, cudaStream_t st) {
+    const int L = d.field_L, B = std::max(L, kFieldNS), nb = (d.pp.n_tiles + B - 1) / B;
+    const dim3 grid((unsigned)((long)nb * (nb + 1) / 2 * (B / std::min(L, kFieldNS))), d.field_parts);
+    const float4 *pq = (const float4*)d.posq_s, *op = (const float4*)(kind == 0 ? d.dipt_s : d.vec_s);
+    const unsigned blocks = (unsigned)((d.n_pad + 127) / 128);
+    if (kind == 1) {
+        k_field_items<1, kFieldNS><<<grid, 32, 0, st>>>(d.pp, L, pq, op, d.tctr_s, d.text_s, d.pos_s, d.exs_off,
+                                                        d.exs_j, d.exs_s, d.exs_tiles, d.n_pad, fix_of(d));
+        k_field_done<1><<<blocks, 128, 0, st>>>(d.pp, 0, pq, op, nullptr, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
+                                                d.exs_s, d.n_pad, d.fixacc, 1.0 / d.fix_scale, d.partial);
+    } else {
+        k_field_items<0, kFieldNS><<<grid, 32, 0, st>>>(d.pp, L, pq, op, d.tctr_s, d.text_s, d.pos_s, d.exs_off,
+                                                        d.exs_j, d.exs_m, d.exs_tiles, d.n_pad, fix_of(d));
+        k_field_done<0><<<blocks, 128, 0, st>>>(d.pp, kind == 2 ? 1 : 0, pq, op, (const float4*)d.dipt_s, d.pos_s,
+                                                d.exs_off, d.exs_j, d.exs_m, d.exs_s, d.n_pad, d.fixacc,
+                                                1.0 / d.fix_scale, d.partial);
+    }
+}
+
+template <>
+void launch_field<double>(const Dev& d, int kind, cudaStream_t st) {
+    const size_t smem = field_smem<double>(d.pp.band_tiles);
     // Field kernels run on the spatially sorted records.
     if (kind == 0 || kind == 2) {
-        cudaFuncSetAttribute(k_field_sym<R, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_field_sym<R, 0><<<band_pairs(d), kSymThreads, smem, st>>>(
-            d.pp, (const V4*)d.posq_s, (const V4*)(kind == 0 ? d.dipt_s : d.vec_s), d.tctr_s, d.text_s, d.pos_s,
-            d.exs_off, d.exs_j, d.exs_m, d.exs_s, d.exs_tiles, d.n_pad, d.partial, fix_of(d),
-            kind == 2 ? (const V4*)d.dipt_s : nullptr);
+        cudaFuncSetAttribute(k_field_sym<double, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k_field_sym<double, 0><<<band_pairs(d), kSymThreads, smem, st>>>(
+            d.pp, (const double4*)d.posq_s, (const double4*)(kind == 0 ? d.dipt_s : d.vec_s), d.tctr_s, d.text_s,
+            d.pos_s, d.exs_off, d.exs_j, d.exs_m, d.exs_s, d.exs_tiles, d.n_pad, d.partial,
+            kind == 2 ? (const double4*)d.dipt_s : nullptr);
     } else {
-        cudaFuncSetAttribute(k_field_sym<R, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_field_sym<R, 1><<<band_pairs(d), kSymThreads, smem, st>>>(
-            d.pp, (const V4*)d.posq_s, (const V4*)d.vec_s, d.tctr_s, d.text_s, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
-            d.exs_s, d.exs_tiles, d.n_pad, d.partial, fix_of(d), nullptr);
+        cudaFuncSetAttribute(k_field_sym<double, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k_field_sym<double, 1><<<band_pairs(d), kSymThreads, smem, st>>>(
+            d.pp, (const double4*)d.posq_s, (const double4*)d.vec_s, d.tctr_s, d.text_s, d.pos_s, d.exs_off, d.exs_j,
+            d.exs_m, d.exs_s, d.exs_tiles, d.n_pad, d.partial, nullptr);
     }
-    if (sizeof(R) == 4) fix_flush(d, 3, st);
-    else slot_sum(d, 3, st);
+    slot_sum(d, 3, st);
 }
 
 template <class R>
@@ -1865,8 +2004,6 @@ void launch_energy(const Dev& d, cudaStream_t st) {
     else slot_sum(d, 6, st);
 }
 
-template void launch_field<float>(const Dev&, int, cudaStream_t);
-template void launch_field<double>(const Dev&, int, cudaStream_t);
 template void launch_energy<float>(const Dev&, cudaStream_t);
 template void launch_energy<double>(const Dev&, cudaStream_t);
 
