@@ -797,11 +797,10 @@ void run_energy(tdp_handle* h) {
     size_t k = kernel_begin(h, 1);
     launch_energy<R>(d, st);
     kernel_end(h, k);
-    launch_energy_done(d, st);
     record(h, 4);
     launch_torque_gather(d, st);
     record(h, 5);
-    h->launches += 4;
+    h->launches += 4 + (sizeof(R) == 4 ? 2 : 0);
 }
 
 void finish_timing(tdp_handle* h) {
@@ -1184,12 +1183,25 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
                 }
             d.field_parts = 1;
             while (d.field_parts < 8 && 2 * d.field_parts * visits <= 9L * 148) d.field_parts *= 2;
-            const long adds = std::max(2L * d.pp.n_bands, d.field_parts * (groups + (nt + d.field_L - 1) / d.field_L));
+            const long adds = d.field_parts * (groups + (nt + d.field_L - 1) / d.field_L);
             int lg = 0;
             while ((1L << lg) < adds) lg++;
             const int bits = std::min(32, 40 - lg);
             d.fix_scale = std::ldexp(1.0, bits);
             d.fix_limit = std::ldexp(1.0, 23);
+            // The energy kernel's items (one I tile, 12 warps an SM).
+            const long evisits = (long)nt * (nt + 1) / 2, eresident = 12L * 148;
+            for (int L : {16, 8, 4, 2})
+                if (evisits >= 7 * L * eresident) {
+                    d.energy_L = L;
+                    break;
+                }
+            while (d.energy_parts < 8 && 2 * d.energy_parts * evisits <= 9L * 148) d.energy_parts *= 2;
+            const long echunks = (nt + d.energy_L - 1) / d.energy_L;
+            d.n_eblk = (int)(echunks * (echunks + 1) / 2 * d.energy_L * d.energy_parts);
+            lg = 0;
+            while ((1L << lg) < d.energy_parts * (nt + echunks)) lg++;
+            d.fix_scale_energy = std::ldexp(1.0, std::min(32, 40 - lg));
         }
 
         std::vector<int> eoff(n + 1, 0), ej;
@@ -1229,8 +1241,10 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
         d.thole = dalloc<double>(n, o);
         d.axis = dalloc<int4>(n, o);
         d.posq = dalloc<char>(rsz * d.n_pad, o);
-        d.dipt = dalloc<char>(rsz * d.n_pad, o);
-        d.ind = dalloc<char>(rsz * d.n_pad, o);
+        if (h->precision == TDP_PRECISION_DOUBLE) {   // index-order records of the plain form's energy kernel
+            d.dipt = dalloc<char>(rsz * d.n_pad, o);
+            d.ind = dalloc<char>(rsz * d.n_pad, o);
+        }
         d.yz = dalloc<double2>(d.n_pad, o);
         d.tctr = dalloc<double4>(d.n_pad / kTile, o);
         d.text = dalloc<double4>(d.n_pad / kTile, o);
@@ -1253,10 +1267,13 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
         d.hist = dalloc<double>(n3 * h->extrap.size(), o);
         d.partial = dalloc<double>((size_t)d.nslot * 6 * d.n_pad, o);
         if (d.fix_scale > 0.0) {
-            d.fixacc = dalloc<unsigned long long>(6 * (size_t)d.n_pad, o);
+            d.fixacc = dalloc<unsigned long long>(6 * (size_t)d.n_pad + 1, o);
+            d.axis_cap = std::max(1 << 16, 16 * n);
+            d.axis_pairs = dalloc<int2>(d.axis_cap, o);
+            d.axis_count = dalloc<int>(1, o);
             d.fix_err = dalloc<int>(1, o);
         }
-        d.energy_partial = dalloc<double>((size_t)d.n_eblk, o);
+        d.energy_partial = dalloc<double>((size_t)d.n_eblk + d.n_pad / 128, o);
         d.fpair = dalloc<double>(n3, o);
         d.torque = dalloc<double>(n3, o);
         d.ftotal = dalloc<double>(n3, o);

@@ -134,7 +134,7 @@ __global__ void k_rotate(int n, const double* __restrict__ pos, const double* __
     v.y = (R)d.y;
     v.z = (R)d.z;
     v.w = (R)thole[i];
-    dipt[i] = v;
+    if (sizeof(R) == 8) dipt[i] = v;   // read in index order by the plain form's energy kernel only
     dipt_s[rank[i]] = v;
 }
 
@@ -475,12 +475,20 @@ __global__ void k_eps_scalar(int n, int nblk, const double* __restrict__ eps_par
     if (threadIdx.x == 0) scal[slot] = sqrt(ee / (double)n);
 }
 
-// Induced dipoles packed for the energy kernel.
+// Induced dipoles packed for the energy kernel, by slot where rank is given.
 template <class R>
-__global__ void k_pack_ind(int n, const double* __restrict__ mu, typename Vec4T<R>::type* __restrict__ out) {
+__global__ void k_pack_ind(int n, const int* __restrict__ rank, const double* __restrict__ mu,
+                           typename Vec4T<R>::type* __restrict__ out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    store_vec<R>(out, i, ld3(mu + 3 * i), 0.0);
+    store_vec<R>(out, rank ? rank[i] : i, ld3(mu + 3 * i), 0.0);
+}
+
+// *out = the sum of m parts, in one block.
+__global__ void k_energy_total(int m, const double* __restrict__ parts, double* __restrict__ out) {
+    __shared__ double red[40];
+    const double e = sum_partials(parts, m, red);
+    if (threadIdx.x == 0) *out = e;
 }
 
 // Pair forces/torques and the total energy from the energy-kernel partials.
@@ -813,7 +821,12 @@ void launch_eps_scalar(const Dev& d, int slot, cudaStream_t st) {
 }
 template <class R>
 void launch_pack_ind(const Dev& d, cudaStream_t st) {
-    k_pack_ind<R><<<d.nvb, kVecThreads, 0, st>>>(d.n, d.mu, (typename Vec4T<R>::type*)d.ind);
+    typedef typename Vec4T<R>::type V4;
+    if (sizeof(R) == 4) k_pack_ind<R><<<d.nvb, kVecThreads, 0, st>>>(d.n, d.rank, d.mu, (V4*)d.vec_s);
+    else k_pack_ind<R><<<d.nvb, kVecThreads, 0, st>>>(d.n, nullptr, d.mu, (V4*)d.ind);
+}
+void launch_energy_total(const Dev& d, int m, const double* parts, cudaStream_t st) {
+    k_energy_total<<<1, kVecThreads, 0, st>>>(m, parts, d.energy);
 }
 void launch_energy_done(const Dev& d, cudaStream_t st) {
     k_energy_done<<<d.nvb, kVecThreads, 0, st>>>(d.n, d.nsplit, d.n_pad, d.n_eblk, d.partial, d.energy_partial,

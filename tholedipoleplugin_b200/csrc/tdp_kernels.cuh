@@ -10,7 +10,7 @@ namespace tdp {
 // whole number of bands, nslot partial-sum slots that the pair kernels write
 // (plain all-pairs form: one per band, added into slot 0 before anything reads
 // them), nsplit slots that their consumers add, n_eblk energy partials = one
-// per band pair, nvb blocks of the O(N) kernels).
+// per band pair or item, nvb blocks of the O(N) kernels).
 constexpr int kMuHist = 4;
 
 struct Dev {
@@ -70,7 +70,7 @@ struct Dev {
     double* hist = nullptr;      // extrapolation orders, korder*n*3
     double* partial = nullptr;   // nslot*6*n_pad pair-kernel partial sums (scratch)
     // Mixed all-pairs form: the field and energy kernels add their per-band
-    // sums into one 64-bit fixed-point accumulator (6*n_pad, units of
+    // sums into one 64-bit fixed-point accumulator (6*n_pad + 1, units of
     // 1/fix_scale; integer addition makes the result independent of the order)
     // that a flush kernel converts into partial slot 0 and clears (nsplit = 1).
     // A sum of magnitude >= fix_limit sets *fix_err instead of wrapping.
@@ -80,6 +80,12 @@ struct Dev {
     // Mixed all-pairs field kernel: J tiles per item and parts of each walk
     // (field_items).
     int field_L = 1, field_parts = 1;
+    // The same of the mixed energy kernel, and its accumulator's scale.
+    int energy_L = 1, energy_parts = 1;
+    double fix_scale_energy = 0.0;
+    int2* axis_pairs = nullptr;   // pairs close to the x axis, evaluated apart
+    int* axis_count = nullptr;
+    int axis_cap = 0;
     double* energy_partial = nullptr;
     double* fpair = nullptr;
     double* torque = nullptr;
@@ -101,7 +107,12 @@ constexpr int kFieldNS = 2;
 template <class R> void launch_field(const Dev& d, int kind, cudaStream_t st);
 template <> void launch_field<float>(const Dev& d, int kind, cudaStream_t st);
 template <> void launch_field<double>(const Dev& d, int kind, cudaStream_t st);
+// Pair forces, torques (index order) and the energy from the records of
+// launch_pack_ind.
 template <class R> void launch_energy(const Dev& d, cudaStream_t st);
+template <> void launch_energy<float>(const Dev& d, cudaStream_t st);
+template <> void launch_energy<double>(const Dev& d, cudaStream_t st);
+void launch_energy_total(const Dev& d, int m, const double* parts, cudaStream_t st);
 template <class R> void launch_fixed_done(const Dev& d, cudaStream_t st);
 template <class R> void launch_warm_start(const Dev& d, cudaStream_t st);
 // mu = sum_k c[k] mu_hist[k] over the first nh history entries.

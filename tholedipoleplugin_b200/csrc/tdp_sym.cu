@@ -2,9 +2,9 @@
 // mutual-field matvec, energy/force/torque), each unordered pair evaluated
 // once with both of its sides.
 //
-// Work decomposition.  The mixed form's field kernel takes warp-sized items
-// (k_field_items).  For the others atoms form 32-atom tiles and tiles form bands of
-// band_tiles tiles.  One CTA (4 warps) owns a band pair (p, q), p <= q, and
+// Work decomposition.  Atoms form 32-atom tiles.  The mixed form's kernels take
+// warp-sized items (k_field_items, k_energy_items).  In the plain form's, tiles
+// form bands of band_tiles tiles and one CTA (4 warps) owns a band pair (p, q), p <= q, and
 // evaluates every tile pair (I in band p, J in band q, I <= J).  A warp holds
 // the atoms of its I tile(s) in registers (lane = atom) and walks the atoms of
 // J along the diagonals of the tile pair, the J-side sums travelling with them
@@ -1088,20 +1088,58 @@ __device__ __forceinline__ void energy_walk(const PairParams& P, const double* _
 }
 
 // ---------------------------------------------------------------------------
-// Packed FP32 energy walk (mixed form, non-SLOW tile pairs): the lane's I
-// atom against J atoms m and m + 16 of the tile at once (m = (lane + s) & 15,
-// s = 0..15), the pair routine of pair_energy_sides<R, 3> in f32x2 halves.
-// The J-side sums ride packed (lo: atom m, hi: atom m + 16) and rotate one
-// lane per step; after 16 steps lanes l and l ^ 16 hold the two copies of the
-// sums of atoms l & 15 and (l & 15) + 16, added by one xor-16 shuffle.
+// Mixed-form energy / force / torque walk: the lane's I atom against J atoms m
+// and m + 16 of the tile at once (m = (lane + s) & 15) in f32x2 halves, the
+// J-side sums riding packed and rotating one lane per step as in the field
+// walks.
+//
+// Orientation.  The reference's pair routine has I = lower index, K = higher,
+// d = p_K - p_I.  Tiles here are in spatial order, so a pair may come with its
+// roles exchanged.  That flips Z and Y of the quasi-internal frame (a rotation
+// by pi about X, under which every vector expression of the routine is
+// covariant) and leaves X; what remains is that the terms linear in a charge
+// change sign, and the sign of the force.  So a pair whose I atom has the
+// higher index is evaluated with both charges negated (their product is not)
+// and the force negated: the sign bit of (index of J - index of I) xor-ed in.
+//
+// MODE 0, 1: the pair routine (RTDF.cpp:129-366) in the lab frame, for unit
+// scales and rInvVec[4] = 0 (the default, see TDP_FLAG_DD_FORCE_R4).  What is
+// left of the quasi-internal frame is its X row, the axis its multipole
+// algebra treats as the bond axis (component 0); with x = a u^3, e = exp(-x),
+// tc = 1 - e, w = 1 - (1 + x) e, t0 = 1 - (1 + 3x/2) e, l = 2 (Mutual) or 0:
+//   V_ij  = (q_j/r^2 - 3 (m_j0 + w u_j0)/r^3) X + (m_j + tc u_j)/r^3
+//   V_ji  = (-q_i/r^2 - 3 (m_i0 + w u_i0)/r^3) X + (m_i + tc u_i)/r^3
+//   Vd_ij = (tc q_j/r^2 - 3 w (m_j0 + l u_j0)/r^3) X + tc (m_j + l u_j)/r^3, Vd_ji alike
+//   S   = m_i x V_ij + m_j x V_ji + u_i x Vd_ij + u_j x Vd_ji
+//   f   = (S x X)/r + (q_i q_j/r^2 - 2 (q_i m_j0 - q_j m_i0 + t0 (q_i u_j0 - q_j u_i0))/r^3) X
+//   E   = q_i q_j/r + (q_j m_i0 - q_i m_j0 + tc (q_j u_i0 - q_i u_j0))/(2 r^2) + (m_i.V_ij + m_j.V_ji)/2
+//   F_I -= perm(f), F_J += perm(f), tau_I = -perm(m_i x V_ij), tau_J = -perm(m_j x V_ji)
+// with perm(v) = (v_y, v_z, v_x), the reference's permuted back rotation
+// (:150-159).  The parts of S without X cancel pairwise, so S = K x X with
+// K = a m_i + b m_j + c u_i + d u_j (a, b, c, d the X coefficients of V_ij,
+// V_ji, Vd_ij, Vd_ji) and S x X = (K.X) X - K.  Torques and the dipole energy
+// are linear in V with an atom's own dipole fixed: the walk sums V and the
+// caller takes one cross and one dot product per atom.  MODE 0 is the walk of
+// tile pairs that no damping reaches (tc = w = t0 = 1): with P = m + u and
+// k = l - 1, K = a P_i + b P_j + g u_j0 u_i + g u_i0 u_j, g = -3 k/r^3.
+// X is (d_y^2 + d_z^2, -d_x d_y, -d_x d_z)/(r sqrt(d_y^2 + d_z^2)) where the
+// pair's y or z coordinates differ (:584); pairs within 1e-5 nm of the x axis
+// take the reference's test and Gram-Schmidt as is.
+// MODE 2: the quasi-internal frame routine itself (TDP_FLAG_DD_FORCE_R4).
 // ---------------------------------------------------------------------------
-struct EPackedTile {
+struct EItemTile {
     float4 p0[16], p1[16];   // (x, x', y, y'), (z, z', q, q')   (' = atom m + 16)
-    float4 d0[16], d1[16];   // (mx, mx', my, my'), (mz, mz', t, t')
+    float4 d0[16], d1[16];   // (dx, dx', dy, dy'), (dz, dz', t, t'): m, or m + u in MODE 0
     float4 u0[16], u1[16];   // (ux, ux', uy, uy'), (uz, uz', 1/t, 1/t')
+    int2 id[16];             // atom indices
 };
 
-__device__ __forceinline__ void stage_epacked(EPackedTile& T, int lane, float4 p, float4 d, float4 u) {
+// FP64 positions of the J tile (open systems' charge energy).
+struct EItemPos {
+    double x[32], y[32], z[32];
+};
+
+__device__ __forceinline__ void stage_eitem(EItemTile& T, int lane, float4 p, float4 d, float4 u, int id) {
     const int m = lane & 15, h = lane >> 4;
     float* p0 = reinterpret_cast<float*>(&T.p0[m]);
     float* p1 = reinterpret_cast<float*>(&T.p1[m]);
@@ -1121,296 +1159,10 @@ __device__ __forceinline__ void stage_epacked(EPackedTile& T, int lane, float4 p
     u0[2 + h] = u.y;
     u1[h] = u.z;
     u1[2 + h] = 1.0f / d.w;
+    reinterpret_cast<int*>(&T.id[m])[h] = id;
 }
 
-
-template <bool FOLD>
-__device__ __forceinline__ void energy_walk_x2(const PairParams& P, const double* __restrict__ pos,
-                                               const double2* __restrict__ yz, const EPackedTile& T, int lane,
-                                               int i, int jbase, float oix, float oiy, float oiz, float4 pi,
-                                               float4 di, float4 ui, unsigned fm, float damp_r2, float rv4p,
-                                               float rv4f, bool mutual, float f[6], float gg[6], float& en) {
-    const int nxt = (lane + 1) & 31;
-    const int nmax = P.n_tiles * 32 - 1;
-    const f2 OX = bc2(oix), OY = bc2(oiy), OZ = bc2(oiz);
-    const f2 QI0 = bc2(pi.w), MIX = bc2(di.x), MIY = bc2(di.y), MIZ = bc2(di.z);
-    const f2 UIX = bc2(ui.x), UIY = bc2(ui.y), UIZ = bc2(ui.z);
-    const float ti = di.w, iti = 1.0f / di.w;
-    const f2 ITI = bc2(iti), ONE = bc2(1.0f), HALF = bc2(0.5f);
-    const f2 RV4P = bc2(rv4p), RV4F = bc2(rv4f);
-    f2 Lx = 0, Ly = 0, Lz = 0, Ix = 0, Iy = 0, Iz = 0, NTx = 0, NTy = 0, NTz = 0;
-    if (FOLD) {
-        Lx = bc2(-(float)P.box[0]);
-        Ly = bc2(-(float)P.box[1]);
-        Lz = bc2(-(float)P.box[2]);
-        Ix = bc2((float)P.inv_box[0]);
-        Iy = bc2((float)P.inv_box[1]);
-        Iz = bc2((float)P.inv_box[2]);
-        NTx = bc2(-(float)(P.half_box_tol[0] * P.half_box_tol[0]));
-        NTy = bc2(-(float)(P.half_box_tol[1] * P.half_box_tol[1]));
-        NTz = bc2(-(float)(P.half_box_tol[2] * P.half_box_tol[2]));
-    }
-    // Torques from summed V (pair_energy_lab, VSUM): TX.. sum V_ij, UX.. V_ji.
-    f2 FX = 0, FY = 0, FZ = 0, TX = 0, TY = 0, TZ = 0, EN = 0;        // I side
-    f2 GX = 0, GY = 0, GZ = 0, UX = 0, UY = 0, UZ = 0;                // J side (packed atoms m, m + 16)
-#pragma unroll 1
-    for (int s = 0; s < 16; s++) {
-        const int m = (lane + s) & 15;
-        const float4 a = T.p0[m], b = T.p1[m], c = T.d0[m], d = T.d1[m], e = T.u0[m], h = T.u1[m];
-        f2 DX = sub2(pk2(a.x, a.y), OX), DY = sub2(pk2(a.z, a.w), OY), DZ = sub2(pk2(b.x, b.y), OZ);
-        const int ja = jbase + m, jb = ja + 16;
-        if (FOLD) {
-            // As in xslot_pairs: one sign-bit AND of the d^2 - t^2 words flags
-            // the pairs within the margin of half a box.
-            f2 neg = ~0ull;
-            if (fm & 1u) {
-                DX = fold2(DX, Lx, Ix);
-                neg &= fma2(DX, DX, NTx);
-            }
-            if (fm & 2u) {
-                DY = fold2(DY, Ly, Iy);
-                neg &= fma2(DY, DY, NTy);
-            }
-            if (fm & 4u) {
-                DZ = fold2(DZ, Lz, Iz);
-                neg &= fma2(DZ, DZ, NTz);
-            }
-            const f2 flag = ~neg & 0x8000000080000000ull;
-            if (flag) {
-                const bool amb_a = (flag >> 31) & 1ull, amb_b = (flag >> 63) != 0ull;
-                float ax, bx, ay, by, az, bz;
-                un2(DX, ax, bx);
-                un2(DY, ay, by);
-                un2(DZ, az, bz);
-                if (amb_a) {
-                    d3 q = exact_delta(P, pos, i, ja);
-                    ax = (float)q.x;
-                    ay = (float)q.y;
-                    az = (float)q.z;
-                }
-                if (amb_b) {
-                    d3 q = exact_delta(P, pos, i, jb);
-                    bx = (float)q.x;
-                    by = (float)q.y;
-                    bz = (float)q.z;
-                }
-                DX = pk2(ax, bx);
-                DY = pk2(ay, by);
-                DZ = pk2(az, bz);
-            }
-        }
-        const f2 R2 = dot2(DX, DY, DZ, DX, DY, DZ);
-        float r2a, r2b, dya, dyb, dza, dzb;
-        un2(R2, r2a, r2b);
-        un2(DY, dya, dyb);
-        un2(DZ, dza, dzb);
-        const bool yza = yz_differ<float>(dya, dza, yz, i, ja, nmax);
-        const bool yzb = yz_differ<float>(dyb, dzb, yz, i, jb, nmax);
-        const f2 RINV = pk2(rsqrtf(r2a), rsqrtf(r2b));
-        // QI frame: Z along d; X from Z + x^ or y^ (the reference's yz test), Gram-Schmidt; Y = Z x X.
-        const f2 ZX = mul2(DX, RINV), ZY = mul2(DY, RINV), ZZ = mul2(DZ, RINV);
-        f2 XX = add2(ZX, pk2(yza ? 1.0f : 0.0f, yzb ? 1.0f : 0.0f));
-        f2 XY = add2(ZY, pk2(yza ? 0.0f : 1.0f, yzb ? 0.0f : 1.0f));
-        f2 XZ = ZZ;
-        const f2 NDT = neg2(dot2(ZX, ZY, ZZ, XX, XY, XZ));
-        XX = fma2(ZX, NDT, XX);
-        XY = fma2(ZY, NDT, XY);
-        XZ = fma2(ZZ, NDT, XZ);
-        float xna, xnb;
-        un2(dot2(XX, XY, XZ, XX, XY, XZ), xna, xnb);
-        const f2 SN = pk2(xna > 0.0f ? rsqrtf(xna) : 1.0f, xnb > 0.0f ? rsqrtf(xnb) : 1.0f);
-        XX = mul2(XX, SN);
-        XY = mul2(XY, SN);
-        XZ = mul2(XZ, SN);
-        const f2 YX = fma2(ZY, XZ, neg2(mul2(ZZ, XY)));
-        const f2 YY = fma2(ZZ, XX, neg2(mul2(ZX, XZ)));
-        const f2 YZ = fma2(ZX, XY, neg2(mul2(ZY, XX)));
-        // Rotated multipoles.
-        const f2 UJX = pk2(e.x, e.y), UJY = pk2(e.z, e.w), UJZ = pk2(h.x, h.y);
-        const f2 MJX = pk2(c.x, c.y), MJY = pk2(c.z, c.w), MJZ = pk2(d.x, d.y);
-        const f2 uI0 = dot2(XX, XY, XZ, UIX, UIY, UIZ), uI1 = dot2(YX, YY, YZ, UIX, UIY, UIZ),
-                 uI2 = dot2(ZX, ZY, ZZ, UIX, UIY, UIZ);
-        const f2 uJ0 = dot2(XX, XY, XZ, UJX, UJY, UJZ), uJ1 = dot2(YX, YY, YZ, UJX, UJY, UJZ),
-                 uJ2 = dot2(ZX, ZY, ZZ, UJX, UJY, UJZ);
-        const f2 QJ0 = pk2(b.z, b.w);
-        const f2 QI1 = dot2(XX, XY, XZ, MIX, MIY, MIZ), QI2 = dot2(YX, YY, YZ, MIX, MIY, MIZ),
-                 QI3 = dot2(ZX, ZY, ZZ, MIX, MIY, MIZ);
-        const f2 QJ1 = dot2(XX, XY, XZ, MJX, MJY, MJZ), QJ2 = dot2(YX, YY, YZ, MJX, MJY, MJZ),
-                 QJ3 = dot2(ZX, ZY, ZZ, MJX, MJY, MJZ);
-        const f2 rv1 = RINV, rv2 = mul2(RINV, RINV), rv3 = mul2(rv2, RINV);
-        const f2 rv4 = fma2(RV4P, mul2(rv3, RINV), RV4F);
-        // Thole factors (1 beyond damp_r2 or where t_i t_j <= 1e-5, as the reference).
-        f2 tc = ONE, td0 = ONE, td1 = ONE, dtc = ONE, dtd0 = ONE, dtd1 = ONE;
-        if (r2a < damp_r2 || r2b < damp_r2) {
-            const f2 R = mul2(R2, RINV);
-            const f2 U = mul2(mul2(R, ITI), pk2(h.z, h.w));
-            const f2 AM = pk2(fminf(ti, d.z), fminf(ti, d.w));
-            const f2 AU3 = mul2(AM, mul2(U, mul2(U, U)));
-            float xa, xb;
-            un2(AU3, xa, xb);
-            const bool da = r2a < damp_r2 && fabsf(ti * d.z) > 1.0e-5f;
-            const bool db = r2b < damp_r2 && fabsf(ti * d.w) > 1.0e-5f;
-            const f2 EX = pk2(da ? __expf(-xa) : 0.0f, db ? __expf(-xb) : 0.0f);
-            const f2 AUs = pk2(da ? xa : 0.0f, db ? xb : 0.0f);   // no inf/NaN into the products
-            const f2 NEX = neg2(EX);
-            tc = add2(ONE, NEX);
-            td1 = tc;
-            td0 = fma2(NEX, fma2(bc2(1.5f), AUs, ONE), ONE);
-            dtc = td0;
-            dtd0 = fma2(NEX, fma2(mul2(bc2(1.5f), AUs), AUs, add2(ONE, AUs)), ONE);
-            dtd1 = fma2(NEX, add2(ONE, AUs), ONE);
-        }
-        // Interaction terms (mS = iS = 1).
-        f2 eP = rv1, dP = mul2(bc2(-0.5f), rv2);
-        f2 Vij0 = mul2(eP, QJ0), Vji0 = mul2(eP, QI0), VijR0 = mul2(dP, QJ0), VjiR0 = mul2(dP, QI0);
-        eP = rv2;
-        f2 eU = mul2(rv2, tc);
-        dP = neg2(rv3);
-        f2 dU = mul2(mul2(bc2(-2.0f), rv3), dtc);
-        Vij0 = sub2(Vij0, fma2(eP, QJ1, mul2(eU, uJ0)));
-        const f2 Vji1n = mul2(eP, QI0);   // -Vji1 so far (subtracted below: exact)
-        VijR0 = sub2(VijR0, fma2(dP, QJ1, mul2(dU, uJ0)));
-        f2 VjiR1 = mul2(rv3, QI0);        // -(dP QI0), dP = -rv3: exact
-        f2 Vjid0 = neg2(mul2(eU, QI0));
-        f2 Vij1 = mul2(eP, QJ0);
-        Vji0 = add2(Vji0, fma2(eP, QI1, mul2(eU, uI0)));
-        f2 VijR1 = mul2(dP, QJ0);
-        VjiR0 = add2(VjiR0, fma2(dP, QI1, mul2(dU, uI0)));
-        f2 Vijd0 = mul2(eU, QJ0);
-        eP = mul2(bc2(-2.0f), rv3);
-        eU = mul2(eP, td0);
-        dP = mul2(bc2(3.0f), rv4);
-        dU = mul2(mul2(bc2(6.0f), rv4), dtd0);
-        Vij1 = add2(Vij1, fma2(eP, QJ1, mul2(eU, uJ0)));
-        f2 Vji1 = sub2(fma2(eP, QI1, mul2(eU, uI0)), Vji1n);
-        VijR1 = add2(VijR1, fma2(dP, QJ1, mul2(dU, uJ0)));
-        VjiR1 = add2(VjiR1, fma2(dP, QI1, mul2(dU, uI0)));
-        Vijd0 = fma2(eU, QJ1, Vijd0);
-        Vjid0 = fma2(eU, QI1, Vjid0);
-        eP = rv3;
-        eU = mul2(rv3, td1);
-        dP = mul2(bc2(-1.5f), rv4);
-        dU = mul2(mul2(bc2(-3.0f), rv4), dtd1);
-        const f2 Vij2 = fma2(eP, QJ2, mul2(eU, uJ1)), Vji2 = fma2(eP, QI2, mul2(eU, uI1));
-        const f2 VijR2 = fma2(dP, QJ2, mul2(dU, uJ1)), VjiR2 = fma2(dP, QI2, mul2(dU, uI1));
-        const f2 Vijd1 = mul2(eU, QJ2), Vjid1 = mul2(eU, QI2);
-        const f2 Vij3 = fma2(eP, QJ3, mul2(eU, uJ2)), Vji3 = fma2(eP, QI3, mul2(eU, uI2));
-        const f2 VijR3 = fma2(dP, QJ3, mul2(dU, uJ2)), VjiR3 = fma2(dP, QI3, mul2(dU, uI2));
-        const f2 Vijd2 = mul2(eU, QJ3), Vjid2 = mul2(eU, QI3);
-
-        f2 fIZ = fma2(QI0, VijR0, fma2(QI1, VijR1, fma2(QI2, VijR2, mul2(QI3, VijR3))));
-        f2 fJZ = fma2(QJ0, VjiR0, fma2(QJ1, VjiR1, fma2(QJ2, VjiR2, mul2(QJ3, VjiR3))));
-        const f2 EIX = sub2(mul2(QI3, Vij1), mul2(QI1, Vij3));
-        const f2 EIY = sub2(mul2(QI1, Vij2), mul2(QI2, Vij1));
-        const f2 EJX = sub2(mul2(QJ3, Vji1), mul2(QJ1, Vji3));
-        const f2 EJY = sub2(mul2(QJ1, Vji2), mul2(QJ2, Vji1));
-        f2 iEIX = sub2(mul2(uI2, Vijd0), mul2(uI0, Vijd2));
-        f2 iEJX = sub2(mul2(uJ2, Vjid0), mul2(uJ0, Vjid2));
-        f2 iEIY = sub2(mul2(uI0, Vijd1), mul2(uI1, Vijd0));
-        f2 iEJY = sub2(mul2(uJ0, Vjid1), mul2(uJ1, Vjid0));
-        if (mutual) {
-            f2 eC = mul2(mul2(bc2(-4.0f), rv3), td0);
-            f2 dC = mul2(mul2(bc2(6.0f), rv4), dtd0);
-            iEIX = fma2(mul2(eC, uI2), uJ0, iEIX);
-            iEJX = fma2(mul2(eC, uJ2), uI0, iEJX);
-            iEIY = sub2(iEIY, mul2(mul2(eC, uI1), uJ0));
-            iEJY = sub2(iEJY, mul2(mul2(eC, uJ1), uI0));
-            fIZ = fma2(mul2(dC, uI0), uJ0, fIZ);
-            fJZ = fma2(mul2(dC, uJ0), uI0, fJZ);
-            eC = mul2(mul2(bc2(2.0f), rv3), td1);
-            dC = mul2(mul2(bc2(-3.0f), rv4), dtd1);
-            iEIX = sub2(iEIX, mul2(mul2(eC, uI0), uJ2));
-            iEJX = sub2(iEJX, mul2(mul2(eC, uJ0), uI2));
-            iEIY = fma2(mul2(eC, uI0), uJ1, iEIY);
-            iEJY = fma2(mul2(eC, uJ0), uI1, iEJY);
-            const f2 uu = fma2(uI1, uJ1, mul2(uI2, uJ2));
-            fIZ = fma2(dC, uu, fIZ);
-            fJZ = fma2(dC, uu, fJZ);
-        }
-        // nqf = -qf (the QI-frame force); every sign flip below is exact.
-        const f2 nqf0 = neg2(mul2(RINV, add2(add2(EIY, EJY), add2(iEIY, iEJY))));
-        const f2 nqf1 = mul2(RINV, add2(add2(EIX, EJX), add2(iEIX, iEJX)));
-        const f2 nqf2 = add2(fJZ, fIZ);
-        // Back rotation with the reference's permuted matrix: nfv = -fv.
-        const f2 nfvx = fma2(YY, nqf0, fma2(ZY, nqf1, mul2(XY, nqf2)));
-        const f2 nfvy = fma2(YZ, nqf0, fma2(ZZ, nqf1, mul2(XZ, nqf2)));
-        const f2 nfvz = fma2(YX, nqf0, fma2(ZX, nqf1, mul2(XX, nqf2)));
-        {
-            const f2 EIZ = sub2(mul2(QI2, Vij3), mul2(QI3, Vij2));
-            // Torque of the QI-frame vector -E_I, rotated back (sign folded into the sub).
-            TX = sub2(TX, fma2(YY, EIX, fma2(ZY, EIY, mul2(XY, EIZ))));
-            TY = sub2(TY, fma2(YZ, EIX, fma2(ZZ, EIY, mul2(XZ, EIZ))));
-            TZ = sub2(TZ, fma2(YX, EIX, fma2(ZX, EIY, mul2(XX, EIZ))));
-            FX = add2(FX, nfvx);
-            FY = add2(FY, nfvy);
-            FZ = add2(FZ, nfvz);
-            f2 eq = fma2(QI0, Vij0, mul2(QJ0, Vji0));
-            eq = fma2(QI1, Vij1, fma2(QJ1, Vji1, eq));
-            eq = fma2(QI2, Vij2, fma2(QJ2, Vji2, eq));
-            eq = fma2(QI3, Vij3, fma2(QJ3, Vji3, eq));
-            EN = fma2(HALF, eq, EN);
-        }
-        {
-            const f2 EJZ = sub2(mul2(QJ2, Vji3), mul2(QJ3, Vji2));
-            UX = sub2(UX, fma2(YY, EJX, fma2(ZY, EJY, mul2(XY, EJZ))));
-            UY = sub2(UY, fma2(YZ, EJX, fma2(ZZ, EJY, mul2(XZ, EJZ))));
-            UZ = sub2(UZ, fma2(YX, EJX, fma2(ZX, EJY, mul2(XX, EJZ))));
-            GX = sub2(GX, nfvx);
-            GY = sub2(GY, nfvy);
-            GZ = sub2(GZ, nfvz);
-        }
-        // Rotate the packed J-side sums one lane (64-bit shuffles).
-        GX = __shfl_sync(kFull, GX, nxt);
-        GY = __shfl_sync(kFull, GY, nxt);
-        GZ = __shfl_sync(kFull, GZ, nxt);
-        UX = __shfl_sync(kFull, UX, nxt);
-        UY = __shfl_sync(kFull, UY, nxt);
-        UZ = __shfl_sync(kFull, UZ, nxt);
-    }
-    float lo, hi;
-    const f2* Is[7] = {&FX, &FY, &FZ, &TX, &TY, &TZ, &EN};
-    float* Io[7] = {&f[0], &f[1], &f[2], &f[3], &f[4], &f[5], &en};
-#pragma unroll
-    for (int k = 0; k < 7; k++) {
-        un2(*Is[k], lo, hi);
-        *Io[k] += lo + hi;
-    }
-    // Lane l now holds (atom l & 15, atom (l & 15) + 16); lane l ^ 16 the other copy.
-    const f2 Js[6] = {GX, GY, GZ, UX, UY, UZ};
-#pragma unroll
-    for (int k = 0; k < 6; k++) {
-        un2(Js[k], lo, hi);
-        const float olo = __shfl_xor_sync(kFull, lo, 16), ohi = __shfl_xor_sync(kFull, hi, 16);
-        gg[k] += lane < 16 ? lo + olo : hi + ohi;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Packed FP32 energy walk for tile pairs that no Thole damping reaches (every
-// damping factor 1), with unit scales and rInvVec[4] = 0 (the default, see
-// TDP_FLAG_DD_FORCE_R4).  It computes the reference's pair routine
-// (RTDF.cpp:129-366) in the lab frame.  With all damping factors 1 the
-// permanent and induced coefficients of calculateElectrostaticPairIxn merge
-// and every rInvVec[4] term vanishes; what is left of the quasi-internal
-// frame is its X row, the axis its multipole algebra treats as the bond axis
-// (component 0).  With P = m + u and W = m + 2u (W = m without the
-// induced-induced terms, i.e. unless Mutual), X-components written _0:
-//   E   = q_i q_j / r + (q_j (P_i0 + m_i0) - q_i (P_j0 + m_j0)) / (2 r^2)
-//         + (m_i.P_j + m_j.P_i - 3 (m_i0 P_j0 + m_j0 P_i0)) / (2 r^3)
-//   V_ij = (q_j/r^2 - 3 P_j0/r^3) X + P_j/r^3,  V_ji = (-q_i/r^2 - 3 P_i0/r^3) X + P_i/r^3
-//   Vd_ij, Vd_ji: the same with W for P
-//   S   = m_i x V_ij + m_j x V_ji + u_i x Vd_ij + u_j x Vd_ji
-//   f   = (S x X) / r + (q_i q_j / r^2 - 2 (q_i P_j0 - q_j P_i0) / r^3) X
-//   F_i -= perm(f), F_j += perm(f), tau_i = -perm(m_i x V_ij), tau_j = -perm(m_j x V_ji)
-// where perm(v) = (v_y, v_z, v_x) is the reference's permuted back rotation
-// (:150-159).  This is an exact rewrite (FP64 transcriptions of both agree to
-// rounding), with X from the frame test as there: X = (x^ - Z_x Z)/|.| when
-// the pair's y or z coordinates differ (:584), written here as
-// (d_y^2 + d_z^2, -d_x d_y, -d_x d_z) / (r sqrt(d_y^2 + d_z^2)); pairs within
-// 1e-5 nm of the x axis take the reference's test and Gram-Schmidt as is.
-// ---------------------------------------------------------------------------
 __device__ __forceinline__ f2 xneg2(f2 a) { return a ^ 0x8000000080000000ull; }
-
 
 // X row of formQIRotationMatrix (RTDF.cpp:580-593) for one pair, as the
 // general walk forms it.
@@ -1431,23 +1183,291 @@ __device__ __forceinline__ void qi_frame_x(float dx, float dy, float dz, float r
     xz *= s;
 }
 
-template <bool FOLD>
-__device__ __forceinline__ void energy_walk_x2_fast(const PairParams& P, const double* __restrict__ pos,
-                                                    const double2* __restrict__ yz, const EPackedTile& T, int lane,
-                                                    int i, int jbase, float oix, float oiy, float oiz, float4 pi,
-                                                    float4 di, float4 ui, unsigned fm, bool mutual, float f[6],
-                                                    float gg[6], float& en) {
+// formQIRotationMatrix's test on the raw positions by slot, pI.y != pK.y ||
+// pI.z != pK.z (RTDF.cpp:584): displacements above 1e-5 nm decide it; below
+// that the raw FP64 coordinates are compared.
+__device__ __forceinline__ bool yz_differ_slot(float dy, float dz, const double* __restrict__ pos, int i, int j) {
+    if (fabsf(dy) > 1e-5f || fabsf(dz) > 1e-5f) return true;
+    return pos[3 * (size_t)i + 1] != pos[3 * (size_t)j + 1] || pos[3 * (size_t)i + 2] != pos[3 * (size_t)j + 2];
+}
+
+// The index-order records of the atoms (FP32 offsets from the centres of the
+// 32-atom tiles in index order), and the sorted ones by slot.
+struct IndexRecords {
+    const float4* posq;
+    const double4* tctr;
+    const float4 *posq_s, *dipt_s, *ind_s;
+};
+
+// p_j - p_i of slots i and j (atoms id_i, id_j) from the index-order records,
+// whose rounding does not change when the atoms are sorted anew.
+__device__ __forceinline__ void index_delta(const PairParams& P, const IndexRecords& R, const double* __restrict__ pos,
+                                            int i, int j, int id_i, int id_j, float& dx, float& dy, float& dz) {
+    const bool swap = id_i > id_j;
+    const int lo = swap ? id_j : id_i, hi = swap ? id_i : id_j;
+    const float4 a = R.posq[lo], b = R.posq[hi];
+    const double4 ca = R.tctr[lo >> 5], cb = R.tctr[hi >> 5];
+    double c[3] = {cb.x - ca.x, cb.y - ca.y, cb.z - ca.z};
+    const float pa[3] = {a.x, a.y, a.z}, pb[3] = {b.x, b.y, b.z};
+    float d[3];
+    bool near_half = false;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        if (P.periodic) c[k] = fold_d(c[k], P.box[k], P.inv_box[k]);
+        d[k] = pb[k] - (pa[k] - (float)c[k]);
+        if (P.periodic) {
+            d[k] = fold_f(d[k], (float)P.box[k], (float)P.inv_box[k]);
+            near_half = near_half || fabsf(d[k]) >= (float)P.half_box_tol[k];
+        }
+    }
+    if (near_half) {
+        const d3 e = exact_delta(P, pos, swap ? j : i, swap ? i : j);
+        d[0] = (float)e.x;
+        d[1] = (float)e.y;
+        d[2] = (float)e.z;
+    }
+    dx = swap ? -d[0] : d[0];
+    dy = swap ? -d[1] : d[1];
+    dz = swap ? -d[2] : d[2];
+}
+
+// The pair routine in its quasi-internal frame (RTDF.cpp:129-366) on both
+// halves, given the frame's X row: -f (added to I's force, subtracted from
+// K's), the vectors that come off the two torques, and twice the energy.
+struct QiPair {
+    f2 nfx, nfy, nfz, tx, ty, tz, ux, uy, uz, e2;
+};
+
+__device__ __forceinline__ QiPair qi_pair2(const PairParams& P, f2 DX, f2 DY, f2 DZ, f2 R2, f2 RINV, float r2a,
+                                           float r2b, f2 XX, f2 XY, f2 XZ, f2 QIS, f2 MIX, f2 MIY, f2 MIZ, f2 UIX,
+                                           f2 UIY, f2 UIZ, float ti, float iti, f2 QJS, f2 MJX, f2 MJY, f2 MJZ, f2 UJX,
+                                           f2 UJY, f2 UJZ, float tja, float tjb, float itja, float itjb) {
+    const f2 RV4P = bc2(P.rinv4_power), RV4F = bc2(P.rinv4_fill), ITI = bc2(iti), ONE = bc2(1.0f);
+    const float damp_r2 = P.damp_r2;
+    // QI frame: Z along d, Y = Z x X.
+    const f2 ZX = mul2(DX, RINV), ZY = mul2(DY, RINV), ZZ = mul2(DZ, RINV);
+    const f2 YX = fma2(ZY, XZ, neg2(mul2(ZZ, XY)));
+    const f2 YY = fma2(ZZ, XX, neg2(mul2(ZX, XZ)));
+    const f2 YZ = fma2(ZX, XY, neg2(mul2(ZY, XX)));
+    // Rotated multipoles.
+    const f2 uI0 = dot2(XX, XY, XZ, UIX, UIY, UIZ), uI1 = dot2(YX, YY, YZ, UIX, UIY, UIZ),
+             uI2 = dot2(ZX, ZY, ZZ, UIX, UIY, UIZ);
+    const f2 uJ0 = dot2(XX, XY, XZ, UJX, UJY, UJZ), uJ1 = dot2(YX, YY, YZ, UJX, UJY, UJZ),
+             uJ2 = dot2(ZX, ZY, ZZ, UJX, UJY, UJZ);
+            const f2 QI1 = dot2(XX, XY, XZ, MIX, MIY, MIZ), QI2 = dot2(YX, YY, YZ, MIX, MIY, MIZ),
+             QI3 = dot2(ZX, ZY, ZZ, MIX, MIY, MIZ);
+    const f2 QJ1 = dot2(XX, XY, XZ, MJX, MJY, MJZ), QJ2 = dot2(YX, YY, YZ, MJX, MJY, MJZ),
+             QJ3 = dot2(ZX, ZY, ZZ, MJX, MJY, MJZ);
+    const f2 rv1 = RINV, rv2 = mul2(RINV, RINV), rv3 = mul2(rv2, RINV);
+    const f2 rv4 = fma2(RV4P, mul2(rv3, RINV), RV4F);
+    // Thole factors (1 beyond damp_r2 or where t_i t_j <= 1e-5, as the reference).
+    f2 tc = ONE, td0 = ONE, td1 = ONE, dtc = ONE, dtd0 = ONE, dtd1 = ONE;
+    if (r2a < damp_r2 || r2b < damp_r2) {
+        const f2 R = mul2(R2, RINV);
+        const f2 U = mul2(mul2(R, ITI), pk2(itja, itjb));
+        const f2 AM = pk2(fminf(ti, tja), fminf(ti, tjb));
+        const f2 AU3 = mul2(AM, mul2(U, mul2(U, U)));
+        float xa, xb;
+        un2(AU3, xa, xb);
+        const bool da = r2a < damp_r2 && fabsf(ti * tja) > 1.0e-5f;
+        const bool db = r2b < damp_r2 && fabsf(ti * tjb) > 1.0e-5f;
+        const f2 EX = pk2(da ? __expf(-xa) : 0.0f, db ? __expf(-xb) : 0.0f);
+        const f2 AUs = pk2(da ? xa : 0.0f, db ? xb : 0.0f);   // no inf/NaN into the products
+        const f2 NEX = neg2(EX);
+        tc = add2(ONE, NEX);
+        td1 = tc;
+        td0 = fma2(NEX, fma2(bc2(1.5f), AUs, ONE), ONE);
+        dtc = td0;
+        dtd0 = fma2(NEX, fma2(mul2(bc2(1.5f), AUs), AUs, add2(ONE, AUs)), ONE);
+        dtd1 = fma2(NEX, add2(ONE, AUs), ONE);
+    }
+    // Interaction terms (mS = iS = 1).
+    f2 eP = rv1, dP = mul2(bc2(-0.5f), rv2);
+    f2 Vij0 = mul2(eP, QJS), Vji0 = mul2(eP, QIS), VijR0 = mul2(dP, QJS), VjiR0 = mul2(dP, QIS);
+    eP = rv2;
+    f2 eU = mul2(rv2, tc);
+    dP = neg2(rv3);
+    f2 dU = mul2(mul2(bc2(-2.0f), rv3), dtc);
+    Vij0 = sub2(Vij0, fma2(eP, QJ1, mul2(eU, uJ0)));
+    const f2 Vji1n = mul2(eP, QIS);   // -Vji1 so far (subtracted below: exact)
+    VijR0 = sub2(VijR0, fma2(dP, QJ1, mul2(dU, uJ0)));
+    f2 VjiR1 = mul2(rv3, QIS);        // -(dP QIS), dP = -rv3: exact
+    f2 Vjid0 = neg2(mul2(eU, QIS));
+    f2 Vij1 = mul2(eP, QJS);
+    Vji0 = add2(Vji0, fma2(eP, QI1, mul2(eU, uI0)));
+    f2 VijR1 = mul2(dP, QJS);
+    VjiR0 = add2(VjiR0, fma2(dP, QI1, mul2(dU, uI0)));
+    f2 Vijd0 = mul2(eU, QJS);
+    eP = mul2(bc2(-2.0f), rv3);
+    eU = mul2(eP, td0);
+    dP = mul2(bc2(3.0f), rv4);
+    dU = mul2(mul2(bc2(6.0f), rv4), dtd0);
+    Vij1 = add2(Vij1, fma2(eP, QJ1, mul2(eU, uJ0)));
+    f2 Vji1 = sub2(fma2(eP, QI1, mul2(eU, uI0)), Vji1n);
+    VijR1 = add2(VijR1, fma2(dP, QJ1, mul2(dU, uJ0)));
+    VjiR1 = add2(VjiR1, fma2(dP, QI1, mul2(dU, uI0)));
+    Vijd0 = fma2(eU, QJ1, Vijd0);
+    Vjid0 = fma2(eU, QI1, Vjid0);
+    eP = rv3;
+    eU = mul2(rv3, td1);
+    dP = mul2(bc2(-1.5f), rv4);
+    dU = mul2(mul2(bc2(-3.0f), rv4), dtd1);
+    const f2 Vij2 = fma2(eP, QJ2, mul2(eU, uJ1)), Vji2 = fma2(eP, QI2, mul2(eU, uI1));
+    const f2 VijR2 = fma2(dP, QJ2, mul2(dU, uJ1)), VjiR2 = fma2(dP, QI2, mul2(dU, uI1));
+    const f2 Vijd1 = mul2(eU, QJ2), Vjid1 = mul2(eU, QI2);
+    const f2 Vij3 = fma2(eP, QJ3, mul2(eU, uJ2)), Vji3 = fma2(eP, QI3, mul2(eU, uI2));
+    const f2 VijR3 = fma2(dP, QJ3, mul2(dU, uJ2)), VjiR3 = fma2(dP, QI3, mul2(dU, uI2));
+    const f2 Vijd2 = mul2(eU, QJ3), Vjid2 = mul2(eU, QI3);
+
+    f2 fIZ = fma2(QIS, VijR0, fma2(QI1, VijR1, fma2(QI2, VijR2, mul2(QI3, VijR3))));
+    f2 fJZ = fma2(QJS, VjiR0, fma2(QJ1, VjiR1, fma2(QJ2, VjiR2, mul2(QJ3, VjiR3))));
+    const f2 EIX = sub2(mul2(QI3, Vij1), mul2(QI1, Vij3));
+    const f2 EIY = sub2(mul2(QI1, Vij2), mul2(QI2, Vij1));
+    const f2 EJX = sub2(mul2(QJ3, Vji1), mul2(QJ1, Vji3));
+    const f2 EJY = sub2(mul2(QJ1, Vji2), mul2(QJ2, Vji1));
+    f2 iEIX = sub2(mul2(uI2, Vijd0), mul2(uI0, Vijd2));
+    f2 iEJX = sub2(mul2(uJ2, Vjid0), mul2(uJ0, Vjid2));
+    f2 iEIY = sub2(mul2(uI0, Vijd1), mul2(uI1, Vijd0));
+    f2 iEJY = sub2(mul2(uJ0, Vjid1), mul2(uJ1, Vjid0));
+    if (P.mutual) {
+        f2 eC = mul2(mul2(bc2(-4.0f), rv3), td0);
+        f2 dC = mul2(mul2(bc2(6.0f), rv4), dtd0);
+        iEIX = fma2(mul2(eC, uI2), uJ0, iEIX);
+        iEJX = fma2(mul2(eC, uJ2), uI0, iEJX);
+        iEIY = sub2(iEIY, mul2(mul2(eC, uI1), uJ0));
+        iEJY = sub2(iEJY, mul2(mul2(eC, uJ1), uI0));
+        fIZ = fma2(mul2(dC, uI0), uJ0, fIZ);
+        fJZ = fma2(mul2(dC, uJ0), uI0, fJZ);
+        eC = mul2(mul2(bc2(2.0f), rv3), td1);
+        dC = mul2(mul2(bc2(-3.0f), rv4), dtd1);
+        iEIX = sub2(iEIX, mul2(mul2(eC, uI0), uJ2));
+        iEJX = sub2(iEJX, mul2(mul2(eC, uJ0), uI2));
+        iEIY = fma2(mul2(eC, uI0), uJ1, iEIY);
+        iEJY = fma2(mul2(eC, uJ0), uI1, iEJY);
+        const f2 uu = fma2(uI1, uJ1, mul2(uI2, uJ2));
+        fIZ = fma2(dC, uu, fIZ);
+        fJZ = fma2(dC, uu, fJZ);
+    }
+    // nqf = -qf (the QI-frame force); every sign flip below is exact.
+    const f2 nqf0 = neg2(mul2(RINV, add2(add2(EIY, EJY), add2(iEIY, iEJY))));
+    const f2 nqf1 = mul2(RINV, add2(add2(EIX, EJX), add2(iEIX, iEJX)));
+    const f2 nqf2 = add2(fJZ, fIZ);
+    // Back rotation with the reference's permuted matrix: nfv = -fv.
+    const f2 nfvx = fma2(YY, nqf0, fma2(ZY, nqf1, mul2(XY, nqf2)));
+    const f2 nfvy = fma2(YZ, nqf0, fma2(ZZ, nqf1, mul2(XZ, nqf2)));
+    const f2 nfvz = fma2(YX, nqf0, fma2(ZX, nqf1, mul2(XX, nqf2)));
+    QiPair o;
+    o.nfx = nfvx;
+    o.nfy = nfvy;
+    o.nfz = nfvz;
+    const f2 EIZ = sub2(mul2(QI2, Vij3), mul2(QI3, Vij2)), EJZ = sub2(mul2(QJ2, Vji3), mul2(QJ3, Vji2));
+    o.tx = fma2(YY, EIX, fma2(ZY, EIY, mul2(XY, EIZ)));
+    o.ty = fma2(YZ, EIX, fma2(ZZ, EIY, mul2(XZ, EIZ)));
+    o.tz = fma2(YX, EIX, fma2(ZX, EIY, mul2(XX, EIZ)));
+    o.ux = fma2(YY, EJX, fma2(ZY, EJY, mul2(XY, EJZ)));
+    o.uy = fma2(YZ, EJX, fma2(ZZ, EJY, mul2(XZ, EJZ)));
+    o.uz = fma2(YX, EJX, fma2(ZX, EJY, mul2(XX, EJZ)));
+    o.e2 = fma2(QI3, Vij3, fma2(QJ3, Vji3, fma2(QI2, Vij2, fma2(QJ2, Vji2, fma2(QI1, Vij1, fma2(QJ1, Vji1,
+               fma2(QIS, Vij0, mul2(QJS, Vji0))))))));
+    return o;
+}
+
+// Pairs within these distances of the x axis (squared, nm^2) go to the list of
+// k_axis_pairs (tile pairs within the damping range) or take index_delta
+// (beyond it, where the pair forces are small).
+constexpr float kNearAxis2 = 3.6e-5f, kNearAxisFar2 = 2.5e-7f;
+
+// Pairs (slots) that a walk left to k_axis_pairs.  Sized for 16 an atom; past
+// that a pair stays in its walk.
+struct AxisList {
+    int2* pairs;
+    int* count;
+    int cap;
+};
+
+__device__ __forceinline__ bool axis_push(const AxisList& A, int i, int j) {
+    const int k = atomicAdd(A.count, 1);
+    if (k >= A.cap) return false;
+    A.pairs[k] = make_int2(i, j);
+    return true;
+}
+
+// The listed pairs close to the x axis, each by itself: X's azimuth is that of
+// (d_y, d_z), so such a pair amplifies every rounding on the way to it by
+// r / |(d_y, d_z)|.  It takes the reference's orientation (lower index first)
+// and Gram-Schmidt sequence and the index-order displacement, so that its
+// result depends neither on the spatial sort nor on the walk that met it.
+// Both atoms' forces and torques, and the energy (word 6 n_pad), go into the
+// accumulator.
+__global__ void k_axis_pairs(PairParams P, IndexRecords R, AxisList axis, const int* __restrict__ order,
+                             const double* __restrict__ pos, FixAcc fix, int n_pad) {
+    const int count = min(*axis.count, axis.cap);
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
+        const int2 ij = axis.pairs[q];
+        const int id_i = order[ij.x], id_j = order[ij.y];
+        const int lo = id_i < id_j ? ij.x : ij.y, hi = id_i < id_j ? ij.y : ij.x;
+        float dx, dy, dz;
+        index_delta(P, R, pos, lo, hi, min(id_i, id_j), max(id_i, id_j), dx, dy, dz);
+        const float4 pl = R.posq_s[lo], dl = R.dipt_s[lo], ul = R.ind_s[lo];
+        const float4 ph = R.posq_s[hi], dh = R.dipt_s[hi], uh = R.ind_s[hi];
+        const f2 DX = bc2(dx), DY = bc2(dy), DZ = bc2(dz), R2 = dot2(DX, DY, DZ, DX, DY, DZ);
+        float r2, t;
+        un2(R2, r2, t);
+        const f2 RINV = bc2(rsqrtf(r2));
+        const f2 ZX = mul2(DX, RINV), ZY = mul2(DY, RINV), ZZ = mul2(DZ, RINV);
+        const bool yz = yz_differ_slot(dy, dz, pos, lo, hi);
+        f2 XX = add2(ZX, bc2(yz ? 1.0f : 0.0f)), XY = add2(ZY, bc2(yz ? 0.0f : 1.0f)), XZ = ZZ;
+        const f2 NDT = neg2(dot2(ZX, ZY, ZZ, XX, XY, XZ));
+        XX = fma2(ZX, NDT, XX);
+        XY = fma2(ZY, NDT, XY);
+        XZ = fma2(ZZ, NDT, XZ);
+        float xn;
+        un2(dot2(XX, XY, XZ, XX, XY, XZ), xn, t);
+        const f2 SN = bc2(xn > 0.0f ? rsqrtf(xn) : 1.0f);
+        XX = mul2(XX, SN);
+        XY = mul2(XY, SN);
+        XZ = mul2(XZ, SN);
+        const QiPair o =
+            qi_pair2(P, DX, DY, DZ, R2, RINV, r2, r2, XX, XY, XZ, bc2(pl.w), bc2(dl.x), bc2(dl.y), bc2(dl.z), bc2(ul.x),
+                     bc2(ul.y), bc2(ul.z), dl.w, 1.0f / dl.w, bc2(ph.w), bc2(dh.x), bc2(dh.y), bc2(dh.z), bc2(uh.x),
+                     bc2(uh.y), bc2(uh.z), dh.w, dh.w, 1.0f / dh.w, 1.0f / dh.w);
+        const f2 I[6] = {o.nfx, o.nfy, o.nfz, xneg2(o.tx), xneg2(o.ty), xneg2(o.tz)};
+        const f2 K[6] = {xneg2(o.nfx), xneg2(o.nfy), xneg2(o.nfz), xneg2(o.ux), xneg2(o.uy), xneg2(o.uz)};
+        for (int c = 0; c < 6; c++) {
+            float v, w;
+            un2(I[c], v, t);
+            un2(K[c], w, t);
+            fix_add(fix, (size_t)c * n_pad + lo, v);
+            fix_add(fix, (size_t)c * n_pad + hi, w);
+        }
+        float e;
+        un2(o.e2, e, t);
+        fix_add(fix, 6 * (size_t)n_pad, 0.5f * e);
+    }
+}
+
+// f: I side (force; sum of V, or the torque in MODE 2), g: the same for J atom
+// ((lane + s1) & 15) | (lane & 16).
+// OPEN: the charge-charge energy in FP64 (xi: the I atom's position, XJ: the J
+// atoms'), from the FP32 1/r by one Newton step.  The energy of an open system
+// is the small remainder of charge sums that grow with n^2 (20 e^2/nm of
+// 1.6e6 at 3,993 atoms): in FP32 the roundings of 1/r and of the sum left
+// 1e-6 to 5e-6 of it.
+template <int MODE, bool FOLD, bool MASK, bool OPEN>
+__device__ __forceinline__ void energy_item_walk(const PairParams& P, const double* __restrict__ pos,
+                                                 const IndexRecords& R, const AxisList& axis, const EItemTile& T, int lane, int i, int id, int jbase, float oix,
+                                                 float oiy, float oiz, float4 pi, float4 di, float4 ui, unsigned mk,
+                                                 unsigned fm, float damp_r2, int s0, int s1, float (&f)[6],
+                                                 float (&g)[6], float& en, d3 xi, const EItemPos* XJ, double& en64) {
     const int nxt = (lane + 1) & 31;
-    const int nmax = P.n_tiles * 32 - 1;
     const f2 OX = bc2(oix), OY = bc2(oiy), OZ = bc2(oiz);
-    const float kap = mutual ? 1.0f : -1.0f;   // W = P + kap u
-    const f2 KAP = bc2(kap);
-    const f2 QI0 = bc2(pi.w), NQI0 = bc2(-pi.w);
-    const f2 MIX = bc2(di.x), MIY = bc2(di.y), MIZ = bc2(di.z);
+    const f2 QI = bc2(pi.w), HALF = bc2(0.5f), NTHREE = bc2(-3.0f), ONE = bc2(1.0f);
+    // MODE 0: P_i in place of m_i.
+    const f2 MIX = bc2(MODE == 0 ? di.x + ui.x : di.x), MIY = bc2(MODE == 0 ? di.y + ui.y : di.y),
+             MIZ = bc2(MODE == 0 ? di.z + ui.z : di.z);
     const f2 UIX = bc2(ui.x), UIY = bc2(ui.y), UIZ = bc2(ui.z);
-    const float pix = di.x + ui.x, piy = di.y + ui.y, piz = di.z + ui.z;
-    const f2 PIX = bc2(pix), PIY = bc2(piy), PIZ = bc2(piz);
-    const f2 HALF = bc2(0.5f), NTHREE = bc2(-3.0f), NTWO = bc2(-2.0f);
+    const float ti = di.w, iti = 1.0f / di.w;
+    const bool mutual = P.mutual != 0;
     f2 Lx = 0, Ly = 0, Lz = 0, Ix = 0, Iy = 0, Iz = 0, NTx = 0, NTy = 0, NTz = 0;
     if (FOLD) {
         Lx = bc2(-(float)P.box[0]);
@@ -1460,16 +1480,18 @@ __device__ __forceinline__ void energy_walk_x2_fast(const PairParams& P, const d
         NTy = bc2(-(float)(P.half_box_tol[1] * P.half_box_tol[1]));
         NTz = bc2(-(float)(P.half_box_tol[2] * P.half_box_tol[2]));
     }
-    // Torques from summed V (pair_energy_lab, VSUM): TX.. sum V_ij, UX.. V_ji.
     f2 FX = 0, FY = 0, FZ = 0, TX = 0, TY = 0, TZ = 0, EN = 0;        // I side
     f2 GX = 0, GY = 0, GZ = 0, UX = 0, UY = 0, UZ = 0;                // J side (packed atoms m, m + 16)
 #pragma unroll 1
-    for (int s = 0; s < 16; s++) {
+    for (int s = s0; s < s1; s++) {
         const int m = (lane + s) & 15;
         const float4 a = T.p0[m], b = T.p1[m], c = T.d0[m], d = T.d1[m], e = T.u0[m], h = T.u1[m];
+        const int2 jd = T.id[m];
         f2 DX = sub2(pk2(a.x, a.y), OX), DY = sub2(pk2(a.z, a.w), OY), DZ = sub2(pk2(b.x, b.y), OZ);
         const int ja = jbase + m, jb = ja + 16;
         if (FOLD) {
+            // As in xslot_pairs: one sign-bit AND of the d^2 - t^2 words flags
+            // the pairs within the margin of half a box.
             f2 neg = ~0ull;
             if (fm & 1u) {
                 DX = fold2(DX, Lx, Ix);
@@ -1485,19 +1507,18 @@ __device__ __forceinline__ void energy_walk_x2_fast(const PairParams& P, const d
             }
             const f2 flag = ~neg & 0x8000000080000000ull;
             if (flag) {
-                const bool amb_a = (flag >> 31) & 1ull, amb_b = (flag >> 63) != 0ull;
                 float ax, bx, ay, by, az, bz;
                 un2(DX, ax, bx);
                 un2(DY, ay, by);
                 un2(DZ, az, bz);
-                if (amb_a) {
-                    d3 q = exact_delta(P, pos, i, ja);
+                if (((flag >> 31) & 1ull) && i < P.n && ja < P.n) {
+                    const d3 q = exact_delta(P, pos, i, ja);
                     ax = (float)q.x;
                     ay = (float)q.y;
                     az = (float)q.z;
                 }
-                if (amb_b) {
-                    d3 q = exact_delta(P, pos, i, jb);
+                if ((flag >> 63) && i < P.n && jb < P.n) {
+                    const d3 q = exact_delta(P, pos, i, jb);
                     bx = (float)q.x;
                     by = (float)q.y;
                     bz = (float)q.z;
@@ -1507,70 +1528,158 @@ __device__ __forceinline__ void energy_walk_x2_fast(const PairParams& P, const d
                 DZ = pk2(az, bz);
             }
         }
-        float r2a, r2b, ra, rb;
-        un2(dot2(DX, DY, DZ, DX, DY, DZ), r2a, r2b);
-        const f2 RINV = pk2(rsqrtf(r2a), rsqrtf(r2b));
+        // Orientation: sign bits set where the I atom has the higher index.
+        const f2 SG = pk2(__int_as_float((jd.x - id) & 0x80000000), __int_as_float((jd.y - id) & 0x80000000));
+        const f2 QJS = pk2(b.z, b.w) ^ SG, QIS = QI ^ SG;
+        const f2 MJX = pk2(c.x, c.y), MJY = pk2(c.z, c.w), MJZ = pk2(d.x, d.y);
+        const f2 UJX = pk2(e.x, e.y), UJY = pk2(e.z, e.w), UJZ = pk2(h.x, h.y);
         const f2 RHO2 = fma2(DY, DY, mul2(DZ, DZ));
+        const f2 R2 = fma2(DX, DX, RHO2);
+        float r2a, r2b, ra, rb;
+        un2(R2, r2a, r2b);
         un2(RHO2, ra, rb);
-        // Frame X row (see above).
+        if (MASK) {
+            r2a = (mk >> m) & 1u ? r2a : INFINITY;
+            r2b = (mk >> (m + 16)) & 1u ? r2b : INFINITY;
+        }
+        f2 RINV = pk2(rsqrtf(r2a), rsqrtf(r2b));
+        // Frame X row.
         const f2 XS = mul2(RINV, pk2(rsqrtf(ra), rsqrtf(rb)));
         const f2 NDXS = mul2(xneg2(DX), XS);
         f2 XX = mul2(RHO2, XS), XY = mul2(NDXS, DY), XZ = mul2(NDXS, DZ);
-        if (ra <= 1.0e-10f || rb <= 1.0e-10f) {
-            float dxa, dxb, dya, dyb, dza, dzb, rva, rvb, xxa, xxb, xya, xyb, xza, xzb;
-            un2(DX, dxa, dxb);
-            un2(DY, dya, dyb);
-            un2(DZ, dza, dzb);
-            un2(RINV, rva, rvb);
-            un2(XX, xxa, xxb);
-            un2(XY, xya, xyb);
-            un2(XZ, xza, xzb);
-            if (ra <= 1.0e-10f) qi_frame_x(dxa, dya, dza, rva, yz_differ<float>(dya, dza, yz, i, ja, nmax), xxa, xya, xza);
-            if (rb <= 1.0e-10f) qi_frame_x(dxb, dyb, dzb, rvb, yz_differ<float>(dyb, dzb, yz, i, jb, nmax), xxb, xyb, xzb);
-            XX = pk2(xxa, xxb);
-            XY = pk2(xya, xyb);
-            XZ = pk2(xza, xzb);
+        constexpr float kAxis2 = MODE == 0 ? kNearAxisFar2 : kNearAxis2;
+        if (ra <= kAxis2 || rb <= kAxis2) {
+            float xr[2], rv[2], xx[2], xy[2], xz[2], dx[2], dy[2], dz[2];
+            un2(DX, dx[0], dx[1]);
+            un2(DY, dy[0], dy[1]);
+            un2(DZ, dz[0], dz[1]);
+            un2(RINV, rv[0], rv[1]);
+            un2(XX, xx[0], xx[1]);
+            un2(XY, xy[0], xy[1]);
+            un2(XZ, xz[0], xz[1]);
+            xr[0] = ra;
+            xr[1] = rb;
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                if (xr[k] > kAxis2) continue;
+                const int j = k ? jb : ja;
+                float& r2 = k ? r2b : r2a;
+                if (MODE == 0) {
+                    index_delta(P, R, pos, i, j, id, k ? jd.y : jd.x, dx[k], dy[k], dz[k]);
+                    const float h2 = fmaf(dy[k], dy[k], dz[k] * dz[k]);
+                    rv[k] = rsqrtf(fmaf(dx[k], dx[k], h2));
+                    const float s = rv[k] * rsqrtf(h2);
+                    xx[k] = h2 * s;
+                    xy[k] = -dx[k] * s * dy[k];
+                    xz[k] = -dx[k] * s * dz[k];
+                    xr[k] = h2;
+                } else if (r2 < INFINITY && axis_push(axis, i, j)) {
+                    r2 = INFINITY;
+                    rv[k] = 0.0f;
+                }
+                if (xr[k] <= 1.0e-10f)
+                    qi_frame_x(dx[k], dy[k], dz[k], rv[k], yz_differ_slot(dy[k], dz[k], pos, i, j), xx[k], xy[k],
+                               xz[k]);
+            }
+            RINV = pk2(rv[0], rv[1]);
+            XX = pk2(xx[0], xx[1]);
+            XY = pk2(xy[0], xy[1]);
+            XZ = pk2(xz[0], xz[1]);
         }
-        const f2 QJ0 = pk2(b.z, b.w);
-        const f2 MJX = pk2(c.x, c.y), MJY = pk2(c.z, c.w), MJZ = pk2(d.x, d.y);
-        const f2 UJX = pk2(e.x, e.y), UJY = pk2(e.z, e.w), UJZ = pk2(h.x, h.y);
-        const f2 PJX = add2(MJX, UJX), PJY = add2(MJY, UJY), PJZ = add2(MJZ, UJZ);
-        const f2 PI0 = dot2(XX, XY, XZ, PIX, PIY, PIZ), UI0 = dot2(XX, XY, XZ, UIX, UIY, UIZ);
-        const f2 PJ0 = dot2(XX, XY, XZ, PJX, PJY, PJZ), UJ0 = dot2(XX, XY, XZ, UJX, UJY, UJZ);
-        const f2 rv2 = mul2(RINV, RINV), rv3 = mul2(rv2, RINV);
-        const f2 NR3X3 = mul2(NTHREE, rv3);
-        // Energy: the charge terms here; the dipole terms 0.5 (m_i.V_ij +
-        // m_j.V_ji) come from the V sums after the walk (pair_energy_lab, VSUM).
-        {
-            const f2 qq = mul2(QI0, QJ0);
-            const f2 cp = fma2(QJ0, PI0, mul2(NQI0, PJ0));
-            EN = fma2(RINV, qq, fma2(mul2(HALF, rv2), cp, EN));
-        }
-        const f2 rv2QJ0 = mul2(rv2, QJ0), rv2NQI0 = mul2(rv2, NQI0);
-        // S = K x X with K = a m_i + b m_j + c u_i + d u_j (pair_energy_lab):
-        // the torques need m_i x V_ij and m_j x V_ji, the force only K.
-        const f2 aJ = fma2(NR3X3, PJ0, rv2QJ0);
-        const f2 bI = fma2(NR3X3, PI0, rv2NQI0);
-        // V_ij (I torque) and V_ji (J torque), summed; the cross products with
-        // m_i and m_j come once per atom after the walk.
-        TX = fma2(aJ, XX, fma2(rv3, PJX, TX));
-        TY = fma2(aJ, XY, fma2(rv3, PJY, TY));
-        TZ = fma2(aJ, XZ, fma2(rv3, PJZ, TZ));
-        UX = fma2(bI, XX, fma2(rv3, PIX, UX));
-        UY = fma2(bI, XY, fma2(rv3, PIY, UY));
-        UZ = fma2(bI, XZ, fma2(rv3, PIZ, UZ));
-        {
-            const f2 cJ = fma2(NR3X3, fma2(KAP, UJ0, PJ0), rv2QJ0);
-            const f2 dI = fma2(NR3X3, fma2(KAP, UI0, PI0), rv2NQI0);
-            const f2 KX = fma2(aJ, MIX, fma2(bI, MJX, fma2(cJ, UIX, mul2(dI, UJX))));
-            const f2 KY = fma2(aJ, MIY, fma2(bI, MJY, fma2(cJ, UIY, mul2(dI, UJY))));
-            const f2 KZ = fma2(aJ, MIZ, fma2(bI, MJZ, fma2(cJ, UIZ, mul2(dI, UJZ))));
-            const f2 qf2 = fma2(mul2(NTWO, rv3), fma2(QI0, PJ0, xneg2(mul2(QJ0, PI0))), mul2(rv2QJ0, QI0));
-            // f = (S x X) / r + qf2 X = (rinv K.X + qf2) X - rinv K.
-            const f2 CF = fma2(RINV, dot2(KX, KY, KZ, XX, XY, XZ), qf2);
-            const f2 NRINV = xneg2(RINV);
-            const f2 FVX = fma2(CF, XX, mul2(NRINV, KX)), FVY = fma2(CF, XY, mul2(NRINV, KY)),
-                     FVZ = fma2(CF, XZ, mul2(NRINV, KZ));
+        if constexpr (MODE == 2) {
+            const QiPair o = qi_pair2(P, DX, DY, DZ, R2, RINV, r2a, r2b, XX, XY, XZ, QIS, MIX, MIY, MIZ, UIX, UIY, UIZ,
+                                      ti, iti, QJS, MJX, MJY, MJZ, UJX, UJY, UJZ, d.z, d.w, h.z, h.w);
+            const f2 SFX = o.nfx ^ SG, SFY = o.nfy ^ SG, SFZ = o.nfz ^ SG;
+            FX = add2(FX, SFX);
+            FY = add2(FY, SFY);
+            FZ = add2(FZ, SFZ);
+            GX = sub2(GX, SFX);
+            GY = sub2(GY, SFY);
+            GZ = sub2(GZ, SFZ);
+            TX = sub2(TX, o.tx);
+            TY = sub2(TY, o.ty);
+            TZ = sub2(TZ, o.tz);
+            UX = sub2(UX, o.ux);
+            UY = sub2(UY, o.uy);
+            UZ = sub2(UZ, o.uz);
+            EN = fma2(HALF, o.e2, EN);
+        } else {
+            const f2 MI0 = dot2(XX, XY, XZ, MIX, MIY, MIZ), UI0 = dot2(XX, XY, XZ, UIX, UIY, UIZ);
+            const f2 MJ0 = dot2(XX, XY, XZ, MJX, MJY, MJZ), UJ0 = dot2(XX, XY, XZ, UJX, UJY, UJZ);
+            const f2 rv2 = mul2(RINV, RINV), rv3 = mul2(rv2, RINV);
+            const f2 NR3 = mul2(NTHREE, rv3), R3T = add2(rv3, rv3);
+            const f2 qq = mul2(QIS, QJS);
+            const f2 RQJ = mul2(rv2, QJS), RQI = mul2(rv2, xneg2(QIS));
+            f2 KX, KY, KZ, QF, RAD;   // K, radial force term, 2 r^2 (E without q_i q_j/r and the V terms)
+            if constexpr (MODE == 0) {
+                RAD = fma2(QJS, MI0, mul2(xneg2(QIS), MJ0));
+                const f2 A = fma2(NR3, MJ0, RQJ), B = fma2(NR3, MI0, RQI);
+                TX = fma2(A, XX, fma2(rv3, MJX, TX));
+                TY = fma2(A, XY, fma2(rv3, MJY, TY));
+                TZ = fma2(A, XZ, fma2(rv3, MJZ, TZ));
+                UX = fma2(B, XX, fma2(rv3, MIX, UX));
+                UY = fma2(B, XY, fma2(rv3, MIY, UY));
+                UZ = fma2(B, XZ, fma2(rv3, MIZ, UZ));
+                const f2 NRK = mutual ? NR3 : xneg2(NR3);
+                const f2 CI = mul2(NRK, UJ0), CJ = mul2(NRK, UI0);
+                KX = fma2(A, MIX, fma2(B, MJX, fma2(CI, UIX, mul2(CJ, UJX))));
+                KY = fma2(A, MIY, fma2(B, MJY, fma2(CI, UIY, mul2(CJ, UJY))));
+                KZ = fma2(A, MIZ, fma2(B, MJZ, fma2(CI, UIZ, mul2(CJ, UJZ))));
+                QF = fma2(R3T, RAD, mul2(rv2, qq));
+            } else {
+                // Thole factors (1 beyond damp_r2 or where t_i t_j <= 1e-5, as the reference).
+                f2 TC = ONE, W = ONE, T0 = ONE;
+                if (r2a < damp_r2 || r2b < damp_r2) {
+                    const f2 U = mul2(mul2(mul2(R2, RINV), bc2(iti)), pk2(h.z, h.w));
+                    const f2 AU3 = mul2(pk2(fminf(ti, d.z), fminf(ti, d.w)), mul2(U, mul2(U, U)));
+                    float xa, xb;
+                    un2(AU3, xa, xb);
+                    const bool da = r2a < damp_r2 && fabsf(ti * d.z) > 1.0e-5f;
+                    const bool db = r2b < damp_r2 && fabsf(ti * d.w) > 1.0e-5f;
+                    const f2 NEX = pk2(da ? -__expf(-xa) : 0.0f, db ? -__expf(-xb) : 0.0f);
+                    const f2 X3 = pk2(da ? xa : 0.0f, db ? xb : 0.0f);   // no inf/NaN into the products
+                    TC = add2(ONE, NEX);
+                    W = fma2(NEX, add2(X3, ONE), ONE);
+                    T0 = fma2(NEX, fma2(bc2(1.5f), X3, ONE), ONE);
+                }
+                const f2 CM = fma2(QJS, MI0, mul2(xneg2(QIS), MJ0)), CU = fma2(QJS, UI0, mul2(xneg2(QIS), UJ0));
+                RAD = fma2(TC, CU, CM);
+                const f2 A = fma2(NR3, fma2(W, UJ0, MJ0), RQJ), B = fma2(NR3, fma2(W, UI0, MI0), RQI);
+                const f2 R3C = mul2(rv3, TC);
+                TX = fma2(A, XX, fma2(rv3, MJX, fma2(R3C, UJX, TX)));
+                TY = fma2(A, XY, fma2(rv3, MJY, fma2(R3C, UJY, TY)));
+                TZ = fma2(A, XZ, fma2(rv3, MJZ, fma2(R3C, UJZ, TZ)));
+                UX = fma2(B, XX, fma2(rv3, MIX, fma2(R3C, UIX, UX)));
+                UY = fma2(B, XY, fma2(rv3, MIY, fma2(R3C, UIY, UY)));
+                UZ = fma2(B, XZ, fma2(rv3, MIZ, fma2(R3C, UIZ, UZ)));
+                const f2 LAM = bc2(mutual ? 2.0f : 0.0f), NRW = mul2(NR3, W);
+                const f2 CI = fma2(NRW, fma2(LAM, UJ0, MJ0), mul2(TC, RQJ));
+                const f2 CJ = fma2(NRW, fma2(LAM, UI0, MI0), mul2(TC, RQI));
+                KX = fma2(A, MIX, fma2(B, MJX, fma2(CI, UIX, mul2(CJ, UJX))));
+                KY = fma2(A, MIY, fma2(B, MJY, fma2(CI, UIY, mul2(CJ, UJY))));
+                KZ = fma2(A, MIZ, fma2(B, MJZ, fma2(CI, UIZ, mul2(CJ, UJZ))));
+                QF = fma2(R3T, fma2(T0, CU, CM), mul2(rv2, qq));
+            }
+            if constexpr (OPEN) {
+                EN = fma2(mul2(HALF, rv2), RAD, EN);
+                float rva, rvb;
+                un2(RINV, rva, rvb);
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    const int jj = m + 16 * k;
+                    const double x = XJ->x[jj] - xi.x, y = XJ->y[jj] - xi.y, z = XJ->z[jj] - xi.z;
+                    const double r2 = x * x + y * y + z * z, y0 = (double)(k ? rvb : rva);
+                    const double r1 = y0 + (0.5 * y0) * (1.0 - (r2 * y0) * y0);
+                    en64 += ((double)pi.w * (double)(k ? b.w : b.z)) * r1;
+                }
+            } else {
+                EN = fma2(RINV, qq, fma2(mul2(HALF, rv2), RAD, EN));
+            }
+            // f = (rinv K.X + QF) X - rinv K, with the orientation's sign.
+            const f2 CF = fma2(RINV, dot2(KX, KY, KZ, XX, XY, XZ), QF) ^ SG;
+            const f2 NR = xneg2(RINV) ^ SG;
+            const f2 FVX = fma2(CF, XX, mul2(NR, KX)), FVY = fma2(CF, XY, mul2(NR, KY)),
+                     FVZ = fma2(CF, XZ, mul2(NR, KZ));
             FX = sub2(FX, FVY);
             FY = sub2(FY, FVZ);
             FZ = sub2(FZ, FVX);
@@ -1586,45 +1695,246 @@ __device__ __forceinline__ void energy_walk_x2_fast(const PairParams& P, const d
         UZ = __shfl_sync(kFull, UZ, nxt);
     }
     float lo, hi;
-    const f2* Is[4] = {&FX, &FY, &FZ, &EN};
-    float* Io[4] = {&f[0], &f[1], &f[2], &en};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        un2(*Is[k], lo, hi);
-        *Io[k] += lo + hi;
-    }
-    float v[3];
-    const f2 Vs[3] = {TX, TY, TZ};
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        un2(Vs[k], lo, hi);
-        v[k] = lo + hi;
-    }
-    // tau_I = -perm(m_i x sum V_ij); dipole energy 0.5 m_i.sum V_ij.
-    en += 0.5f * (di.x * v[0] + di.y * v[1] + di.z * v[2]);
-    f[3] -= di.z * v[0] - di.x * v[2];
-    f[4] -= di.x * v[1] - di.y * v[0];
-    f[5] -= di.y * v[2] - di.z * v[1];
-    const f2 Js[6] = {GX, GY, GZ, UX, UY, UZ};
-    float w[6];
+    const f2 Is[6] = {FX, FY, FZ, TX, TY, TZ}, Js[6] = {GX, GY, GZ, UX, UY, UZ};
 #pragma unroll
     for (int k = 0; k < 6; k++) {
+        un2(Is[k], lo, hi);
+        f[k] = lo + hi;
+        // Lanes l and l ^ 16 hold the two copies of atoms (m, m + 16).
         un2(Js[k], lo, hi);
         const float olo = __shfl_xor_sync(kFull, lo, 16), ohi = __shfl_xor_sync(kFull, hi, 16);
-        w[k] = lane < 16 ? lo + olo : hi + ohi;
+        g[k] = lane < 16 ? lo + olo : hi + ohi;
     }
-    gg[0] += w[0];
-    gg[1] += w[1];
-    gg[2] += w[2];
-    // Lane l now holds J atom l: tau_J = -perm(m_j x sum V_ji).
-    const int m = lane & 15, h = lane >> 4;
-    const float mjx = reinterpret_cast<const float*>(&T.d0[m])[h];
-    const float mjy = reinterpret_cast<const float*>(&T.d0[m])[2 + h];
-    const float mjz = reinterpret_cast<const float*>(&T.d1[m])[h];
-    gg[3] -= mjz * w[3] - mjx * w[5];
-    gg[4] -= mjx * w[4] - mjy * w[3];
-    gg[5] -= mjy * w[5] - mjz * w[4];
-    en += 0.5f * (mjx * w[3] + mjy * w[4] + mjz * w[5]);
+    un2(EN, lo, hi);
+    en = lo + hi;
+}
+
+// Sum of V -> torque -perm(m x V) and the dipole energy 0.5 m.V (MODE 0, 1).
+__device__ __forceinline__ float torque_of_v(float4 m, float (&f)[6]) {
+    const float vx = f[3], vy = f[4], vz = f[5];
+    f[3] = -(m.z * vx - m.x * vz);
+    f[4] = -(m.x * vy - m.y * vx);
+    f[5] = -(m.y * vz - m.z * vy);
+    return 0.5f * (m.x * vx + m.y * vy + m.z * vz);
+}
+
+__device__ __forceinline__ void copy16_async(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+// The J records of an item's next tile, fetched while the current one is walked.
+struct EItemRaw {
+    float4 p[32], d[32], u[32];
+};
+
+// Mixed-form energy kernel: warp items as in k_field_items, one I tile against
+// J tiles [c L, c L + L), in the spatial order of the field kernels (compact
+// tiles: few tile pairs fold or reach the damping range, and the FP32 offsets
+// are short).  Pairs that do not count (self, padding, the second visit on a
+// diagonal tile, listed partners) are masked out; k_energy_items_done
+// evaluates the partners.  GENERAL: MODE 2 for every tile pair.  OPEN: no
+// box, the charge energy in FP64.
+//
+// Bound by the FP32 pipe (82 FMA-pipe f32x2 instructions a step of two pairs
+// in MODE 0, about 100 in MODE 1).  The band-pair kernel before it ran in
+// index order: its tiles were as long as the input's rows (3.3 nm on a
+// lattice), so most tile pairs folded, and those within the damping range
+// took the quasi-internal frame walk (about 230).  Before -> now (the done
+// kernels included): 31 -> 27 us at 648 atoms, 210 -> 83 at 3,993, 535 -> 409
+// at 12,288, 24,200 -> 20,300 at 98,304.
+template <bool GENERAL, bool OPEN>
+__global__ void __launch_bounds__(32, 12) k_energy_items(
+    PairParams P, int L, const float4* __restrict__ posq, const float4* __restrict__ dipt,
+    const float4* __restrict__ indv, const int* __restrict__ order, const double4* __restrict__ tctr,
+    const double4* __restrict__ text, const double* __restrict__ pos, const int* __restrict__ exc_off,
+    const int* __restrict__ exc_j, const double* __restrict__ exc_m, const double* __restrict__ exc_s,
+    const int2* __restrict__ exc_tiles, IndexRecords R, AxisList axis, int n_pad,
+    double* __restrict__ energy_partial, FixAcc fix) {
+    __shared__ EItemTile T;
+    __shared__ EItemRaw raw;
+    __shared__ EItemPos XJ[1];
+    __shared__ double s_my[6][32];
+    const int lane = threadIdx.x;
+    int p, q;
+    band_pair(blockIdx.x / L, p, q);
+    const int I = p * L + blockIdx.x % L, J0 = q * L, J1 = min(J0 + L, P.n_tiles);
+    const size_t item = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
+    int J = max(J0, I);
+    if (I >= P.n_tiles || J >= J1) {
+        if (lane == 0) energy_partial[item] = 0.0;
+        return;
+    }
+    const int s0 = 16 * blockIdx.y / gridDim.y, s1 = 16 * (blockIdx.y + 1) / gridDim.y;
+    const float damp_r2 = P.damp_r2;
+    const auto fetch = [&](int t) {
+        copy16_async(&raw.p[lane], posq + t * 32 + lane);
+        copy16_async(&raw.d[lane], dipt + t * 32 + lane);
+        copy16_async(&raw.u[lane], indv + t * 32 + lane);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(J);
+    const int i = I * 32 + lane;
+    const float4 pi = posq[i], di = dipt[i], ui = indv[i];
+    const int id = order[i];
+    d3 xi = {0.0, 0.0, 0.0};
+    if (OPEN) xi = ld3(pos + 3 * (size_t)i);
+    const int2 et = exc_tiles[I];
+    int e0 = 0, e1 = 0;
+    unsigned own = 0u;
+    if (i < P.n) {
+        own = ~0u;
+        e0 = exc_off[i];
+        e1 = exc_off[i + 1];
+    }
+    float gdx = 0.f, gdy = 0.f, gdz = 0.f;
+    unsigned gfl = 0u;
+    if (lane < L && J0 + lane < P.n_tiles) {
+        const TileGeom g = tile_geom(P, tctr[I], text[I], tctr[J0 + lane], text[J0 + lane]);
+        gdx = (float)g.dcx;
+        gdy = (float)g.dcy;
+        gdz = (float)g.dcz;
+        gfl = g.fmask | (g.fold ? 8u : 0u) | (g.near ? 16u : 0u);
+    }
+#pragma unroll
+    for (int k = 0; k < 6; k++) s_my[k][lane] = 0.0;
+    double energy = 0.0;
+    for (; J < J1; J++) {
+        const int jbase = J * 32, jid = order[jbase + lane];
+        const float dx = __shfl_sync(kFull, gdx, J - J0), dy = __shfl_sync(kFull, gdy, J - J0),
+                    dz = __shfl_sync(kFull, gdz, J - J0);
+        const unsigned fl = __shfl_sync(kFull, gfl, J - J0);
+        unsigned mk = own;
+        if (J == P.n_tiles - 1 && (P.n & 31)) mk &= (1u << (P.n & 31)) - 1u;
+        if (I == J) mk &= ~((2u << lane) - 1u);   // each pair of a diagonal tile once: j > i
+        if (J >= et.x && J <= et.y)
+            for (int e = e0; e < e1; e++) {
+                const unsigned off = (unsigned)(exc_j[e] - jbase);
+                if (off < 32u && (exc_m[e] != 1.0 || exc_s[e] != 1.0)) mk &= ~(1u << off);
+            }
+        const bool masked = __any_sync(kFull, mk != ~0u);
+        const bool plain = !GENERAL && !masked && !(fl & 16u);   // MODE 0
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+        {
+            const float4 pj = raw.p[lane], uj = raw.u[lane];
+            float4 dj = raw.d[lane];
+            if (plain) {
+                dj.x += uj.x;
+                dj.y += uj.y;
+                dj.z += uj.z;
+            }
+            stage_eitem(T, lane, pj, dj, uj, jid);
+            if (OPEN) {
+                const d3 x = ld3(pos + 3 * (size_t)(jbase + lane));
+                XJ->x[lane] = x.x;
+                XJ->y[lane] = x.y;
+                XJ->z[lane] = x.z;
+            }
+        }
+        __syncwarp();
+        if (J + 1 < J1) fetch(J + 1);
+        const float ox = pi.x - dx, oy = pi.y - dy, oz = pi.z - dz;
+        float f[6], g[6], en;
+#define TDP_EWALK(M, F, K) \
+    energy_item_walk<M, F, K, OPEN>(P, pos, R, axis, T, lane, i, id, jbase, ox, oy, oz, pi, di, ui, mk, fl, damp_r2, \
+                                    s0, s1, f, g, en, xi, XJ, energy)
+        if constexpr (GENERAL) {
+            TDP_EWALK(2, true, true);
+        } else if (plain) {
+            if (fl & 8u) TDP_EWALK(0, true, false);
+            else TDP_EWALK(0, false, false);
+        } else if (masked) {
+            TDP_EWALK(1, true, true);
+        } else if (fl & 8u) {
+            TDP_EWALK(1, true, false);
+        } else {
+            TDP_EWALK(1, false, false);
+        }
+#undef TDP_EWALK
+        const int jl = ((lane + s1) & 15) | (lane & 16);
+        if constexpr (!GENERAL) en += torque_of_v(di, f) + torque_of_v(dipt[jbase + jl], g);
+        energy += (double)en;
+#pragma unroll
+        for (int k = 0; k < 6; k++) {
+            fix_add(fix, (size_t)k * n_pad + jbase + jl, g[k]);
+            s_my[k][lane] += (double)f[k];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 6; k++) fix_add(fix, (size_t)k * n_pad + i, s_my[k][lane]);
+    energy = warp_sum(energy);
+    if (lane == 0) energy_partial[item] = energy;
+}
+
+// Fixed-point force and torque sums -> FP64 in index order, clearing them,
+// plus each slot's listed partners one-sided with their scales (FP64 pair
+// routine on the pair records; the pair's energy counts on its lower index),
+// and the block's share of the item energies, summed in order into
+// energy_block[blockIdx.x].
+__global__ void k_energy_items_done(PairParams P, const float4* __restrict__ posq, const float4* __restrict__ dipt,
+                                    const float4* __restrict__ indv, const int* __restrict__ order,
+                                    const double* __restrict__ pos, const int* __restrict__ exc_off,
+                                    const int* __restrict__ exc_j, const double* __restrict__ exc_m,
+                                    const double* __restrict__ exc_s, IndexRecords R, int* __restrict__ axis_count,
+                                    int n_pad, unsigned long long* __restrict__ acc, double inv_scale, int n_items, const double* __restrict__ energy_item,
+                                    double* __restrict__ fpair, double* __restrict__ torque,
+                                    double* __restrict__ energy_block) {
+    __shared__ double red[40];
+    const int per = (n_items + gridDim.x - 1) / gridDim.x;
+    const int a0 = min(n_items, blockIdx.x * per), a1 = min(n_items, a0 + per);
+    double energy = 0.0;
+    for (int a = a0 + threadIdx.x; a < a1; a += blockDim.x) energy += energy_item[a];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {   // the listed pairs' energy; the list is empty again
+        energy += (double)(long long)acc[6 * (size_t)n_pad] * inv_scale;
+        acc[6 * (size_t)n_pad] = 0ull;
+        *axis_count = 0;
+    }
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n_pad) {
+        double v[6];
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+            v[c] = (double)(long long)acc[(size_t)c * n_pad + k] * inv_scale;
+            acc[(size_t)c * n_pad + k] = 0ull;
+        }
+        if (k < P.n) {
+            const int id = order[k];
+            const double4 p = make_double4(0, 0, 0, posq[k].w);
+            const float4 df = dipt[k], uf = indv[k];
+            const EAtom<double> me = eatom<double>(p, make_double4(df.x, df.y, df.z, df.w),
+                                                   make_double4(uf.x, uf.y, uf.z, 0));
+            for (int e = exc_off[k]; e < exc_off[k + 1]; e++) {
+                const double mS = exc_m[e], iS = exc_s[e];
+                if ((mS == 0.0 && iS == 0.0) || (mS == 1.0 && iS == 1.0)) continue;
+                const int j = exc_j[e];
+                const float4 dj = dipt[j], uj = indv[j];
+                const EAtom<double> other = eatom<double>(make_double4(0, 0, 0, posq[j].w),
+                                                          make_double4(dj.x, dj.y, dj.z, dj.w),
+                                                          make_double4(uj.x, uj.y, uj.z, 0));
+                float dx, dy, dz;
+                index_delta(P, R, pos, k, j, id, order[j], dx, dy, dz);
+                const d3 d = {(double)dx, (double)dy, (double)dz};
+                const double r2 = dot(d, d);
+                const bool yzd = pos[3 * (size_t)k + 1] != pos[3 * (size_t)j + 1] ||
+                                 pos[3 * (size_t)k + 2] != pos[3 * (size_t)j + 2];
+                const double dr2 = (double)P.damp_r2, p4 = P.rinv4_power, f4 = P.rinv4_fill;
+                if (id < order[j])
+                    pair_energy<double, true>(d.x, d.y, d.z, r2, yzd, me, other, mS, iS, dr2, p4, f4, P.mutual != 0,
+                                              v[0], v[1], v[2], v[3], v[4], v[5], energy);
+                else
+                    pair_energy<double, false>(-d.x, -d.y, -d.z, r2, yzd, other, me, mS, iS, dr2, p4, f4,
+                                               P.mutual != 0, v[0], v[1], v[2], v[3], v[4], v[5], energy);
+            }
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                fpair[3 * (size_t)id + c] = v[c];
+                torque[3 * (size_t)id + c] = v[3 + c];
+            }
+        }
+    }
+    energy = block_sum(energy, red);
+    if (threadIdx.x == 0) energy_block[blockIdx.x] = energy;
 }
 
 // Partner pairs of a SLOW tile pair with their (M, I) scales, each side once:
@@ -1691,8 +2001,7 @@ __global__ void __launch_bounds__(kSymThreads, 3) k_energy_sym(
     const typename Vec4T<R>::type* __restrict__ indv, const double2* __restrict__ yz, const double4* __restrict__ tctr,
     const double4* __restrict__ text, const double* __restrict__ pos, const int* __restrict__ exc_off,
     const int* __restrict__ exc_j, const double* __restrict__ exc_m, const double* __restrict__ exc_s,
-    const int2* __restrict__ exc_tiles, int n_pad, double* __restrict__ partial, double* __restrict__ energy_partial,
-    FixAcc fix) {
+    const int2* __restrict__ exc_tiles, int n_pad, double* __restrict__ partial, double* __restrict__ energy_partial) {
     typedef typename Vec4T<R>::type V4;
     extern __shared__ __align__(16) unsigned char smem[];
     const int BT = P.band_tiles, NA = BT * 32;
@@ -1703,7 +2012,6 @@ __global__ void __launch_bounds__(kSymThreads, 3) k_energy_sym(
     V4* s_pos = reinterpret_cast<V4*>(s_ext + BT);
     V4* s_dip = s_pos + NA;
     V4* s_ind = s_dip + NA;
-    __shared__ EPackedTile s_ept[sizeof(R) == 4 ? kSymWarps : 1];   // packed walk's J tile (mixed form)
 
     int p, q;
     band_pair(blockIdx.x, p, q);
@@ -1750,19 +2058,6 @@ __global__ void __launch_bounds__(kSymThreads, 3) k_energy_sym(
             }
         }
         const EAtom<R> me = eatom<R>(pi, di, ui);
-        // FP32 form: the round's BT tile-pair geometries (FP64 arithmetic), one
-        // per lane, read by shuffles instead of every lane repeating each.
-        float gdx = 0.f, gdy = 0.f, gdz = 0.f;
-        unsigned gfl = 0u;
-        if constexpr (sizeof(R) == 4) {
-            if (wact && lane < BT) {
-                const TileGeom g0 = tile_geom(P, cA, eA, s_ctr[lane], s_ext[lane]);
-                gdx = (float)g0.dcx;
-                gdy = (float)g0.dcy;
-                gdz = (float)g0.dcz;
-                gfl = g0.fmask | (g0.fold ? 8u : 0u) | (g0.near ? 16u : 0u);
-            }
-        }
         for (int c = 0; c < 6; c++) my[c] = 0.0;
         for (int t = 0; t < BT; t++) {
             const int Jl = (t + warp * stride) % BT;
@@ -1771,56 +2066,16 @@ __global__ void __launch_bounds__(kSymThreads, 3) k_energy_sym(
                 const double4 cB = s_ctr[Jl];
                 const bool diag = I == J;
                 const bool slow = diag || (J == P.n_tiles - 1 && (P.n & 31)) || (J >= et.x && J <= et.y);
-                TileGeom g;
+                const TileGeom g = tile_geom(P, cA, eA, cB, s_ext[Jl]);
                 R oix, oiy, oiz;
-                if constexpr (sizeof(R) == 4) {
-                    const float dx = __shfl_sync(kFull, gdx, Jl), dy = __shfl_sync(kFull, gdy, Jl),
-                                dz = __shfl_sync(kFull, gdz, Jl);
-                    const unsigned fl = __shfl_sync(kFull, gfl, Jl);
-                    oix = pi.x - dx;
-                    oiy = pi.y - dy;
-                    oiz = pi.z - dz;
-                    if (slow) {
-                        g = tile_geom(P, cA, eA, cB, s_ext[Jl]);   // the partner walk's FP64 geometry
-                    } else {
-                        g.fmask = fl & 7u;
-                        g.fold = (fl >> 3) & 1u;
-                        g.near = (fl >> 4) & 1u;
-                    }
-                } else {
-                    g = tile_geom(P, cA, eA, cB, s_ext[Jl]);
-                    shift_into<R>(g, cA, cB, pi.x, pi.y, pi.z, oix, oiy, oiz);
-                }
+                shift_into<R>(g, cA, cB, pi.x, pi.y, pi.z, oix, oiy, oiz);
                 const int jbase = J * 32;
                 const V4* sp = s_pos + Jl * 32;
                 const V4* sd = s_dip + Jl * 32;
                 const V4* su = s_ind + Jl * 32;
                 const unsigned partners = slow ? partner_bits(exc_j, e0, e1, jbase) : 0u;
                 R f[6] = {0, 0, 0, 0, 0, 0}, gg[6] = {0, 0, 0, 0, 0, 0}, en = 0;
-                bool packed = false;
-                if constexpr (sizeof(R) == 4) {
-                    if (!slow) {
-                        packed = true;
-                        __syncwarp();
-                        stage_epacked(s_ept[warp], lane, sp[lane], sd[lane], su[lane]);
-                        __syncwarp();
-                        if (!g.near && P.lab_energy) {
-                            if (g.fold)
-                                energy_walk_x2_fast<true>(P, pos, yz, s_ept[warp], lane, i, jbase, oix, oiy, oiz, pi,
-                                                          di, ui, g.fmask, P.mutual != 0, f, gg, en);
-                            else
-                                energy_walk_x2_fast<false>(P, pos, yz, s_ept[warp], lane, i, jbase, oix, oiy, oiz, pi,
-                                                           di, ui, g.fmask, P.mutual != 0, f, gg, en);
-                        } else if (g.fold)
-                            energy_walk_x2<true>(P, pos, yz, s_ept[warp], lane, i, jbase, oix, oiy, oiz, pi, di, ui,
-                                                 g.fmask, damp_r2, rv4p, rv4f, P.mutual != 0, f, gg, en);
-                        else
-                            energy_walk_x2<false>(P, pos, yz, s_ept[warp], lane, i, jbase, oix, oiy, oiz, pi, di, ui,
-                                                  g.fmask, damp_r2, rv4p, rv4f, P.mutual != 0, f, gg, en);
-                    }
-                }
-                if (packed) {
-                } else if (slow) {
+                if (slow) {
                     if (g.fold) {
                         energy_walk<R, true, true>(P, pos, yz, sp, sd, su, lane, i, jbase, oix, oiy, oiz, me, diag,
                                                    partners, damp_r2, rv4p, rv4f, f, gg, en);
@@ -1865,8 +2120,6 @@ __global__ void __launch_bounds__(kSymThreads, 3) k_energy_sym(
             if (p == q) {
                 double* acc = s_acc + 6 * (Il * 32 + lane);
                 for (int c = 0; c < 6; c++) acc[c] += my[c];
-            } else if (sizeof(R) == 4) {
-                for (int c = 0; c < 6; c++) fix_add(fix, (size_t)c * n_pad + i, my[c]);
             } else {
                 const size_t b = (size_t)q * 6 * n_pad;
                 for (int c = 0; c < 6; c++) partial[b + (size_t)c * n_pad + i] = my[c];
@@ -1876,10 +2129,7 @@ __global__ void __launch_bounds__(kSymThreads, 3) k_energy_sym(
     }
     const size_t b = (size_t)p * 6 * n_pad;
     for (int k = threadIdx.x; k < NA; k += kSymThreads)
-        for (int c = 0; c < 6; c++) {
-            if (sizeof(R) == 4) fix_add(fix, (size_t)c * n_pad + qa0 + k, s_acc[6 * k + c]);
-            else partial[b + (size_t)c * n_pad + qa0 + k] = s_acc[6 * k + c];
-        }
+        for (int c = 0; c < 6; c++) partial[b + (size_t)c * n_pad + qa0 + k] = s_acc[6 * k + c];
     // CTA energy, summed in thread order (padding atoms contribute exactly 0).
     double e = warp_sum(my[6]);
     __shared__ double s_red[kSymWarps];
@@ -1908,23 +2158,7 @@ size_t energy_smem(int BT) {
 
 int band_pairs(const Dev& d) { return d.pp.n_bands * (d.pp.n_bands + 1) / 2; }
 
-// Fixed-point accumulator -> partial slot 0 (ncomp components of n_pad), clearing it.
-__global__ void k_fix_flush(size_t count, unsigned long long* __restrict__ acc, double inv_scale,
-                            double* __restrict__ out) {
-    size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= count) return;
-    long long v = (long long)acc[k];
-    acc[k] = 0ull;
-    out[k] = (double)v * inv_scale;
-}
-
 FixAcc fix_of(const Dev& d) { return FixAcc{d.fixacc, d.fix_err, d.fix_scale, d.fix_limit}; }
-
-void fix_flush(const Dev& d, int ncomp, cudaStream_t st) {
-    if (!d.fixacc) return;
-    const size_t count = (size_t)ncomp * d.n_pad;
-    k_fix_flush<<<(unsigned)((count + 255) / 256), 256, 0, st>>>(count, d.fixacc, 1.0 / d.fix_scale, d.partial);
-}
 
 // Plain form: the slots of every sum, in slot order, into slot 0, one thread
 // per sum.  The consumers used to add an atom's slots themselves, 3 x n_bands
@@ -1992,19 +2226,45 @@ void launch_field<double>(const Dev& d, int kind, cudaStream_t st) {
     slot_sum(d, 3, st);
 }
 
-template <class R>
-void launch_energy(const Dev& d, cudaStream_t st) {
-    typedef typename Vec4T<R>::type V4;
-    const size_t smem = energy_smem<R>(d.pp.band_tiles);
-    cudaFuncSetAttribute(k_energy_sym<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_energy_sym<R><<<band_pairs(d), kSymThreads, smem, st>>>(
-        d.pp, (const V4*)d.posq, (const V4*)d.dipt, (const V4*)d.ind, d.yz, d.tctr, d.text, d.pos, d.exc_off, d.exc_j,
-        d.exc_m, d.exc_s, d.exc_tiles, d.n_pad, d.partial, d.energy_partial, fix_of(d));
-    if (sizeof(R) == 4) fix_flush(d, 6, st);
-    else slot_sum(d, 6, st);
+template <>
+void launch_energy<float>(const Dev& d, cudaStream_t st) {
+    const int L = d.energy_L, nb = (d.pp.n_tiles + L - 1) / L;
+    const dim3 grid((unsigned)((long)nb * (nb + 1) / 2 * L), d.energy_parts);
+    const float4 *pq = (const float4*)d.posq_s, *dp = (const float4*)d.dipt_s, *u = (const float4*)d.vec_s;
+    FixAcc fix = fix_of(d);
+    fix.scale = d.fix_scale_energy;
+    const IndexRecords rec{(const float4*)d.posq, d.tctr, pq, dp, u};
+    const AxisList axis{d.axis_pairs, d.axis_count, d.axis_cap};
+    if (d.pp.lab_energy && !d.pp.periodic)
+        k_energy_items<false, true><<<grid, 32, 0, st>>>(d.pp, L, pq, dp, u, d.order, d.tctr_s, d.text_s, d.pos_s,
+                                                         d.exs_off, d.exs_j, d.exs_m, d.exs_s, d.exs_tiles, rec, axis,
+                                                         d.n_pad, d.energy_partial, fix);
+    else if (d.pp.lab_energy)
+        k_energy_items<false, false><<<grid, 32, 0, st>>>(d.pp, L, pq, dp, u, d.order, d.tctr_s, d.text_s, d.pos_s, d.exs_off,
+                                                   d.exs_j, d.exs_m, d.exs_s, d.exs_tiles, rec, axis, d.n_pad,
+                                                   d.energy_partial, fix);
+    else
+        k_energy_items<true, false><<<grid, 32, 0, st>>>(d.pp, L, pq, dp, u, d.order, d.tctr_s, d.text_s, d.pos_s, d.exs_off,
+                                                  d.exs_j, d.exs_m, d.exs_s, d.exs_tiles, rec, axis, d.n_pad,
+                                                  d.energy_partial, fix);
+    k_axis_pairs<<<148, 64, 0, st>>>(d.pp, rec, axis, d.order, d.pos_s, fix, d.n_pad);
+    k_energy_items_done<<<d.n_pad / 128, 128, 0, st>>>(d.pp, pq, dp, u, d.order, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
+                                                       d.exs_s, rec, d.axis_count, d.n_pad, d.fixacc,
+                                                       1.0 / fix.scale, d.n_eblk,
+                                                       d.energy_partial, d.fpair, d.torque,
+                                                       d.energy_partial + d.n_eblk);
+    launch_energy_total(d, d.n_pad / 128, d.energy_partial + d.n_eblk, st);
 }
 
-template void launch_energy<float>(const Dev&, cudaStream_t);
-template void launch_energy<double>(const Dev&, cudaStream_t);
+template <>
+void launch_energy<double>(const Dev& d, cudaStream_t st) {
+    const size_t smem = energy_smem<double>(d.pp.band_tiles);
+    cudaFuncSetAttribute(k_energy_sym<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_energy_sym<double><<<band_pairs(d), kSymThreads, smem, st>>>(
+        d.pp, (const double4*)d.posq, (const double4*)d.dipt, (const double4*)d.ind, d.yz, d.tctr, d.text, d.pos,
+        d.exc_off, d.exc_j, d.exc_m, d.exc_s, d.exc_tiles, d.n_pad, d.partial, d.energy_partial);
+    slot_sum(d, 6, st);
+    launch_energy_done(d, st);
+}
 
 }  // namespace tdp
