@@ -70,6 +70,12 @@ struct BatchArgs {
     const int2* users;  // (frame atom, role), global
     const double* coef; // extrapolation coefficients
     int* queue;
+    // Pair coefficients of the induced-induced tensor (rr3, rr5, I scale
+    // included), thread-private rows: CTA b's thread t keeps its step s at
+    // pair_coef[(b * coef_steps + s) * blockDim.x + t].  NULL: recomputed in
+    // every matvec.
+    double2* pair_coef;
+    int coef_steps;
     double* forces;     // n*3, written
     double* mu_out;     // n*3 induced dipoles
     double* energy;     // per cluster
@@ -115,6 +121,7 @@ struct Cl {
     int *eoff, *ej;
     R *em, *es;
     double *lab64, *q64, *th64;   // FP64 lab-frame dipoles (3 per atom), charges, Thole factors
+    double2* coef;   // this thread's pair coefficients, one row per step of blockDim.x (NULL: none)
     int M;
 };
 
@@ -155,7 +162,28 @@ __device__ Cl<R> carve(char* base, int M, int X, int korder) {
     c.lab64 = dd; dd += 3 * M;
     c.q64 = dd; dd += M;
     c.th64 = dd;
+    c.coef = nullptr;
     return c;
+}
+
+// The thread's rows of A.pair_coef.
+template <class R>
+__device__ __forceinline__ void use_coefs(Cl<R>& c, const BatchArgs& A) {
+    if (A.pair_coef) c.coef = A.pair_coef + (size_t)blockIdx.x * A.coef_steps * blockDim.x + threadIdx.x;
+}
+
+// A cluster of n atoms on a CTA of `threads`: the largest number of J atoms on
+// one thread over a whole pair pass (all rounds of split), as pairs of J atoms
+// (rows of a pass).
+__host__ __device__ inline int coef_rows(int n, int threads, int lmax) {
+    int rows = 0;
+    for (int base = 0; base < n; base += threads) {
+        const int na = n - base < threads ? n - base : threads;
+        const int T = threads < na * lmax ? threads : na * lmax;
+        const int L = T / na > 1 ? T / na : 1;
+        rows += (n + 2 * L - 1) / (2 * L);
+    }
+    return rows;
 }
 
 // Block sum in a fixed order (deterministic for a given CTA size).
@@ -305,17 +333,117 @@ __device__ __forceinline__ void matvec_lane_x2(const Cl<float>& c, int n, int i,
     fz += lo + hi;
 }
 
+// The lane's part of the matvec from the stored coefficients of its pairs
+// (store_coefs): J atoms ja = l + 2 L s and ja + L in step s, one 16-byte row
+// a step in the mixed form (rr3, rr3', rr5, rr5' as floats) and two in the
+// plain form.  A half without a pair holds zeros.  The coefficients do not
+// change through a solve: a step costs 14 operations a pair and a read of the
+// thread's own row from L2 in place of the distance, 1/r, the damping
+// exponential and the scale lookup (the solve of a 102-atom cluster, per SM:
+// 150 -> 67 us in the mixed form, now two CTAs an SM, 223 -> 103 us in the
+// plain one; 1024 clusters of 4-64 waters with the energy pass below 1.73 ->
+// 1.03 ms and 2.10 -> 1.25 ms).
+__device__ __forceinline__ void matvec_lane_coef(const Cl<float>& c, const double2*& row, int n, int i, int l, int L,
+                                                 float& fx, float& fy, float& fz) {
+    const float4 pi = c.posq[i];
+    const f2 OX = bc2(pi.x), OY = bc2(pi.y), OZ = bc2(pi.z);
+    f2 FX = 0, FY = 0, FZ = 0;
+#pragma unroll 2
+    for (int ja = l; ja < n; ja += 2 * L, row += blockDim.x) {
+        const int jb = min(ja + L, n - 1);
+        const float4 k = *reinterpret_cast<const float4*>(row);
+        const float4 pa = c.posq[ja], va = c.vec[ja], pb = c.posq[jb], vb = c.vec[jb];
+        const f2 DX = sub2(pk2(pa.x, pb.x), OX), DY = sub2(pk2(pa.y, pb.y), OY), DZ = sub2(pk2(pa.z, pb.z), OZ);
+        const f2 VX = pk2(va.x, vb.x), VY = pk2(va.y, vb.y), VZ = pk2(va.z, vb.z);
+        const f2 DD = mul2(pk2(k.z, k.w), fma2(VX, DX, fma2(VY, DY, mul2(VZ, DZ)))), NR3 = pk2(-k.x, -k.y);
+        FX = fma2(NR3, VX, fma2(DD, DX, FX));
+        FY = fma2(NR3, VY, fma2(DD, DY, FY));
+        FZ = fma2(NR3, VZ, fma2(DD, DZ, FZ));
+    }
+    float lo, hi;
+    un2(FX, lo, hi);
+    fx = lo + hi;
+    un2(FY, lo, hi);
+    fy = lo + hi;
+    un2(FZ, lo, hi);
+    fz = lo + hi;
+}
+__device__ __forceinline__ void matvec_lane_coef(const Cl<double>& c, const double2*& row, int n, int i, int l, int L,
+                                                 double& fx, double& fy, double& fz) {
+    const double4 pi = c.posq[i];
+    for (int ja = l; ja < n; ja += 2 * L, row += 2 * blockDim.x)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int j = min(ja + h * L, n - 1);
+            const double2 k = row[h * blockDim.x];
+            const double4 pj = c.posq[j], vj = c.vec[j];
+            const double dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
+            const double dd = k.y * (vj.x * dx + vj.y * dy + vj.z * dz);
+            fx += dd * dx - k.x * vj.x;
+            fy += dd * dy - k.x * vj.y;
+            fz += dd * dz - k.x * vj.z;
+        }
+}
+
+// The coefficients of the lane's pairs of atom i, from the form's pair records.
+template <class R>
+__device__ __forceinline__ void store_coefs(const Cl<R>& c, double2*& row, int n, int i, int l, int L, R damp_r2) {
+    const typename Vec4T<R>::type pi = c.posq[i];
+    const R ti = c.dipt[i].w;
+    for (int ja = l; ja < n; ja += 2 * L) {
+        R k3[2] = {0, 0}, k5[2] = {0, 0};
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int j = ja + h * L;
+            if (j >= n || j == i) continue;
+            R m, s;
+            pair_scales(c, i, j, m, s);
+            if (s == R(0)) continue;
+            const typename Vec4T<R>::type pj = c.posq[j];
+            const R dx = pj.x - pi.x, dy = pj.y - pi.y, dz = pj.z - pi.z;
+            const R r2 = dx * dx + dy * dy + dz * dz;
+            const R rinv = rsqrt_r(r2), rinv2 = rinv * rinv;
+            R rr3 = rinv * rinv2, rr5 = R(3) * rr3 * rinv2;
+            damp_field(r2, rinv, ti, c.dipt[j].w, damp_r2, rr3, rr5);
+            k3[h] = s * rr3;
+            k5[h] = s * rr5;
+        }
+        if constexpr (sizeof(R) == 4) {
+            *reinterpret_cast<float4*>(row) = make_float4(k3[0], k3[1], k5[0], k5[1]);
+            row += blockDim.x;
+        } else {
+            row[0] = make_double2(k3[0], k5[0]);
+            row[blockDim.x] = make_double2(k3[1], k5[1]);
+            row += 2 * blockDim.x;
+        }
+    }
+}
+
+// store_coefs over the cluster (each thread writes what it alone reads).
+template <class R>
+__device__ __forceinline__ void cluster_coefs(const Cl<R>& c, int n, int lmax, R damp_r2) {
+    if (!c.coef) return;
+    double2* row = c.coef;
+    for (int base = 0; base < n; base += blockDim.x) {
+        const Split sp = split(min(n - base, (int)blockDim.x), lmax);
+        if (sp.act) store_coefs(c, row, n, base + sp.a, sp.l, sp.L, damp_r2);
+    }
+}
+
 // out[i] = sum_j I_ij T_ij v_j with v in c.vec (the mutual field of the operand).
 // Ends with a CTA barrier: out is complete and visible on return.
 template <class R>
 __device__ void cluster_matvec(const Cl<R>& c, int n, int lmax, R damp_r2, double* out) {
     typedef typename Vec4T<R>::type V4;
+    const double2* row = c.coef;
     for (int base = 0; base < n; base += blockDim.x) {
         const int na = min(n - base, (int)blockDim.x);
         const Split sp = split(na, lmax);
         const int i = base + sp.a;
         R fx = 0, fy = 0, fz = 0;
-        if constexpr (sizeof(R) == 4) {
+        if (row) {
+            if (sp.act) matvec_lane_coef(c, row, n, i, sp.l, sp.L, fx, fy, fz);
+        } else if constexpr (sizeof(R) == 4) {
             if (sp.act) matvec_lane_x2(c, n, i, sp.l, sp.L, (float)damp_r2, fx, fy, fz);
         } else if (sp.act) {
             const V4 pi = c.posq[i];
@@ -567,6 +695,121 @@ __device__ __forceinline__ void cluster_field_any(const Cl<R>& c, const BatchArg
     else cluster_fixed_field(c, A, n, damp_r2);
 }
 
+// One ordered pair of the energy pass in the lab frame (FP64, unit scales, 1/r^4
+// terms zero): the expressions of the box path's energy items, damping
+// included, with the charges negated and the force's sign turned where the
+// atom has the higher index.  Adds atom i's force to f and V_ij to v, and
+// half of the pair's charge terms to en; the torque -perm(m_i x sum V) and the
+// dipole energy 0.5 m_i.sum V follow once per lane.  About 140 FP64 operations
+// where the quasi-internal frame routine takes 450 (the energy pass of a
+// 102-atom cluster 73 -> 36 us mixed, 58 -> 34 us plain).
+struct LabAtom {
+    double q, mx, my, mz, ux, uy, uz, t;
+};
+__device__ __forceinline__ void lab_pair_one_side(double dx, double dy, double dz, double r2, double rho2,
+                                                  const LabAtom& I, const LabAtom& J, double sg, double lam,
+                                                  double damp_r2, double f[3], double v[3], double& en) {
+    const double rinv = rsqrt(r2), xs = rinv * rsqrt(rho2), ndxs = -dx * xs;
+    const double xx = rho2 * xs, xy = ndxs * dy, xz = ndxs * dz;
+    const double qi = sg * I.q, qj = sg * J.q;
+    const double mi0 = xx * I.mx + xy * I.my + xz * I.mz, ui0 = xx * I.ux + xy * I.uy + xz * I.uz;
+    const double mj0 = xx * J.mx + xy * J.my + xz * J.mz, uj0 = xx * J.ux + xy * J.uy + xz * J.uz;
+    double tc = 1.0, w = 1.0, t0 = 1.0;
+    if (r2 < damp_r2) {
+        const double dmp = I.t * J.t;
+        if (fabs(dmp) > 1.0e-5) {
+            const double a = I.t < J.t ? I.t : J.t, u = r2 * rinv / dmp, x = a * u * u * u, e = exp(-x);
+            tc = 1.0 - e;
+            w = 1.0 - (1.0 + x) * e;
+            t0 = 1.0 - (1.0 + 1.5 * x) * e;
+        }
+    }
+    const double rv2 = rinv * rinv, rv3 = rv2 * rinv, nr3 = -3.0 * rv3, r3c = rv3 * tc;
+    const double rqj = rv2 * qj, rqi = -rv2 * qi, qq = qi * qj;
+    const double cm = qj * mi0 - qi * mj0, cu = qj * ui0 - qi * uj0;
+    en += 0.5 * (rinv * qq + 0.5 * rv2 * (cm + tc * cu));
+    const double A = rqj + nr3 * (mj0 + w * uj0), B = rqi + nr3 * (mi0 + w * ui0);
+    const double C = tc * rqj + nr3 * w * (mj0 + lam * uj0), D = tc * rqi + nr3 * w * (mi0 + lam * ui0);
+    v[0] += A * xx + rv3 * J.mx + r3c * J.ux;
+    v[1] += A * xy + rv3 * J.my + r3c * J.uy;
+    v[2] += A * xz + rv3 * J.mz + r3c * J.uz;
+    const double kx = A * I.mx + B * J.mx + C * I.ux + D * J.ux;
+    const double ky = A * I.my + B * J.my + C * I.uy + D * J.uy;
+    const double kz = A * I.mz + B * J.mz + C * I.uz + D * J.uz;
+    const double cf = rinv * (kx * xx + ky * xy + kz * xz) + rv2 * qq + 2.0 * rv3 * (cm + t0 * cu);
+    f[0] -= sg * (cf * xy - rinv * ky);
+    f[1] -= sg * (cf * xz - rinv * kz);
+    f[2] -= sg * (cf * xx - rinv * kx);
+}
+
+// The lane's part of atom i's energy, force and torque (f[0..2], f[3..5]) in
+// FP64: unit-scale pairs off the x axis in the lab frame, the others -- listed
+// partners (after the walk, so that they do not stall it), pairs on the axis,
+// and every pair with 1/r^4 terms -- by the reference's routine.
+template <class R>
+__device__ __forceinline__ void energy_lane64(const Cl<R>& c, const BatchArgs& A, int n, int i, int l, int L,
+                                              double f[6], double& en) {
+    const bool lab_ok = A.rinv4_power == 0.0 && A.rinv4_fill == 0.0, mutual = A.polarization == TDP_MUTUAL;
+    const LabAtom I{c.q64[i], c.lab64[3 * i], c.lab64[3 * i + 1], c.lab64[3 * i + 2],
+                    c.mu[3 * i], c.mu[3 * i + 1], c.mu[3 * i + 2], c.th64[i]};
+    const double pix = c.pos[3 * i], piy = c.pos[3 * i + 1], piz = c.pos[3 * i + 2];
+    const double lam = mutual ? 2.0 : 0.0;
+    const auto general = [&](int j, double m, double s) {
+        const double dx = c.pos[3 * j] - pix, dy = c.pos[3 * j + 1] - piy, dz = c.pos[3 * j + 2] - piz;
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        const bool yzd = piy != c.pos[3 * j + 1] || piz != c.pos[3 * j + 2];
+        const EAtom<double> me{I.q, I.mx, I.my, I.mz, I.ux, I.uy, I.uz, I.t};
+        const EAtom<double> other{c.q64[j], c.lab64[3 * j], c.lab64[3 * j + 1], c.lab64[3 * j + 2],
+                                  c.mu[3 * j], c.mu[3 * j + 1], c.mu[3 * j + 2], c.th64[j]};
+        if (i < j)
+            pair_energy<double, true>(dx, dy, dz, r2, yzd, me, other, m, s, A.damp_r2, A.rinv4_power, A.rinv4_fill,
+                                      mutual, f[0], f[1], f[2], f[3], f[4], f[5], en);
+        else
+            pair_energy<double, false>(-dx, -dy, -dz, r2, yzd, other, me, m, s, A.damp_r2, A.rinv4_power,
+                                       A.rinv4_fill, mutual, f[0], f[1], f[2], f[3], f[4], f[5], en);
+    };
+    const unsigned long long mask = c.emask[i];
+    double v[3] = {0.0, 0.0, 0.0};
+    bool aside = false;
+    for (int j = l; j < n; j += L) {
+        if (j == i) continue;
+        const unsigned o = (unsigned)(j - i + 32);
+        if (o < 63u ? (mask >> o) & 1ull : mask >> 63) {
+            // On (or perhaps on) the exception list.
+            R m, s;
+            pair_scales(c, i, j, m, s);
+            if (m != R(1) || s != R(1)) continue;
+        }
+        const double dx = c.pos[3 * j] - pix, dy = c.pos[3 * j + 1] - piy, dz = c.pos[3 * j + 2] - piz;
+        const double rho2 = dy * dy + dz * dz;
+        if (!lab_ok || rho2 < 1.0e-12) {
+            aside = true;
+            continue;
+        }
+        const LabAtom J{c.q64[j], c.lab64[3 * j], c.lab64[3 * j + 1], c.lab64[3 * j + 2],
+                        c.mu[3 * j], c.mu[3 * j + 1], c.mu[3 * j + 2], c.th64[j]};
+        lab_pair_one_side(dx, dy, dz, dx * dx + rho2, rho2, I, J, i < j ? 1.0 : -1.0, lam, A.damp_r2, f, v, en);
+    }
+    en += 0.5 * (I.mx * v[0] + I.my * v[1] + I.mz * v[2]);
+    f[3] -= I.mz * v[0] - I.mx * v[2];
+    f[4] -= I.mx * v[1] - I.my * v[0];
+    f[5] -= I.my * v[2] - I.mz * v[1];
+    if (aside)
+        for (int j = l; j < n; j += L) {
+            if (j == i) continue;
+            const double dy = c.pos[3 * j + 1] - piy, dz = c.pos[3 * j + 2] - piz;
+            if (lab_ok && !(dy * dy + dz * dz < 1.0e-12)) continue;
+            R m, s;
+            pair_scales(c, i, j, m, s);
+            if (m != R(1) || s != R(1)) continue;
+            general(j, 1.0, 1.0);
+        }
+    for (int e = c.eoff[i] + l; e < c.eoff[i + 1]; e += L) {
+        const double m = (double)c.em[e], s = (double)c.es[e];
+        if ((m != 1.0 || s != 1.0) && (m != 0.0 || s != 0.0)) general(c.ej[e], m, s);
+    }
+}
+
 // Mutual polarization: CG in y = mu / sqrt(alpha) on (I - S T S) y = S E from
 // mu = alpha E (c.mu), stopping on the RMS Jacobi-step change (true residual
 // confirmed) at target or after cap iterations; leaves mu in c.mu.
@@ -639,7 +882,8 @@ template <class R>
 __global__ void __launch_bounds__(512) k_batch(BatchArgs A) {
     typedef typename Vec4T<R>::type V4;
     extern __shared__ __align__(32) char smem_raw[];
-    const Cl<R> c = carve<R>(smem_raw, A.max_atoms, A.max_exc, A.korder);
+    Cl<R> c = carve<R>(smem_raw, A.max_atoms, A.max_exc, A.korder);
+    use_coefs(c, A);
     __shared__ int s_slot;
     const R damp_r2 = (R)A.damp_r2;
     const R rv4p = (R)A.rinv4_power, rv4f = (R)A.rinv4_fill;
@@ -662,6 +906,7 @@ __global__ void __launch_bounds__(512) k_batch(BatchArgs A) {
         cluster_load(c, A, a0, n);
         cluster_lab(c, A, a0, n);
         cluster_field_any(c, A, n, damp_r2);
+        if (A.polarization != TDP_DIRECT) cluster_coefs(c, n, A.lmax, damp_r2);
 
         // ---- induced dipoles ---------------------------------------------------------------
         int it = 0;
@@ -714,59 +959,15 @@ __global__ void __launch_bounds__(512) k_batch(BatchArgs A) {
         double* frc = c.w;
         double* trq = c.w + 3 * c.M;
         double en = 0.0;
-        const bool e64 = sizeof(R) == 4 && A.fp64_passes;
-        const bool lab_ok = A.rinv4_power == 0.0 && A.rinv4_fill == 0.0;
+        const bool e64 = sizeof(R) == 8 || A.fp64_passes;
         for (int base = 0; base < n; base += blockDim.x) {
             const int na = min(n - base, (int)blockDim.x);
             const Split sp = split(na, A.lmax);
             const int i = base + sp.a;
             double f[6] = {0, 0, 0, 0, 0, 0};
             if (sp.act && e64) {
-                // FP64 pair arithmetic on the FP64 records; pairs beyond the
-                // damping range with unit scales take the lab-frame form.
-                const EAtom<double> me{c.q64[i], c.lab64[3 * i], c.lab64[3 * i + 1], c.lab64[3 * i + 2],
-                                       c.mu[3 * i], c.mu[3 * i + 1], c.mu[3 * i + 2], c.th64[i]};
-                const double pix = c.pos[3 * i], piy = c.pos[3 * i + 1], piz = c.pos[3 * i + 2];
-                const bool mutual = A.polarization == TDP_MUTUAL;
-                for (int j = sp.l; j < n; j += sp.L) {
-                    if (j == i) continue;
-                    R mr, sr;
-                    pair_scales(c, i, j, mr, sr);
-                    const double m = mr, s = sr;
-                    if (m == 0.0 && s == 0.0) continue;
-                    const EAtom<double> other{c.q64[j], c.lab64[3 * j], c.lab64[3 * j + 1], c.lab64[3 * j + 2],
-                                              c.mu[3 * j], c.mu[3 * j + 1], c.mu[3 * j + 2], c.th64[j]};
-                    const double dx = c.pos[3 * j] - pix, dy = c.pos[3 * j + 1] - piy, dz = c.pos[3 * j + 2] - piz;
-                    const double r2 = dx * dx + dy * dy + dz * dz;
-                    bool yzd = fabs(dy) > 1e-5 || fabs(dz) > 1e-5;
-                    if (!yzd) yzd = (piy != c.pos[3 * j + 1]) || (piz != c.pos[3 * j + 2]);
-                    double fx = 0, fy = 0, fz = 0, tx = 0, ty = 0, tz = 0, e = 0;
-                    if (lab_ok && m == 1.0 && s == 1.0 && !(r2 < A.damp_r2)) {
-                        double gx = 0, gy = 0, gz = 0, ux = 0, uy = 0, uz = 0;
-                        const double kap = mutual ? 1.0 : -1.0;
-                        if (i < j)
-                            pair_energy_lab<double>(dx, dy, dz, r2, yzd, me, other, kap, fx, fy, fz, tx, ty, tz, gx, gy,
-                                                    gz, ux, uy, uz, e);
-                        else
-                            pair_energy_lab<double>(-dx, -dy, -dz, r2, yzd, other, me, kap, gx, gy, gz, ux, uy, uz, fx,
-                                                    fy, fz, tx, ty, tz, e);
-                        if (i > j) e = 0.0;
-                    } else if (i < j) {
-                        pair_energy<double, true>(dx, dy, dz, r2, yzd, me, other, m, s, A.damp_r2, A.rinv4_power,
-                                                  A.rinv4_fill, mutual, fx, fy, fz, tx, ty, tz, e);
-                    } else {
-                        pair_energy<double, false>(-dx, -dy, -dz, r2, yzd, other, me, m, s, A.damp_r2, A.rinv4_power,
-                                                   A.rinv4_fill, mutual, fx, fy, fz, tx, ty, tz, e);
-                    }
-                    f[0] += fx;
-                    f[1] += fy;
-                    f[2] += fz;
-                    f[3] += tx;
-                    f[4] += ty;
-                    f[5] += tz;
-                    en += e;
-                }
-            } else if (sp.act) {
+                energy_lane64(c, A, n, i, sp.l, sp.L, f, en);
+            } else if (sizeof(R) == 4 && sp.act) {
                 const V4 pi = c.posq[i], di = c.dipt[i], ui = c.vec[i];
                 const EAtom<R> me{pi.w, di.x, di.y, di.z, ui.x, ui.y, ui.z, di.w};
                 const double yi = c.pos[3 * i + 1], zi = c.pos[3 * i + 2];
@@ -897,7 +1098,8 @@ __device__ __forceinline__ void cluster_apply_t(const Cl<R>& c, int n, int lmax,
 template <class R>
 __global__ void __launch_bounds__(512) k_batch_adjoint(BatchArgs A, AdjArgs G) {
     extern __shared__ __align__(32) char smem_raw[];
-    const Cl<R> c = carve<R>(smem_raw, A.max_atoms, A.max_exc, A.korder);
+    Cl<R> c = carve<R>(smem_raw, A.max_atoms, A.max_exc, A.korder);
+    use_coefs(c, A);
     const AdjCl g = carve_adj<R>(smem_raw, A.max_atoms, A.max_exc, A.korder);
     __shared__ int s_slot;
     const R damp_r2 = (R)A.damp_r2;
@@ -942,6 +1144,7 @@ __global__ void __launch_bounds__(512) k_batch_adjoint(BatchArgs A, AdjArgs G) {
         const double gE = G.gE ? G.gE[cid] : 0.0;
         // Permanent field of the forward into c.E (also sets c.mu = alpha E).
         cluster_field_any(c, A, n, damp_r2);
+        if (A.polarization == TDP_MUTUAL) cluster_coefs(c, n, A.lmax, damp_r2);
         for (int k = threadIdx.x; k < 3 * n; k += blockDim.x) g.etm[k] = c.E[k];
 
         // ---- g_tau = M^T g (k_torque_vjp) -------------------------------------------------
@@ -1110,6 +1313,10 @@ struct tdp_batch {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double last_ms = 0.0;
     bool have_results = false;
+    // Workspace of the stored pair coefficients, for the largest tile shape
+    // that stays within kCoefLimit (larger ones recompute them).
+    double2* coef_space = nullptr;
+    size_t coef_capacity = 0;
     // Reverse pass (allocated on the first tdp_batch_adjoint).
     AdjArgs adj{};
     int adj_ctas = 0;
@@ -1126,6 +1333,9 @@ struct TileShape {
 const TileShape kShapes[] = {{64, 4},  {64, 16},  {128, 4},  {128, 8},  {128, 16}, {128, 32},
                              {256, 4}, {256, 8},  {256, 16}, {256, 32}, {512, 8},  {512, 32}};
 constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
+// Every resident CTA's coefficients should stay in the 126 MB L2 with what
+// else the launch reads; at 192 atoms they take 45 MB (mixed) or 90 MB.
+constexpr size_t kCoefLimit = (size_t)112 << 20;
 
 int batch_fail(tdp_batch* b, const TdpError& e) {
     if (b) b->err = e.msg;
@@ -1155,9 +1365,25 @@ int grid_for(tdp_batch* b, int threads) {
     return std::max(1, std::min(b->nc, per_sm * b->num_sms));
 }
 
+// Rows (16 bytes a thread) of the stored pair coefficients of the largest cluster.
+int coef_steps(const tdp_batch* b, int threads, int lmax) {
+    return coef_rows(b->max_atoms, threads, lmax) * (b->precision == TDP_PRECISION_DOUBLE ? 2 : 1);
+}
+size_t coef_bytes(const tdp_batch* b, int threads, int lmax, int ctas) {
+    return sizeof(double2) * (size_t)coef_steps(b, threads, lmax) * threads * ctas;
+}
+
+// A launch's coefficient rows, where the workspace holds them.
+void set_coefs(const tdp_batch* b, BatchArgs& a, int threads, int lmax, int ctas) {
+    const bool fits = coef_bytes(b, threads, lmax, ctas) <= b->coef_capacity;
+    a.pair_coef = fits ? b->coef_space : nullptr;
+    a.coef_steps = coef_steps(b, threads, lmax);
+}
+
 void launch(tdp_batch* b, int threads, int lmax, int ctas, cudaStream_t st) {
     BatchArgs a = b->args;
     a.lmax = lmax;
+    set_coefs(b, a, threads, lmax, ctas);
     size_t smem = smem_for(b);
     TDP_CUDA(cudaMemsetAsync(a.queue, 0, sizeof(int), st));
     if (b->precision == TDP_PRECISION_DOUBLE) k_batch<double><<<ctas, threads, smem, st>>>(a);
@@ -1209,6 +1435,17 @@ double time_launch(tdp_batch* b, int threads, int lmax, int ctas, int reps) {
 // pins the shape instead.
 void autotune(tdp_batch* b) {
     b->tune_ms.assign(kNumShapes, -1.0);
+    if (b->polarization != TDP_DIRECT && !b->coef_space) {
+        size_t most = 0;
+        for (const TileShape& s : kShapes) {
+            const size_t need = coef_bytes(b, s.threads, s.lmax, grid_for(b, s.threads));
+            if (need <= kCoefLimit) most = std::max(most, need);
+        }
+        if (most) {
+            b->coef_space = reinterpret_cast<double2*>(dalloc<char>(most, b->owned));
+            b->coef_capacity = most;
+        }
+    }
     int pin_t = 0, pin_l = 0;
     if (const char* env = getenv("TDP_BATCH_TILE")) sscanf(env, "%d,%d", &pin_t, &pin_l);
     double best = 1e300;
@@ -1587,6 +1824,7 @@ int tdp_batch_adjoint(tdp_batch* b, const double* dL_dF, const double* dL_dE, in
         TDP_CUDA(cudaMemsetAsync(g.queue, 0, sizeof(int), st));
         BatchArgs a = b->args;
         a.lmax = lmax;
+        set_coefs(b, a, threads, lmax, b->adj_ctas);
         if (b->precision == TDP_PRECISION_DOUBLE) k_batch_adjoint<double><<<b->adj_ctas, threads, smem, st>>>(a, args);
         else k_batch_adjoint<float><<<b->adj_ctas, threads, smem, st>>>(a, args);
         TDP_CUDA(cudaGetLastError());
