@@ -22,15 +22,10 @@
 // T (alpha gbar_(k+1)); then lambda = sum_k alpha gbar_k takes the place of
 // the adjoint solution in b, dL/dalpha = sum_k gbar_k . (E + T mu_(k-1)) and
 // c_t = sum_(k>=1) d/dt of (alpha gbar_k)^T T mu_(k-1).
-// For fixed geometry and damping the pair routine's energy, forces and
-// torques are bilinear in the two atoms' multipoles (every term is one
-// quantity of atom I times one of atom K), so the derivative with respect to
-// one atom's multipoles is the pair function evaluated with those multipoles
-// set to unit vectors; the Thole-factor derivative flows through the damping
-// factors and is taken with a one-direction dual number.  Damping terms are
-// recomputed in every pass rather than stored.  Pairs beyond the damping
-// range with unit scales (nearly all of a box) take the closed-form lab-frame
-// VJP (pair_vjp_lab), a few times cheaper.  Every pair is visited from both
+// The pair VJP is written out in closed form from the routine's lab-frame
+// form, damping and scales included (pair_vjp_me); pairs on the x axis and the
+// 1/r^4 option go through the routine itself (visit_pair_routine).  Damping
+// terms are recomputed in every pass rather than stored.  Every pair is visited from both
 // atoms (each atom owns kLanes threads), so no atomics are needed.
 #include "tholedipole_b200.h"
 #include <algorithm>
@@ -117,7 +112,7 @@ __global__ void __launch_bounds__(kVjpTile, 12) k_pair_vjp_fast(PairParams P, At
     const W u0 = {(T)A.mu[3 * mi], (T)A.mu[3 * mi + 1], (T)A.mu[3 * mi + 2]};
     const W g0 = {(T)g[3 * mi], (T)g[3 * mi + 1], (T)g[3 * mi + 2]};
     const W t0 = {(T)gT[3 * mi], (T)gT[3 * mi + 1], (T)gT[3 * mi + 2]};
-    const T kap = P.mutual ? T(1) : T(-1), tgE = (T)gE;
+    const T lam = P.mutual ? T(2) : T(0), tgE = (T)gE;
     const double damp_r2 = P.damp_r2 == 0.0f ? 0.0 : (double)P.damp_r2;
     double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     int ns = 0;
@@ -142,7 +137,7 @@ __global__ void __launch_bounds__(kVjpTile, 12) k_pair_vjp_fast(PairParams P, At
         __syncwarp();
         if (!act) continue;
         const int cnt = min(kVjpTile, P.n - base);
-        T part[7] = {0, 0, 0, 0, 0, 0, 0};
+        T part[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         for (int jj = 0; jj < cnt; jj++) {
             const int j = base + jj;
             if (j == me) continue;
@@ -154,14 +149,12 @@ __global__ void __launch_bounds__(kVjpTile, 12) k_pair_vjp_fast(PairParams P, At
             const bool yzd = (myz.x != yj.x) || (myz.y != yj.y);
             const double r2 = d.x * d.x + d.y * d.y + d.z * d.z;
             if (!(r2 < damp_r2) && yzd && d.y * d.y + d.z * d.z > 0.0) {
-                const W dj = {(T)d.x, (T)d.y, (T)d.z};
+                const T sg = meI ? T(1) : T(-1);
+                const W dj = {sg * (T)d.x, sg * (T)d.y, sg * (T)d.z};
                 const W mj = {s_v[0][jj], s_v[1][jj], s_v[2][jj]}, uj = {s_v[3][jj], s_v[4][jj], s_v[5][jj]};
                 const W gj = {s_v[6][jj], s_v[7][jj], s_v[8][jj]}, tj = {s_v[9][jj], s_v[10][jj], s_v[11][jj]};
-                const T qj = s_q[jj];
-                T o[7];
-                if (meI) pair_vjp_lab<T>(dj, q0, m0, u0, qj, mj, uj, kap, tgE, g0, gj, t0, tj, true, o);
-                else pair_vjp_lab<T>(dj, qj, mj, uj, q0, m0, u0, kap, tgE, gj, g0, tj, t0, false, o);
-                for (int a = 0; a < 7; a++) part[a] += o[a];
+                pair_vjp_me<T, false>(dj, sg, q0, m0, u0, T(0), s_q[jj], mj, uj, T(0), T(1), T(1), T(0), lam, tgE, g0,
+                                      gj, t0, tj, part);
             } else {
                 // The count goes on past the row (the list users then scan all
                 // partners of this atom).
