@@ -1157,8 +1157,7 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
                 throw TdpError{TDP_ERR_INVALID_ARGUMENT,
                                "Ewald mode: the Thole damping at the cutoff exceeds 1e-12 (cutoff too short for the "
                                "largest Thole factor)"};
-            // Real space in partial slot 0, reciprocal space + self in slot 1.
-            d.nslot = d.nsplit = 2;
+            d.nslot = d.nsplit = 1;
             d.n_eblk = 1;
         } else if (h->precision == TDP_PRECISION_MIXED && !variational) {
             // Mixed all-pairs form: the band sums go into the fixed-point

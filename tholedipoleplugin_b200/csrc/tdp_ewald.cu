@@ -65,6 +65,8 @@ struct EwParams {
     double rc2;             // cutoff^2
     double selfc;           // 4 alpha^3 / (3 sqrt(pi))
     int cap;                // neighbour-list row capacity
+    int split;              // warps (and partial-sum slots) per I tile
+    float damp_r2f;         // FP32 walks: squared distance beyond which damping is below rounding
 };
 
 struct PmeGrid {
@@ -347,24 +349,6 @@ __device__ __forceinline__ void stage_packed(EwPackedTile& T, int lane, float4 p
     reinterpret_cast<float*>(&T.it[m])[h] = 1.0f / v.w;
 }
 
-// Whether a J atom (record offsets p in J's frame) can lie within the cutoff
-// of any atom of the I tile, whose centre sits at -dc in J's frame with
-// half-extents e: the distance to the I tile's box, minimum image when the
-// tile pair folds, against the cutoff plus 1e-3 nm (no pair the walk would
-// count is dropped by FP32 rounding).
-__device__ __forceinline__ bool near_i_tile(const PairParams& P, float px, float py, float pz, const float* dc,
-                                            const float* e, float rcm2, bool fold) {
-    float a[3] = {px + dc[0], py + dc[1], pz + dc[2]};
-    float g2 = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        if (fold) a[k] = fold_f(a[k], (float)P.box[k], (float)P.inv_box[k]);
-        const float g = fmaxf(fabsf(a[k]) - e[k], 0.0f);
-        g2 += g * g;
-    }
-    return g2 < rcm2;
-}
-
 // Minimum-image displacement of J's tile centre from I's, FP32 (mixed form).
 __device__ __forceinline__ void tile_dc(const PairParams& P, double4 cA, double4 cB, float* dc) {
     dc[0] = (float)fold1(cB.x - cA.x, P.box[0], P.inv_box[0]);
@@ -372,10 +356,13 @@ __device__ __forceinline__ void tile_dc(const PairParams& P, double4 cA, double4
     dc[2] = (float)fold1(cB.z - cA.z, P.box[2], P.inv_box[2]);
 }
 
-template <int KIND, bool FOLD>
+// Steps [m0, m1) of the packed tile.  DAMP: some pair may lie within the
+// damping range; MASK: bits 2m and 2m + 1 of mk say whether the pairs count.
+template <int KIND, bool FOLD, bool DAMP, bool MASK>
 __device__ __forceinline__ void ew_field_walk_x2(const PairParams& P, const EwParams& E, const EwPackedTile& T,
                                                  float ox, float oy, float oz, float ti, float iti, float rc2,
-                                                 float damp_r2, int nsteps, float& fx, float& fy, float& fz) {
+                                                 unsigned mk, int m0, int m1, float& fx, float& fy, float& fz) {
+    const float damp_r2 = E.damp_r2f;
     const f2 OX = bc2(ox), OY = bc2(oy), OZ = bc2(oz);
     const f2 ALPHA = bc2((float)E.alpha), NA2 = bc2((float)(-E.alpha * E.alpha));
     const f2 CA = bc2((float)E.ca), A2 = bc2((float)E.a2), ONE = bc2(1.0f), THREE = bc2(3.0f), NEG = bc2(-1.0f);
@@ -392,7 +379,7 @@ __device__ __forceinline__ void ew_field_walk_x2(const PairParams& P, const EwPa
     const f2 MAGIC = bc2(12582912.0f), NMAGIC = bc2(-12582912.0f);
     f2 FX = 0, FY = 0, FZ = 0;
 #pragma unroll 2
-    for (int m = 0; m < nsteps; m++) {
+    for (int m = m0; m < m1; m++) {
         const float4 a = T.p0[m], b = T.p1[m], c = T.v0[m], d = T.v1[m];
         const float2 it = T.it[m];
         f2 DX = sub2(pk2(a.x, a.y), OX), DY = sub2(pk2(a.z, a.w), OY), DZ = sub2(pk2(b.x, b.y), OZ);
@@ -404,7 +391,11 @@ __device__ __forceinline__ void ew_field_walk_x2(const PairParams& P, const EwPa
         const f2 R2 = fma2(DX, DX, fma2(DY, DY, mul2(DZ, DZ)));
         float r2a, r2b;
         un2(R2, r2a, r2b);
-        const bool act_a = r2a < rc2, act_b = r2b < rc2;
+        bool act_a = r2a < rc2, act_b = r2b < rc2;
+        if (MASK) {
+            act_a = act_a && ((mk >> (2 * m)) & 1u);
+            act_b = act_b && ((mk >> (2 * m + 1)) & 1u);
+        }
         if (!__any_sync(kFull, act_a || act_b)) continue;
         r2a = act_a ? r2a : 1e30f;
         r2b = act_b ? r2b : 1e30f;
@@ -426,7 +417,7 @@ __device__ __forceinline__ void ew_field_walk_x2(const PairParams& P, const EwPa
         const f2 G1 = mul2(CA, EX);
         f2 B1 = mul2(add2(B0, G1), RINV2);
         f2 B2 = mul2(fma2(THREE, B1, mul2(G1, A2)), RINV2);
-        if (r2a < damp_r2 || r2b < damp_r2) {
+        if (DAMP && (r2a < damp_r2 || r2b < damp_r2)) {
             // -(1 - l3) b1 and -(1 - l5) b2 with u = r / (t_i t_j), a = min(t_i, t_j).
             const f2 U = mul2(mul2(R, ITI), pk2(it.x, it.y));
             const f2 AM = pk2(fminf(ti, d.z), fminf(ti, d.w));
@@ -471,111 +462,170 @@ __device__ __forceinline__ void ew_field_walk_x2(const PairParams& P, const EwPa
     fz += lo + hi;
 }
 
+// Compaction of the J atoms that can lie within the cutoff of the I tile's
+// box: those within the damping range of it first.  Returns the lane's place
+// (32: dropped), the two counts in nn (damping range) and nt (all).
+__device__ __forceinline__ int near_first(const PairParams& P, float px, float py, float pz, const float* dc,
+                                          const float* e, float rcm2, float dm2, bool fold, int lane, int& nn,
+                                          int& nt) {
+    float a[3] = {px + dc[0], py + dc[1], pz + dc[2]};
+    float g2 = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        if (fold) a[k] = fold_f(a[k], (float)P.box[k], (float)P.inv_box[k]);
+        const float g = fmaxf(fabsf(a[k]) - e[k], 0.0f);
+        g2 += g * g;
+    }
+    const unsigned in = __ballot_sync(kFull, g2 < rcm2), dn = __ballot_sync(kFull, g2 < rcm2 && g2 < dm2);
+    const unsigned below = (1u << lane) - 1u;
+    nn = __popc(dn);
+    nt = __popc(in);
+    if ((dn >> lane) & 1u) return __popc(dn & below);
+    if ((in >> lane) & 1u) return nn + __popc(in & ~dn & below);
+    return 32;
+}
+
+// Pairs of a SLOW tile pair that count, for the lane's I atom: bit s for J
+// atom jbase + s (not self, not padding, not a listed partner).
+__device__ __forceinline__ unsigned pair_mask(const PairParams& P, const int* __restrict__ exs_j, int e0, int e1,
+                                              int i, int jbase) {
+    if (i >= P.n) return 0u;
+    unsigned mk = ~partner_bits(exs_j, e0, e1, jbase);
+    if (P.n - jbase < 32) mk &= (1u << (P.n - jbase)) - 1u;
+    if ((unsigned)(i - jbase) < 32u) mk &= ~(1u << (i - jbase));
+    return mk;
+}
+
+// Real-space field: warp w of tile I (one-warp blocks, E.split of them a tile)
+// takes list entries w, w + split, ... and leaves its sums in slot w of the
+// real-space partials; ew_real_field adds the slots and the listed partners.
+// Few-tile systems split finely enough to fill the GPU, large ones end evenly
+// (four warps a block left 2.2 waves at 41,472 atoms).
 template <class R, int KIND>
-__global__ void __launch_bounds__(kEwThreads) k_ew_field(PairParams P, EwParams E,
-                                                         const typename Vec4T<R>::type* __restrict__ posq_s,
-                                                         const typename Vec4T<R>::type* __restrict__ src,
-                                                         const double4* __restrict__ tctr,
-                                                         const double4* __restrict__ text,
-                                                         const double* __restrict__ pos_s,
-                                                         const int* __restrict__ exs_off, const int* __restrict__ exs_j,
-                                                         const double* __restrict__ exs_m,
-                                                         const double* __restrict__ exs_s, const int* __restrict__ list,
-                                                         const int* __restrict__ count, int n_pad,
-                                                         double* __restrict__ out,
-                                                         const typename Vec4T<R>::type* __restrict__ lab) {
+__global__ void __launch_bounds__(32) k_ew_field(PairParams P, EwParams E,
+                                                 const typename Vec4T<R>::type* __restrict__ posq_s,
+                                                 const typename Vec4T<R>::type* __restrict__ src,
+                                                 const double4* __restrict__ tctr, const double4* __restrict__ text,
+                                                 const int* __restrict__ exs_off, const int* __restrict__ exs_j,
+                                                 const int* __restrict__ list, const int* __restrict__ count, int n_pad,
+                                                 double* __restrict__ out) {
     typedef typename Vec4T<R>::type V4;
-    __shared__ V4 s_pos[kEwWarps][32], s_vec[kEwWarps][32];
-    __shared__ EwPackedTile s_pk[sizeof(R) == 4 ? kEwWarps : 1];
-    __shared__ double s_red[kEwWarps][3][32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // One I tile per CTA; warp w takes list entries w, w + 4, ...; the four
-    // partial sums are added in warp order.
-    const int I = blockIdx.x;
+    __shared__ V4 s_pos[sizeof(R) == 8 ? 32 : 1], s_vec[sizeof(R) == 8 ? 32 : 1];
+    __shared__ EwPackedTile s_pk[1];
+    const int lane = threadIdx.x;
+    const int I = blockIdx.x / E.split, w = blockIdx.x % E.split;
     const int i = I * 32 + lane;
     const V4 pi = posq_s[i], vi = src[i];
     const double4 cA = tctr[I];
     const double4 eAd = text[I];
     const float eA[3] = {(float)eAd.x, (float)eAd.y, (float)eAd.z};
-    const float rcm = (float)sqrt(E.rc2) + 1e-3f;
+    const float rcm = (float)sqrt(E.rc2) + 1e-3f, dm = sqrtf(E.damp_r2f) + 1e-3f;
     const int e0 = i < P.n ? exs_off[i] : 0, e1 = i < P.n ? exs_off[i + 1] : 0;
     const R rc2 = (R)E.rc2, damp_r2 = (R)P.damp_r2;
     double fx = 0.0, fy = 0.0, fz = 0.0;
     const int cnt = count[I];
-    for (int t = warp; t < cnt; t += kEwWarps) {
+    for (int t = w; t < cnt; t += E.split) {
         const int ent = list[(size_t)I * E.cap + t];
-        const int J = ent & kTileMask;
+        const int J = ent & kTileMask, jbase = J * 32;
         const bool fold = (ent >> 30) & 1, slow = ((unsigned)ent >> 31) & 1u;
         const double4 cB = tctr[J];
-        __syncwarp();
-        const V4 pj = posq_s[J * 32 + lane], vj = src[J * 32 + lane];
-        int nsteps = 16;
-        bool staged = false;
-        if constexpr (sizeof(R) == 4) {
-            if (!slow) {
-                // Only the J atoms within the cutoff of the I tile's box,
-                // compacted; an odd count is padded with a multipole-free copy.
-                float dc[3];
-                tile_dc(P, cA, cB, dc);
-                const bool act = near_i_tile(P, (float)pj.x, (float)pj.y, (float)pj.z, dc, eA, rcm * rcm, fold);
-                const unsigned mk = __ballot_sync(kFull, act);
-                const int nact = __popc(mk), k = __popc(mk & ((1u << lane) - 1u));
-                if (act) stage_packed(s_pk[warp], k, pj, vj);
-                if ((nact & 1) && act && k == nact - 1)
-                    stage_packed(s_pk[warp], nact, make_float4(pj.x, pj.y, pj.z, 0.0f), make_float4(0.0f, 0.0f, 0.0f, vj.w));
-                nsteps = (nact + 1) >> 1;
-                staged = true;
-            }
-        }
-        if (!staged) {
-            s_pos[warp][lane] = pj;
-            s_vec[warp][lane] = vj;
-        }
-        __syncwarp();
+        const V4 pj = posq_s[jbase + lane], vj = src[jbase + lane];
         R ox, oy, oz;
         tile_shift<R>(P, cA, cB, pi.x, pi.y, pi.z, ox, oy, oz);
         R tx = 0, ty = 0, tz = 0;
+        __syncwarp();
         if constexpr (sizeof(R) == 4) {
-            if (!slow) {
-                const float iti = 1.0f / (float)vi.w;
-                if (fold) ew_field_walk_x2<KIND, true>(P, E, s_pk[warp], ox, oy, oz, vi.w, iti, rc2, damp_r2, nsteps, tx, ty, tz);
-                else ew_field_walk_x2<KIND, false>(P, E, s_pk[warp], ox, oy, oz, vi.w, iti, rc2, damp_r2, nsteps, tx, ty, tz);
-                fx += (double)tx;
-                fy += (double)ty;
-                fz += (double)tz;
-                continue;
+            const float iti = 1.0f / vi.w;
+            if (slow) {
+                stage_packed(s_pk[0], lane, pj, vj);
+                __syncwarp();
+                const unsigned mk = pair_mask(P, exs_j, e0, e1, i, jbase);
+                ew_field_walk_x2<KIND, true, true, true>(P, E, s_pk[0], ox, oy, oz, vi.w, iti, rc2, mk, 0, 16, tx, ty,
+                                                         tz);
+            } else {
+                float dc[3];
+                tile_dc(P, cA, cB, dc);
+                int nn, nt;
+                const int k = near_first(P, pj.x, pj.y, pj.z, dc, eA, rcm * rcm, dm * dm, fold, lane, nn, nt);
+                if (k < 32) stage_packed(s_pk[0], k, pj, vj);
+                // An odd count is padded with a multipole-free copy.
+                if ((nt & 1) && k == nt - 1)
+                    stage_packed(s_pk[0], nt, make_float4(pj.x, pj.y, pj.z, 0.0f),
+                                 make_float4(0.0f, 0.0f, 0.0f, vj.w));
+                __syncwarp();
+                const int mn = (nn + 1) >> 1, mt = (nt + 1) >> 1;
+                if (fold) {
+                    ew_field_walk_x2<KIND, true, true, false>(P, E, s_pk[0], ox, oy, oz, vi.w, iti, rc2, 0u, 0, mn, tx,
+                                                              ty, tz);
+                    ew_field_walk_x2<KIND, true, false, false>(P, E, s_pk[0], ox, oy, oz, vi.w, iti, rc2, 0u, mn, mt,
+                                                               tx, ty, tz);
+                } else {
+                    ew_field_walk_x2<KIND, false, true, false>(P, E, s_pk[0], ox, oy, oz, vi.w, iti, rc2, 0u, 0, mn,
+                                                               tx, ty, tz);
+                    ew_field_walk_x2<KIND, false, false, false>(P, E, s_pk[0], ox, oy, oz, vi.w, iti, rc2, 0u, mn, mt,
+                                                                tx, ty, tz);
+                }
             }
-        }
-        if (slow) {
-            const unsigned part = partner_bits(exs_j, e0, e1, J * 32);
-            if (fold) ew_field_walk<R, KIND, true, true>(P, E, s_pos[warp], s_vec[warp], i, J * 32, ox, oy, oz, vi.w, part, rc2, damp_r2, tx, ty, tz);
-            else ew_field_walk<R, KIND, false, true>(P, E, s_pos[warp], s_vec[warp], i, J * 32, ox, oy, oz, vi.w, part, rc2, damp_r2, tx, ty, tz);
-        } else if (fold) {
-            ew_field_walk<R, KIND, true, false>(P, E, s_pos[warp], s_vec[warp], i, J * 32, ox, oy, oz, vi.w, 0u, rc2, damp_r2, tx, ty, tz);
         } else {
-            ew_field_walk<R, KIND, false, false>(P, E, s_pos[warp], s_vec[warp], i, J * 32, ox, oy, oz, vi.w, 0u, rc2, damp_r2, tx, ty, tz);
+            s_pos[lane] = pj;
+            s_vec[lane] = vj;
+            __syncwarp();
+            if (slow) {
+                const unsigned part = partner_bits(exs_j, e0, e1, jbase);
+                if (fold) ew_field_walk<R, KIND, true, true>(P, E, s_pos, s_vec, i, jbase, ox, oy, oz, vi.w, part, rc2, damp_r2, tx, ty, tz);
+                else ew_field_walk<R, KIND, false, true>(P, E, s_pos, s_vec, i, jbase, ox, oy, oz, vi.w, part, rc2, damp_r2, tx, ty, tz);
+            } else if (fold) {
+                ew_field_walk<R, KIND, true, false>(P, E, s_pos, s_vec, i, jbase, ox, oy, oz, vi.w, 0u, rc2, damp_r2, tx, ty, tz);
+            } else {
+                ew_field_walk<R, KIND, false, false>(P, E, s_pos, s_vec, i, jbase, ox, oy, oz, vi.w, 0u, rc2, damp_r2, tx, ty, tz);
+            }
         }
         fx += (double)tx;
         fy += (double)ty;
         fz += (double)tz;
     }
-    s_red[warp][0][lane] = fx;
-    s_red[warp][1][lane] = fy;
-    s_red[warp][2][lane] = fz;
-    __syncthreads();
-    if (warp != 0) return;
-    for (int w = 1; w < kEwWarps; w++) {
-        fx += s_red[w][0][lane];
-        fy += s_red[w][1][lane];
-        fz += s_red[w][2][lane];
-    }
-    if (i < P.n)
-        ew_field_exceptions<R, KIND>(P, E, pos_s, posq_s, src, exs_off, exs_j, exs_m, exs_s, i, (double)vi.w, fx, fy,
-                                     fz, lab);
-    else fx = fy = fz = 0.0;
-    out[i] = fx;
-    out[(size_t)n_pad + i] = fy;
-    out[2 * (size_t)n_pad + i] = fz;
+    double* o = out + 3 * (size_t)w * n_pad;
+    const bool real = i < P.n;
+    o[i] = real ? fx : 0.0;
+    o[(size_t)n_pad + i] = real ? fy : 0.0;
+    o[2 * (size_t)n_pad + i] = real ? fz : 0.0;
+}
+
+// Listed partners and their scales, for the kernels that add up real space.
+struct EwExceptions {
+    const int *off, *j;
+    const double *m, *s;
+};
+
+// Real-space field of slot k: the split sums in order, then the partners.
+template <class R, int KIND>
+__device__ __forceinline__ d3 ew_real_field(const PairParams& P, const EwParams& E, const double* __restrict__ part,
+                                            int n_pad, const EwExceptions& X, const double* __restrict__ pos_s,
+                                            const typename Vec4T<R>::type* __restrict__ posq_s,
+                                            const typename Vec4T<R>::type* __restrict__ src,
+                                            const typename Vec4T<R>::type* __restrict__ lab, int k) {
+    double f[3] = {0.0, 0.0, 0.0};
+    for (int w = 0; w < E.split; w++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) f[c] += part[(3 * (size_t)w + c) * n_pad + k];
+    ew_field_exceptions<R, KIND>(P, E, pos_s, posq_s, src, X.off, X.j, X.m, X.s, k, (double)src[k].w, f[0], f[1], f[2],
+                                 lab);
+    return {f[0], f[1], f[2]};
+}
+
+// The variational NoCutoff model's field: real space alone.
+template <class R, int KIND>
+__global__ void k_ew_real_done(PairParams P, EwParams E, const double* __restrict__ part, int n_pad, EwExceptions X,
+                               const double* __restrict__ pos_s, const typename Vec4T<R>::type* __restrict__ posq_s,
+                               const typename Vec4T<R>::type* __restrict__ src,
+                               const typename Vec4T<R>::type* __restrict__ lab, double* __restrict__ out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n_pad) return;
+    const d3 f = k < P.n ? ew_real_field<R, KIND>(P, E, part, n_pad, X, pos_s, posq_s, src, lab, k)
+                         : d3{0.0, 0.0, 0.0};
+    out[k] = f.x;
+    out[(size_t)n_pad + k] = f.y;
+    out[2 * (size_t)n_pad + k] = f.z;
 }
 
 // ---------------------------------------------------------------------------
@@ -736,11 +786,12 @@ __device__ __forceinline__ void pair_ewald2(f2 DX, f2 DY, f2 DZ, f2 QI, f2 IX, f
     GZ = fma2(A, DZ, fma2(NK1, fma2(QJ, DZ, JZ), GZ));
 }
 
-template <bool FOLD>
+template <bool FOLD, bool DAMP, bool MASK>
 __device__ __forceinline__ void ew_force_walk_x2(const PairParams& P, const EwParams& E, const EwPackedForceTile& T,
                                                  float ox, float oy, float oz, float qi, float4 di, float4 ui,
-                                                 float iti, float rc2, float damp_r2, int nsteps, float& en, float* f,
-                                                 float* g) {
+                                                 float iti, float rc2, unsigned mk, int m0, int m1, float& en,
+                                                 float* f, float* g) {
+    const float damp_r2 = E.damp_r2f;
     const f2 OX = bc2(ox), OY = bc2(oy), OZ = bc2(oz);
     const f2 ALPHA = bc2((float)E.alpha), NA2 = bc2((float)(-E.alpha * E.alpha));
     const f2 CA = bc2((float)E.ca), A2 = bc2((float)E.a2), ONE = bc2(1.0f), THREE = bc2(3.0f),
@@ -760,7 +811,7 @@ __device__ __forceinline__ void ew_force_walk_x2(const PairParams& P, const EwPa
     const f2 MAGIC = bc2(12582912.0f), NMAGIC = bc2(-12582912.0f);
     f2 EN = 0, FX = 0, FY = 0, FZ = 0, GX = 0, GY = 0, GZ = 0;
 #pragma unroll 1
-    for (int m = 0; m < nsteps; m++) {
+    for (int m = m0; m < m1; m++) {
         const float4 a = T.p0[m], b = T.p1[m], c = T.d0[m], d = T.d1[m], u = T.u0[m], v = T.u1[m];
         const float2 it = T.it[m];
         f2 DX = sub2(pk2(a.x, a.y), OX), DY = sub2(pk2(a.z, a.w), OY), DZ = sub2(pk2(b.x, b.y), OZ);
@@ -772,7 +823,11 @@ __device__ __forceinline__ void ew_force_walk_x2(const PairParams& P, const EwPa
         const f2 R2 = fma2(DX, DX, fma2(DY, DY, mul2(DZ, DZ)));
         float r2a, r2b;
         un2(R2, r2a, r2b);
-        const bool act_a = r2a < rc2, act_b = r2b < rc2;
+        bool act_a = r2a < rc2, act_b = r2b < rc2;
+        if (MASK) {
+            act_a = act_a && ((mk >> (2 * m)) & 1u);
+            act_b = act_b && ((mk >> (2 * m + 1)) & 1u);
+        }
         if (!__any_sync(kFull, act_a || act_b)) continue;
         r2a = act_a ? r2a : 1e30f;
         r2b = act_b ? r2b : 1e30f;
@@ -798,7 +853,7 @@ __device__ __forceinline__ void ew_force_walk_x2(const PairParams& P, const EwPa
         G1 = mul2(G1, A2);
         const f2 B3 = mul2(fma2(FIVE, B2, G1), RINV2);
         f2 D1 = ZERO, D2 = ZERO, D3 = ZERO;
-        const bool damp = r2a < damp_r2 || r2b < damp_r2;
+        const bool damp = DAMP && (r2a < damp_r2 || r2b < damp_r2);
         if (damp) {
             const f2 U = mul2(mul2(R, ITI), pk2(it.x, it.y));
             const f2 AM = pk2(fminf(di.w, d.z), fminf(di.w, d.w));
@@ -851,92 +906,87 @@ __device__ __forceinline__ void ew_force_walk_x2(const PairParams& P, const EwPa
     g[2] += lo + hi;
 }
 
+// Real-space energy/force: warps and slots as in k_ew_field, six components a
+// slot and one energy a warp.
 template <class R>
-__global__ void __launch_bounds__(kEwThreads) k_ew_force(PairParams P, EwParams E,
-                                                         const typename Vec4T<R>::type* __restrict__ posq_s,
-                                                         const typename Vec4T<R>::type* __restrict__ dipt_s,
-                                                         const typename Vec4T<R>::type* __restrict__ vec_s,
-                                                         const double4* __restrict__ tctr,
-                                                         const double4* __restrict__ text,
-                                                         const double* __restrict__ pos_s,
-                                                         const int* __restrict__ exs_off, const int* __restrict__ exs_j,
-                                                         const double* __restrict__ exs_m,
-                                                         const double* __restrict__ exs_s, const int* __restrict__ list,
-                                                         const int* __restrict__ count, int n_pad,
-                                                         double* __restrict__ out, double* __restrict__ tile_energy) {
+__global__ void __launch_bounds__(32) k_ew_force(PairParams P, EwParams E,
+                                                 const typename Vec4T<R>::type* __restrict__ posq_s,
+                                                 const typename Vec4T<R>::type* __restrict__ dipt_s,
+                                                 const typename Vec4T<R>::type* __restrict__ vec_s,
+                                                 const double4* __restrict__ tctr, const double4* __restrict__ text,
+                                                 const int* __restrict__ exs_off, const int* __restrict__ exs_j,
+                                                 const int* __restrict__ list, const int* __restrict__ count, int n_pad,
+                                                 double* __restrict__ out, double* __restrict__ warp_energy) {
     typedef typename Vec4T<R>::type V4;
-    __shared__ V4 s_pos[kEwWarps][32], s_dip[kEwWarps][32], s_ind[kEwWarps][32];
-    __shared__ EwPackedForceTile s_pk[sizeof(R) == 4 ? kEwWarps : 1];
-    __shared__ double s_red[kEwWarps][7][32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // One I tile per CTA; warps split the neighbour list (see k_ew_field).
-    const int I = blockIdx.x;
+    __shared__ V4 s_pos[sizeof(R) == 8 ? 32 : 1], s_dip[sizeof(R) == 8 ? 32 : 1], s_ind[sizeof(R) == 8 ? 32 : 1];
+    __shared__ EwPackedForceTile s_pk[1];
+    const int lane = threadIdx.x;
+    const int I = blockIdx.x / E.split, w = blockIdx.x % E.split;
     const int i = I * 32 + lane;
     const V4 pi = posq_s[i], di = dipt_s[i], ui = vec_s[i];
     const double4 cA = tctr[I];
     const double4 eAd = text[I];
     const float eA[3] = {(float)eAd.x, (float)eAd.y, (float)eAd.z};
-    const float rcm = (float)sqrt(E.rc2) + 1e-3f;
+    const float rcm = (float)sqrt(E.rc2) + 1e-3f, dm = sqrtf(E.damp_r2f) + 1e-3f;
     const int e0 = i < P.n ? exs_off[i] : 0, e1 = i < P.n ? exs_off[i + 1] : 0;
     const R rc2 = (R)E.rc2, damp_r2 = (R)P.damp_r2;
     double F[3] = {0, 0, 0}, G[3] = {0, 0, 0}, en = 0.0;
     const int cnt = count[I];
-    for (int t = warp; t < cnt; t += kEwWarps) {
+    for (int t = w; t < cnt; t += E.split) {
         const int ent = list[(size_t)I * E.cap + t];
-        const int J = ent & kTileMask;
+        const int J = ent & kTileMask, jbase = J * 32;
         const bool fold = (ent >> 30) & 1, slow = ((unsigned)ent >> 31) & 1u;
         const double4 cB = tctr[J];
-        __syncwarp();
-        const V4 pj = posq_s[J * 32 + lane], dj = dipt_s[J * 32 + lane], uj = vec_s[J * 32 + lane];
-        int nsteps = 16;
-        bool staged = false;
-        if constexpr (sizeof(R) == 4) {
-            if (!slow) {
-                // Only the J atoms within the cutoff of the I tile's box,
-                // compacted; an odd count is padded with a multipole-free copy.
-                float dc[3];
-                tile_dc(P, cA, cB, dc);
-                const bool act = near_i_tile(P, (float)pj.x, (float)pj.y, (float)pj.z, dc, eA, rcm * rcm, fold);
-                const unsigned mk = __ballot_sync(kFull, act);
-                const int nact = __popc(mk), k = __popc(mk & ((1u << lane) - 1u));
-                if (act) stage_packed_force(s_pk[warp], k, pj, dj, uj);
-                if ((nact & 1) && act && k == nact - 1)
-                    stage_packed_force(s_pk[warp], nact, make_float4(pj.x, pj.y, pj.z, 0.0f),
-                                       make_float4(0.0f, 0.0f, 0.0f, dj.w), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
-                nsteps = (nact + 1) >> 1;
-                staged = true;
-            }
-        }
-        if (!staged) {
-            s_pos[warp][lane] = pj;
-            s_dip[warp][lane] = dj;
-            s_ind[warp][lane] = uj;
-        }
-        __syncwarp();
+        const V4 pj = posq_s[jbase + lane], dj = dipt_s[jbase + lane], uj = vec_s[jbase + lane];
         R ox, oy, oz;
         tile_shift<R>(P, cA, cB, pi.x, pi.y, pi.z, ox, oy, oz);
         R f[3] = {0, 0, 0}, g[3] = {0, 0, 0}, e = 0;
+        __syncwarp();
         if constexpr (sizeof(R) == 4) {
-            if (!slow) {
-                const float iti = 1.0f / (float)di.w;
-                if (fold) ew_force_walk_x2<true>(P, E, s_pk[warp], ox, oy, oz, pi.w, di, ui, iti, rc2, damp_r2, nsteps, e, f, g);
-                else ew_force_walk_x2<false>(P, E, s_pk[warp], ox, oy, oz, pi.w, di, ui, iti, rc2, damp_r2, nsteps, e, f, g);
-                for (int c = 0; c < 3; c++) {
-                    F[c] += (double)f[c];
-                    G[c] += (double)g[c];
+            const float iti = 1.0f / di.w;
+            if (slow) {
+                stage_packed_force(s_pk[0], lane, pj, dj, uj);
+                __syncwarp();
+                const unsigned mk = pair_mask(P, exs_j, e0, e1, i, jbase);
+                ew_force_walk_x2<true, true, true>(P, E, s_pk[0], ox, oy, oz, pi.w, di, ui, iti, rc2, mk, 0, 16, e, f,
+                                                   g);
+            } else {
+                float dc[3];
+                tile_dc(P, cA, cB, dc);
+                int nn, nt;
+                const int k = near_first(P, pj.x, pj.y, pj.z, dc, eA, rcm * rcm, dm * dm, fold, lane, nn, nt);
+                if (k < 32) stage_packed_force(s_pk[0], k, pj, dj, uj);
+                if ((nt & 1) && k == nt - 1)
+                    stage_packed_force(s_pk[0], nt, make_float4(pj.x, pj.y, pj.z, 0.0f),
+                                       make_float4(0.0f, 0.0f, 0.0f, dj.w), make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+                __syncwarp();
+                const int mn = (nn + 1) >> 1, mt = (nt + 1) >> 1;
+                if (fold) {
+                    ew_force_walk_x2<true, true, false>(P, E, s_pk[0], ox, oy, oz, pi.w, di, ui, iti, rc2, 0u, 0, mn,
+                                                        e, f, g);
+                    ew_force_walk_x2<true, false, false>(P, E, s_pk[0], ox, oy, oz, pi.w, di, ui, iti, rc2, 0u, mn, mt,
+                                                         e, f, g);
+                } else {
+                    ew_force_walk_x2<false, true, false>(P, E, s_pk[0], ox, oy, oz, pi.w, di, ui, iti, rc2, 0u, 0, mn,
+                                                         e, f, g);
+                    ew_force_walk_x2<false, false, false>(P, E, s_pk[0], ox, oy, oz, pi.w, di, ui, iti, rc2, 0u, mn,
+                                                          mt, e, f, g);
                 }
-                en += (double)e;
-                continue;
             }
-        }
-        if (slow) {
-            const unsigned part = partner_bits(exs_j, e0, e1, J * 32);
-            if (fold) ew_force_walk<R, true, true>(P, E, s_pos[warp], s_dip[warp], s_ind[warp], i, J * 32, ox, oy, oz, pi.w, di, ui, part, rc2, damp_r2, e, f, g);
-            else ew_force_walk<R, false, true>(P, E, s_pos[warp], s_dip[warp], s_ind[warp], i, J * 32, ox, oy, oz, pi.w, di, ui, part, rc2, damp_r2, e, f, g);
-        } else if (fold) {
-            ew_force_walk<R, true, false>(P, E, s_pos[warp], s_dip[warp], s_ind[warp], i, J * 32, ox, oy, oz, pi.w, di, ui, 0u, rc2, damp_r2, e, f, g);
         } else {
-            ew_force_walk<R, false, false>(P, E, s_pos[warp], s_dip[warp], s_ind[warp], i, J * 32, ox, oy, oz, pi.w, di, ui, 0u, rc2, damp_r2, e, f, g);
+            s_pos[lane] = pj;
+            s_dip[lane] = dj;
+            s_ind[lane] = uj;
+            __syncwarp();
+            if (slow) {
+                const unsigned part = partner_bits(exs_j, e0, e1, jbase);
+                if (fold) ew_force_walk<R, true, true>(P, E, s_pos, s_dip, s_ind, i, jbase, ox, oy, oz, pi.w, di, ui, part, rc2, damp_r2, e, f, g);
+                else ew_force_walk<R, false, true>(P, E, s_pos, s_dip, s_ind, i, jbase, ox, oy, oz, pi.w, di, ui, part, rc2, damp_r2, e, f, g);
+            } else if (fold) {
+                ew_force_walk<R, true, false>(P, E, s_pos, s_dip, s_ind, i, jbase, ox, oy, oz, pi.w, di, ui, 0u, rc2, damp_r2, e, f, g);
+            } else {
+                ew_force_walk<R, false, false>(P, E, s_pos, s_dip, s_ind, i, jbase, ox, oy, oz, pi.w, di, ui, 0u, rc2, damp_r2, e, f, g);
+            }
         }
         for (int c = 0; c < 3; c++) {
             F[c] += (double)f[c];
@@ -944,31 +994,14 @@ __global__ void __launch_bounds__(kEwThreads) k_ew_force(PairParams P, EwParams 
         }
         en += (double)e;
     }
+    const bool real = i < P.n;
+    double* o = out + 6 * (size_t)w * n_pad;
     for (int c = 0; c < 3; c++) {
-        s_red[warp][c][lane] = F[c];
-        s_red[warp][3 + c][lane] = G[c];
+        o[(size_t)c * n_pad + i] = real ? F[c] : 0.0;
+        o[(size_t)(3 + c) * n_pad + i] = real ? G[c] : 0.0;
     }
-    s_red[warp][6][lane] = en;
-    __syncthreads();
-    if (warp != 0) return;
-    for (int w = 1; w < kEwWarps; w++) {
-        for (int c = 0; c < 3; c++) {
-            F[c] += s_red[w][c][lane];
-            G[c] += s_red[w][3 + c][lane];
-        }
-        en += s_red[w][6][lane];
-    }
-    if (i < P.n) {
-        ew_force_exceptions<R>(P, E, pos_s, posq_s, dipt_s, vec_s, exs_off, exs_j, exs_m, exs_s, i, en, F, G);
-    } else {
-        F[0] = F[1] = F[2] = G[0] = G[1] = G[2] = en = 0.0;
-    }
-    for (int c = 0; c < 3; c++) {
-        out[(size_t)c * n_pad + i] = F[c];
-        out[(size_t)(3 + c) * n_pad + i] = G[c];
-    }
-    en = warp_sum(en);
-    if (lane == 0) tile_energy[I] = en;
+    en = warp_sum(real ? en : 0.0);
+    if (lane == 0) warp_energy[blockIdx.x] = en;
 }
 
 // ---------------------------------------------------------------------------
@@ -1190,10 +1223,13 @@ __global__ void k_pme_influence(PmeGrid G, double alpha, const double* __restric
     C[k] = (R)c;
 }
 
-// Field -grad phi at every atom (+ self term selfc * d) into partial slot 1;
-// FORCE: force q E + (d.grad) E in components 0..2 and E in 3..5.
+// Field -grad phi at every atom, self term selfc * d and real space (KIND 0 or
+// 1), the whole field into partial slot 0; FORCE: force q E + (d.grad) E in
+// components 0..2 and E in 3..5, for k_ew_finish.
 template <class R, class GT, int KIND, bool FORCE>
-__global__ void k_pme_gather(PmeGrid G, int n, int n_pad, double selfc, const double* __restrict__ pos_s,
+__global__ void k_pme_gather(PairParams P, EwParams EP, const double* __restrict__ real_part, EwExceptions X,
+                             const typename Vec4T<R>::type* __restrict__ lab_s, PmeGrid G, int n, int n_pad,
+                             double selfc, const double* __restrict__ pos_s,
                              const typename Vec4T<R>::type* __restrict__ posq_s,
                              const typename Vec4T<R>::type* __restrict__ dipt_s,
                              const typename Vec4T<R>::type* __restrict__ vec_s, const GT* __restrict__ phi,
@@ -1248,9 +1284,11 @@ __global__ void k_pme_gather(PmeGrid G, int n, int n_pad, double selfc, const do
             const typename Vec4T<R>::type v = vec_s[k];
             dd = {(double)v.x, (double)v.y, (double)v.z};
         }
-        out[k] = E[0] + selfc * dd.x;
-        out[(size_t)n_pad + k] = E[1] + selfc * dd.y;
-        out[2 * (size_t)n_pad + k] = E[2] + selfc * dd.z;
+        const d3 r = ew_real_field<R, KIND == 2 ? 0 : KIND>(P, EP, real_part, n_pad, X, pos_s, posq_s,
+                                                            KIND == 0 ? dipt_s : vec_s, lab_s, k);
+        out[k] = r.x + (E[0] + selfc * dd.x);
+        out[(size_t)n_pad + k] = r.y + (E[1] + selfc * dd.y);
+        out[2 * (size_t)n_pad + k] = r.z + (E[2] + selfc * dd.z);
     } else {
         // dE_b/dx_a = -sum phi d_a d_b Th  (hab above, scaled by sc_a sc_b)
         double H[3][3];
@@ -1311,24 +1349,28 @@ __global__ void k_ew_finish(int n, int n_pad, const int* __restrict__ rank, cons
                             const typename Vec4T<R>::type* __restrict__ posq_s,
                             const typename Vec4T<R>::type* __restrict__ dipt_s,
                             const typename Vec4T<R>::type* __restrict__ vec_s, const double* __restrict__ lab,
-                            const double* __restrict__ pol, double alpha, double selfc, int recip,
-                            double* __restrict__ fpair, double* __restrict__ torque, double* __restrict__ epart,
+                            const double* __restrict__ pol, double alpha, double selfc, int recip, PairParams PP,
+                            EwParams EP, const double* __restrict__ real_part, EwExceptions X,
+                            const double* __restrict__ pos_s, double* __restrict__ fpair, double* __restrict__ torque, double* __restrict__ epart,
                             int subtract = 0) {
     __shared__ double red[40];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     double e = 0.0;
     if (i < n) {
         const int k = rank[i];
-        const size_t s1 = 6 * (size_t)n_pad;
-        double F[3], G[3];
-        for (int c = 0; c < 3; c++) {
-            F[c] = partial[(size_t)c * n_pad + k];
-            G[c] = partial[(size_t)(3 + c) * n_pad + k];
-            if (recip) {
-                F[c] += partial[s1 + (size_t)c * n_pad + k];
-                G[c] += partial[s1 + (size_t)(3 + c) * n_pad + k];
+        // Real space: the split sums in order, then the listed partners.
+        double F[3] = {0, 0, 0}, G[3] = {0, 0, 0};
+        for (int w = 0; w < EP.split; w++)
+            for (int c = 0; c < 3; c++) {
+                F[c] += real_part[(6 * (size_t)w + c) * n_pad + k];
+                G[c] += real_part[(6 * (size_t)w + 3 + c) * n_pad + k];
             }
-        }
+        ew_force_exceptions<R>(PP, EP, pos_s, posq_s, dipt_s, vec_s, X.off, X.j, X.m, X.s, k, e, F, G);
+        if (recip)
+            for (int c = 0; c < 3; c++) {
+                F[c] += partial[(size_t)c * n_pad + k];
+                G[c] += partial[(size_t)(3 + c) * n_pad + k];
+            }
         const typename Vec4T<R>::type P = dipt_s[k], U = vec_s[k];
         const d3 u = {(double)U.x, (double)U.y, (double)U.z};
         const d3 t = {(double)P.x + u.x, (double)P.y + u.y, (double)P.z + u.z};
@@ -1337,7 +1379,7 @@ __global__ void k_ew_finish(int n, int n_pad, const int* __restrict__ rank, cons
         G[1] += selfc * t.y;
         G[2] += selfc * t.z;
         const double q = (double)posq_s[k].w;
-        e = -alpha / kSqrtPi * q * q - 2.0 * alpha * alpha * alpha / (3.0 * kSqrtPi) * dot(t, t);
+        e += -alpha / kSqrtPi * q * q - 2.0 * alpha * alpha * alpha / (3.0 * kSqrtPi) * dot(t, t);
         if (subtract) {
             // The induced dipoles' own pass: its forces come off the total;
             // nothing acts on the permanent dipoles, and no induction term.
@@ -1401,6 +1443,12 @@ int smooth_size(int n) {
     }
 }
 
+// damp_r2 is where a u^3 reaches 50.  The packed FP32 walks stop at 27: there
+// (1 + a u^3) e^(-a u^3) = 5e-11, below half an ulp of the erfc kernels the
+// correction is subtracted from (0.006 of the bare ones or more within the
+// cutoffs the mode allows).
+float fp32_damp_r2(float damp_r2) { return damp_r2 * (float)std::pow(27.0 / 50.0, 2.0 / 3.0); }
+
 void check_cufft(cufftResult r, const char* what) {
     if (r != CUFFT_SUCCESS) throw TdpError{TDP_ERR_CUDA, std::string(what) + ": cuFFT error " + std::to_string((int)r)};
 }
@@ -1426,7 +1474,9 @@ struct Ewald {
     int* count = nullptr;
     int* overflow = nullptr;
     int* h_overflow = nullptr;
-    double* tile_energy = nullptr;
+    double* warp_energy = nullptr;
+    double* real_part = nullptr;   // real-space sums by slot: split * 6 * n_pad
+    int split = 1;
     double* atom_epart = nullptr;
     int n_atom_blk = 1;
     // Grid (planned on the first ewald_prepare).  The solver passes run on
@@ -1503,7 +1553,14 @@ Ewald* ewald_create(const Dev& d, int precision, bool vacuum, bool direct) {
         e->list = dalloc<int>((size_t)nt * e->cap, e->owned);
         e->count = dalloc<int>(nt, e->owned);
         e->overflow = dalloc<int>(1, e->owned);
-        e->tile_energy = dalloc<double>(nt, e->owned);
+        // Warps per I tile: at most nine rounds of the 20 resident warps an SM,
+        // no more than 32 (MD step with 4, 8, 16, 32: 910, 722, 650, 626 us at
+        // 6,591 atoms, 1691, 1374, 1219, 1177 at 24,000, 2818, 2284, 2032, 2008
+        // at 52,728, 2750, 2746, 2851, 3006 at 98,304).
+        e->split = 4;
+        while (e->split < 32 && (long)nt * e->split * 2 <= 9L * 20 * 148) e->split *= 2;
+        e->real_part = dalloc<double>((size_t)e->split * 6 * d.n_pad, e->owned);
+        e->warp_energy = dalloc<double>((size_t)nt * e->split, e->owned);
         e->n_atom_blk = std::max(1, (d.n + kVecThreads - 1) / kVecThreads);
         e->atom_epart = dalloc<double>(e->n_atom_blk, e->owned);
         TDP_CUDA(cudaMallocHost(&e->h_overflow, sizeof(int)));
@@ -1528,6 +1585,8 @@ void ewald_prepare(Ewald* e, const Dev& d, const double box[3], double cutoff, d
         e->E.rc2 = INFINITY;
         e->E.selfc = 0.0;
         e->E.cap = e->cap;
+        e->E.split = e->split;
+        e->E.damp_r2f = fp32_damp_r2(d.pp.damp_r2);
         e->n_rec_blk = 0;
         return;
     }
@@ -1569,6 +1628,8 @@ void ewald_prepare(Ewald* e, const Dev& d, const double box[3], double cutoff, d
     e->E.rc2 = cutoff * cutoff;
     e->E.selfc = 4.0 * a * a * a / (3.0 * kSqrtPi);
     e->E.cap = e->cap;
+    e->E.split = e->split;
+    e->E.damp_r2f = fp32_damp_r2(d.pp.damp_r2);
     if (box[0] != e->box[0] || box[1] != e->box[1] || box[2] != e->box[2]) {
         for (int k = 0; k < 3; k++) {
             e->box[k] = box[k];
@@ -1580,7 +1641,6 @@ void ewald_prepare(Ewald* e, const Dev& d, const double box[3], double cutoff, d
         influence(e, e->it, st);
         if (e->precision != TDP_PRECISION_DOUBLE) influence(e, e->en64, st);
     }
-    (void)d;
 }
 
 void ewald_params(const Ewald* e, double* alpha, int grid[3]) {
@@ -1633,13 +1693,31 @@ void pme_potential(Ewald* e, const Dev& d, FftGrid& g, bool energy, cudaStream_t
     else check_cufft(cufftExecC2R(g.inv, (cufftComplex*)g.cplx, (float*)g.real), "cufftExecC2R");
 }
 
+EwExceptions exceptions_of(const Dev& d) { return {d.exs_off, d.exs_j, d.exs_m, d.exs_s}; }
+
 template <class R, int KIND>
 void real_field(Ewald* e, const Dev& d, const void* src, cudaStream_t st, const void* lab = nullptr) {
     typedef typename Vec4T<R>::type V4;
-    const int blocks = d.pp.n_tiles;
-    k_ew_field<R, KIND><<<blocks, kEwThreads, 0, st>>>(d.pp, e->E, (const V4*)d.posq_s, (const V4*)src, d.tctr_s,
-                                                      d.text_s, d.pos_s, d.exs_off, d.exs_j, d.exs_m, d.exs_s, e->list, e->count,
-                                                      d.n_pad, d.partial, (const V4*)lab);
+    k_ew_field<R, KIND><<<d.pp.n_tiles * e->split, 32, 0, st>>>(
+        d.pp, e->E, (const V4*)d.posq_s, (const V4*)src, d.tctr_s, d.text_s, d.exs_off, d.exs_j, e->list, e->count,
+        d.n_pad, e->real_part);
+    e->launches++;
+    if (!e->vacuum) return;
+    k_ew_real_done<R, KIND><<<nblk((size_t)d.n_pad, 128), 128, 0, st>>>(d.pp, e->E, e->real_part, d.n_pad,
+                                                                        exceptions_of(d), d.pos_s,
+                                                                        (const V4*)d.posq_s, (const V4*)src,
+                                                                        (const V4*)lab, d.partial);
+    e->launches++;
+}
+
+// Reciprocal field of `dip` (KIND 0) or vec_s (KIND 1) on grid e->it, the self
+// term and real space, into partial slot 0.
+template <class R, int KIND>
+void gather_field(Ewald* e, const Dev& d, const void* dip, cudaStream_t st, const void* lab = nullptr) {
+    typedef typename Vec4T<R>::type V4;
+    k_pme_gather<R, R, KIND, false><<<nblk((size_t)d.n_pad, 128), 128, 0, st>>>(
+        d.pp, e->E, e->real_part, exceptions_of(d), (const V4*)lab, e->G, d.n, d.n_pad, e->E.selfc, d.pos_s,
+        (const V4*)d.posq_s, (const V4*)dip, (const V4*)d.vec_s, (const R*)e->it.real, d.partial);
     e->launches++;
 }
 
@@ -1666,25 +1744,18 @@ void ewald_fixed_field(Ewald* e, const Dev& d, cudaStream_t st, const void* oper
     TDP_CUDA(cudaGetLastError());
     if (e->vacuum) return;
     pme_potential<R, R, 0>(e, d, e->it, false, st, nullptr, dip);
-    k_pme_gather<R, R, 0, false><<<nblk((size_t)d.n_pad, 128), 128, 0, st>>>(
-        e->G, d.n, d.n_pad, e->E.selfc, d.pos_s, (const V4*)d.posq_s, dip, (const V4*)d.vec_s,
-        (const R*)e->it.real, d.partial + 3 * (size_t)d.n_pad);
-    e->launches++;
+    gather_field<R, 0>(e, d, dip, st, operand ? d.dipt_s : nullptr);
     TDP_CUDA(cudaGetLastError());
 }
 
 template <class R>
 void ewald_matvec(Ewald* e, const Dev& d, cudaStream_t st) {
-    typedef typename Vec4T<R>::type V4;
     e->launches = 0;
     real_field<R, 1>(e, d, d.vec_s, st);
     TDP_CUDA(cudaGetLastError());
     if (e->vacuum) return;
     pme_potential<R, R, 1>(e, d, e->it, false, st);
-    k_pme_gather<R, R, 1, false><<<nblk((size_t)d.n_pad, 128), 128, 0, st>>>(
-        e->G, d.n, d.n_pad, e->E.selfc, d.pos_s, (const V4*)d.posq_s, (const V4*)d.dipt_s, (const V4*)d.vec_s,
-        (const R*)e->it.real, d.partial + 3 * (size_t)d.n_pad);
-    e->launches++;
+    gather_field<R, 1>(e, d, d.dipt_s, st);
     TDP_CUDA(cudaGetLastError());
 }
 
@@ -1697,22 +1768,23 @@ template <class R>
 void energy_pass(Ewald* e, const Dev& d, const typename Vec4T<R>::type* posq, const typename Vec4T<R>::type* dipt,
                  double plasma, int subtract, cudaStream_t st) {
     typedef typename Vec4T<R>::type V4;
-    k_ew_force<R><<<d.pp.n_tiles, kEwThreads, 0, st>>>(d.pp, e->E, posq, dipt, (const V4*)d.vec_s, d.tctr_s,
-                                                       d.text_s, d.pos_s, d.exs_off, d.exs_j, d.exs_m, d.exs_s,
-                                                       e->list, e->count, d.n_pad, d.partial, e->tile_energy);
+    k_ew_force<R><<<d.pp.n_tiles * e->split, 32, 0, st>>>(d.pp, e->E, posq, dipt, (const V4*)d.vec_s, d.tctr_s,
+                                                          d.text_s, d.exs_off, d.exs_j, e->list, e->count, d.n_pad,
+                                                          e->real_part, e->warp_energy);
     if (!e->vacuum) {
         FftGrid& g = e->energy_grid();
         pme_potential<R, double, 2>(e, d, g, true, st, posq, dipt);
         k_pme_gather<R, double, 2, true><<<nblk((size_t)d.n_pad, 128), 128, 0, st>>>(
-            e->G, d.n, d.n_pad, e->E.selfc, d.pos_s, posq, dipt, (const V4*)d.vec_s, (const double*)g.real,
-            d.partial + 6 * (size_t)d.n_pad);
+            d.pp, e->E, e->real_part, exceptions_of(d), (const V4*)nullptr, e->G, d.n, d.n_pad, e->E.selfc, d.pos_s,
+            posq, dipt, (const V4*)d.vec_s, (const double*)g.real, d.partial);
     }
     k_ew_finish<R><<<e->n_atom_blk, kVecThreads, 0, st>>>(d.n, d.n_pad, d.rank, d.partial, posq, dipt,
                                                           (const V4*)d.vec_s, d.lab, d.alpha, e->alpha, e->E.selfc,
-                                                          e->vacuum ? 0 : 1, d.fpair, d.torque, e->atom_epart,
+                                                          e->vacuum ? 0 : 1, d.pp, e->E, e->real_part,
+                                                          exceptions_of(d), d.pos_s, d.fpair, d.torque, e->atom_epart,
                                                           subtract);
-    k_ew_energy_sum<<<1, kVecThreads, 0, st>>>(d.pp.n_tiles, e->tile_energy, e->n_rec_blk, e->rec_epart,
-                                               e->n_atom_blk, e->atom_epart, plasma, d.energy, subtract);
+    k_ew_energy_sum<<<1, 1024, 0, st>>>(d.pp.n_tiles * e->split, e->warp_energy, e->n_rec_blk, e->rec_epart,
+                                        e->n_atom_blk, e->atom_epart, plasma, d.energy, subtract);
     e->launches += e->vacuum ? 3 : 4;
 }
 

@@ -32,13 +32,13 @@ void ewald_params(const Ewald* e, double* alpha, int grid[3]);
 // Neighbour list of the sorted tiles within the cutoff (part of
 // ewald_fixed_field; alone for a caller that only runs matvecs).
 void ewald_build_list(Ewald* e, const Dev& d, cudaStream_t st);
-// Permanent field E_M of the sorted records into partial slots 0 (real
-// space) and 1 (reciprocal + self); builds the neighbour list first.
+// Permanent field E_M of the sorted records into partial slot 0; builds the
+// neighbour list first.
 // operand (the fused start of a warm-started solve): dipole records
 // P = m + mu0 in place of m, giving E_M + T mu0 (covalent partners split
 // into their M and I scales).
 template <class R> void ewald_fixed_field(Ewald* e, const Dev& d, cudaStream_t st, const void* operand = nullptr);
-// Periodic field T v of the operand in vec_s into partial slots 0 and 1.
+// Periodic field T v of the operand in vec_s into partial slot 0.
 template <class R> void ewald_matvec(Ewald* e, const Dev& d, cudaStream_t st);
 // Energy, forces (fpair) and torques (torque) at the converged dipoles d.mu;
 // plasma = -pi Q^2 / (2 V alpha^2) is added to the energy.  direct: the

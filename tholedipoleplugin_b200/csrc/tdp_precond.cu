@@ -3,8 +3,7 @@
 //
 // Every vector here is FP64 (n*3, atom order); B's matvec is the Ewald mode's
 // (tdp_ewald.cu) in the form's arithmetic, reading the packed operand in
-// vec_s and leaving real space in partial slot 0 and reciprocal space plus
-// self term in slot 1.  Reductions are block partials summed in a fixed order
+// vec_s and leaving the field in partial slot 0.  Reductions are block partials summed in a fixed order
 // by the next kernel, so an application is deterministic.
 #include "tdp_ewald.cuh"
 #include "tdp_frames.cuh"
@@ -93,9 +92,9 @@ __global__ void k_pc_q(int n, const int* __restrict__ rank, int n_pad, const dou
     if (i < n) {
         const int k = rank[i];
         d3 f;
-        f.x = partial[k] + partial[3 * (size_t)n_pad + k];
-        f.y = partial[(size_t)n_pad + k] + partial[4 * (size_t)n_pad + k];
-        f.z = partial[2 * (size_t)n_pad + k] + partial[5 * (size_t)n_pad + k];
+        f.x = partial[k];
+        f.y = partial[(size_t)n_pad + k];
+        f.z = partial[2 * (size_t)n_pad + k];
         f = f - M * csurf;
         const d3 p = ld3(pin + 3 * i);
         const d3 q = p - f * salpha[i];
