@@ -157,12 +157,17 @@ __global__ void k_ew_tiles(PairParams P, EwParams E, const double4* __restrict__
     const bool ragged = (P.n & 31) != 0;
     const int last = P.n_tiles - 1;
     int written = 0;
+    // The next 32 tiles' boxes are read during the test of the current ones.
+    double4 nc = tctr[min(lane, last)], ne = text[min(lane, last)];
     for (int J0 = 0; J0 < P.n_tiles; J0 += 32) {
         const int J = J0 + lane;
+        const double4 cB = nc, eB = ne;
+        const int nx = min(J + 32, last);
+        nc = tctr[nx];
+        ne = text[nx];
         bool keep = false;
         unsigned flags = 0u;
         if (J < P.n_tiles) {
-            const double4 cB = tctr[J], eB = text[J];
             double dc[3] = {cB.x - cA.x, cB.y - cA.y, cB.z - cA.z};
             const double ea[3] = {eA.x, eA.y, eA.z}, eb[3] = {eB.x, eB.y, eB.z};
             double g2 = 0.0;
@@ -278,11 +283,11 @@ __device__ __forceinline__ void ew_field_exceptions(const PairParams& P, const E
                                                     const typename Vec4T<R>::type* __restrict__ src,
                                                     const int* __restrict__ exs_off, const int* __restrict__ exs_j,
                                                     const double* __restrict__ exs_m, const double* __restrict__ exs_s,
-                                                    int i, double ti, double& fx, double& fy, double& fz,
-                                                    const typename Vec4T<R>::type* __restrict__ lab = nullptr) {
+                                                    int i, double ti, int lane, int lanes, double& fx, double& fy,
+                                                    double& fz, const typename Vec4T<R>::type* __restrict__ lab) {
     const int e0 = exs_off[i], e1 = exs_off[i + 1];
     const d3 pi = ld3(pos_s + 3 * i);
-    for (int e = e0; e < e1; e++) {
+    for (int e = e0 + lane; e < e1; e += lanes) {
         const int j = exs_j[e];
         const double sc = KIND == 0 ? exs_m[e] : exs_s[e];
         d3 pj = ld3(pos_s + 3 * j);
@@ -597,20 +602,20 @@ struct EwExceptions {
     const double *m, *s;
 };
 
-// Real-space field of slot k: the split sums in order, then the partners.
+// Real-space field of slot k, part `lane` of `lanes`: the split sums lane,
+// lane + lanes, ... and the partners likewise.
 template <class R, int KIND>
-__device__ __forceinline__ d3 ew_real_field(const PairParams& P, const EwParams& E, const double* __restrict__ part,
+__device__ __forceinline__ void ew_real_field(const PairParams& P, const EwParams& E, const double* __restrict__ part,
                                             int n_pad, const EwExceptions& X, const double* __restrict__ pos_s,
                                             const typename Vec4T<R>::type* __restrict__ posq_s,
                                             const typename Vec4T<R>::type* __restrict__ src,
-                                            const typename Vec4T<R>::type* __restrict__ lab, int k) {
-    double f[3] = {0.0, 0.0, 0.0};
-    for (int w = 0; w < E.split; w++)
+                                            const typename Vec4T<R>::type* __restrict__ lab, int k, int lane,
+                                            int lanes, double f[3]) {
+    for (int w = lane; w < E.split; w += lanes)
 #pragma unroll
         for (int c = 0; c < 3; c++) f[c] += part[(3 * (size_t)w + c) * n_pad + k];
-    ew_field_exceptions<R, KIND>(P, E, pos_s, posq_s, src, X.off, X.j, X.m, X.s, k, (double)src[k].w, f[0], f[1], f[2],
-                                 lab);
-    return {f[0], f[1], f[2]};
+    ew_field_exceptions<R, KIND>(P, E, pos_s, posq_s, src, X.off, X.j, X.m, X.s, k, (double)src[k].w, lane, lanes,
+                                 f[0], f[1], f[2], lab);
 }
 
 // The variational NoCutoff model's field: real space alone.
@@ -621,11 +626,9 @@ __global__ void k_ew_real_done(PairParams P, EwParams E, const double* __restric
                                const typename Vec4T<R>::type* __restrict__ lab, double* __restrict__ out) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n_pad) return;
-    const d3 f = k < P.n ? ew_real_field<R, KIND>(P, E, part, n_pad, X, pos_s, posq_s, src, lab, k)
-                         : d3{0.0, 0.0, 0.0};
-    out[k] = f.x;
-    out[(size_t)n_pad + k] = f.y;
-    out[2 * (size_t)n_pad + k] = f.z;
+    double f[3] = {0.0, 0.0, 0.0};
+    if (k < P.n) ew_real_field<R, KIND>(P, E, part, n_pad, X, pos_s, posq_s, src, lab, k, 0, 1, f);
+    for (int c = 0; c < 3; c++) out[(size_t)c * n_pad + k] = f[c];
 }
 
 // ---------------------------------------------------------------------------
@@ -1076,15 +1079,49 @@ __device__ __forceinline__ void atom_splines(const PmeGrid& G, const double* __r
 
 __device__ __forceinline__ int wrap(int g, int K) { return g < 0 ? g + K : g; }
 
+// Spread and gather: five consecutive lanes share an atom (six atoms a warp),
+// lane c on the grid points floor(u_z) - c, so that the five points of a row
+// -- consecutive in memory -- go out in one instruction.  With one thread an
+// atom every lane of an instruction hit another sector: 12.3e6 atomics of
+// 98,304 atoms took 72 us, now 27; at 6,591 atoms 13 -> 5 us, the gather with
+// the partners it took over 20 -> 11 us.
+constexpr int kPmeAtoms = 6;                     // atoms per warp
+constexpr int kPmeThreads = 128;
+constexpr int kPmeBlockAtoms = kPmeAtoms * kPmeThreads / 32;
+
+// Atom of the thread (-1: none) and its z point.
+__device__ __forceinline__ int pme_atom(int count, int& c) {
+    const int warp = (blockIdx.x * kPmeThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    const int k = warp * kPmeAtoms + lane / kOrder;
+    c = lane % kOrder;
+    return lane < kPmeAtoms * kOrder && k < count ? k : -1;
+}
+
+// Value of z point c out of a spline's five.
+template <class R>
+__device__ __forceinline__ R pick5(const R* v, int c) {
+    return c == 0 ? v[0] : c == 1 ? v[1] : c == 2 ? v[2] : c == 3 ? v[3] : v[4];
+}
+
+// Sum over the atom's five lanes, in lane order, valid on lane 0 of the five.
+template <class T>
+__device__ __forceinline__ T sum5(T v) {
+    const T a = __shfl_down_sync(kFull, v, 1), b = __shfl_down_sync(kFull, v, 2), c = __shfl_down_sync(kFull, v, 3),
+            d = __shfl_down_sync(kFull, v, 4);
+    return (((v + a) + b) + c) + d;
+}
+
 // KIND 0: (q, p) from posq_s/dipt_s; 1: (0, v) from vec_s; 2: (q, p + mu).
 template <class R, int KIND>
-__global__ void k_pme_spread(PmeGrid G, int n, const double* __restrict__ pos_s,
-                             const typename Vec4T<R>::type* __restrict__ posq_s,
-                             const typename Vec4T<R>::type* __restrict__ dipt_s,
-                             const typename Vec4T<R>::type* __restrict__ vec_s,
-                             unsigned long long* __restrict__ gfix, double* __restrict__ gdbl) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
+__global__ void __launch_bounds__(kPmeThreads) k_pme_spread(PmeGrid G, int n, const double* __restrict__ pos_s,
+                                                            const typename Vec4T<R>::type* __restrict__ posq_s,
+                                                            const typename Vec4T<R>::type* __restrict__ dipt_s,
+                                                            const typename Vec4T<R>::type* __restrict__ vec_s,
+                                                            unsigned long long* __restrict__ gfix,
+                                                            double* __restrict__ gdbl) {
+    int c;
+    const int k = pme_atom(n, c);
+    if (k < 0) return;
     int base[3];
     R th[3][kOrder], d1[3][kOrder], d2[3][kOrder];
     atom_splines<R, false>(G, pos_s, k, base, th, d1, d2);
@@ -1105,6 +1142,8 @@ __global__ void k_pme_spread(PmeGrid G, int n, const double* __restrict__ pos_s,
     dx *= (R)G.sc[0];
     dy *= (R)G.sc[1];
     dz *= (R)G.sc[2];
+    const int gz = wrap(base[2] - c, G.K[2]);
+    const R tz = pick5(th[2], c), dtz = pick5(d1[2], c);
 #pragma unroll
     for (int a = 0; a < kOrder; a++) {
         const int gx = wrap(base[0] - a, G.K[0]);
@@ -1114,33 +1153,38 @@ __global__ void k_pme_spread(PmeGrid G, int n, const double* __restrict__ pos_s,
             const R A = th[0][a] * th[1][b];
             const R S = q * A + dx * d1[0][a] * th[1][b] + dy * th[0][a] * d1[1][b];
             const R Z = dz * A;
-            const size_t row = ((size_t)gx * G.K[1] + gy) * G.K[2];
-#pragma unroll
-            for (int c = 0; c < kOrder; c++) {
-                const int gz = wrap(base[2] - c, G.K[2]);
-                const R v = S * th[2][c] + Z * d1[2][c];
-                if (sizeof(R) == 4)
-                    atomicAdd(gfix + row + gz, (unsigned long long)__float2ll_rn((float)v * 4294967296.0f));
-                else
-                    atomicAdd(gdbl + row + gz, (double)v);
-            }
+            const size_t at = ((size_t)gx * G.K[1] + gy) * G.K[2] + gz;
+            const R v = S * tz + Z * dtz;
+            if (sizeof(R) == 4)
+                atomicAdd(gfix + at, (unsigned long long)__float2ll_rn((float)v * 4294967296.0f));
+            else
+                atomicAdd(gdbl + at, (double)v);
         }
     }
 }
 
-// Fixed-point grid to G (FP32 for the solver passes, FP64 for the energy
-// pass), clearing it for the next spread.
-template <class G>
-__global__ void k_pme_fix_to_real(size_t ng, unsigned long long* __restrict__ gfix, G* __restrict__ out) {
-    size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= ng) return;
-    long long v = (long long)gfix[k];
-    gfix[k] = 0ull;
-    out[k] = (G)((double)v * kFixInv);
+// Fixed-point grid to FP32 (solver passes) or FP64 (energy pass), four words a
+// thread, clearing it for the next spread.
+__device__ __forceinline__ double fix_to_double(unsigned long long u) { return (double)(long long)u * kFixInv; }
+__global__ void k_pme_fix_to_f64x4(size_t ng, unsigned long long* __restrict__ gfix, double* __restrict__ out) {
+    const size_t k = 4 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
+    if (k + 3 < ng) {
+        ulonglong2* g2 = reinterpret_cast<ulonglong2*>(gfix + k);
+        const ulonglong2 a = g2[0], b = g2[1];
+        g2[0] = make_ulonglong2(0ull, 0ull);
+        g2[1] = make_ulonglong2(0ull, 0ull);
+        double2* o = reinterpret_cast<double2*>(out + k);
+        o[0] = make_double2(fix_to_double(a.x), fix_to_double(a.y));
+        o[1] = make_double2(fix_to_double(b.x), fix_to_double(b.y));
+    } else {
+        for (size_t j = k; j < ng; j++) {
+            out[j] = fix_to_double(gfix[j]);
+            gfix[j] = 0ull;
+        }
+    }
 }
 
-// FP32 version, four words per thread: v 2^-32 = hi + lo 2^-32 with hi the
-// signed upper and lo the unsigned lower 32 bits (two 32-bit conversions).
+// FP32: v 2^-32 = hi + lo 2^-32 with hi the signed upper and lo the unsigned lower 32 bits (two 32-bit conversions).
 __device__ __forceinline__ float fix_to_float(unsigned long long u) {
     const int hi = (int)(long long)(u >> 32);
     const unsigned lo = (unsigned)u;
@@ -1227,51 +1271,63 @@ __global__ void k_pme_influence(PmeGrid G, double alpha, const double* __restric
 // 1), the whole field into partial slot 0; FORCE: force q E + (d.grad) E in
 // components 0..2 and E in 3..5, for k_ew_finish.
 template <class R, class GT, int KIND, bool FORCE>
-__global__ void k_pme_gather(PairParams P, EwParams EP, const double* __restrict__ real_part, EwExceptions X,
+__global__ void __launch_bounds__(kPmeThreads) k_pme_gather(PairParams P, EwParams EP, const double* __restrict__ real_part, EwExceptions X,
                              const typename Vec4T<R>::type* __restrict__ lab_s, PmeGrid G, int n, int n_pad,
                              double selfc, const double* __restrict__ pos_s,
                              const typename Vec4T<R>::type* __restrict__ posq_s,
                              const typename Vec4T<R>::type* __restrict__ dipt_s,
                              const typename Vec4T<R>::type* __restrict__ vec_s, const GT* __restrict__ phi,
                              double* __restrict__ out) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n_pad) return;
-    if (k >= n) {
-        for (int c = 0; c < (FORCE ? 6 : 3); c++) out[(size_t)c * n_pad + k] = 0.0;
-        return;
-    }
+    int c;
+    const int at = pme_atom(n_pad, c), k = at >= 0 && at < n ? at : 0;   // idle lanes take atom 0 and write nothing
     int base[3];
     R th[3][kOrder], d1[3][kOrder], d2[3][kOrder];
     atom_splines<R, FORCE>(G, pos_s, k, base, th, d1, d2);
-    R ex = 0, ey = 0, ez = 0, hxx = 0, hyy = 0, hzz = 0, hxy = 0, hxz = 0, hyz = 0;
+    const int gz = wrap(base[2] - c, G.K[2]);
+    // Row sums of phi with the x and y weights; the z weights come after.
+    R px = 0, py = 0, pz = 0, pxx = 0, pyy = 0, pxy = 0;
 #pragma unroll
     for (int a = 0; a < kOrder; a++) {
         const int gx = wrap(base[0] - a, G.K[0]);
 #pragma unroll
         for (int b = 0; b < kOrder; b++) {
             const int gy = wrap(base[1] - b, G.K[1]);
-            const size_t row = ((size_t)gx * G.K[1] + gy) * G.K[2];
-            R s0 = 0, s1 = 0, s2 = 0;   // sum_c phi th_z, phi d1_z, phi d2_z
-#pragma unroll
-            for (int c = 0; c < kOrder; c++) {
-                const R p = (R)phi[row + wrap(base[2] - c, G.K[2])];
-                s0 += p * th[2][c];
-                s1 += p * d1[2][c];
-                if (FORCE) s2 += p * d2[2][c];
-            }
-            const R tx = th[0][a], ty = th[1][b], gxv = d1[0][a], gyv = d1[1][b];
-            ex -= gxv * ty * s0;
-            ey -= tx * gyv * s0;
-            ez -= tx * ty * s1;
+            const R p = (R)phi[((size_t)gx * G.K[1] + gy) * G.K[2] + gz];
+            const R tx = th[0][a] * p, gxv = d1[0][a] * p;
+            px += gxv * th[1][b];
+            py += tx * d1[1][b];
+            pz += tx * th[1][b];
             if (FORCE) {
-                hxx -= d2[0][a] * ty * s0;
-                hyy -= tx * d2[1][b] * s0;
-                hzz -= tx * ty * s2;
-                hxy -= gxv * gyv * s0;
-                hxz -= gxv * ty * s1;
-                hyz -= tx * gyv * s1;
+                pxx += d2[0][a] * p * th[1][b];
+                pyy += tx * d2[1][b];
+                pxy += gxv * d1[1][b];
             }
         }
+    }
+    const R tz = pick5(th[2], c), dtz = pick5(d1[2], c), ddz = FORCE ? pick5(d2[2], c) : R(0);
+    const R ex = -sum5(px * tz), ey = -sum5(py * tz), ez = -sum5(pz * dtz);
+    R hxx = 0, hyy = 0, hzz = 0, hxy = 0, hxz = 0, hyz = 0;
+    if (FORCE) {
+        hxx = -sum5(pxx * tz);
+        hyy = -sum5(pyy * tz);
+        hzz = -sum5(pz * ddz);
+        hxy = -sum5(pxy * tz);
+        hxz = -sum5(px * dtz);
+        hyz = -sum5(py * dtz);
+    }
+    // Real space of the atom, its slots and partners shared by the five lanes.
+    d3 real = {0.0, 0.0, 0.0};
+    if (!FORCE) {
+        double f[3] = {0.0, 0.0, 0.0};
+        if (at >= 0 && at < n)
+            ew_real_field<R, KIND == 2 ? 0 : KIND>(P, EP, real_part, n_pad, X, pos_s, posq_s,
+                                                   KIND == 0 ? dipt_s : vec_s, lab_s, k, c, kOrder, f);
+        real = {sum5(f[0]), sum5(f[1]), sum5(f[2])};
+    }
+    if (at < 0 || c != 0) return;
+    if (at >= n) {
+        for (int u = 0; u < (FORCE ? 6 : 3); u++) out[(size_t)u * n_pad + at] = 0.0;
+        return;
     }
     const double sx = G.sc[0], sy = G.sc[1], sz = G.sc[2];
     double E[3] = {(double)ex * sx, (double)ey * sy, (double)ez * sz};
@@ -1284,11 +1340,9 @@ __global__ void k_pme_gather(PairParams P, EwParams EP, const double* __restrict
             const typename Vec4T<R>::type v = vec_s[k];
             dd = {(double)v.x, (double)v.y, (double)v.z};
         }
-        const d3 r = ew_real_field<R, KIND == 2 ? 0 : KIND>(P, EP, real_part, n_pad, X, pos_s, posq_s,
-                                                            KIND == 0 ? dipt_s : vec_s, lab_s, k);
-        out[k] = r.x + (E[0] + selfc * dd.x);
-        out[(size_t)n_pad + k] = r.y + (E[1] + selfc * dd.y);
-        out[2 * (size_t)n_pad + k] = r.z + (E[2] + selfc * dd.z);
+        out[k] = real.x + (E[0] + selfc * dd.x);
+        out[(size_t)n_pad + k] = real.y + (E[1] + selfc * dd.y);
+        out[2 * (size_t)n_pad + k] = real.z + (E[2] + selfc * dd.z);
     } else {
         // dE_b/dx_a = -sum phi d_a d_b Th  (hab above, scaled by sc_a sc_b)
         double H[3][3];
@@ -1351,11 +1405,18 @@ __global__ void k_ew_finish(int n, int n_pad, const int* __restrict__ rank, cons
                             const typename Vec4T<R>::type* __restrict__ vec_s, const double* __restrict__ lab,
                             const double* __restrict__ pol, double alpha, double selfc, int recip, PairParams PP,
                             EwParams EP, const double* __restrict__ real_part, EwExceptions X,
-                            const double* __restrict__ pos_s, double* __restrict__ fpair, double* __restrict__ torque, double* __restrict__ epart,
+                            const double* __restrict__ pos_s, int n_we, const double* __restrict__ warp_energy,
+                            int n_re, const double* __restrict__ rec_energy, double* __restrict__ fpair, double* __restrict__ torque, double* __restrict__ epart,
                             int subtract = 0) {
     __shared__ double red[40];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     double e = 0.0;
+    // The block's share of the real- and reciprocal-space energies.
+    const int pw = (n_we + gridDim.x - 1) / gridDim.x, pr = (n_re + gridDim.x - 1) / gridDim.x;
+    for (int a = blockIdx.x * pw + threadIdx.x; a < min(n_we, (int)(blockIdx.x + 1) * pw); a += blockDim.x)
+        e += warp_energy[a];
+    for (int a = blockIdx.x * pr + threadIdx.x; a < min(n_re, (int)(blockIdx.x + 1) * pr); a += blockDim.x)
+        e += rec_energy[a];
     if (i < n) {
         const int k = rank[i];
         // Real space: the split sums in order, then the listed partners.
@@ -1400,14 +1461,11 @@ __global__ void k_ew_finish(int n, int n_pad, const int* __restrict__ rank, cons
     if (threadIdx.x == 0) epart[blockIdx.x] = e;
 }
 
-// *out = s + plasma, or with subtract *out -= s + plasma.
-__global__ void k_ew_energy_sum(int n_a, const double* __restrict__ a, int n_b, const double* __restrict__ b, int n_c,
-                                const double* __restrict__ c, double plasma, double* __restrict__ out,
-                                int subtract = 0) {
+// *out = s + plasma, or with subtract *out -= s + plasma; s: the sum of m parts.
+__global__ void k_ew_energy_sum(int m, const double* __restrict__ parts, double plasma, double* __restrict__ out,
+                                int subtract) {
     __shared__ double red[40];
-    double s = sum_partials(a, n_a, red);
-    s += sum_partials(b, n_b, red);
-    s += sum_partials(c, n_c, red);
+    const double s = sum_partials(parts, m, red);
     if (threadIdx.x == 0) *out = subtract ? *out - (s + plasma) : s + plasma;
 }
 
@@ -1666,7 +1724,7 @@ void pme_potential(Ewald* e, const Dev& d, FftGrid& g, bool energy, cudaStream_t
     const size_t nc = (size_t)e->K[0] * e->K[1] * (e->K[2] / 2 + 1);
     const bool fix = sizeof(R) == 4;   // the mixed form spreads into the fixed-point grid
     if (!fix) TDP_CUDA(cudaMemsetAsync(g.real, 0, ng * sizeof(double), st));
-    k_pme_spread<R, KIND><<<nblk((size_t)d.n, 128), 128, 0, st>>>(e->G, d.n, d.pos_s, posq, dipt,
+    k_pme_spread<R, KIND><<<nblk((size_t)d.n, kPmeBlockAtoms), kPmeThreads, 0, st>>>(e->G, d.n, d.pos_s, posq, dipt,
                                                                    (const V4*)d.vec_s, e->gfix,
                                                                    fix ? nullptr : (double*)g.real);
     e->launches++;
@@ -1674,7 +1732,7 @@ void pme_potential(Ewald* e, const Dev& d, FftGrid& g, bool energy, cudaStream_t
         if (sizeof(GT) == 4)
             k_pme_fix_to_f32x4<<<nblk((ng + 3) / 4, 256), 256, 0, st>>>(ng, e->gfix, (float*)g.real);
         else
-            k_pme_fix_to_real<GT><<<nblk(ng, 256), 256, 0, st>>>(ng, e->gfix, (GT*)g.real);
+            k_pme_fix_to_f64x4<<<nblk((ng + 3) / 4, 256), 256, 0, st>>>(ng, e->gfix, (double*)g.real);
         e->launches++;
     }
     check_cufft(cufftSetStream(g.fwd, st), "cufftSetStream");
@@ -1715,7 +1773,7 @@ void real_field(Ewald* e, const Dev& d, const void* src, cudaStream_t st, const 
 template <class R, int KIND>
 void gather_field(Ewald* e, const Dev& d, const void* dip, cudaStream_t st, const void* lab = nullptr) {
     typedef typename Vec4T<R>::type V4;
-    k_pme_gather<R, R, KIND, false><<<nblk((size_t)d.n_pad, 128), 128, 0, st>>>(
+    k_pme_gather<R, R, KIND, false><<<nblk((size_t)d.n_pad, kPmeBlockAtoms), kPmeThreads, 0, st>>>(
         d.pp, e->E, e->real_part, exceptions_of(d), (const V4*)lab, e->G, d.n, d.n_pad, e->E.selfc, d.pos_s,
         (const V4*)d.posq_s, (const V4*)dip, (const V4*)d.vec_s, (const R*)e->it.real, d.partial);
     e->launches++;
@@ -1774,17 +1832,18 @@ void energy_pass(Ewald* e, const Dev& d, const typename Vec4T<R>::type* posq, co
     if (!e->vacuum) {
         FftGrid& g = e->energy_grid();
         pme_potential<R, double, 2>(e, d, g, true, st, posq, dipt);
-        k_pme_gather<R, double, 2, true><<<nblk((size_t)d.n_pad, 128), 128, 0, st>>>(
+        k_pme_gather<R, double, 2, true><<<nblk((size_t)d.n_pad, kPmeBlockAtoms), kPmeThreads, 0, st>>>(
             d.pp, e->E, e->real_part, exceptions_of(d), (const V4*)nullptr, e->G, d.n, d.n_pad, e->E.selfc, d.pos_s,
             posq, dipt, (const V4*)d.vec_s, (const double*)g.real, d.partial);
     }
     k_ew_finish<R><<<e->n_atom_blk, kVecThreads, 0, st>>>(d.n, d.n_pad, d.rank, d.partial, posq, dipt,
                                                           (const V4*)d.vec_s, d.lab, d.alpha, e->alpha, e->E.selfc,
                                                           e->vacuum ? 0 : 1, d.pp, e->E, e->real_part,
-                                                          exceptions_of(d), d.pos_s, d.fpair, d.torque, e->atom_epart,
+                                                          exceptions_of(d), d.pos_s, d.pp.n_tiles * e->split,
+                                                          e->warp_energy, e->n_rec_blk, e->rec_epart, d.fpair,
+                                                          d.torque, e->atom_epart,
                                                           subtract);
-    k_ew_energy_sum<<<1, 1024, 0, st>>>(d.pp.n_tiles * e->split, e->warp_energy, e->n_rec_blk, e->rec_epart,
-                                        e->n_atom_blk, e->atom_epart, plasma, d.energy, subtract);
+    k_ew_energy_sum<<<1, kVecThreads, 0, st>>>(e->n_atom_blk, e->atom_epart, plasma, d.energy, subtract);
     e->launches += e->vacuum ? 3 : 4;
 }
 
