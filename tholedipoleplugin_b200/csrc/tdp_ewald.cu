@@ -20,7 +20,7 @@
 // partners) are masked out of the tile walk and evaluated separately in FP64.
 //
 // Work layout.  Atoms are in the spatially sorted slots of the field kernels
-// (molecules along a Morton curve, 32-atom tiles).  A neighbour list of tiles
+// (molecules along a Hilbert curve, 32-atom tiles).  A neighbour list of tiles
 // (J tiles whose bounding box comes within the cutoff of I's, minimum image)
 // is rebuilt at every evaluation.  One warp owns an I tile (lane = atom), walks
 // its J tiles with the J records staged in shared memory and broadcast one per
