@@ -61,6 +61,13 @@ __device__ __forceinline__ void band_pair(int k, int& p, int& q) {
     p = k - qq * (qq + 1) / 2;
 }
 
+// FP32 walks end the damping where the exponent x = a u^3 is 25, half of what
+// P.damp_r2 stands for: the largest departure of a factor from 1 there is
+// (1 + x + 1.5 x^2) exp(-x) = 1.4e-8, under half an ulp of 1 (3.0e-8), so every
+// FP32 factor beyond is 1 either way, and fewer tile pairs take the damped
+// walk (its range is 0.58 instead of 0.73 nm for water).
+constexpr float kDampRange32 = 0.62996f;   // (25/50)^(2/3)
+
 // Geometry of a tile pair: displacement of J's centre from I's (FP64, minimum
 // image), whether any pair needs per-pair folding, whether any pair can be
 // within the damping range.
@@ -71,7 +78,8 @@ struct TileGeom {
     unsigned fmask;   // dimensions in which some pair may need folding (bit k: dimension k)
 };
 
-__device__ __forceinline__ TileGeom tile_geom(const PairParams& P, double4 cA, double4 eA, double4 cB, double4 eB) {
+__device__ __forceinline__ TileGeom tile_geom(const PairParams& P, double damp_r2, double4 cA, double4 eA, double4 cB,
+                                              double4 eB) {
     TileGeom g;
     g.dcx = cB.x - cA.x;
     g.dcy = cB.y - cA.y;
@@ -94,7 +102,7 @@ __device__ __forceinline__ TileGeom tile_geom(const PairParams& P, double4 cA, d
     double gx = fmax(fabs(g.dcx) - eA.x - eB.x, 0.0);
     double gy = fmax(fabs(g.dcy) - eA.y - eB.y, 0.0);
     double gz = fmax(fabs(g.dcz) - eA.z - eB.z, 0.0);
-    g.near = gx * gx + gy * gy + gz * gz < (double)P.damp_r2;
+    g.near = gx * gx + gy * gy + gz * gz < damp_r2;
     return g;
 }
 
@@ -541,7 +549,7 @@ __global__ void __launch_bounds__(32, 16) k_field_items(
     const int I0 = a * NS, J0 = c * L, J1 = min(J0 + L, P.n_tiles);
     if (I0 >= P.n_tiles || J1 <= max(J0, I0)) return;
     const int s0 = 16 * blockIdx.y / gridDim.y, s1 = 16 * (blockIdx.y + 1) / gridDim.y;
-    const float damp_r2 = P.damp_r2;
+    const float damp_r2 = kDampRange32 * P.damp_r2;
 
     float4 pi[NS], vi[NS];
     int2 et[NS];
@@ -571,7 +579,7 @@ __global__ void __launch_bounds__(32, 16) k_field_items(
     {
         const int k = lane / L, I = I0 + k, J = J0 + lane % L;
         if (k < NS && I < P.n_tiles && J < P.n_tiles) {
-            const TileGeom g = tile_geom(P, tctr[I], text[I], tctr[J], text[J]);
+            const TileGeom g = tile_geom(P, (double)damp_r2, tctr[I], text[I], tctr[J], text[J]);
             gdx = (float)g.dcx;
             gdy = (float)g.dcy;
             gdz = (float)g.dcz;
@@ -820,7 +828,7 @@ __device__ __forceinline__ void slot_against(ISlot<R>& a, const PairParams& P, b
                                              const int* __restrict__ exc_j) {
     a.valid = a.act && J < P.n_tiles && (!same_band || Jl >= a.Il);
     if (!a.valid) return;
-    const TileGeom g = tile_geom(P, cA, eA, cB, eB);
+    const TileGeom g = tile_geom(P, (double)P.damp_r2, cA, eA, cB, eB);
     shift_into<R>(g, cA, cB, a.pi.x, a.pi.y, a.pi.z, a.ox, a.oy, a.oz);
     a.fold = g.fold;
     a.fmask = g.fmask;
@@ -941,7 +949,7 @@ __global__ void __launch_bounds__(kSymThreads, 3) k_field_sym(
                 if (!s1.valid || !s1.slow) continue;
                 R* f1 = k == 0 ? fa : fb;
                 const double4 cA = s_ic[2 * warp + k];
-                const TileGeom g1 = tile_geom(P, cA, s_ie[2 * warp + k], cB, eB);
+                const TileGeom g1 = tile_geom(P, (double)P.damp_r2, cA, s_ie[2 * warp + k], cB, eB);
                 if (s1.fold)
                     field_partners<R, KIND, true>(P, pos, posq, jvec, sp, sv, exc_off, exc_j, exc_m, exc_s, g1, cA,
                                                   cB, lane, s1.i, s1.I * 32, jbase, s1.e0, s1.e1, s1.ox, s1.oy, s1.oz,
@@ -1766,7 +1774,7 @@ __global__ void __launch_bounds__(32, 12) k_energy_items(
         return;
     }
     const int s0 = 16 * blockIdx.y / gridDim.y, s1 = 16 * (blockIdx.y + 1) / gridDim.y;
-    const float damp_r2 = P.damp_r2;
+    const float damp_r2 = kDampRange32 * P.damp_r2;
     const auto fetch = [&](int t) {
         copy16_async(&raw.p[lane], posq + t * 32 + lane);
         copy16_async(&raw.d[lane], dipt + t * 32 + lane);
@@ -1790,7 +1798,7 @@ __global__ void __launch_bounds__(32, 12) k_energy_items(
     float gdx = 0.f, gdy = 0.f, gdz = 0.f;
     unsigned gfl = 0u;
     if (lane < L && J0 + lane < P.n_tiles) {
-        const TileGeom g = tile_geom(P, tctr[I], text[I], tctr[J0 + lane], text[J0 + lane]);
+        const TileGeom g = tile_geom(P, (double)damp_r2, tctr[I], text[I], tctr[J0 + lane], text[J0 + lane]);
         gdx = (float)g.dcx;
         gdy = (float)g.dcy;
         gdz = (float)g.dcz;
@@ -2066,7 +2074,7 @@ __global__ void __launch_bounds__(kSymThreads, 3) k_energy_sym(
                 const double4 cB = s_ctr[Jl];
                 const bool diag = I == J;
                 const bool slow = diag || (J == P.n_tiles - 1 && (P.n & 31)) || (J >= et.x && J <= et.y);
-                const TileGeom g = tile_geom(P, cA, eA, cB, s_ext[Jl]);
+                const TileGeom g = tile_geom(P, (double)P.damp_r2, cA, eA, cB, s_ext[Jl]);
                 R oix, oiy, oiz;
                 shift_into<R>(g, cA, cB, pi.x, pi.y, pi.z, oix, oiy, oiz);
                 const int jbase = J * 32;
