@@ -1380,10 +1380,12 @@ __device__ __forceinline__ QiPair qi_pair2(const PairParams& P, f2 DX, f2 DY, f2
     return o;
 }
 
-// Pairs within these distances of the x axis (squared, nm^2) go to the list of
-// k_axis_pairs (tile pairs within the damping range) or take index_delta
-// (beyond it, where the pair forces are small).
-constexpr float kNearAxis2 = 3.6e-5f, kNearAxisFar2 = 2.5e-7f;
+// Pairs this close to the x axis (kNearAxis2, nm^2) and no further apart than
+// sqrt(kAxisListRange2) = 1.5 times the damping range go to the list of
+// k_axis_pairs.  Further pairs have smaller forces: within kNearAxisFar2 they
+// keep the lab form and take index_delta.  The line is drawn for each pair, not
+// for its tiles, so that a new spatial order moves no pair across it.
+constexpr float kNearAxis2 = 3.6e-5f, kNearAxisFar2 = 4.0e-6f, kAxisListRange2 = 2.2f;
 
 // Pairs (slots) that a walk left to k_axis_pairs.  Sized for 16 an atom; past
 // that a pair stays in its walk.
@@ -1463,8 +1465,8 @@ __global__ void k_axis_pairs(PairParams P, IndexRecords R, AxisList axis, const 
 // 1e-6 to 5e-6 of it.
 template <int MODE, bool FOLD, bool MASK, bool OPEN>
 __device__ __forceinline__ void energy_item_walk(const PairParams& P, const double* __restrict__ pos,
-                                                 const IndexRecords& R, const AxisList& axis, const EItemTile& T, int lane, int i, int id, int jbase, float oix,
-                                                 float oiy, float oiz, float4 pi, float4 di, float4 ui, unsigned mk,
+                                                 const IndexRecords& R, const AxisList& axis, const EItemTile& T,
+                                                 int lane, int i, int id, int jbase, float oix, float oiy, float oiz, float4 pi, float4 di, float4 ui, unsigned mk,
                                                  unsigned fm, float damp_r2, int s0, int s1, float (&f)[6],
                                                  float (&g)[6], float& en, d3 xi, const EItemPos* XJ, double& en64) {
     const int nxt = (lane + 1) & 31;
@@ -1555,8 +1557,7 @@ __device__ __forceinline__ void energy_item_walk(const PairParams& P, const doub
         const f2 XS = mul2(RINV, pk2(rsqrtf(ra), rsqrtf(rb)));
         const f2 NDXS = mul2(xneg2(DX), XS);
         f2 XX = mul2(RHO2, XS), XY = mul2(NDXS, DY), XZ = mul2(NDXS, DZ);
-        constexpr float kAxis2 = MODE == 0 ? kNearAxisFar2 : kNearAxis2;
-        if (ra <= kAxis2 || rb <= kAxis2) {
+        if (ra <= kNearAxis2 || rb <= kNearAxis2) {
             float xr[2], rv[2], xx[2], xy[2], xz[2], dx[2], dy[2], dz[2];
             un2(DX, dx[0], dx[1]);
             un2(DY, dy[0], dy[1]);
@@ -1569,10 +1570,16 @@ __device__ __forceinline__ void energy_item_walk(const PairParams& P, const doub
             xr[1] = rb;
 #pragma unroll
             for (int k = 0; k < 2; k++) {
-                if (xr[k] > kAxis2) continue;
                 const int j = k ? jb : ja;
                 float& r2 = k ? r2b : r2a;
-                if (MODE == 0) {
+                const bool listed = MODE == 2 || r2 < kAxisListRange2 * P.damp_r2;
+                if (xr[k] > (listed ? kNearAxis2 : kNearAxisFar2)) continue;
+                if (listed) {
+                    if (r2 < INFINITY && axis_push(axis, i, j)) {
+                        r2 = INFINITY;
+                        rv[k] = 0.0f;
+                    }
+                } else if (r2 < INFINITY) {
                     index_delta(P, R, pos, i, j, id, k ? jd.y : jd.x, dx[k], dy[k], dz[k]);
                     const float h2 = fmaf(dy[k], dy[k], dz[k] * dz[k]);
                     rv[k] = rsqrtf(fmaf(dx[k], dx[k], h2));
@@ -1581,9 +1588,6 @@ __device__ __forceinline__ void energy_item_walk(const PairParams& P, const doub
                     xy[k] = -dx[k] * s * dy[k];
                     xz[k] = -dx[k] * s * dz[k];
                     xr[k] = h2;
-                } else if (r2 < INFINITY && axis_push(axis, i, j)) {
-                    r2 = INFINITY;
-                    rv[k] = 0.0f;
                 }
                 if (xr[k] <= 1.0e-10f)
                     qi_frame_x(dx[k], dy[k], dz[k], rv[k], yz_differ_slot(dy[k], dz[k], pos, i, j), xx[k], xy[k],
