@@ -1133,13 +1133,24 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
             int v = atoi(e);
             if ((v == 1 || v == 2 || v == 4 || v == 8 || v == 16) && v <= widest) band = v;
         }
+        // Plain form's field kernel: bands of two tiles up to 512 tiles (one
+        // warp a CTA), four beyond, where the slots of the narrow bands would
+        // take more memory than the energy kernel's (matvec with 2 and 4: 83
+        // and 81 us at 3,993 atoms, 372 and 385 at 12,288, 2096 and 2031 at
+        // 31,944).  Too few CTAs for 16 an SM: the walks are split (2, 4, 8,
+        // 16 parts: 45, 32, 27, 28 us at 648 atoms, 45, 34, 30, 37 at 1,029,
+        // 51, 52, 57, 77 at 2,187).
+        const int fband = nt <= 512 ? 2 : 4, fbands = (nt + fband - 1) / fband;
+        d.field_L = fband;
+        d.field_parts = 1;
+        while (d.field_parts < 8 && (long)d.field_parts * fbands * (fbands + 1) / 2 <= 8L * 148) d.field_parts *= 2;
         const int pad = kTile * std::max(4, band);
         d.n = n;
         d.n_pad = std::max(pad, ((n + pad - 1) / pad) * pad);
         d.nvb = std::max(1, (n + kVecThreads - 1) / kVecThreads);
         d.pp.band_tiles = band;
         d.pp.n_bands = (nt + band - 1) / band;
-        d.nslot = d.pp.n_bands;
+        d.nslot = std::max(d.pp.n_bands, (fbands * d.field_parts + 1) / 2);   // of six components (energy) or three
         d.nsplit = 1;
         d.n_eblk = d.pp.n_bands * (d.pp.n_bands + 1) / 2;
         const bool variational = (h->flags & TDP_FLAG_VARIATIONAL) != 0;

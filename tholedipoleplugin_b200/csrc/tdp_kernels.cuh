@@ -8,7 +8,7 @@ namespace tdp {
 
 // All device buffers of one system (sizes: n atoms, n_pad = n rounded up to a
 // whole number of bands, nslot partial-sum slots that the pair kernels write
-// (plain all-pairs form: one per band, added into slot 0 before anything reads
+// (plain all-pairs form: one per band and part, added into slot 0 before anything reads
 // them), nsplit slots that their consumers add, n_eblk energy partials = one
 // per band pair or item, nvb blocks of the O(N) kernels).
 constexpr int kMuHist = 4;
@@ -77,8 +77,8 @@ struct Dev {
     unsigned long long* fixacc = nullptr;
     int* fix_err = nullptr;
     double fix_scale = 0.0, fix_limit = 0.0;
-    // Mixed all-pairs field kernel: J tiles per item and parts of each walk
-    // (field_items).
+    // All-pairs field kernels: J tiles per item (plain form: tiles per band) and
+    // parts of each walk.
     int field_L = 1, field_parts = 1;
     // The same of the mixed energy kernel, and its accumulator's scale.
     int energy_L = 1, energy_parts = 1;

@@ -393,47 +393,4 @@ __device__ __forceinline__ void pair_energy(R dx, R dy, R dz, R r2, bool yz_diff
                                          mutual, fx, fy, fz, tx, ty, tz, d0, d1, d2, d3, d4, d5, en);
 }
 
-// Both sides of the mutual-field pair: the field at i from v_j and the field
-// at j from v_i (the dipole-field tensor is even in d), I scale applied by the
-// caller.
-template <class R, bool DAMP = true>
-__device__ __forceinline__ void pair_matvec2(R dx, R dy, R dz, R r2, R vix, R viy, R viz, R vjx, R vjy, R vjz, R ti,
-                                             R tj, R damp_r2, R& fix, R& fiy, R& fiz, R& fjx, R& fjy, R& fjz) {
-    R rinv = rsqrt_r(r2);
-    R rinv2 = rinv * rinv;
-    R rr3 = rinv * rinv2;
-    R rr5 = R(3) * rr3 * rinv2;
-    if (DAMP) damp_field(r2, rinv, ti, tj, damp_r2, rr3, rr5);
-    R ddj = rr5 * (vjx * dx + vjy * dy + vjz * dz);
-    R ddi = rr5 * (vix * dx + viy * dy + viz * dz);
-    fix += ddj * dx - rr3 * vjx;
-    fiy += ddj * dy - rr3 * vjy;
-    fiz += ddj * dz - rr3 * vjz;
-    fjx += ddi * dx - rr3 * vix;
-    fjy += ddi * dy - rr3 * viy;
-    fjz += ddi * dz - rr3 * viz;
-}
-
-// Both sides of the permanent-field pair (calculateFixedDipoleFieldPairIxn,
-// RTDF.cpp:678-713), M scale applied by the caller:
-//   E_i -= d (rr3 q_j - rr5 mu_j.d) + mu_j rr3,  E_j += d (rr3 q_i + rr5 mu_i.d) - mu_i rr3.
-template <class R, bool DAMP = true>
-__device__ __forceinline__ void pair_fixed2(R dx, R dy, R dz, R r2, R qi, R mix, R miy, R miz, R qj, R mjx, R mjy,
-                                            R mjz, R ti, R tj, R damp_r2, R& fix, R& fiy, R& fiz, R& fjx, R& fjy,
-                                            R& fjz) {
-    R rinv = rsqrt_r(r2);
-    R rinv2 = rinv * rinv;
-    R rr3 = rinv * rinv2;
-    R rr5 = R(3) * rr3 * rinv2;
-    if (DAMP) damp_field(r2, rinv, ti, tj, damp_r2, rr3, rr5);
-    R a = rr3 * qj - rr5 * (mjx * dx + mjy * dy + mjz * dz);
-    R b = rr3 * qi + rr5 * (mix * dx + miy * dy + miz * dz);
-    fix -= dx * a + mjx * rr3;
-    fiy -= dy * a + mjy * rr3;
-    fiz -= dz * a + mjz * rr3;
-    fjx += dx * b - mix * rr3;
-    fjy += dy * b - miy * rr3;
-    fjz += dz * b - miz * rr3;
-}
-
 }  // namespace tdp

@@ -4,37 +4,38 @@
 //
 // Work decomposition.  Atoms form 32-atom tiles.  The mixed form's kernels take
 // warp-sized items (k_field_items, k_energy_items).  In the plain form's, tiles
-// form bands of band_tiles tiles and one CTA (4 warps) owns a band pair (p, q), p <= q, and
-// evaluates every tile pair (I in band p, J in band q, I <= J).  A warp holds
+// form bands and one CTA owns a band pair (p, q), p <= q, and evaluates every
+// tile pair (I in band p, J in band q, I <= J).  A warp holds
 // the atoms of its I tile(s) in registers (lane = atom) and walks the atoms of
 // J along the diagonals of the tile pair, the J-side sums travelling with them
 // from lane to lane by shuffles, so that at the end each lane holds the
-// J-side sums of "its" J atom.  The scalar walks (FP64 form, and SLOW tile
-// pairs) pair lane l with J atom (l + s) mod 32 at step s.  The mixed form's
+// J-side sums of "its" J atom.  The FP64 walks pair lane l with J atom
+// (l + s) mod 32 at step s.  The mixed form's
 // packed walks (f32x2, tdp_f32x2.cuh) pair lane l with J atoms m and m + 16,
 // m = (l + s) mod 16, in the two halves of each register; lanes l and l ^ 16
 // then hold two copies of the same J sums, added by one xor-16 exchange.
 //
-// J-side sums of band q.  Field kernels: each warp sums into its own area of
-// shared memory, the four areas are added in warp order at the end.  Energy
+// J-side sums of band q.  Plain field kernel: each warp sums into its own area
+// of shared memory, the areas are added in warp order at the end.  Plain energy
 // kernel: one FP64 area; the warps visit disjoint J tiles within each window
 // of band_tiles / 4 steps and a barrier separates the windows, so the order
 // of the additions is fixed.
 //
-// Output.  Plain form: partial sums go to slot s of a [n_bands][components]
+// Output.  Plain form: partial sums go to slot s of a [slots][components]
 // [n_pad] FP64 buffer -- CTA (p, q) writes the I-side sums of band p into
-// slot q and the J-side sums of band q into slot p -- and k_slot_sum adds an
-// atom's slots in slot order.  Mixed form: every CTA adds its band sums into
-// one 64-bit fixed-point accumulator (integer addition, independent of the
-// order).  Either way results are bitwise deterministic.
+// slot q and the J-side sums of band q into slot p -- and k_field_slots and
+// k_slot_sum add an atom's slots in slot order.  Mixed form: every warp adds its
+// sums into one 64-bit fixed-point accumulator (integer addition, independent
+// of the order).  Either way results are bitwise deterministic.
 //
 // Tile pairs are classified as in the reference's arithmetic requires: FOLD
 // where the tiles' extents reach half a box (per-pair minimum image with an
 // FP64 fallback near the half-box boundary), DAMP where some pair may lie
-// within the Thole damping range, SLOW on the diagonal tile, the ragged last
-// tile and tiles holding covalent partners.  In SLOW tile pairs, self and
-// padding pairs and the partners are masked out of the diagonal walk; each
-// partner pair is then evaluated once per side with its M/I scales.
+// within the Thole damping range, MASK (SLOW in the plain energy kernel) on the
+// diagonal tile, the ragged last tile and tiles holding covalent partners.
+// There self and padding pairs and the partners are left out of the walk; each
+// partner pair is evaluated once per side with its M/I scales, by the kernel
+// that collects the sums or (plain energy kernel) after the walk.
 #include "tdp_frames.cuh"
 #include "tdp_f32x2.cuh"
 #include "tdp_kernels.cuh"
@@ -204,72 +205,88 @@ __device__ __forceinline__ void fix_add(const FixAcc& F, size_t k, double v) {
 // Field kernels: KIND 0 = permanent field (records: posq + lab dipole/thole),
 // KIND 1 = mutual-field matvec T*v (records: posq + v/thole).
 // ---------------------------------------------------------------------------
-template <class R, int KIND, bool FOLD, bool SLOW, bool DAMP>
-__device__ __forceinline__ void field_walk(const PairParams& P, const double* __restrict__ pos,
-                                           const typename Vec4T<R>::type* __restrict__ sp,
-                                           const typename Vec4T<R>::type* __restrict__ sv, int lane, int i, int jbase,
-                                           R oix, R oiy, R oiz, R qi, typename Vec4T<R>::type vi, bool diag,
-                                           unsigned partners, R damp_r2, R& fx, R& fy, R& fz, R& gx, R& gy, R& gz) {
-    const int nxt = (lane + 1) & 31;
-#pragma unroll 2
-    for (int s = 0; s < 32; s++) {
-        const int jj = (lane + s) & 31;
-        const typename Vec4T<R>::type pj = sp[jj];
-        const typename Vec4T<R>::type vj = sv[jj];
-        const int j = jbase + jj;
-        R dx, dy, dz;
-        pair_delta<R, FOLD>(P, pos, i, j, pj.x, pj.y, pj.z, oix, oiy, oiz, dx, dy, dz);
-        R r2 = dx * dx + dy * dy + dz * dz;
-        if (SLOW && skip_pair(s, lane, i, j, P.n, partners, jj, diag)) r2 = (R)INFINITY;
-        if (KIND == 0)
-            pair_fixed2<R, DAMP>(dx, dy, dz, r2, qi, vi.x, vi.y, vi.z, pj.w, vj.x, vj.y, vj.z, vi.w, vj.w, damp_r2, fx,
-                                 fy, fz, gx, gy, gz);
-        else
-            pair_matvec2<R, DAMP>(dx, dy, dz, r2, vi.x, vi.y, vi.z, vj.x, vj.y, vj.z, vi.w, vj.w, damp_r2, fx, fy, fz,
-                                  gx, gy, gz);
-        gx = __shfl_sync(kFull, gx, nxt);
-        gy = __shfl_sync(kFull, gy, nxt);
-        gz = __shfl_sync(kFull, gz, nxt);
-    }
+// 1/sqrt(x) of a positive normal x: the hardware's approximation and one
+// third-order (Halley) step, y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2: five
+// FP64 operations and no special cases.  y^2 is exact (the approximation's low
+// 32 bits are zero), so e carries no rounding of it.
+__device__ __forceinline__ double rsqrt_step(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y * y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
 }
 
-// Two I tiles against the same J tile: every J record read from shared
-// memory and every shuffle of the J-side sums serves two pairs, and the two
-// pair evaluations are independent instruction streams.
-template <class R, int KIND, bool FOLD, bool SLOW, bool DAMP>
-__device__ __forceinline__ void field_walk2(const PairParams& P, const double* __restrict__ pos,
-                                            const typename Vec4T<R>::type* __restrict__ sp,
-                                            const typename Vec4T<R>::type* __restrict__ sv, int lane, int jbase,
-                                            int ia, R oax, R oay, R oaz, R qa, typename Vec4T<R>::type va, bool diag_a,
-                                            unsigned part_a, int ib, R obx, R oby, R obz, R qb,
-                                            typename Vec4T<R>::type vb, bool diag_b, unsigned part_b, R damp_r2,
-                                            R* fa, R* fb, R* g) {
+// fold_d without its rounding instruction: round to nearest by the 1.5 * 2^52
+// constant.  Only an exact tie rounds differently, so displacements that end
+// within half_box_tol of half a box are folded again by fold_d.
+__device__ __forceinline__ double fold_magic(double d, double L, double invL, int tol_hi) {
+    const double magic = 6755399441055744.0;
+    const double t = __dadd_rn(__fma_rn(d, invL, magic), -magic);
+    const double f = __fma_rn(-t, L, d);
+    return (__double2hiint(f) & 0x7fffffff) >= tol_hi ? fold_d(d, L, invL) : f;
+}
+
+// The plain form's J records, one 16-byte piece of every atom after the other:
+// a warp reads 32 consecutive pieces without bank conflicts (8 wavefronts for
+// a 32-byte record of each lane, against 16 when the records lie whole).
+
+struct Rec64 {
+    double2 *xy, *zx, *yz, *qt;   // (x, y), (z, vx), (vy, vz), (q, t)
+    double* c;                    // 1 / t^3
+};
+
+// Two I atoms of a lane against the J tile at j0: both sides of every pair.
+// MASK: bit jj of m[k] is the pair (slot k, J atom jj); the other walks take all.
+template <int KIND, bool FOLD, bool DAMP, bool MASK>
+__device__ __forceinline__ void field_walk64(const PairParams& P, const Rec64& T, int lane, int j0,
+                                             const double (&o)[2][3], const double (&v)[2][3], const double (&q)[2],
+                                             const double (&ti)[2], const double (&c3)[2], const unsigned (&m)[2], unsigned fold, int s0,
+                                             int s1, double (&f)[2][3], double (&g)[3]) {
     const int nxt = (lane + 1) & 31;
-#pragma unroll 2
-    for (int s = 0; s < 32; s++) {
+    const int tx = __double2hiint(P.half_box_tol[0]), ty = __double2hiint(P.half_box_tol[1]),
+              tz = __double2hiint(P.half_box_tol[2]);
+#pragma unroll 1
+    for (int s = s0; s < s1; s++) {
         const int jj = (lane + s) & 31;
-        const typename Vec4T<R>::type pj = sp[jj];
-        const typename Vec4T<R>::type vj = sv[jj];
-        const int j = jbase + jj;
-        R dax, day, daz, dbx, dby, dbz;
-        pair_delta<R, FOLD>(P, pos, ia, j, pj.x, pj.y, pj.z, oax, oay, oaz, dax, day, daz);
-        pair_delta<R, FOLD>(P, pos, ib, j, pj.x, pj.y, pj.z, obx, oby, obz, dbx, dby, dbz);
-        R ra = dax * dax + day * day + daz * daz;
-        R rb = dbx * dbx + dby * dby + dbz * dbz;
-        if (SLOW) {
-            if (skip_pair(s, lane, ia, j, P.n, part_a, jj, diag_a)) ra = (R)INFINITY;
-            if (skip_pair(s, lane, ib, j, P.n, part_b, jj, diag_b)) rb = (R)INFINITY;
-        }
-        if (KIND == 0) {
-            pair_fixed2<R, DAMP>(dax, day, daz, ra, qa, va.x, va.y, va.z, pj.w, vj.x, vj.y, vj.z, va.w, vj.w,
-                                 damp_r2, fa[0], fa[1], fa[2], g[0], g[1], g[2]);
-            pair_fixed2<R, DAMP>(dbx, dby, dbz, rb, qb, vb.x, vb.y, vb.z, pj.w, vj.x, vj.y, vj.z, vb.w, vj.w,
-                                 damp_r2, fb[0], fb[1], fb[2], g[0], g[1], g[2]);
-        } else {
-            pair_matvec2<R, DAMP>(dax, day, daz, ra, va.x, va.y, va.z, vj.x, vj.y, vj.z, va.w, vj.w, damp_r2, fa[0],
-                                  fa[1], fa[2], g[0], g[1], g[2]);
-            pair_matvec2<R, DAMP>(dbx, dby, dbz, rb, vb.x, vb.y, vb.z, vj.x, vj.y, vj.z, vb.w, vj.w, damp_r2, fb[0],
-                                  fb[1], fb[2], g[0], g[1], g[2]);
+        const double2 xy = T.xy[j0 + jj], zx = T.zx[j0 + jj], yz = T.yz[j0 + jj];
+        double2 qt = make_double2(0.0, 0.0);
+        if (KIND == 0 || DAMP) qt = T.qt[j0 + jj];
+        const double wx = zx.y, wy = yz.x, wz = yz.y;
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            double dx = xy.x - o[k][0], dy = xy.y - o[k][1], dz = zx.x - o[k][2];
+            if (FOLD) {
+                if (fold & 1u) dx = fold_magic(dx, P.box[0], P.inv_box[0], tx);
+                if (fold & 2u) dy = fold_magic(dy, P.box[1], P.inv_box[1], ty);
+                if (fold & 4u) dz = fold_magic(dz, P.box[2], P.inv_box[2], tz);
+            }
+            const double r2 = dx * dx + dy * dy + dz * dz;
+            double rinv = rsqrt_step(r2);
+            if (MASK) rinv = (m[k] >> jj) & 1u ? rinv : 0.0;
+            const double rinv2 = rinv * rinv;
+            double rr3 = rinv * rinv2;
+            double rr5 = 3.0 * rr3 * rinv2;
+            if (DAMP && r2 < (double)P.damp_r2 && ti[k] * qt.y != 0.0) {
+                // x = min(t_i, t_j) (r / (t_i t_j))^3
+                const double x = fmin(ti[k], qt.y) * (r2 * r2 * rinv) * (c3[k] * T.c[j0 + jj]);
+                if (x < 50.0) {
+                    const double ex = exp(-x);
+                    rr3 *= 1.0 - ex;
+                    rr5 *= 1.0 - (1.0 + x) * ex;
+                }
+            }
+            double a = rr5 * (wx * dx + wy * dy + wz * dz);
+            double b = rr5 * (v[k][0] * dx + v[k][1] * dy + v[k][2] * dz);
+            if (KIND == 0) {
+                a = fma(-rr3, qt.x, a);
+                b = fma(rr3, q[k], b);
+            }
+            f[k][0] = fma(a, dx, fma(-rr3, wx, f[k][0]));
+            f[k][1] = fma(a, dy, fma(-rr3, wy, f[k][1]));
+            f[k][2] = fma(a, dz, fma(-rr3, wz, f[k][2]));
+            g[0] = fma(b, dx, fma(-rr3, v[k][0], g[0]));
+            g[1] = fma(b, dy, fma(-rr3, v[k][1], g[1]));
+            g[2] = fma(b, dz, fma(-rr3, v[k][2], g[2]));
         }
         g[0] = __shfl_sync(kFull, g[0], nxt);
         g[1] = __shfl_sync(kFull, g[1], nxt);
@@ -649,11 +666,41 @@ __global__ void __launch_bounds__(32, 16) k_field_items(
         for (int d = 0; d < 3; d++) fix_add(fix, (size_t)d * n_pad + (I0 + k) * 32 + lane, s_my[3 * k + d][lane]);
 }
 
-// Fixed-point sums -> partial slot 0, clearing them, plus the covalent
-// partners that k_field_items masked out, one-sided with their scales (FP64
-// displacement and arithmetic on the pair records).  kind 0: M scale; 1: I
-// scale; 2 (fused start, operand P = m + mu0): M field(q, P) + (I - M) T mu0
-// with mu0 = P - m, the second term also where M = 1.
+// Atom k's covalent partner e, which the walks masked out, one-sided with its
+// scale (FP64 displacement and arithmetic on the pair records).  KIND 0: M
+// scale; 1: I scale; fused (KIND 0, operand P = m + mu0): M field(q, P) +
+// (I - M) T mu0 with mu0 = P - m, the second term also where M = 1.
+template <int KIND, class V4>
+__device__ __forceinline__ void add_partner(const PairParams& P, int fused, const V4* __restrict__ posq,
+                                            const V4* __restrict__ jvec, const V4* __restrict__ lab,
+                                            const double* __restrict__ pos, const int* __restrict__ exc_j,
+                                            const double* __restrict__ exc_m, const double* __restrict__ exc_s, int k,
+                                            int e, double ti, double (&f)[3]) {
+    const double sc = KIND == 0 ? exc_m[e] : exc_s[e], ds = fused ? exc_s[e] - sc : 0.0;
+    if ((sc == 0.0 || sc == 1.0) && ds == 0.0) return;
+    const int j = exc_j[e];
+    const d3 d = exact_delta(P, pos, k, j);
+    const double r2 = dot(d, d);
+    const V4 vj = jvec[j];
+    double t[3] = {0.0, 0.0, 0.0};
+    if (KIND == 0)
+        pair_fixed<double, true>(d.x, d.y, d.z, r2, (double)posq[j].w, (double)vj.x, (double)vj.y, (double)vj.z, ti,
+                                 (double)vj.w, (double)P.damp_r2, t[0], t[1], t[2]);
+    else
+        pair_matvec<double, true>(d.x, d.y, d.z, r2, (double)vj.x, (double)vj.y, (double)vj.z, ti, (double)vj.w,
+                                  (double)P.damp_r2, t[0], t[1], t[2]);
+    if (sc != 1.0)
+        for (int c = 0; c < 3; c++) f[c] += sc * t[c];
+    if (ds != 0.0) {
+        const V4 mj = lab[j];
+        double u[3] = {0.0, 0.0, 0.0};
+        pair_matvec<double, true>(d.x, d.y, d.z, r2, (double)vj.x - (double)mj.x, (double)vj.y - (double)mj.y,
+                                  (double)vj.z - (double)mj.z, ti, (double)vj.w, (double)P.damp_r2, u[0], u[1], u[2]);
+        for (int c = 0; c < 3; c++) f[c] += ds * u[c];
+    }
+}
+
+// Fixed-point sums -> partial slot 0, clearing them, plus the partner pairs.
 template <int KIND>
 __global__ void k_field_done(PairParams P, int fused, const float4* __restrict__ posq, const float4* __restrict__ jvec,
                              const float4* __restrict__ lab, const double* __restrict__ pos,
@@ -670,325 +717,189 @@ __global__ void k_field_done(PairParams P, int fused, const float4* __restrict__
     }
     if (k < P.n) {
         const double ti = (double)jvec[k].w;
-        for (int e = exc_off[k]; e < exc_off[k + 1]; e++) {
-            const double sc = KIND == 0 ? exc_m[e] : exc_s[e], ds = fused ? exc_s[e] - sc : 0.0;
-            if ((sc == 0.0 || sc == 1.0) && ds == 0.0) continue;
-            const int j = exc_j[e];
-            const d3 d = exact_delta(P, pos, k, j);
-            const double r2 = dot(d, d);
-            const float4 vj = jvec[j];
-            double t[3] = {0.0, 0.0, 0.0};
-            if (KIND == 0)
-                pair_fixed<double, true>(d.x, d.y, d.z, r2, (double)posq[j].w, (double)vj.x, (double)vj.y,
-                                         (double)vj.z, ti, (double)vj.w, (double)P.damp_r2, t[0], t[1], t[2]);
-            else
-                pair_matvec<double, true>(d.x, d.y, d.z, r2, (double)vj.x, (double)vj.y, (double)vj.z, ti,
-                                          (double)vj.w, (double)P.damp_r2, t[0], t[1], t[2]);
-            if (sc != 1.0)
-                for (int c = 0; c < 3; c++) f[c] += sc * t[c];
-            if (ds != 0.0) {
-                const float4 mj = lab[j];
-                double u[3] = {0.0, 0.0, 0.0};
-                pair_matvec<double, true>(d.x, d.y, d.z, r2, (double)vj.x - (double)mj.x, (double)vj.y - (double)mj.y,
-                                          (double)vj.z - (double)mj.z, ti, (double)vj.w, (double)P.damp_r2, u[0],
-                                          u[1], u[2]);
-                for (int c = 0; c < 3; c++) f[c] += ds * u[c];
-            }
-        }
+        for (int e = exc_off[k]; e < exc_off[k + 1]; e++)
+            add_partner<KIND>(P, fused, posq, jvec, lab, pos, exc_j, exc_m, exc_s, k, e, ti, f);
     }
 #pragma unroll
     for (int c = 0; c < 3; c++) out[(size_t)c * n_pad + k] = f[c];
 }
 
-// Partner pairs of a SLOW tile pair, each side once with its scale (M for
-// the permanent field, I for the matvec): lane l adds, for its I atom, the
-// partners in J, and for atom l of J (not on the diagonal tile), the partners
-// in I.
-template <class R, int KIND, bool FOLD>
-__device__ __forceinline__ void field_partners(const PairParams& P, const double* __restrict__ pos,
-                                               const typename Vec4T<R>::type* __restrict__ posq,
-                                               const typename Vec4T<R>::type* __restrict__ jvec,
-                                               const typename Vec4T<R>::type* __restrict__ sp,
-                                               const typename Vec4T<R>::type* __restrict__ sv,
-                                               const int* __restrict__ exc_off, const int* __restrict__ exc_j,
-                                               const double* __restrict__ exc_m, const double* __restrict__ exc_s,
-                                               const TileGeom& g, double4 cA, double4 cB, int lane, int i, int ibase,
-                                               int jbase, int e0, int e1, R oix, R oiy, R oiz, R qi,
-                                               typename Vec4T<R>::type vi, bool diag, R damp_r2, R& fx, R& fy, R& fz,
-                                               R& gx, R& gy, R& gz,
-                                               const typename Vec4T<R>::type* __restrict__ lab = nullptr) {
-    typedef typename Vec4T<R>::type V4;
-    // With lab (the fused start of a warm-started solve, KIND 0) the operand
-    // is P = m + mu0 and a partner pair adds M * field(q, P) + (I - M) * T mu0
-    // = M * field(q, m) + I * T mu0, with mu0 = P - m.
-    const bool fused = KIND == 0 && lab != nullptr;
-#pragma unroll 1
-    for (int e = e0; e < e1; e++) {
-        unsigned off = (unsigned)(exc_j[e] - jbase);
-        if (off >= 32u) continue;
-        R sc = (R)(KIND == 0 ? exc_m[e] : exc_s[e]);
-        const R si = (R)exc_s[e];
-        if (sc == R(0) && (!fused || si == R(0))) continue;
-        const V4 pj = sp[off], vj = sv[off];
-        R dx, dy, dz;
-        pair_delta<R, FOLD>(P, pos, i, jbase + off, pj.x, pj.y, pj.z, oix, oiy, oiz, dx, dy, dz);
-        R r2 = dx * dx + dy * dy + dz * dz;
-        R tx = 0, ty = 0, tz = 0;
-        if (KIND == 0) pair_fixed<R, true>(dx, dy, dz, r2, pj.w, vj.x, vj.y, vj.z, vi.w, vj.w, damp_r2, tx, ty, tz);
-        else pair_matvec<R, true>(dx, dy, dz, r2, vj.x, vj.y, vj.z, vi.w, vj.w, damp_r2, tx, ty, tz);
-        fx += sc * tx;
-        fy += sc * ty;
-        fz += sc * tz;
-        if (fused && si != sc) {
-            const V4 mj = lab[jbase + off];
-            R ux = 0, uy = 0, uz = 0;
-            pair_matvec<R, true>(dx, dy, dz, r2, vj.x - mj.x, vj.y - mj.y, vj.z - mj.z, vi.w, vj.w, damp_r2, ux, uy,
-                                 uz);
-            fx += (si - sc) * ux;
-            fy += (si - sc) * uy;
-            fz += (si - sc) * uz;
-        }
-    }
-    if (diag) return;
-    const int jl = jbase + lane;
-    if (jl >= P.n) return;
-    const V4 pl = sp[lane], vl = sv[lane];
-#pragma unroll 1
-    for (int e = exc_off[jl]; e < exc_off[jl + 1]; e++) {
-        const int a = exc_j[e];
-        if ((unsigned)(a - ibase) >= 32u) continue;
-        R sc = (R)(KIND == 0 ? exc_m[e] : exc_s[e]);
-        const R si = (R)exc_s[e];
-        if (sc == R(0) && (!fused || si == R(0))) continue;
-        const V4 pa = posq[a], va = jvec[a];
-        R ox, oy, oz;
-        shift_into<R>(g, cA, cB, pa.x, pa.y, pa.z, ox, oy, oz);
-        R dx, dy, dz;  // p_a - p_jl
-        pair_delta<R, FOLD>(P, pos, jl, a, ox, oy, oz, pl.x, pl.y, pl.z, dx, dy, dz);
-        R r2 = dx * dx + dy * dy + dz * dz;
-        R tx = 0, ty = 0, tz = 0;
-        if (KIND == 0) pair_fixed<R, true>(dx, dy, dz, r2, pa.w, va.x, va.y, va.z, vl.w, va.w, damp_r2, tx, ty, tz);
-        else pair_matvec<R, true>(dx, dy, dz, r2, va.x, va.y, va.z, vl.w, va.w, damp_r2, tx, ty, tz);
-        gx += sc * tx;
-        gy += sc * ty;
-        gz += sc * tz;
-        if (fused && si != sc) {
-            const V4 ma = lab[a];
-            R ux = 0, uy = 0, uz = 0;
-            pair_matvec<R, true>(dx, dy, dz, r2, va.x - ma.x, va.y - ma.y, va.z - ma.z, vl.w, va.w, damp_r2, ux, uy,
-                                 uz);
-            gx += (si - sc) * ux;
-            gy += (si - sc) * uy;
-            gz += (si - sc) * uz;
-        }
-    }
-}
-
-// One I tile of a warp (lane = atom) and its state against the current J
-// tile.  The tile's centre and extent stay in shared memory (s_ic, s_ie).
-template <class R>
-struct ISlot {
-    typename Vec4T<R>::type pi, vi;
-    int2 et;
-    int Il, I, i, e0, e1;
-    bool act;
-    // Against the current J tile.
-    bool valid, diag, slow, fold, near;
-    unsigned partners, fmask;
-    R ox, oy, oz;
-};
-
-template <class R>
-__device__ __forceinline__ void load_slot(ISlot<R>& a, const PairParams& P, int p, int BT, int Il, int lane,
-                                          const typename Vec4T<R>::type* __restrict__ posq,
-                                          const typename Vec4T<R>::type* __restrict__ jvec,
-                                          const int* __restrict__ exc_off, const int2* __restrict__ exc_tiles) {
-    a.Il = Il;
-    a.I = p * BT + Il;
-    a.act = Il < BT && a.I < P.n_tiles;
-    a.i = a.I * 32 + lane;
-    a.pi = {};
-    a.vi = {};
-    a.et = make_int2(1 << 30, -1);
-    a.e0 = a.e1 = 0;
-    if (a.act) {
-        a.pi = posq[a.i];
-        a.vi = jvec[a.i];
-        a.et = exc_tiles[a.I];
-        if (a.i < P.n) {
-            a.e0 = exc_off[a.i];
-            a.e1 = exc_off[a.i + 1];
-        }
-    }
-}
-
-template <class R>
-__device__ __forceinline__ void slot_against(ISlot<R>& a, const PairParams& P, bool same_band, int J, int Jl,
-                                             double4 cA, double4 eA, double4 cB, double4 eB,
-                                             const int* __restrict__ exc_j) {
-    a.valid = a.act && J < P.n_tiles && (!same_band || Jl >= a.Il);
-    if (!a.valid) return;
-    const TileGeom g = tile_geom(P, (double)P.damp_r2, cA, eA, cB, eB);
-    shift_into<R>(g, cA, cB, a.pi.x, a.pi.y, a.pi.z, a.ox, a.oy, a.oz);
-    a.fold = g.fold;
-    a.fmask = g.fmask;
-    a.near = g.near;
-    a.diag = a.I == J;
-    a.slow = a.diag || (J == P.n_tiles - 1 && (P.n & 31)) || (J >= a.et.x && J <= a.et.y);
-    a.partners = a.slow ? partner_bits(exc_j, a.e0, a.e1, J * 32) : 0u;
-}
-
-// Plain form.  3 CTAs per SM (168 registers), which halves the walks' register
-// spills (measured 2-4 % faster than 4).
-template <class R, int KIND>
-__global__ void __launch_bounds__(kSymThreads, 3) k_field_sym(
-    PairParams P, const typename Vec4T<R>::type* __restrict__ posq, const typename Vec4T<R>::type* __restrict__ jvec,
-    const double4* __restrict__ tctr, const double4* __restrict__ text, const double* __restrict__ pos,
-    const int* __restrict__ exc_off, const int* __restrict__ exc_j, const double* __restrict__ exc_m,
-    const double* __restrict__ exc_s, const int2* __restrict__ exc_tiles, int n_pad, double* __restrict__ partial,
-    const typename Vec4T<R>::type* __restrict__ lab) {
-    typedef typename Vec4T<R>::type V4;
+// Plain form: one CTA per band pair and part of the walks, BT / 2 warps with
+// two I tiles each (see the top of the file).  Sums into slots of `partial`, part
+// y's from slot y * bands on.
+//
+// Bound by the latency of the FP64 chain: 37 FP64 operations a pair (43 with
+// the damped and masked tiles) keep the FP64 pipe 55 % busy with 16 warps an SM.
+// Hence two independent pairs a step, no unrolling (unrolled twice, the five
+// walks no longer share the instruction cache: 452 instead of 385 us), and
+// everything a walk does not need reread per J tile to stay at 122 registers.
+// The kernel before (one I tile a warp in narrow bands, whole 32-byte records,
+// library 1/sqrt and floor) against this one, matvec: 47 -> 30 us at 1,029
+// atoms, 227 -> 83 at 3,993, 516 -> 372 at 12,288, 2265 -> 2031 at 31,944.
+template <int KIND>
+__global__ void __launch_bounds__(128, 4)
+    k_field_bands(PairParams P, int BT, const double4* __restrict__ posq, const double4* __restrict__ jvec,
+                  const double4* __restrict__ tctr, const double4* __restrict__ text, const int* __restrict__ exc_off,
+                  const int* __restrict__ exc_j, const double* __restrict__ exc_scale,
+                  const int2* __restrict__ exc_tiles, int n_pad, double* __restrict__ partial) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int BT = P.band_tiles, NA = BT * 32;
-    double* s_iacc = reinterpret_cast<double*>(smem);              // 6 * kSymThreads: I-side sums, two slots
-    double4* s_ctr = reinterpret_cast<double4*>(s_iacc + 6 * kSymThreads);  // BT
-    double4* s_ext = s_ctr + BT;                                   // BT
-    double4* s_ic = s_ext + BT;                                    // 2 * kSymWarps: the warps' I tiles
-    double4* s_ie = s_ic + 2 * kSymWarps;
-    V4* s_pos = reinterpret_cast<V4*>(s_ie + 2 * kSymWarps);       // NA
-    V4* s_vec = s_pos + NA;                                        // NA
-    R* s_acc = reinterpret_cast<R*>(s_vec + NA);                   // kSymWarps * 3 * NA: J-side sums per warp
+    const int NA = BT * 32, warps = BT / 2;
+    Rec64 T;
+    T.xy = reinterpret_cast<double2*>(smem);
+    T.zx = T.xy + NA;
+    T.yz = T.zx + NA;
+    T.qt = T.yz + NA;
+    T.c = reinterpret_cast<double*>(T.qt + NA);
+    double4* s_geo = reinterpret_cast<double4*>(T.c + NA);
+    double* s_acc = reinterpret_cast<double*>(s_geo + warps * 2 * BT);   // [warp][component][NA]: J-side sums
 
     int p, q;
     band_pair(blockIdx.x, p, q);
+    const int s0 = 32 * blockIdx.y / gridDim.y, s1 = 32 * (blockIdx.y + 1) / gridDim.y;
+    const int bands = (P.n_tiles + BT - 1) / BT;
+    partial += (size_t)blockIdx.y * bands * 3 * n_pad;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int qa0 = q * NA;
-    for (int k = threadIdx.x; k < NA; k += kSymThreads) {
-        s_pos[k] = posq[qa0 + k];
-        s_vec[k] = jvec[qa0 + k];
+    for (int k = threadIdx.x; k < NA; k += blockDim.x) {
+        const double4 a = posq[q * NA + k], b = jvec[q * NA + k];
+        T.xy[k] = make_double2(a.x, a.y);
+        T.zx[k] = make_double2(a.z, b.x);
+        T.yz[k] = make_double2(b.y, b.z);
+        T.qt[k] = make_double2(a.w, b.w);
+        T.c[k] = 1.0 / (b.w * b.w * b.w);
     }
-    for (int k = threadIdx.x; k < kSymWarps * 3 * NA; k += kSymThreads) s_acc[k] = R(0);
-    for (int k = threadIdx.x; k < BT; k += kSymThreads) {
-        s_ctr[k] = tctr[q * BT + k];
-        s_ext[k] = text[q * BT + k];
-    }
-    double* my = s_iacc + 6 * threadIdx.x;
-    R* wacc = s_acc + warp * 3 * NA;
-    __syncthreads();
+    for (int k = threadIdx.x; k < warps * 3 * NA; k += blockDim.x) s_acc[k] = 0.0;
 
-    // Each warp sums its J-side contributions in its own area, so the warps
-    // never wait for one another until the final combination.
-    const R damp_r2 = (R)P.damp_r2;
-    const int stride = BT >= kSymWarps ? BT / kSymWarps : 1;
-    // A warp's I tiles are warp, warp + 4, warp + 8, ...; a round takes two of them.
-    const int rounds = (BT + 2 * kSymWarps - 1) / (2 * kSymWarps);
-    for (int r = 0; r < rounds; r++) {
-        ISlot<R> a, b;
-        load_slot<R>(a, P, p, BT, warp + 2 * kSymWarps * r, lane, posq, jvec, exc_off, exc_tiles);
-        load_slot<R>(b, P, p, BT, warp + 2 * kSymWarps * r + kSymWarps, lane, posq, jvec, exc_off, exc_tiles);
-        __syncwarp();
-        if (lane < 2) {
-            const ISlot<R>& s1 = lane == 0 ? a : b;
-            s_ic[2 * warp + lane] = s1.act ? tctr[s1.I] : make_double4(0, 0, 0, 0);
-            s_ie[2 * warp + lane] = s1.act ? text[s1.I] : make_double4(0, 0, 0, 0);
+    // The warp's 2 x BT tile-pair geometries, one per lane: the whole-box image
+    // of the tile pair and its flags.
+    const int I0 = p * BT + 2 * warp;
+    {
+        const int I = I0 + lane / BT, J = q * BT + lane % BT;
+        if (lane < 2 * BT) {
+            double4 s = make_double4(0, 0, 0, 0);
+            unsigned fl = 0u;
+            if (I < P.n_tiles && J < P.n_tiles) {
+                const double4 cA = tctr[I], cB = tctr[J];
+                const TileGeom g = tile_geom(P, (double)P.damp_r2, cA, text[I], cB, text[J]);
+                s.x = (cB.x - cA.x) - g.dcx;
+                s.y = (cB.y - cA.y) - g.dcy;
+                s.z = (cB.z - cA.z) - g.dcz;
+                fl = g.fmask | (g.fold ? 8u : 0u) | (g.near ? 16u : 0u);
+            }
+            s.w = __hiloint2double(0, (int)fl);
+            s_geo[warp * 2 * BT + lane] = s;
         }
-        __syncwarp();
-        for (int c = 0; c < 6; c++) my[c] = 0.0;
-        for (int t = 0; t < BT; t++) {
-            const int Jl = (t + warp * stride) % BT;
-            const int J = q * BT + Jl;
-            const double4 cB = s_ctr[Jl], eB = s_ext[Jl];
-            slot_against<R>(a, P, p == q, J, Jl, s_ic[2 * warp], s_ie[2 * warp], cB, eB, exc_j);
-            slot_against<R>(b, P, p == q, J, Jl, s_ic[2 * warp + 1], s_ie[2 * warp + 1], cB, eB, exc_j);
-            if (!(a.valid || b.valid)) continue;
-            const int jbase = J * 32;
-            const V4* sp = s_pos + Jl * 32;
-            const V4* sv = s_vec + Jl * 32;
-            R fa[3] = {0, 0, 0}, fb[3] = {0, 0, 0}, g[3] = {0, 0, 0};
-            if (a.valid && b.valid) {
-                const bool slow = a.slow || b.slow, fold = a.fold || b.fold;
-                const bool near = a.near || b.near;
-#define TDP_FWALK2(F, S, D)                                                                                        \
-    field_walk2<R, KIND, F, S, D>(P, pos, sp, sv, lane, jbase, a.i, a.ox, a.oy, a.oz, a.pi.w, a.vi, a.diag,     \
-                                  a.partners, b.i, b.ox, b.oy, b.oz, b.pi.w, b.vi, b.diag, b.partners, damp_r2, fa, \
-                                  fb, g)
-                if (slow) {
-                    if (fold) TDP_FWALK2(true, true, true);
-                    else TDP_FWALK2(false, true, true);
-                } else if (fold) {
-                    if (near) TDP_FWALK2(true, false, true);
-                    else TDP_FWALK2(true, false, false);
-                } else if (near) {
-                    TDP_FWALK2(false, false, true);
-                } else {
-                    TDP_FWALK2(false, false, false);
-                }
-#undef TDP_FWALK2
-            } else {
-                const ISlot<R>& s1 = a.valid ? a : b;
-                R* f1 = a.valid ? fa : fb;
-#define TDP_FWALK(F, S, D)                                                                                        \
-    field_walk<R, KIND, F, S, D>(P, pos, sp, sv, lane, s1.i, jbase, s1.ox, s1.oy, s1.oz, s1.pi.w, s1.vi, s1.diag, \
-                                 s1.partners, damp_r2, f1[0], f1[1], f1[2], g[0], g[1], g[2])
-                if (s1.slow) {
-                    if (s1.fold) TDP_FWALK(true, true, true);
-                    else TDP_FWALK(false, true, true);
-                } else if (s1.fold) {
-                    if (s1.near) TDP_FWALK(true, false, true);
-                    else TDP_FWALK(true, false, false);
-                } else if (s1.near) {
-                    TDP_FWALK(false, false, true);
-                } else {
-                    TDP_FWALK(false, false, false);
-                }
-#undef TDP_FWALK
-            }
-            // Partner pairs of each SLOW slot, each side once.
-            for (int k = 0; k < 2; k++) {
-                const ISlot<R>& s1 = k == 0 ? a : b;
-                if (!s1.valid || !s1.slow) continue;
-                R* f1 = k == 0 ? fa : fb;
-                const double4 cA = s_ic[2 * warp + k];
-                const TileGeom g1 = tile_geom(P, (double)P.damp_r2, cA, s_ie[2 * warp + k], cB, eB);
-                if (s1.fold)
-                    field_partners<R, KIND, true>(P, pos, posq, jvec, sp, sv, exc_off, exc_j, exc_m, exc_s, g1, cA,
-                                                  cB, lane, s1.i, s1.I * 32, jbase, s1.e0, s1.e1, s1.ox, s1.oy, s1.oz,
-                                                  s1.pi.w, s1.vi, s1.diag, damp_r2, f1[0], f1[1], f1[2], g[0], g[1],
-                                                  g[2], lab);
-                else
-                    field_partners<R, KIND, false>(P, pos, posq, jvec, sp, sv, exc_off, exc_j, exc_m, exc_s, g1, cA,
-                                                   cB, lane, s1.i, s1.I * 32, jbase, s1.e0, s1.e1, s1.ox, s1.oy,
-                                                   s1.oz, s1.pi.w, s1.vi, s1.diag, damp_r2, f1[0], f1[1], f1[2], g[0],
-                                                   g[1], g[2], lab);
-            }
-            R* acc = wacc + 3 * (Jl * 32 + lane);
-            for (int c = 0; c < 3; c++) {
-                acc[c] += g[c];
-                my[c] += (double)fa[c];
-                my[3 + c] += (double)fb[c];
-            }
-        }
-        // I-side sums: slot q of band p; on the diagonal band, slot p, where
-        // the J-side sums of the same atoms are added below.
+    }
+    double v[2][3];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int I = I0 + k;
+        const double4 b = I < P.n_tiles ? jvec[I * 32 + lane] : make_double4(0, 0, 0, 0);
+        v[k][0] = b.x;
+        v[k][1] = b.y;
+        v[k][2] = b.z;
+    }
+    __syncthreads();
+    double f[2][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+    double* acc = s_acc + warp * 3 * NA;
+    for (int t = 0; t < BT; t++) {
+        const int J = q * BT + t, jbase = J * 32;
+        if (J >= P.n_tiles || I0 > J || I0 >= P.n_tiles) continue;
+        // What a walk needs of the I atoms beside their operands is read anew
+        // for each J tile (L1), so that it takes no registers in between.
+        double o[2][3], qi[2], ti[2], c3[2];
+        unsigned mk[2], fl = 0u;
+        bool masked = false;
+        const unsigned real = J == P.n_tiles - 1 && (P.n & 31) ? (1u << (P.n & 31)) - 1u : ~0u;
+#pragma unroll
         for (int k = 0; k < 2; k++) {
-            const ISlot<R>& s1 = k == 0 ? a : b;
-            if (!s1.act) continue;
-            const size_t base = (size_t)q * 3 * n_pad;
-            for (int c = 0; c < 3; c++) partial[base + (size_t)c * n_pad + s1.i] = my[3 * k + c];
+            const int I = I0 + k, i = I * 32 + lane;
+            const double4 s = s_geo[(warp * 2 + k) * BT + t];
+            const double4 a = I < P.n_tiles ? posq[i] : make_double4(0, 0, 0, 0);
+            o[k][0] = a.x + s.x;
+            o[k][1] = a.y + s.y;
+            o[k][2] = a.z + s.z;
+            qi[k] = a.w;
+            ti[k] = I < P.n_tiles ? jvec[i].w : 0.0;
+            c3[k] = 1.0 / (ti[k] * ti[k] * ti[k]);
+            fl |= (unsigned)__double2loint(s.w);
+            mk[k] = I <= J && i < P.n ? real : 0u;
+            if (I == J) mk[k] &= ~((2u << lane) - 1u);   // each pair of a diagonal tile once: j > i
+            if (I < P.n_tiles && i < P.n) {
+                const int2 et = exc_tiles[I];
+                if (J >= et.x && J <= et.y)
+                    for (int e = exc_off[i]; e < exc_off[i + 1]; e++) {
+                        const unsigned off = (unsigned)(exc_j[e] - jbase);
+                        if (off < 32u && exc_scale[e] != 1.0) mk[k] &= ~(1u << off);
+                    }
+            }
+            masked = masked || mk[k] != ~0u;
+        }
+        double g[3] = {0.0, 0.0, 0.0};
+        const int j0 = t * 32;
+#define TDP_FWALK64(F, D, M) field_walk64<KIND, F, D, M>(P, T, lane, j0, o, v, qi, ti, c3, mk, fl, s0, s1, f, g)
+        if (__any_sync(kFull, masked)) {
+            TDP_FWALK64(true, true, true);
+        } else if (fl & 8u) {
+            if (fl & 16u) TDP_FWALK64(true, true, false);
+            else TDP_FWALK64(true, false, false);
+        } else if (fl & 16u) {
+            TDP_FWALK64(false, true, false);
+        } else {
+            TDP_FWALK64(false, false, false);
+        }
+#undef TDP_FWALK64
+        const int jl = j0 + ((lane + s1) & 31);   // the J atom whose sums the lane holds now
+#pragma unroll
+        for (int c = 0; c < 3; c++) acc[c * NA + jl] += g[c];
+        __syncwarp();
+    }
+    // I-side sums: slot q of band p; on the diagonal band they join the J-side
+    // sums of the same atoms.
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        if (I0 + k >= P.n_tiles) continue;
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            if (p == q) acc[c * NA + (2 * warp + k) * 32 + lane] += f[k][c];
+            else partial[((size_t)q * 3 + c) * n_pad + (I0 + k) * 32 + lane] = f[k][c];
         }
     }
     __syncthreads();
-    const size_t base = (size_t)p * 3 * n_pad;
-    for (int k = threadIdx.x; k < NA; k += kSymThreads) {
-        const int a = qa0 + k;
-        const bool own = p == q && (a >> 5) < P.n_tiles;
+    for (int k = threadIdx.x; k < NA; k += blockDim.x)
+#pragma unroll
         for (int c = 0; c < 3; c++) {
-            double v = 0.0;
-            for (int w = 0; w < kSymWarps; w++) v += (double)s_acc[w * 3 * NA + 3 * k + c];
-            if (own) v += partial[base + (size_t)c * n_pad + a];
-            partial[base + (size_t)c * n_pad + a] = v;
+            double s = 0.0;
+            for (int w = 0; w < warps; w++) s += s_acc[(w * 3 + c) * NA + k];
+            partial[((size_t)p * 3 + c) * n_pad + q * NA + k] = s;
         }
+}
+
+// Plain form: an atom's slots, in slot order, into slot 0, and its partner
+// pairs.  A CTA takes 32 atoms: warp c adds component c's slots (coalesced), and
+// the three warps share the partners.
+template <int KIND>
+__global__ void __launch_bounds__(96)
+    k_field_slots(PairParams P, int fused, const double4* __restrict__ posq, const double4* __restrict__ jvec,
+                  const double4* __restrict__ lab, const double* __restrict__ pos, const int* __restrict__ exc_off,
+                  const int* __restrict__ exc_j, const double* __restrict__ exc_m, const double* __restrict__ exc_s,
+                  int n_pad, int nslot, double* __restrict__ partial) {
+    __shared__ double s_part[3][3][32];
+    const int lane = threadIdx.x & 31, c = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;
+    double f[3] = {0.0, 0.0, 0.0};
+    if (k < P.n) {
+        const double ti = jvec[k].w;
+        for (int e = exc_off[k] + c; e < exc_off[k + 1]; e += 3)
+            add_partner<KIND>(P, fused, posq, jvec, lab, pos, exc_j, exc_m, exc_s, k, e, ti, f);
     }
+#pragma unroll
+    for (int d = 0; d < 3; d++) s_part[c][d][lane] = f[d];
+    __syncthreads();
+    const size_t count = (size_t)3 * n_pad;
+    double* out = partial + (size_t)c * n_pad + k;
+    double s = 0.0;
+#pragma unroll 8
+    for (int j = 0; j < nslot; j++) s += out[j * count];
+    *out = s + s_part[0][c][lane] + s_part[1][c][lane] + s_part[2][c][lane];
 }
 
 // ---------------------------------------------------------------------------
@@ -2154,11 +2065,8 @@ __global__ void __launch_bounds__(kSymThreads, 3) k_energy_sym(
     }
 }
 
-template <class R>
 size_t field_smem(int BT) {
-    const int NA = 32 * BT;
-    return sizeof(double) * 6 * kSymThreads + sizeof(double4) * (2 * BT + 4 * kSymWarps) +
-           sizeof(typename Vec4T<R>::type) * 2 * NA + sizeof(R) * kSymWarps * 3 * NA;
+    return (size_t)32 * BT * (4 * sizeof(double2) + (1 + 3 * (BT / 2)) * sizeof(double)) + BT * BT * sizeof(double4);
 }
 
 template <class R>
@@ -2188,9 +2096,9 @@ __global__ void k_slot_sum(size_t count, int nslot, double* __restrict__ partial
 }
 
 void slot_sum(const Dev& d, int ncomp, cudaStream_t st) {
-    if (d.nslot < 2) return;
+    if (d.pp.n_bands < 2) return;
     const size_t count = (size_t)ncomp * d.n_pad;
-    k_slot_sum<<<(unsigned)((count + 127) / 128), 128, 0, st>>>(count, d.nslot, d.partial);
+    k_slot_sum<<<(unsigned)((count + 127) / 128), 128, 0, st>>>(count, d.pp.n_bands, d.partial);
 }
 
 }  // namespace
@@ -2221,21 +2129,24 @@ void launch_field<float>(const Dev& d, int kind, cudaStream_t st) {
 
 template <>
 void launch_field<double>(const Dev& d, int kind, cudaStream_t st) {
-    const size_t smem = field_smem<double>(d.pp.band_tiles);
-    // Field kernels run on the spatially sorted records.
-    if (kind == 0 || kind == 2) {
-        cudaFuncSetAttribute(k_field_sym<double, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_field_sym<double, 0><<<band_pairs(d), kSymThreads, smem, st>>>(
-            d.pp, (const double4*)d.posq_s, (const double4*)(kind == 0 ? d.dipt_s : d.vec_s), d.tctr_s, d.text_s,
-            d.pos_s, d.exs_off, d.exs_j, d.exs_m, d.exs_s, d.exs_tiles, d.n_pad, d.partial,
-            kind == 2 ? (const double4*)d.dipt_s : nullptr);
+    const int BT = d.field_L, nb = (d.pp.n_tiles + BT - 1) / BT;
+    const dim3 grid((unsigned)(nb * (nb + 1) / 2), d.field_parts);
+    const size_t smem = field_smem(BT);
+    const double4 *pq = (const double4*)d.posq_s, *op = (const double4*)(kind == 0 ? d.dipt_s : d.vec_s);
+    if (kind == 1) {
+        cudaFuncSetAttribute(k_field_bands<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k_field_bands<1><<<grid, 16 * BT, smem, st>>>(d.pp, BT, pq, op, d.tctr_s, d.text_s, d.exs_off, d.exs_j,
+                                                      d.exs_s, d.exs_tiles, d.n_pad, d.partial);
+        k_field_slots<1><<<d.n_pad / 32, 96, 0, st>>>(d.pp, 0, pq, op, nullptr, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
+                                                      d.exs_s, d.n_pad, nb * d.field_parts, d.partial);
     } else {
-        cudaFuncSetAttribute(k_field_sym<double, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_field_sym<double, 1><<<band_pairs(d), kSymThreads, smem, st>>>(
-            d.pp, (const double4*)d.posq_s, (const double4*)d.vec_s, d.tctr_s, d.text_s, d.pos_s, d.exs_off, d.exs_j,
-            d.exs_m, d.exs_s, d.exs_tiles, d.n_pad, d.partial, nullptr);
+        cudaFuncSetAttribute(k_field_bands<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        k_field_bands<0><<<grid, 16 * BT, smem, st>>>(d.pp, BT, pq, op, d.tctr_s, d.text_s, d.exs_off, d.exs_j,
+                                                      d.exs_m, d.exs_tiles, d.n_pad, d.partial);
+        k_field_slots<0><<<d.n_pad / 32, 96, 0, st>>>(d.pp, kind == 2 ? 1 : 0, pq, op, (const double4*)d.dipt_s,
+                                                      d.pos_s, d.exs_off, d.exs_j, d.exs_m, d.exs_s, d.n_pad,
+                                                      nb * d.field_parts, d.partial);
     }
-    slot_sum(d, 3, st);
 }
 
 template <>
