@@ -10,6 +10,17 @@
 
 namespace tdp {
 
+// 1/sqrt(x) of a positive normal x: the hardware's approximation and one
+// third-order (Halley) step, y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2: five
+// FP64 operations and no special cases.  y^2 is exact (the approximation's low
+// 32 bits are zero), so e carries no rounding of it.
+__device__ __forceinline__ double rsqrt_step(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y * y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
 // Thole damping of 1/r^3 and 3/r^5 as getAndScaleInverseRs (RTDF.cpp:646-676).
 // Pairs with r2 >= damp_r2 have a*u^3 >= 50 and are left undamped there too.
 template <class R>
@@ -283,103 +294,70 @@ __device__ __forceinline__ void pair_energy_sides(R dx, R dy, R dz, R r2, bool y
 // the frame test's (:580-593): (x^ - Z_x Z)/|.| = (d_y^2 + d_z^2, -d_x d_y,
 // -d_x d_z) / (r sqrt(d_y^2 + d_z^2)) when the y or z coordinates differ,
 // the Gram-Schmidt form otherwise.  kap = 1 (Mutual) or -1: W = P + kap u.
-// VSUM: (tx, ty, tz) and (ux, uy, uz) receive V_ij and V_ji in place of the
-// torques, and en only the charge terms.  The torque of an atom is linear in
+// vi and vj receive V_ij and V_ji in place of the torques, and en only the
+// charge terms.  The torque of an atom is linear in
 // V with its own dipole fixed, tau_I = -perm(m_i x sum_j V_ij), and the
 // dipole terms of the energy are 0.5 (m_i.V_ij + m_j.V_ji) (expand m.V with
 // the expressions above: E = q_i q_j / r + (q_j P_i0 - q_i P_j0) / (2 r^2)
 // + (m_i.V_ij + m_j.V_ji) / 2), so a walk can sum V over its partners and
 // take one cross product and one dot product per atom at the end.
-template <class R, bool VSUM = false>
-__device__ __forceinline__ void pair_energy_lab(R dx, R dy, R dz, R r2, bool yz_differ, const EAtom<R>& I,
-                                                const EAtom<R>& K, R kap, R& fx, R& fy, R& fz, R& tx, R& ty, R& tz,
-                                                R& gx, R& gy, R& gz, R& ux, R& uy, R& uz, R& en) {
-    const R rinv = rsqrt_r(r2);
-    const R rho2 = dy * dy + dz * dz;
-    R xx, xy, xz;
-    if (yz_differ && rho2 > R(0)) {
-        const R s = rinv * rsqrt_r(rho2);
+// In S = m_i x V_ij + m_j x V_ji + u_i x Vd_ij + u_j x Vd_ji the rv3 terms
+// cancel pairwise (m_i x P_j + m_j x P_i + u_i x W_j + u_j x W_i = 0), so S =
+// K x X with K = a P_i + b P_j - 3 kap rv3 (u_j0 u_i + u_i0 u_j), a and b the
+// factors of X in V_ij and V_ji, and for the unit X S x X = (K.X) X - K.
+// yz_differ() is asked only for pairs within 1.4e-5 nm of the x axis.
+template <class YZ>
+__device__ __forceinline__ void pair_energy_lab(double dx, double dy, double dz, double qi, const double (&P)[3],
+                                                const double (&u)[3], double qj, const double (&Q)[3],
+                                                const double (&w)[3], double kap, YZ yz_differ, double* f, double* g,
+                                                double* vi, double* vj, double& en) {
+    const double rho2 = dy * dy + dz * dz, rinv = rsqrt_step(dx * dx + rho2);
+    double xx, xy, xz;
+    if (__double2hiint(rho2) > __double2hiint(2.0e-10) || (rho2 > 0.0 && yz_differ())) {
+        const double s = rinv * rsqrt_step(rho2), nd = -dx * s;
         xx = rho2 * s;
-        xy = -dx * dy * s;
-        xz = -dx * dz * s;
+        xy = nd * dy;
+        xz = nd * dz;
     } else {
-        const R zx = dx * rinv, zy = dy * rinv, zz = dz * rinv;
-        xx = zx + (yz_differ ? R(1) : R(0));
-        xy = zy + (yz_differ ? R(0) : R(1));
+        const bool yz = yz_differ();
+        const double zx = dx * rinv, zy = dy * rinv, zz = dz * rinv;
+        xx = zx + (yz ? 1.0 : 0.0);
+        xy = zy + (yz ? 0.0 : 1.0);
         xz = zz;
-        const R dt = zx * xx + zy * xy + zz * xz;
+        const double dt = zx * xx + zy * xy + zz * xz;
         xx -= zx * dt;
         xy -= zy * dt;
         xz -= zz * dt;
-        const R n2 = xx * xx + xy * xy + xz * xz;
-        const R s = n2 > R(0) ? rsqrt_r(n2) : R(1);
+        const double n2 = xx * xx + xy * xy + xz * xz;
+        const double s = n2 > 0.0 ? rsqrt(n2) : 1.0;
         xx *= s;
         xy *= s;
         xz *= s;
     }
-    const R pix = I.mx + I.ux, piy = I.my + I.uy, piz = I.mz + I.uz;
-    const R pjx = K.mx + K.ux, pjy = K.my + K.uy, pjz = K.mz + K.uz;
-    const R qi1 = xx * I.mx + xy * I.my + xz * I.mz, ui0 = xx * I.ux + xy * I.uy + xz * I.uz;
-    const R qj1 = xx * K.mx + xy * K.my + xz * K.mz, uj0 = xx * K.ux + xy * K.uy + xz * K.uz;
-    const R pi0 = qi1 + ui0, pj0 = qj1 + uj0;
-    const R rv2 = rinv * rinv, rv3 = rv2 * rinv;
-    const R qq = I.q * K.q;
-    if (VSUM) {
-        en += rinv * qq + R(0.5) * rv2 * (K.q * pi0 - I.q * pj0);
-    } else {
-        const R t1 = K.q * (pi0 + qi1) - I.q * (pj0 + qj1);
-        const R t2 = I.mx * pjx + I.my * pjy + I.mz * pjz + K.mx * pix + K.my * piy + K.mz * piz -
-                     R(3) * (qi1 * pj0 + qj1 * pi0);
-        en += rinv * qq + R(0.5) * (rv2 * t1 + rv3 * t2);
-    }
-    // V_ij = a X + rv3 P_j, V_ji = b X + rv3 P_i, Vd_ij = c X + rv3 W_j,
-    // Vd_ji = d X + rv3 W_i.  In S = m_i x V_ij + m_j x V_ji + u_i x Vd_ij +
-    // u_j x Vd_ji the rv3 terms cancel pairwise (m_i x P_j + m_j x P_i +
-    // u_i x W_j + u_j x W_i = 0 for P = m + u, W = m + (1 + kap) u), so
-    // S = K x X with K = a m_i + b m_j + c u_i + d u_j, and for the unit X
-    // S x X = (K.X) X - K.
-    const R a = rv2 * K.q - R(3) * rv3 * pj0;
-    const R b = -rv2 * I.q - R(3) * rv3 * pi0;
-    {
-        const R vx = a * xx + rv3 * pjx, vy = a * xy + rv3 * pjy, vz = a * xz + rv3 * pjz;
-        if (VSUM) {
-            tx += vx;
-            ty += vy;
-            tz += vz;
-        } else {
-            tx -= I.mz * vx - I.mx * vz;
-            ty -= I.mx * vy - I.my * vx;
-            tz -= I.my * vz - I.mz * vy;
-        }
-    }
-    {
-        const R vx = b * xx + rv3 * pix, vy = b * xy + rv3 * piy, vz = b * xz + rv3 * piz;
-        if (VSUM) {
-            ux += vx;
-            uy += vy;
-            uz += vz;
-        } else {
-            ux -= K.mz * vx - K.mx * vz;
-            uy -= K.mx * vy - K.my * vx;
-            uz -= K.my * vz - K.mz * vy;
-        }
-    }
-    const R c = rv2 * K.q - R(3) * rv3 * (pj0 + kap * uj0);
-    const R d = -rv2 * I.q - R(3) * rv3 * (pi0 + kap * ui0);
-    const R kx = a * I.mx + b * K.mx + c * I.ux + d * K.ux;
-    const R ky = a * I.my + b * K.my + c * I.uy + d * K.uy;
-    const R kz = a * I.mz + b * K.mz + c * I.uz + d * K.uz;
-    const R qf2 = rv2 * qq - R(2) * rv3 * (I.q * pj0 - K.q * pi0);
-    const R cf = rinv * (kx * xx + ky * xy + kz * xz) + qf2;
-    const R fvx = cf * xx - rinv * kx;
-    const R fvy = cf * xy - rinv * ky;
-    const R fvz = cf * xz - rinv * kz;
-    fx -= fvy;
-    fy -= fvz;
-    fz -= fvx;
-    gx += fvy;
-    gy += fvz;
-    gz += fvx;
+    const double pi0 = xx * P[0] + xy * P[1] + xz * P[2], ui0 = xx * u[0] + xy * u[1] + xz * u[2];
+    const double pj0 = xx * Q[0] + xy * Q[1] + xz * Q[2], uj0 = xx * w[0] + xy * w[1] + xz * w[2];
+    const double rv2 = rinv * rinv, rv3 = rv2 * rinv, n3 = -3.0 * rv3;
+    const double qq = rinv * qi * qj, rad = qj * pi0 - qi * pj0;
+    en += fma(0.5 * rv2, rad, qq);
+    const double a = fma(n3, pj0, rv2 * qj), b = fma(n3, pi0, -(rv2 * qi));
+    vi[0] = fma(a, xx, fma(rv3, Q[0], vi[0]));
+    vi[1] = fma(a, xy, fma(rv3, Q[1], vi[1]));
+    vi[2] = fma(a, xz, fma(rv3, Q[2], vi[2]));
+    vj[0] = fma(b, xx, fma(rv3, P[0], vj[0]));
+    vj[1] = fma(b, xy, fma(rv3, P[1], vj[1]));
+    vj[2] = fma(b, xz, fma(rv3, P[2], vj[2]));
+    const double nk = n3 * kap, c = nk * uj0, d = nk * ui0;
+    const double kx = fma(a, P[0], fma(b, Q[0], fma(c, u[0], d * w[0])));
+    const double ky = fma(a, P[1], fma(b, Q[1], fma(c, u[1], d * w[1])));
+    const double kz = fma(a, P[2], fma(b, Q[2], fma(c, u[2], d * w[2])));
+    const double cf = fma(rinv, kx * xx + ky * xy + kz * xz, fma(rinv, qq, 2.0 * rv3 * rad));
+    const double fvx = fma(cf, xx, -(rinv * kx)), fvy = fma(cf, xy, -(rinv * ky)), fvz = fma(cf, xz, -(rinv * kz));
+    f[0] -= fvy;
+    f[1] -= fvz;
+    f[2] -= fvx;
+    g[0] += fvy;
+    g[1] += fvz;
+    g[2] += fvx;
 }
 
 // One side of the pair: SIDE_I adds the force and torque on I and the pair

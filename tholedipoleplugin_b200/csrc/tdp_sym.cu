@@ -119,49 +119,38 @@ __device__ __forceinline__ d3 exact_delta(const PairParams& P, const double* __r
     return d;
 }
 
-// p_j - p_i from j's record (its own tile frame) and i's record shifted into
-// that frame.
-template <class R, bool FOLD>
-__device__ __forceinline__ void pair_delta(const PairParams& P, const double* __restrict__ pos, int i, int j, R pjx,
-                                           R pjy, R pjz, R oix, R oiy, R oiz, R& dx, R& dy, R& dz) {
+// fold_d without its rounding instruction: round to nearest by the 1.5 * 2^52
+// constant.  Only an exact tie rounds differently, so displacements that end
+// within half_box_tol of half a box are folded again by fold_d.
+__device__ __forceinline__ double fold_magic(double d, double L, double invL, int tol_hi) {
+    const double magic = 6755399441055744.0;
+    const double t = __dadd_rn(__fma_rn(d, invL, magic), -magic);
+    const double f = __fma_rn(-t, L, d);
+    return (__double2hiint(f) & 0x7fffffff) >= tol_hi ? fold_d(d, L, invL) : f;
+}
+
+// p_j - p_i from j's position and i's shifted into j's image; fold: bits of the
+// dimensions that need folding.
+template <bool FOLD>
+__device__ __forceinline__ void pair_delta(const PairParams& P, unsigned fold, double pjx, double pjy, double pjz,
+                                           double oix, double oiy, double oiz, double& dx, double& dy, double& dz) {
     dx = pjx - oix;
     dy = pjy - oiy;
     dz = pjz - oiz;
     if (FOLD) {
-        if (sizeof(R) == 4) {
-            dx = (R)fold_f((float)dx, (float)P.box[0], (float)P.inv_box[0]);
-            dy = (R)fold_f((float)dy, (float)P.box[1], (float)P.inv_box[1]);
-            dz = (R)fold_f((float)dz, (float)P.box[2], (float)P.inv_box[2]);
-            if ((fabs(dx) > (R)P.half_box_tol[0] || fabs(dy) > (R)P.half_box_tol[1] ||
-                 fabs(dz) > (R)P.half_box_tol[2]) && i < P.n && j < P.n) {
-                d3 e = exact_delta(P, pos, i, j);
-                dx = (R)e.x;
-                dy = (R)e.y;
-                dz = (R)e.z;
-            }
-        } else {
-            dx = (R)fold_d((double)dx, P.box[0], P.inv_box[0]);
-            dy = (R)fold_d((double)dy, P.box[1], P.inv_box[1]);
-            dz = (R)fold_d((double)dz, P.box[2], P.inv_box[2]);
-        }
+        if (fold & 1u) dx = fold_magic(dx, P.box[0], P.inv_box[0], __double2hiint(P.half_box_tol[0]));
+        if (fold & 2u) dy = fold_magic(dy, P.box[1], P.inv_box[1], __double2hiint(P.half_box_tol[1]));
+        if (fold & 4u) dz = fold_magic(dz, P.box[2], P.inv_box[2], __double2hiint(P.half_box_tol[2]));
     }
 }
 
-// The record of an I-tile atom shifted into J's frame.  FP32: offsets from the
-// tile centres, shifted by the minimum-image centre displacement; FP64:
-// absolute positions, shifted by the whole-box image the tile pair chose.
-template <class R>
-__device__ __forceinline__ void shift_into(const TileGeom& g, double4 cA, double4 cB, R px, R py, R pz, R& ox, R& oy,
-                                           R& oz) {
-    if (sizeof(R) == 4) {
-        ox = px - (R)g.dcx;
-        oy = py - (R)g.dcy;
-        oz = pz - (R)g.dcz;
-    } else {
-        ox = px + (R)((cB.x - cA.x) - g.dcx);
-        oy = py + (R)((cB.y - cA.y) - g.dcy);
-        oz = pz + (R)((cB.z - cA.z) - g.dcz);
-    }
+// The position of an I-tile atom shifted by the whole-box image that the tile
+// pair chose.
+__device__ __forceinline__ void shift_into(const TileGeom& g, double4 cA, double4 cB, double px, double py, double pz,
+                                           double& ox, double& oy, double& oz) {
+    ox = px + ((cB.x - cA.x) - g.dcx);
+    oy = py + ((cB.y - cA.y) - g.dcy);
+    oz = pz + ((cB.z - cA.z) - g.dcz);
 }
 
 // Pairs of the diagonal walk that are left out: self, padding, listed
@@ -205,27 +194,6 @@ __device__ __forceinline__ void fix_add(const FixAcc& F, size_t k, double v) {
 // Field kernels: KIND 0 = permanent field (records: posq + lab dipole/thole),
 // KIND 1 = mutual-field matvec T*v (records: posq + v/thole).
 // ---------------------------------------------------------------------------
-// 1/sqrt(x) of a positive normal x: the hardware's approximation and one
-// third-order (Halley) step, y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2: five
-// FP64 operations and no special cases.  y^2 is exact (the approximation's low
-// 32 bits are zero), so e carries no rounding of it.
-__device__ __forceinline__ double rsqrt_step(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y * y, 1.0);
-    return fma(y * e, fma(e, 0.375, 0.5), y);
-}
-
-// fold_d without its rounding instruction: round to nearest by the 1.5 * 2^52
-// constant.  Only an exact tie rounds differently, so displacements that end
-// within half_box_tol of half a box are folded again by fold_d.
-__device__ __forceinline__ double fold_magic(double d, double L, double invL, int tol_hi) {
-    const double magic = 6755399441055744.0;
-    const double t = __dadd_rn(__fma_rn(d, invL, magic), -magic);
-    const double f = __fma_rn(-t, L, d);
-    return (__double2hiint(f) & 0x7fffffff) >= tol_hi ? fold_d(d, L, invL) : f;
-}
-
 // The plain form's J records, one 16-byte piece of every atom after the other:
 // a warp reads 32 consecutive pieces without bank conflicts (8 wavefronts for
 // a 32-byte record of each lane, against 16 when the records lie whole).
@@ -243,8 +211,6 @@ __device__ __forceinline__ void field_walk64(const PairParams& P, const Rec64& T
                                              const double (&ti)[2], const double (&c3)[2], const unsigned (&m)[2], unsigned fold, int s0,
                                              int s1, double (&f)[2][3], double (&g)[3]) {
     const int nxt = (lane + 1) & 31;
-    const int tx = __double2hiint(P.half_box_tol[0]), ty = __double2hiint(P.half_box_tol[1]),
-              tz = __double2hiint(P.half_box_tol[2]);
 #pragma unroll 1
     for (int s = s0; s < s1; s++) {
         const int jj = (lane + s) & 31;
@@ -254,12 +220,8 @@ __device__ __forceinline__ void field_walk64(const PairParams& P, const Rec64& T
         const double wx = zx.y, wy = yz.x, wz = yz.y;
 #pragma unroll
         for (int k = 0; k < 2; k++) {
-            double dx = xy.x - o[k][0], dy = xy.y - o[k][1], dz = zx.x - o[k][2];
-            if (FOLD) {
-                if (fold & 1u) dx = fold_magic(dx, P.box[0], P.inv_box[0], tx);
-                if (fold & 2u) dy = fold_magic(dy, P.box[1], P.inv_box[1], ty);
-                if (fold & 4u) dz = fold_magic(dz, P.box[2], P.inv_box[2], tz);
-            }
+            double dx, dy, dz;
+            pair_delta<FOLD>(P, fold, xy.x, xy.y, zx.x, o[k][0], o[k][1], o[k][2], dx, dy, dz);
             const double r2 = dx * dx + dy * dy + dz * dz;
             double rinv = rsqrt_step(r2);
             if (MASK) rinv = (m[k] >> jj) & 1u ? rinv : 0.0;
@@ -934,60 +896,83 @@ __device__ __forceinline__ bool yz_differ(R dy, R dz, const double2* __restrict_
     return d;
 }
 
+// J records of the plain energy kernel in pieces (see Rec64).
+struct ERec64 {
+    double2 *xy, *zq, *mm, *mu, *uu;   // (x, y), (z, q), (mx, my), (mz, ux), (uy, uz)
+    double* t;
+    __device__ __forceinline__ ERec64(double2* s, int n)
+        : xy(s), zq(s + n), mm(s + 2 * n), mu(s + 3 * n), uu(s + 4 * n), t(reinterpret_cast<double*>(s + 5 * n)) {}
+    __device__ __forceinline__ EAtom<double> atom(int k) const {
+        EAtom<double> a;
+        const double2 m = mm[k], x = mu[k], u = uu[k];
+        a.q = zq[k].y;
+        a.mx = m.x;
+        a.my = m.y;
+        a.mz = x.x;
+        a.ux = x.y;
+        a.uy = u.x;
+        a.uz = u.y;
+        a.t = t[k];
+        return a;
+    }
+};
+
 // LAB (non-SLOW tile pairs beyond the damping range only): pair_energy_lab.
-template <class R, bool FOLD, bool SLOW, bool LAB = false>
-__device__ __forceinline__ void energy_walk(const PairParams& P, const double* __restrict__ pos,
-                                            const double2* __restrict__ yz,
-                                            const typename Vec4T<R>::type* __restrict__ sp,
-                                            const typename Vec4T<R>::type* __restrict__ sd,
-                                            const typename Vec4T<R>::type* __restrict__ su, int lane, int i,
-                                            int jbase, R oix, R oiy, R oiz, const EAtom<R>& me, bool diag,
-                                            unsigned partners, R damp_r2, R rv4p, R rv4f, R f[6], R g[6], R& en) {
+template <bool FOLD, bool SLOW, bool LAB = false>
+__device__ __forceinline__ void energy_walk(const PairParams& P, const double2* __restrict__ yz, const ERec64& T, int j0,
+                                            int lane, int i, int jbase, double oix, double oiy, double oiz,
+                                            const EAtom<double>& me, bool diag, unsigned partners, unsigned fold,
+                                            double f[6], double g[6], double& en) {
     const int nxt = (lane + 1) & 31;
     const int nmax = P.n_tiles * 32 - 1;
     // LAB: the walk sums V_ij (I side) and V_ji (J side, rotating with the
     // J atoms) and turns them into torques once at the end (pair_energy_lab).
-    R vi[3] = {0, 0, 0}, vj[3] = {0, 0, 0};
+    double vi[3] = {0, 0, 0}, vj[3] = {0, 0, 0};
+    const double Pi[3] = {me.mx + me.ux, me.my + me.uy, me.mz + me.uz}, ui[3] = {me.ux, me.uy, me.uz};
+    const double kap = P.mutual ? 1.0 : -1.0;
 #pragma unroll 1
     for (int s = 0; s < 32; s++) {
         const int jj = (lane + s) & 31;
         const int j = jbase + jj;
-        const EAtom<R> other = eatom<R>(sp[jj], sd[jj], su[jj]);
-        R dx, dy, dz;
-        pair_delta<R, FOLD>(P, pos, i, j, sp[jj].x, sp[jj].y, sp[jj].z, oix, oiy, oiz, dx, dy, dz);
-        R r2 = dx * dx + dy * dy + dz * dz;
-        if (SLOW && skip_pair(s, lane, i, j, P.n, partners, jj, diag)) r2 = (R)INFINITY;
-        const bool yzd = yz_differ<R>(dy, dz, yz, i, j, nmax);
-        if (LAB) {
-            pair_energy_lab<R, true>(dx, dy, dz, r2, yzd, me, other, P.mutual ? R(1) : R(-1), f[0], f[1], f[2], vi[0],
-                                     vi[1], vi[2], g[0], g[1], g[2], vj[0], vj[1], vj[2], en);
-        } else if (!SLOW || !diag) {
-            pair_energy_sides<R, 3>(dx, dy, dz, r2, yzd, me, other, R(1), R(1), damp_r2, rv4p, rv4f, P.mutual != 0,
-                                    f[0], f[1], f[2], f[3], f[4], f[5], g[0], g[1], g[2], g[3], g[4], g[5], en);
-        } else {
-            // Diagonal tile: the lane's atom is the lower index iff lane + s < 32.
-            const bool lo = lane + s < 32;
-            const EAtom<R> A = lo ? me : other;
-            const EAtom<R> B = lo ? other : me;
-            const R sg = lo ? R(1) : R(-1);
-            R a[6] = {0, 0, 0, 0, 0, 0}, b[6] = {0, 0, 0, 0, 0, 0};
-            pair_energy_sides<R, 3>(sg * dx, sg * dy, sg * dz, r2, yzd, A, B, R(1), R(1), damp_r2, rv4p, rv4f,
-                                    P.mutual != 0, a[0], a[1], a[2], a[3], a[4], a[5], b[0], b[1], b[2], b[3], b[4],
-                                    b[5], en);
-#pragma unroll
-            for (int c = 0; c < 6; c++) {
-                f[c] += lo ? a[c] : b[c];
-                g[c] += lo ? b[c] : a[c];
-            }
-        }
-        if (LAB) {
-            // g[3..5] are untouched by this walk (a full rotation is the identity).
+        const double2 pxy = T.xy[j0 + jj], pzq = T.zq[j0 + jj];
+        double dx, dy, dz;
+        pair_delta<FOLD>(P, fold, pxy.x, pxy.y, pzq.x, oix, oiy, oiz, dx, dy, dz);
+        if constexpr (LAB) {
+            const double2 mm = T.mm[j0 + jj], mu = T.mu[j0 + jj], uu = T.uu[j0 + jj];
+            const double w[3] = {mu.y, uu.x, uu.y}, Q[3] = {mm.x + w[0], mm.y + w[1], mu.x + w[2]};
+            pair_energy_lab(dx, dy, dz, me.q, Pi, ui, pzq.y, Q, w, kap,
+                            [&] { return yz_differ<double>(dy, dz, yz, i, j, nmax); }, f, g, vi, vj, en);
 #pragma unroll
             for (int c = 0; c < 3; c++) {
                 g[c] = __shfl_sync(kFull, g[c], nxt);
                 vj[c] = __shfl_sync(kFull, vj[c], nxt);
             }
         } else {
+            const double damp_r2 = (double)P.damp_r2, rv4p = (double)P.rinv4_power, rv4f = (double)P.rinv4_fill;
+            double r2 = dx * dx + dy * dy + dz * dz;
+            if (SLOW && skip_pair(s, lane, i, j, P.n, partners, jj, diag)) r2 = (double)INFINITY;
+            const bool yzd = yz_differ<double>(dy, dz, yz, i, j, nmax);
+            const EAtom<double> other = T.atom(j0 + jj);
+            if (!SLOW || !diag) {
+                pair_energy_sides<double, 3>(dx, dy, dz, r2, yzd, me, other, 1.0, 1.0, damp_r2, rv4p, rv4f,
+                                             P.mutual != 0, f[0], f[1], f[2], f[3], f[4], f[5], g[0], g[1], g[2], g[3],
+                                             g[4], g[5], en);
+            } else {
+                // Diagonal tile: the lane's atom is the lower index iff lane + s < 32.
+                const bool lo = lane + s < 32;
+                const EAtom<double> A = lo ? me : other;
+                const EAtom<double> B = lo ? other : me;
+                const double sg = lo ? 1.0 : -1.0;
+                double a[6] = {0, 0, 0, 0, 0, 0}, b[6] = {0, 0, 0, 0, 0, 0};
+                pair_energy_sides<double, 3>(sg * dx, sg * dy, sg * dz, r2, yzd, A, B, 1.0, 1.0, damp_r2, rv4p, rv4f,
+                                             P.mutual != 0, a[0], a[1], a[2], a[3], a[4], a[5], b[0], b[1], b[2],
+                                             b[3], b[4], b[5], en);
+#pragma unroll
+                for (int c = 0; c < 6; c++) {
+                    f[c] += lo ? a[c] : b[c];
+                    g[c] += lo ? b[c] : a[c];
+                }
+            }
 #pragma unroll
             for (int c = 0; c < 6; c++) g[c] = __shfl_sync(kFull, g[c], nxt);
         }
@@ -995,14 +980,14 @@ __device__ __forceinline__ void energy_walk(const PairParams& P, const double* _
     if (LAB) {
         // tau = -perm(m x sum V) and the dipole energy 0.5 m.sum V: the lane's
         // I atom, and J atom jbase + lane.
-        const typename Vec4T<R>::type mj = sd[lane];
-        en += R(0.5) * (me.mx * vi[0] + me.my * vi[1] + me.mz * vi[2] + mj.x * vj[0] + mj.y * vj[1] + mj.z * vj[2]);
+        const EAtom<double> mj = T.atom(j0 + lane);
+        en += 0.5 * (me.mx * vi[0] + me.my * vi[1] + me.mz * vi[2] + mj.mx * vj[0] + mj.my * vj[1] + mj.mz * vj[2]);
         f[3] -= me.mz * vi[0] - me.mx * vi[2];
         f[4] -= me.mx * vi[1] - me.my * vi[0];
         f[5] -= me.my * vi[2] - me.mz * vi[1];
-        g[3] -= mj.z * vj[0] - mj.x * vj[2];
-        g[4] -= mj.x * vj[1] - mj.y * vj[0];
-        g[5] -= mj.y * vj[2] - mj.z * vj[1];
+        g[3] -= mj.mz * vj[0] - mj.mx * vj[2];
+        g[4] -= mj.mx * vj[1] - mj.my * vj[0];
+        g[5] -= mj.my * vj[2] - mj.mz * vj[1];
     }
 }
 
@@ -1863,90 +1848,94 @@ __global__ void k_energy_items_done(PairParams P, const float4* __restrict__ pos
 // Partner pairs of a SLOW tile pair with their (M, I) scales, each side once:
 // the lane's I atom with its partners in J (the pair energy is counted on the
 // lower-index side), and atom l of J (off the diagonal) with its partners in I.
-template <class R, bool FOLD>
+template <bool FOLD>
 __device__ __forceinline__ void energy_partners(
-    const PairParams& P, const double* __restrict__ pos, const double2* __restrict__ yz,
-    const typename Vec4T<R>::type* __restrict__ posq, const typename Vec4T<R>::type* __restrict__ dipt,
-    const typename Vec4T<R>::type* __restrict__ indv, const typename Vec4T<R>::type* __restrict__ sp,
-    const typename Vec4T<R>::type* __restrict__ sd, const typename Vec4T<R>::type* __restrict__ su,
+    const PairParams& P, const double2* __restrict__ yz, const double4* __restrict__ posq,
+    const double4* __restrict__ dipt, const double4* __restrict__ indv, const ERec64& T, int j0,
     const int* __restrict__ exc_off, const int* __restrict__ exc_j, const double* __restrict__ exc_m,
     const double* __restrict__ exc_s, const TileGeom& geo, double4 cA, double4 cB, int lane, int i, int ibase,
-    int jbase, int e0, int e1, R oix, R oiy, R oiz, const EAtom<R>& me, bool diag, R damp_r2, R rv4p, R rv4f, R f[6],
-    R g[6], R& en) {
-    typedef typename Vec4T<R>::type V4;
+    int jbase, int e0, int e1, double oix, double oiy, double oiz, const EAtom<double>& me, bool diag, double f[6],
+    double g[6], double& en) {
     const int nmax = P.n_tiles * 32 - 1;
+    const double damp_r2 = (double)P.damp_r2, rv4p = (double)P.rinv4_power, rv4f = (double)P.rinv4_fill;
 #pragma unroll 1
     for (int e = e0; e < e1; e++) {
         unsigned off = (unsigned)(exc_j[e] - jbase);
         if (off >= 32u) continue;
-        const R mS = (R)exc_m[e], iS = (R)exc_s[e];
-        if (mS == R(0) && iS == R(0)) continue;
-        const int j = jbase + (int)off;
-        const EAtom<R> other = eatom<R>(sp[off], sd[off], su[off]);
-        R dx, dy, dz;
-        pair_delta<R, FOLD>(P, pos, i, j, sp[off].x, sp[off].y, sp[off].z, oix, oiy, oiz, dx, dy, dz);
-        const R r2 = dx * dx + dy * dy + dz * dz;
-        const bool yzd = yz_differ<R>(dy, dz, yz, i, j, nmax);
+        const double mS = exc_m[e], iS = exc_s[e];
+        if (mS == 0.0 && iS == 0.0) continue;
+        const int j = jbase + (int)off, k = j0 + (int)off;
+        const EAtom<double> other = T.atom(k);
+        double dx, dy, dz;
+        pair_delta<FOLD>(P, geo.fmask, T.xy[k].x, T.xy[k].y, T.zq[k].x, oix, oiy, oiz, dx, dy, dz);
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        const bool yzd = yz_differ<double>(dy, dz, yz, i, j, nmax);
         if (j > i)
-            pair_energy<R, true>(dx, dy, dz, r2, yzd, me, other, mS, iS, damp_r2, rv4p, rv4f, P.mutual != 0, f[0],
-                                 f[1], f[2], f[3], f[4], f[5], en);
+            pair_energy<double, true>(dx, dy, dz, r2, yzd, me, other, mS, iS, damp_r2, rv4p, rv4f, P.mutual != 0, f[0],
+                                      f[1], f[2], f[3], f[4], f[5], en);
         else
-            pair_energy<R, false>(-dx, -dy, -dz, r2, yzd, other, me, mS, iS, damp_r2, rv4p, rv4f, P.mutual != 0,
-                                  f[0], f[1], f[2], f[3], f[4], f[5], en);
+            pair_energy<double, false>(-dx, -dy, -dz, r2, yzd, other, me, mS, iS, damp_r2, rv4p, rv4f, P.mutual != 0,
+                                       f[0], f[1], f[2], f[3], f[4], f[5], en);
     }
     if (diag) return;
-    const int jl = jbase + lane;
+    const int jl = jbase + lane, kl = j0 + lane;
     if (jl >= P.n) return;
-    const EAtom<R> mine = eatom<R>(sp[lane], sd[lane], su[lane]);
-    R dummy = 0;
+    const EAtom<double> mine = T.atom(kl);
+    double dummy = 0;
 #pragma unroll 1
     for (int e = exc_off[jl]; e < exc_off[jl + 1]; e++) {
         const int a = exc_j[e];
         if ((unsigned)(a - ibase) >= 32u) continue;
-        const R mS = (R)exc_m[e], iS = (R)exc_s[e];
-        if (mS == R(0) && iS == R(0)) continue;
-        const V4 pa = posq[a];
-        const EAtom<R> A = eatom<R>(pa, dipt[a], indv[a]);
-        R ox, oy, oz;
-        shift_into<R>(geo, cA, cB, pa.x, pa.y, pa.z, ox, oy, oz);
-        R dx, dy, dz;  // p_jl - p_a: a (tile I < J) is the lower index
-        pair_delta<R, FOLD>(P, pos, a, jl, sp[lane].x, sp[lane].y, sp[lane].z, ox, oy, oz, dx, dy, dz);
-        const R r2 = dx * dx + dy * dy + dz * dz;
-        const bool yzd = yz_differ<R>(dy, dz, yz, a, jl, nmax);
-        pair_energy<R, false>(dx, dy, dz, r2, yzd, A, mine, mS, iS, damp_r2, rv4p, rv4f, P.mutual != 0, g[0], g[1],
-                              g[2], g[3], g[4], g[5], dummy);
+        const double mS = exc_m[e], iS = exc_s[e];
+        if (mS == 0.0 && iS == 0.0) continue;
+        const double4 pa = posq[a];
+        const EAtom<double> A = eatom<double>(pa, dipt[a], indv[a]);
+        double ox, oy, oz;
+        shift_into(geo, cA, cB, pa.x, pa.y, pa.z, ox, oy, oz);
+        double dx, dy, dz;  // p_jl - p_a: a (tile I < J) is the lower index
+        pair_delta<FOLD>(P, geo.fmask, T.xy[kl].x, T.xy[kl].y, T.zq[kl].x, ox, oy, oz, dx, dy, dz);
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        const bool yzd = yz_differ<double>(dy, dz, yz, a, jl, nmax);
+        pair_energy<double, false>(dx, dy, dz, r2, yzd, A, mine, mS, iS, damp_r2, rv4p, rv4f, P.mutual != 0, g[0],
+                                   g[1], g[2], g[3], g[4], g[5], dummy);
     }
 }
 
-template <class R>
+// Plain form: one CTA per band pair, one warp per I tile at a time (one to four
+// warps).  Bound by the FP64 chain (135 operations a pair, the pipe 54 % busy
+// with 12 warps an SM).  Warps without a tile in narrow bands are not launched,
+// the records lie in conflict-free pieces, and the pairs beyond the damping
+// range take pair_energy_lab: 81 -> 59 us at 1,029 atoms, 427 -> 220 at 3,993,
+// 1205 -> 1130 at 12,288.
 __global__ void __launch_bounds__(kSymThreads, 3) k_energy_sym(
-    PairParams P, const typename Vec4T<R>::type* __restrict__ posq, const typename Vec4T<R>::type* __restrict__ dipt,
-    const typename Vec4T<R>::type* __restrict__ indv, const double2* __restrict__ yz, const double4* __restrict__ tctr,
+    PairParams P, const double4* __restrict__ posq, const double4* __restrict__ dipt,
+    const double4* __restrict__ indv, const double2* __restrict__ yz, const double4* __restrict__ tctr,
     const double4* __restrict__ text, const double* __restrict__ pos, const int* __restrict__ exc_off,
     const int* __restrict__ exc_j, const double* __restrict__ exc_m, const double* __restrict__ exc_s,
     const int2* __restrict__ exc_tiles, int n_pad, double* __restrict__ partial, double* __restrict__ energy_partial) {
-    typedef typename Vec4T<R>::type V4;
     extern __shared__ __align__(16) unsigned char smem[];
     const int BT = P.band_tiles, NA = BT * 32;
     double* s_acc = reinterpret_cast<double*>(smem);              // 6 * NA: J-side sums of band q
-    double* s_iacc = s_acc + 6 * NA;                               // 7 * kSymThreads: I-side sums and energy
-    double4* s_ctr = reinterpret_cast<double4*>(s_iacc + 7 * kSymThreads);
+    double* s_iacc = s_acc + 6 * NA;                               // 7 * threads: I-side sums and energy
+    double4* s_ctr = reinterpret_cast<double4*>(s_iacc + 7 * blockDim.x);
     double4* s_ext = s_ctr + BT;
-    V4* s_pos = reinterpret_cast<V4*>(s_ext + BT);
-    V4* s_dip = s_pos + NA;
-    V4* s_ind = s_dip + NA;
+    const ERec64 T(reinterpret_cast<double2*>(s_ext + BT), NA);
 
     int p, q;
     band_pair(blockIdx.x, p, q);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int qa0 = q * NA;
-    for (int k = threadIdx.x; k < NA; k += kSymThreads) {
-        s_pos[k] = posq[qa0 + k];
-        s_dip[k] = dipt[qa0 + k];
-        s_ind[k] = indv[qa0 + k];
-        for (int c = 0; c < 6; c++) s_acc[6 * k + c] = 0.0;
+    for (int k = threadIdx.x; k < NA; k += blockDim.x) {
+        const double4 a = posq[qa0 + k], b = dipt[qa0 + k], u = indv[qa0 + k];
+        T.xy[k] = make_double2(a.x, a.y);
+        T.zq[k] = make_double2(a.z, a.w);
+        T.mm[k] = make_double2(b.x, b.y);
+        T.mu[k] = make_double2(b.z, u.x);
+        T.uu[k] = make_double2(u.y, u.z);
+        T.t[k] = b.w;
+        for (int c = 0; c < 6; c++) s_acc[c * NA + k] = 0.0;
     }
-    for (int k = threadIdx.x; k < BT; k += kSymThreads) {
+    for (int k = threadIdx.x; k < BT; k += blockDim.x) {
         s_ctr[k] = tctr[q * BT + k];
         s_ext[k] = text[q * BT + k];
     }
@@ -1954,17 +1943,15 @@ __global__ void __launch_bounds__(kSymThreads, 3) k_energy_sym(
     my[6] = 0.0;
     __syncthreads();
 
-    const R damp_r2 = (R)P.damp_r2;
-    const R rv4p = (R)P.rinv4_power, rv4f = (R)P.rinv4_fill;
-    const int stride = BT >= kSymWarps ? BT / kSymWarps : 1;
-    const int rounds = (BT + kSymWarps - 1) / kSymWarps;
+    const int stride = BT / warps;
+    const int rounds = (BT + warps - 1) / warps;
     for (int r = 0; r < rounds; r++) {
-        const int Il = warp + kSymWarps * r;
+        const int Il = warp + warps * r;
         const int I = p * BT + Il;
         const bool wact = Il < BT && I < P.n_tiles;
         const int ibase = I * 32;
         const int i = ibase + lane;
-        V4 pi = {}, di = {}, ui = {};
+        double4 pi = {}, di = {}, ui = {};
         double4 cA = {}, eA = {};
         int2 et = make_int2(1 << 30, -1);
         int e0 = 0, e1 = 0;
@@ -1980,7 +1967,7 @@ __global__ void __launch_bounds__(kSymThreads, 3) k_energy_sym(
                 e1 = exc_off[i + 1];
             }
         }
-        const EAtom<R> me = eatom<R>(pi, di, ui);
+        const EAtom<double> me = eatom<double>(pi, di, ui);
         for (int c = 0; c < 6; c++) my[c] = 0.0;
         for (int t = 0; t < BT; t++) {
             const int Jl = (t + warp * stride) % BT;
@@ -1990,48 +1977,40 @@ __global__ void __launch_bounds__(kSymThreads, 3) k_energy_sym(
                 const bool diag = I == J;
                 const bool slow = diag || (J == P.n_tiles - 1 && (P.n & 31)) || (J >= et.x && J <= et.y);
                 const TileGeom g = tile_geom(P, (double)P.damp_r2, cA, eA, cB, s_ext[Jl]);
-                R oix, oiy, oiz;
-                shift_into<R>(g, cA, cB, pi.x, pi.y, pi.z, oix, oiy, oiz);
-                const int jbase = J * 32;
-                const V4* sp = s_pos + Jl * 32;
-                const V4* sd = s_dip + Jl * 32;
-                const V4* su = s_ind + Jl * 32;
+                double oix, oiy, oiz;
+                shift_into(g, cA, cB, pi.x, pi.y, pi.z, oix, oiy, oiz);
+                const int jbase = J * 32, j0 = Jl * 32;
                 const unsigned partners = slow ? partner_bits(exc_j, e0, e1, jbase) : 0u;
-                R f[6] = {0, 0, 0, 0, 0, 0}, gg[6] = {0, 0, 0, 0, 0, 0}, en = 0;
+                double f[6] = {0, 0, 0, 0, 0, 0}, gg[6] = {0, 0, 0, 0, 0, 0}, en = 0;
+#define TDP_EWALK64(F, S, L) \
+    energy_walk<F, S, L>(P, yz, T, j0, lane, i, jbase, oix, oiy, oiz, me, diag, partners, g.fmask, f, gg, en)
+#define TDP_EPARTNERS64(F)                                                                                       \
+    energy_partners<F>(P, yz, posq, dipt, indv, T, j0, exc_off, exc_j, exc_m, exc_s, g, cA, cB, lane, i, ibase, \
+                       jbase, e0, e1, oix, oiy, oiz, me, diag, f, gg, en)
                 if (slow) {
                     if (g.fold) {
-                        energy_walk<R, true, true>(P, pos, yz, sp, sd, su, lane, i, jbase, oix, oiy, oiz, me, diag,
-                                                   partners, damp_r2, rv4p, rv4f, f, gg, en);
-                        energy_partners<R, true>(P, pos, yz, posq, dipt, indv, sp, sd, su, exc_off, exc_j, exc_m,
-                                                 exc_s, g, cA, cB, lane, i, ibase, jbase, e0, e1, oix, oiy, oiz, me,
-                                                 diag, damp_r2, rv4p, rv4f, f, gg, en);
+                        TDP_EWALK64(true, true, false);
+                        TDP_EPARTNERS64(true);
                     } else {
-                        energy_walk<R, false, true>(P, pos, yz, sp, sd, su, lane, i, jbase, oix, oiy, oiz, me, diag,
-                                                    partners, damp_r2, rv4p, rv4f, f, gg, en);
-                        energy_partners<R, false>(P, pos, yz, posq, dipt, indv, sp, sd, su, exc_off, exc_j, exc_m,
-                                                  exc_s, g, cA, cB, lane, i, ibase, jbase, e0, e1, oix, oiy, oiz, me,
-                                                  diag, damp_r2, rv4p, rv4f, f, gg, en);
+                        TDP_EWALK64(false, true, false);
+                        TDP_EPARTNERS64(false);
                     }
                 } else if (!g.near && P.lab_energy) {
-                    if (g.fold)
-                        energy_walk<R, true, false, true>(P, pos, yz, sp, sd, su, lane, i, jbase, oix, oiy, oiz, me,
-                                                          diag, partners, damp_r2, rv4p, rv4f, f, gg, en);
-                    else
-                        energy_walk<R, false, false, true>(P, pos, yz, sp, sd, su, lane, i, jbase, oix, oiy, oiz, me,
-                                                           diag, partners, damp_r2, rv4p, rv4f, f, gg, en);
+                    if (g.fold) TDP_EWALK64(true, false, true);
+                    else TDP_EWALK64(false, false, true);
                 } else if (g.fold) {
-                    energy_walk<R, true, false>(P, pos, yz, sp, sd, su, lane, i, jbase, oix, oiy, oiz, me, diag,
-                                                partners, damp_r2, rv4p, rv4f, f, gg, en);
+                    TDP_EWALK64(true, false, false);
                 } else {
-                    energy_walk<R, false, false>(P, pos, yz, sp, sd, su, lane, i, jbase, oix, oiy, oiz, me, diag,
-                                                 partners, damp_r2, rv4p, rv4f, f, gg, en);
+                    TDP_EWALK64(false, false, false);
                 }
-                double* acc = s_acc + 6 * (Jl * 32 + lane);
+#undef TDP_EWALK64
+#undef TDP_EPARTNERS64
+                double* acc = s_acc + Jl * 32 + lane;
                 for (int c = 0; c < 6; c++) {
-                    acc[c] += (double)gg[c];
-                    my[c] += (double)f[c];
+                    acc[c * NA] += gg[c];
+                    my[c] += f[c];
                 }
-                my[6] += (double)en;
+                my[6] += en;
             }
             // Within a window of `stride` steps the warps' J tiles are
             // disjoint ((t + warp * stride) % BT), so the shared J-side sums
@@ -2041,8 +2020,8 @@ __global__ void __launch_bounds__(kSymThreads, 3) k_energy_sym(
         }
         if (wact) {
             if (p == q) {
-                double* acc = s_acc + 6 * (Il * 32 + lane);
-                for (int c = 0; c < 6; c++) acc[c] += my[c];
+                double* acc = s_acc + Il * 32 + lane;
+                for (int c = 0; c < 6; c++) acc[c * NA] += my[c];
             } else {
                 const size_t b = (size_t)q * 6 * n_pad;
                 for (int c = 0; c < 6; c++) partial[b + (size_t)c * n_pad + i] = my[c];
@@ -2051,8 +2030,8 @@ __global__ void __launch_bounds__(kSymThreads, 3) k_energy_sym(
         __syncthreads();
     }
     const size_t b = (size_t)p * 6 * n_pad;
-    for (int k = threadIdx.x; k < NA; k += kSymThreads)
-        for (int c = 0; c < 6; c++) partial[b + (size_t)c * n_pad + qa0 + k] = s_acc[6 * k + c];
+    for (int k = threadIdx.x; k < NA; k += blockDim.x)
+        for (int c = 0; c < 6; c++) partial[b + (size_t)c * n_pad + qa0 + k] = s_acc[c * NA + k];
     // CTA energy, summed in thread order (padding atoms contribute exactly 0).
     double e = warp_sum(my[6]);
     __shared__ double s_red[kSymWarps];
@@ -2060,7 +2039,7 @@ __global__ void __launch_bounds__(kSymThreads, 3) k_energy_sym(
     __syncthreads();
     if (threadIdx.x == 0) {
         double s = 0.0;
-        for (int w = 0; w < kSymWarps; w++) s += s_red[w];
+        for (int w = 0; w < warps; w++) s += s_red[w];
         energy_partial[blockIdx.x] = s;
     }
 }
@@ -2069,11 +2048,9 @@ size_t field_smem(int BT) {
     return (size_t)32 * BT * (4 * sizeof(double2) + (1 + 3 * (BT / 2)) * sizeof(double)) + BT * BT * sizeof(double4);
 }
 
-template <class R>
 size_t energy_smem(int BT) {
     const int NA = 32 * BT;
-    return sizeof(double) * (6 * NA + 7 * kSymThreads) + sizeof(double4) * 2 * BT +
-           sizeof(typename Vec4T<R>::type) * 3 * NA;
+    return sizeof(double) * (7 * NA + 7 * kSymThreads) + sizeof(double4) * 2 * BT + sizeof(double2) * 5 * NA;
 }
 
 int band_pairs(const Dev& d) { return d.pp.n_bands * (d.pp.n_bands + 1) / 2; }
@@ -2181,9 +2158,9 @@ void launch_energy<float>(const Dev& d, cudaStream_t st) {
 
 template <>
 void launch_energy<double>(const Dev& d, cudaStream_t st) {
-    const size_t smem = energy_smem<double>(d.pp.band_tiles);
-    cudaFuncSetAttribute(k_energy_sym<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_energy_sym<double><<<band_pairs(d), kSymThreads, smem, st>>>(
+    const size_t smem = energy_smem(d.pp.band_tiles);
+    cudaFuncSetAttribute(k_energy_sym, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_energy_sym<<<band_pairs(d), 32 * std::min(kSymWarps, d.pp.band_tiles), smem, st>>>(
         d.pp, (const double4*)d.posq, (const double4*)d.dipt, (const double4*)d.ind, d.yz, d.tctr, d.text, d.pos,
         d.exc_off, d.exc_j, d.exc_m, d.exc_s, d.exc_tiles, d.n_pad, d.partial, d.energy_partial);
     slot_sum(d, 6, st);
