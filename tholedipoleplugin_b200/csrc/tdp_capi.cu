@@ -35,6 +35,8 @@ thread_local std::string g_create_error;
 
 }  // namespace
 
+constexpr int kEpsRing = 8;
+
 struct tdp_handle {
     int n = 0;
     int method = TDP_NO_CUTOFF;
@@ -68,6 +70,7 @@ struct tdp_handle {
     std::vector<void*> owned;
     cudaStream_t stream = nullptr;
     double* h_scal = nullptr;   // pinned scalar readback
+    double* h_eps = nullptr;    // pinned ring of kEpsRing epsilons, written by the cluster CG kernels
     int* h_fixerr = nullptr;    // pinned copy of the accumulator range flag
     double* h_forces = nullptr; // pinned n*3
     double* d_stage = nullptr;  // device staging for host FP32 positions / query inputs
@@ -450,6 +453,27 @@ double read_scalar(tdp_handle* h, const double* dptr) {
     return *h->h_scal;
 }
 
+// Epsilon `slot`, which a kernel already launched writes to pinned memory:
+// clear_eps() before that launch, wait_eps() after it.  The host sees it some
+// microseconds before a copy and a stream synchronisation would have returned.
+constexpr uint64_t kNoEps = 0xfff8d1e5a11f0001ull;   // a NaN that no arithmetic makes
+double* eps_word(tdp_handle* h, int slot) { return h->h_eps + slot % kEpsRing; }
+void clear_eps(tdp_handle* h, int slot) { std::memcpy(eps_word(h, slot), &kNoEps, sizeof kNoEps); }
+double wait_eps(tdp_handle* h, int slot) {
+    const volatile uint64_t* w = reinterpret_cast<const volatile uint64_t*>(eps_word(h, slot));
+    for (long spin = 1; *w == kNoEps; spin++) {
+        if (spin % 4096) continue;
+        const cudaError_t e = cudaStreamQuery(h->stream);
+        if (e == cudaErrorNotReady) continue;
+        TDP_CUDA(e);
+        if (*w == kNoEps) return read_scalar(h, h->d.scal_eps + slot);   // the stream is empty
+    }
+    const uint64_t bits = *w;
+    double eps;
+    std::memcpy(&eps, &bits, sizeof eps);
+    return eps;
+}
+
 void record(tdp_handle* h, int k) {
     if (h->timing) TDP_CUDA(cudaEventRecord(h->ev[k], h->stream));
 }
@@ -530,35 +554,74 @@ void solve_cg(tdp_handle* h, bool fused = false, bool cold = true) {
     }
     const int cap = h->max_iter;
     int slot = 0;
+    // Up to 16,384 atoms the O(N) work of an iteration is one launch by one
+    // cluster, and the epsilon reaches the host through pinned memory.  Where
+    // the matvec is so short that its parts are split (field_parts), the next
+    // iteration is queued before the host has seen the epsilon; its kernels do
+    // nothing if that shows the solve has stopped.  (Not while the stages are
+    // timed.)
+    const bool one = cg_cluster(d), collect = one && !h->ew && sizeof(R) == 4;
+    const bool ahead = one && !h->ew && d.field_parts > 1 && !h->timing;
+    // The residual of y in scalar slot `slot` (use_partial: of a matvec).
+    const auto start = [&](bool use_partial) {
+        if (one) {
+            clear_eps(h, slot);
+            launch_cg_start<R>(d, slot, use_partial, eps_word(h, slot), st);
+            h->launches += 1;
+            return wait_eps(h, slot);
+        }
+        launch_cg_residual<R>(d, st, use_partial);
+        launch_cg_p<R>(d, -1, slot, st);
+        h->launches += 2;
+        return read_scalar(h, d.scal_eps + slot);
+    };
+    // Queues the iteration from slot `from`; conditional: only if that has not stopped.
+    const auto queue = [&](int from, bool conditional) {
+        const double* stop = conditional ? d.scal_eps + from : nullptr;
+        if (!one) {
+            matvec<R>(h);
+            launch_cg_q(d, st);
+            launch_cg_update(d, from, st);
+            launch_cg_p<R>(d, from, from + 1, st);
+            h->launches += 3;
+            return;
+        }
+        clear_eps(h, from + 1);
+        if (h->ew) {
+            matvec<R>(h);
+        } else {
+            size_t k = kernel_begin(h, 0);
+            launch_cg_matvec<R>(d, stop, h->target_eps, st);
+            kernel_end(h, k);
+            h->launches++;
+            if (!conditional) h->matvecs++;
+        }
+        launch_cg_step<R>(d, from, collect, stop, h->target_eps, eps_word(h, from + 1), st);
+        h->launches++;
+    };
     // Residual of the starting point (mu = alpha E, or the previous solution).
-    if (fused) {
-        launch_cg_residual<R>(d, st, false);
-    } else {
-        matvec<R>(h);
-        launch_cg_residual<R>(d, st);
-    }
-    launch_cg_p<R>(d, -1, slot, st);
-    h->launches += 2;
-    double eps = read_scalar(h, d.scal_eps + slot);
+    if (!fused) matvec<R>(h);
+    double eps = start(!fused);
     double eps_sum = eps;   // residual norms stepped through since the last true residual
-    bool is_true = true;
+    bool is_true = true, queued = false;
     int it = 0;
     h->status = TDP_STATUS_MAX_ITERATIONS;
+    const auto may_step = [&](int done, int at) { return done < cap && (size_t)at + 3 < h->nscal; };
     while (true) {
         if (!std::isfinite(eps)) {
             h->status = TDP_STATUS_NON_FINITE;
             break;
         }
-        if (eps <= h->target_eps || it >= cap || (size_t)slot + 3 >= h->nscal) {
+        if (eps <= h->target_eps || !may_step(it, slot)) {
+            queued = false;   // what was queued does nothing
             const bool drift_ok = eps <= h->target_eps && !h->always_true_residual &&
                                   kDriftPerStep * eps_sum <= h->target_eps - eps;
             if (!is_true && !drift_ok) {
                 launch_cg_mu<R>(d, st, fused ? d.mu0 : nullptr);
+                h->launches += 1;
                 matvec<R>(h);
-                launch_cg_residual<R>(d, st);
-                launch_cg_p<R>(d, -1, ++slot, st);
-                h->launches += 3;
-                eps = read_scalar(h, d.scal_eps + slot);
+                ++slot;
+                eps = start(true);
                 eps_sum = eps;
                 is_true = true;
                 continue;
@@ -566,14 +629,13 @@ void solve_cg(tdp_handle* h, bool fused = false, bool cold = true) {
             if (eps <= h->target_eps) h->status = TDP_STATUS_CONVERGED;
             break;
         }
-        matvec<R>(h);
-        launch_cg_q(d, st);
-        launch_cg_update(d, slot, st);
-        launch_cg_p<R>(d, slot, slot + 1, st);
-        h->launches += 3;
+        if (!queued) queue(slot, false);
+        else h->matvecs++;
         slot++;
         it++;
-        eps = read_scalar(h, d.scal_eps + slot);
+        queued = ahead && may_step(it, slot);
+        if (queued) queue(slot, true);
+        eps = one ? wait_eps(h, slot) : read_scalar(h, d.scal_eps + slot);
         eps_sum += eps;
         is_true = false;
     }
@@ -1379,6 +1441,7 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
             h->pre = precond_create(d, h->precision, rc, 1e-3, inner);
         }
         TDP_CUDA(cudaMallocHost(&h->h_scal, 64 * sizeof(double)));
+        TDP_CUDA(cudaMallocHost(&h->h_eps, kEpsRing * sizeof(double)));
         TDP_CUDA(cudaMallocHost(&h->h_fixerr, sizeof(int)));
         *h->h_fixerr = 0;
         TDP_CUDA(cudaMallocHost(&h->h_forces, std::max<size_t>(n3, 1) * sizeof(double)));
@@ -1405,6 +1468,7 @@ void tdp_destroy(tdp_handle* h) {
     if (h->pre) precond_destroy(h->pre);
     for (void* p : h->owned) cudaFree(p);
     if (h->h_scal) cudaFreeHost(h->h_scal);
+    if (h->h_eps) cudaFreeHost(h->h_eps);
     if (h->h_fixerr) cudaFreeHost(h->h_fixerr);
     if (h->h_forces) cudaFreeHost(h->h_forces);
     for (int k = 0; k < 6; k++)

@@ -124,6 +124,20 @@ template <class R> void launch_cg_residual(const Dev& d, cudaStream_t st, bool u
 template <class R> void launch_pack_total(const Dev& d, cudaStream_t st);
 template <class R> void launch_fused_done(const Dev& d, cudaStream_t st);
 void launch_cg_q(const Dev& d, cudaStream_t st);
+// One CG iteration in two launches for systems that fit a cluster (cg_cluster):
+// the matvec, and everything after it.  stop_eps (may be null): the launches do
+// nothing where *stop_eps shows that the solve has stopped.  host_eps: pinned
+// word that receives the new epsilon.  collect: the all-pairs matvec was
+// launch_cg_matvec.
+bool cg_cluster(const Dev& d);
+template <class R>
+void launch_cg_start(const Dev& d, int slot, bool use_partial, double* host_eps, cudaStream_t st);
+template <class R> void launch_cg_matvec(const Dev& d, const double* stop_eps, double target, cudaStream_t st);
+template <> void launch_cg_matvec<float>(const Dev& d, const double* stop_eps, double target, cudaStream_t st);
+template <> void launch_cg_matvec<double>(const Dev& d, const double* stop_eps, double target, cudaStream_t st);
+template <class R>
+void launch_cg_step(const Dev& d, int slot, bool collect, const double* stop_eps, double target, double* host_eps,
+                    cudaStream_t st);
 void launch_cg_update(const Dev& d, int slot, cudaStream_t st);
 template <class R> void launch_cg_p(const Dev& d, int prev, int slot, cudaStream_t st);
 // mu0 != NULL: the packed operand is mu - mu0 (the final check of a fused start).

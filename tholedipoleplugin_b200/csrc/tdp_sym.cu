@@ -41,9 +41,12 @@
 #include "tdp_kernels.cuh"
 #include "tdp_pairs.cuh"
 
+#include <cooperative_groups.h>
 #include <math.h>
 
 #include <algorithm>
+
+namespace cg = cooperative_groups;
 
 namespace tdp {
 
@@ -170,6 +173,28 @@ __device__ __forceinline__ unsigned partner_bits(const int* __restrict__ exc_j, 
         if (off < 32u) b |= 1u << off;
     }
     return b;
+}
+
+// Whether the solve had stopped before this launch, which was queued before
+// the host knew: eps (may be null) at or below the target, or not finite.
+struct CgStop {
+    const double* eps;
+    double target;
+    __device__ __forceinline__ bool stopped() const {
+        if (!eps) return false;
+        const double e = *eps;
+        return !(e > target && e < (double)INFINITY);
+    }
+};
+
+template <class R>
+__device__ __forceinline__ void store_operand(typename Vec4T<R>::type* v, int k, d3 a, double t) {
+    typename Vec4T<R>::type o;
+    o.x = (R)a.x;
+    o.y = (R)a.y;
+    o.z = (R)a.z;
+    o.w = (R)t;
+    v[k] = o;
 }
 
 // 64-bit fixed-point accumulator of the mixed form (Dev::fixacc).
@@ -508,7 +533,8 @@ __global__ void __launch_bounds__(32, 16) k_field_items(
     PairParams P, int L, const float4* __restrict__ posq, const float4* __restrict__ jvec,
     const double4* __restrict__ tctr, const double4* __restrict__ text, const double* __restrict__ pos,
     const int* __restrict__ exc_off, const int* __restrict__ exc_j, const double* __restrict__ exc_scale,
-    const int2* __restrict__ exc_tiles, int n_pad, FixAcc fix) {
+    const int2* __restrict__ exc_tiles, int n_pad, FixAcc fix, CgStop stop) {
+    if (stop.stopped()) return;
     __shared__ FPackedTile T;
     __shared__ double s_my[3 * NS][32];   // I-side sums
     const int lane = threadIdx.x;
@@ -862,6 +888,180 @@ __global__ void __launch_bounds__(96)
 #pragma unroll 8
     for (int j = 0; j < nslot; j++) s += out[j * count];
     *out = s + s_part[0][c][lane] + s_part[1][c][lane] + s_part[2][c][lane];
+}
+
+// ---------------------------------------------------------------------------
+// One CG iteration after its matvec, in one launch: a cluster of eight CTAs
+// holds every atom's p, r and q in registers between the two scalar products,
+// which cross it through distributed shared memory in a fixed order.  Bound by
+// latency (launch, two cluster barriers, a chain of loads), as the four
+// launches before it were (sums, q, update, p: 4.4 + 4.2 + 5.3 + 5.1 us at 648
+// atoms, 6.1 + 4.7 + 5.3 + 4.9 at 12,288, and a gap after each).  With the
+// epsilon through pinned memory and the next iteration queued ahead, an
+// evaluation went from 436 to 295 us at 648 atoms (mixed), 555 to 474 at 1,029
+// and 5111 to 5033 at 12,288 (FP64), 2369 to 2267 at 12,288 (mixed).
+// ---------------------------------------------------------------------------
+constexpr int kCgCtas = 8, kCgThreads = 512, kCgCap = kCgCtas * kCgThreads;
+
+// The sum over the cluster of a and b, the same in every thread.  buf: two
+// doubles per warp and two for the CTA, used once per launch.
+__device__ __forceinline__ void cluster_sum2(cg::cluster_group& cl, double& a, double& b, double (&buf)[2][17]) {
+    a = warp_sum(a);
+    b = warp_sum(b);
+    const int w = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) {
+        buf[0][w] = a;
+        buf[1][w] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double t = 0.0;
+        for (int k = 0; k < kCgThreads / 32; k++) t += buf[threadIdx.x][k];
+        buf[threadIdx.x][16] = t;
+    }
+    cl.sync();
+    a = b = 0.0;
+#pragma unroll
+    for (int c = 0; c < kCgCtas; c++) {
+        a += *cl.map_shared_rank(&buf[0][16], c);
+        b += *cl.map_shared_rank(&buf[1][16], c);
+    }
+}
+
+struct CgArrays {
+    const int* order;
+    const double *partial, *salpha, *thole, *E;
+    double *y, *r, *p, *scal_rr, *scal_eps, *host_eps;
+    unsigned long long* acc;   // mixed form: the matvec's fixed-point sums, else null
+    double inv_scale;
+    int n, n_pad, slot;        // reads scal[slot], writes scal[slot + 1]
+    CgStop stop;
+};
+
+// q = p - S T S p, a = r.r / p.q, y += a p, r -= a q, p = r + (r'.r' / r.r) p and
+// the next operand S p.  DONE: the matvec's sums still lie in the fixed-point
+// accumulator, and the thread of slot k also evaluates its partner pairs, as
+// k_field_done does.
+template <class R, bool DONE, int M>
+__global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads)
+    k_cg_step(PairParams P, CgArrays A, const typename Vec4T<R>::type* __restrict__ posq,
+              typename Vec4T<R>::type* vec, const double* __restrict__ pos, const int* __restrict__ exc_off,
+              const int* __restrict__ exc_j, const double* __restrict__ exc_m, const double* __restrict__ exc_s) {
+    __shared__ double buf[2][2][17];
+    cg::cluster_group cl = cg::this_cluster();
+    const int k0 = blockIdx.x * kCgThreads + threadIdx.x;
+    const bool stopped = A.stop.stopped();
+    d3 t[M], p[M], r[M];
+    double s[M], pq = 0.0, zero = 0.0;
+    int id[M];
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        const int k = k0 + m * kCgCap;
+        id[m] = -1;
+        double f[3] = {0.0, 0.0, 0.0};
+        if (DONE) {
+            if (k < A.n_pad)
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    f[c] = (double)(long long)A.acc[(size_t)c * A.n_pad + k] * A.inv_scale;
+                    A.acc[(size_t)c * A.n_pad + k] = 0ull;
+                }
+        }
+        if (k >= A.n || stopped) continue;
+        const int i = id[m] = A.order[k];
+        if (DONE) {
+            const double ti = (double)vec[k].w;
+            for (int e = exc_off[k]; e < exc_off[k + 1]; e++)
+                add_partner<1>(P, 0, posq, (const typename Vec4T<R>::type*)vec, (const typename Vec4T<R>::type*)nullptr,
+                               pos, exc_j, exc_m, exc_s, k, e, ti, f);
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; c++) f[c] = A.partial[(size_t)c * A.n_pad + k];
+        }
+        s[m] = A.salpha[i];
+        p[m] = ld3(A.p + 3 * (size_t)i);
+        r[m] = ld3(A.r + 3 * (size_t)i);
+        t[m] = p[m] - d3{f[0], f[1], f[2]} * s[m];   // q
+        pq += dot(p[m], t[m]);
+    }
+    if (stopped) return;   // the same in every CTA
+    cluster_sum2(cl, pq, zero, buf[0]);
+    const double rr = A.scal_rr[A.slot], a = rr / pq;
+    double rn = 0.0, en = 0.0;
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        if (id[m] < 0) continue;
+        double* y = A.y + 3 * (size_t)id[m];
+        const d3 yv = ld3(y) + p[m] * a;
+        y[0] = yv.x;
+        y[1] = yv.y;
+        y[2] = yv.z;
+        r[m] = r[m] - t[m] * a;
+        double* ro = A.r + 3 * (size_t)id[m];
+        ro[0] = r[m].x;
+        ro[1] = r[m].y;
+        ro[2] = r[m].z;
+        const double v = dot(r[m], r[m]);
+        rn += v;
+        en += s[m] * s[m] * v;
+    }
+    cluster_sum2(cl, rn, en, buf[1]);
+    if (k0 == 0) {
+        const double eps = sqrt(en / (double)A.n);
+        A.scal_rr[A.slot + 1] = rn;
+        A.scal_eps[A.slot + 1] = eps;
+        *(volatile double*)A.host_eps = eps;
+    }
+    const double beta = rn / rr;
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        if (id[m] < 0) continue;
+        const int i = id[m];
+        const d3 pv = r[m] + p[m] * beta;
+        double* po = A.p + 3 * (size_t)i;
+        po[0] = pv.x;
+        po[1] = pv.y;
+        po[2] = pv.z;
+        store_operand<R>(vec, k0 + m * kCgCap, pv * s[m], A.thole[i]);
+    }
+    cl.sync();   // no CTA leaves while another reads its sums
+}
+
+// The residual of y: r = p = S (E + T mu) - y (use_partial 0: E holds the field
+// already), the operand S p and the scalars of `slot`.
+template <class R, int M>
+__global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads)
+    k_cg_start(CgArrays A, typename Vec4T<R>::type* __restrict__ vec, int use_partial) {
+    __shared__ double buf[2][17];
+    cg::cluster_group cl = cg::this_cluster();
+    const int k0 = blockIdx.x * kCgThreads + threadIdx.x;
+    double rr = 0.0, ee = 0.0;
+#pragma unroll
+    for (int m = 0; m < M; m++) {
+        const int k = k0 + m * kCgCap;
+        if (k >= A.n) continue;
+        const int i = A.order[k];
+        d3 e = ld3(A.E + 3 * (size_t)i);
+        if (use_partial) e = e + d3{A.partial[k], A.partial[A.n_pad + k], A.partial[2 * (size_t)A.n_pad + k]};
+        const double s = A.salpha[i];
+        const d3 rv = e * s - ld3(A.y + 3 * (size_t)i);
+        double *r = A.r + 3 * (size_t)i, *p = A.p + 3 * (size_t)i;
+        r[0] = p[0] = rv.x;
+        r[1] = p[1] = rv.y;
+        r[2] = p[2] = rv.z;
+        store_operand<R>(vec, k, rv * s, A.thole[i]);
+        const double v = dot(rv, rv);
+        rr += v;
+        ee += s * s * v;
+    }
+    cluster_sum2(cl, rr, ee, buf);
+    if (k0 == 0) {
+        const double eps = sqrt(ee / (double)A.n);
+        A.scal_rr[A.slot] = rr;
+        A.scal_eps[A.slot] = eps;
+        *(volatile double*)A.host_eps = eps;
+    }
+    cl.sync();
 }
 
 // ---------------------------------------------------------------------------
@@ -2092,12 +2292,12 @@ void launch_field<float>(const Dev& d, int kind, cudaStream_t st) {
     const unsigned blocks = (unsigned)((d.n_pad + 127) / 128);
     if (kind == 1) {
         k_field_items<1, kFieldNS><<<grid, 32, 0, st>>>(d.pp, L, pq, op, d.tctr_s, d.text_s, d.pos_s, d.exs_off,
-                                                        d.exs_j, d.exs_s, d.exs_tiles, d.n_pad, fix_of(d));
+                                                        d.exs_j, d.exs_s, d.exs_tiles, d.n_pad, fix_of(d), CgStop{nullptr, 0.0});
         k_field_done<1><<<blocks, 128, 0, st>>>(d.pp, 0, pq, op, nullptr, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
                                                 d.exs_s, d.n_pad, d.fixacc, 1.0 / d.fix_scale, d.partial);
     } else {
         k_field_items<0, kFieldNS><<<grid, 32, 0, st>>>(d.pp, L, pq, op, d.tctr_s, d.text_s, d.pos_s, d.exs_off,
-                                                        d.exs_j, d.exs_m, d.exs_tiles, d.n_pad, fix_of(d));
+                                                        d.exs_j, d.exs_m, d.exs_tiles, d.n_pad, fix_of(d), CgStop{nullptr, 0.0});
         k_field_done<0><<<blocks, 128, 0, st>>>(d.pp, kind == 2 ? 1 : 0, pq, op, (const float4*)d.dipt_s, d.pos_s,
                                                 d.exs_off, d.exs_j, d.exs_m, d.exs_s, d.n_pad, d.fixacc,
                                                 1.0 / d.fix_scale, d.partial);
@@ -2125,6 +2325,87 @@ void launch_field<double>(const Dev& d, int kind, cudaStream_t st) {
                                                       nb * d.field_parts, d.partial);
     }
 }
+
+// The cluster form of the CG kernels holds up to four atoms a thread.
+bool cg_cluster(const Dev& d) { return d.n <= 4 * kCgCap; }
+
+namespace {
+
+CgArrays cg_arrays(const Dev& d, int slot, double* host_eps) {
+    CgArrays A{};
+    A.order = d.order;
+    A.partial = d.partial;
+    A.salpha = d.salpha;
+    A.thole = d.thole;
+    A.E = d.E;
+    A.y = d.y;
+    A.r = d.r;
+    A.p = d.p;
+    A.scal_rr = d.scal_rr;
+    A.scal_eps = d.scal_eps;
+    A.host_eps = host_eps;
+    A.n = d.n;
+    A.n_pad = d.n_pad;
+    A.slot = slot;
+    return A;
+}
+
+template <class R, bool DONE>
+void cg_step(const Dev& d, const CgArrays& A, cudaStream_t st) {
+    typedef typename Vec4T<R>::type V4;
+    const V4* pq = (const V4*)d.posq_s;
+    V4* vec = (V4*)d.vec_s;
+    const int m = (d.n + kCgCap - 1) / kCgCap;
+    if (m <= 1)
+        k_cg_step<R, DONE, 1><<<kCgCtas, kCgThreads, 0, st>>>(d.pp, A, pq, vec, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
+                                                              d.exs_s);
+    else if (m == 2)
+        k_cg_step<R, DONE, 2><<<kCgCtas, kCgThreads, 0, st>>>(d.pp, A, pq, vec, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
+                                                              d.exs_s);
+    else
+        k_cg_step<R, DONE, 4><<<kCgCtas, kCgThreads, 0, st>>>(d.pp, A, pq, vec, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
+                                                              d.exs_s);
+}
+
+}  // namespace
+
+template <class R>
+void launch_cg_start(const Dev& d, int slot, bool use_partial, double* host_eps, cudaStream_t st) {
+    const CgArrays A = cg_arrays(d, slot, host_eps);
+    k_cg_start<R, 4><<<kCgCtas, kCgThreads, 0, st>>>(A, (typename Vec4T<R>::type*)d.vec_s, use_partial ? 1 : 0);
+}
+template void launch_cg_start<float>(const Dev&, int, bool, double*, cudaStream_t);
+template void launch_cg_start<double>(const Dev&, int, bool, double*, cudaStream_t);
+
+// All-pairs matvec without the collection of its sums, which launch_cg_step does.
+template <>
+void launch_cg_matvec<float>(const Dev& d, const double* stop_eps, double target, cudaStream_t st) {
+    const int L = d.field_L, B = std::max(L, kFieldNS), nb = (d.pp.n_tiles + B - 1) / B;
+    const dim3 grid((unsigned)((long)nb * (nb + 1) / 2 * (B / std::min(L, kFieldNS))), d.field_parts);
+    k_field_items<1, kFieldNS><<<grid, 32, 0, st>>>(d.pp, L, (const float4*)d.posq_s, (const float4*)d.vec_s, d.tctr_s,
+                                                    d.text_s, d.pos_s, d.exs_off, d.exs_j, d.exs_s, d.exs_tiles,
+                                                    d.n_pad, fix_of(d), CgStop{stop_eps, target});
+}
+template <>
+void launch_cg_matvec<double>(const Dev& d, const double*, double, cudaStream_t st) {
+    launch_field<double>(d, 1, st);
+}
+
+template <class R>
+void launch_cg_step(const Dev& d, int slot, bool collect, const double* stop_eps, double target, double* host_eps,
+                    cudaStream_t st) {
+    CgArrays A = cg_arrays(d, slot, host_eps);
+    A.stop = CgStop{stop_eps, target};
+    if (sizeof(R) == 4 && collect) {
+        A.acc = d.fixacc;
+        A.inv_scale = 1.0 / d.fix_scale;
+        cg_step<R, true>(d, A, st);
+    } else {
+        cg_step<R, false>(d, A, st);
+    }
+}
+template void launch_cg_step<float>(const Dev&, int, bool, const double*, double, double*, cudaStream_t);
+template void launch_cg_step<double>(const Dev&, int, bool, const double*, double, double*, cudaStream_t);
 
 template <>
 void launch_energy<float>(const Dev& d, cudaStream_t st) {
