@@ -85,7 +85,7 @@ constexpr int kSlowCap = 192;
 // k_pair_vjp_fast at 12 blocks per SM (168 registers, 48 B of spills):
 // 7.3 ms per 12,288-atom adjoint against 7.9 ms at 215 registers and 8.2 ms
 // at 128 (mixed form).
-constexpr int kVjpSplit = 8;
+constexpr int kVjpSplit = 9, kFixedSplit = 16;
 // The FP64 routine out of line, so that the rare overflow of a slow row does
 // not set the fast pass's register budget.
 __device__ __noinline__ void visit_pair_call(const PairParams& P, const AtomData& A, const double* g,
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kVjpTile, 12) k_pair_vjp_fast(PairParams P, At
             if (!meI) d = {-d.x, -d.y, -d.z};
             const double2 yj = s_yz[jj];
             const bool yzd = (myz.x != yj.x) || (myz.y != yj.y);
-            const double r2 = d.x * d.x + d.y * d.y + d.z * d.z;
+            const double r2 = norm2(d);
             if (!(r2 < damp_r2) && yzd && d.y * d.y + d.z * d.z > 0.0) {
                 const T sg = meI ? T(1) : T(-1);
                 const W dj = {sg * (T)d.x, sg * (T)d.y, sg * (T)d.z};
@@ -202,18 +202,15 @@ __global__ void k_pair_vjp_slow(PairParams P, AtomData A, const double* __restri
 // b = d/d(q, lab, t) of lambda . Efix, per atom (out: n*5).  Field at i due to
 // k (RTDF.cpp:698-704): f_ik = -m [d (rr3 q_k - rr5 lab_k.d) + lab_k rr3],
 // d = p_k - p_i.
-// with_dual = 0: the unit-scale pairs' Thole-factor term is left to
-// k_fixed_dual_list (the covalent corrections keep theirs here).
 __global__ void k_fixed_vjp(PairParams P, AtomData A, const double* __restrict__ lam, const int* __restrict__ exc_off,
-                            const int* __restrict__ exc_j, const double* __restrict__ exc_m, double* __restrict__ out,
-                            int with_dual) {
+                            const int* __restrict__ exc_j, const double* __restrict__ exc_m, double* __restrict__ out) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int k = t / kLanes, l = t % kLanes;
     const bool act = k < P.n;
     double acc[5] = {0, 0, 0, 0, 0};
     if (act) {
         for (int i = l; i < P.n; i += kLanes)
-            if (i != k) fixed_vjp_visit(P, A, lam, k, i, 1.0, acc, with_dual != 0);
+            if (i != k) fixed_vjp_visit(P, A, lam, k, i, 1.0, acc);
         for (int e = exc_off[k] + l; e < exc_off[k + 1]; e += kLanes)
             fixed_vjp_visit(P, A, lam, k, exc_j[e], exc_m[e] - 1.0, acc);
     }
@@ -240,17 +237,14 @@ __global__ void k_matvec_t_vjp(PairParams P, AtomData A, const double* __restric
     if (act && l == 0) out[k] = accumulate ? out[k] + acc : acc;
 }
 
-// k_fixed_vjp without the Thole-factor term, over shared-memory J tiles, one
-// thread per atom: undamped pairs in the arithmetic T (FP32 in the mixed
-// form) from an FP64 minimum-image displacement, damped pairs in FP64; the
-// covalent corrections (with their Thole term) in FP64 at the end.  The
+// k_fixed_vjp's undamped pairs, over shared-memory J tiles, one thread per atom,
+// in the arithmetic T (FP32 in the mixed form) from an FP64 minimum-image
+// displacement.  The damped pairs are those of the pair pass's lists and left,
+// with the covalent corrections, to k_fixed_list, so that the loop has no branch and four pairs overlap (820 -> 399 us at 12,288 atoms, and 35 us more in the list kernel).  The
 // J range is split over blockIdx.y as in k_pair_vjp_fast; split s writes
 // part + s * n * 5 and k_sum_splits5 adds the splits in order.
 template <class T>
 __global__ void __launch_bounds__(kVjpTile) k_fixed_vjp_fast(PairParams P, AtomData A, const double* __restrict__ lam,
-                                                            const int* __restrict__ exc_off,
-                                                            const int* __restrict__ exc_j,
-                                                            const double* __restrict__ exc_m,
                                                             double* __restrict__ part) {
     __shared__ double s_pos[3][kVjpTile];
     __shared__ T s_l[3][kVjpTile];
@@ -259,33 +253,27 @@ __global__ void __launch_bounds__(kVjpTile) k_fixed_vjp_fast(PairParams P, AtomD
     const int kk = act ? k : 0;
     const double px = A.pos[3 * kk], py = A.pos[3 * kk + 1], pz = A.pos[3 * kk + 2];
     const double damp_r2 = (double)P.damp_r2;
-    double acc[5] = {0, 0, 0, 0, 0};
+    double acc[4] = {0, 0, 0, 0};
     const int ntile = (P.n + kVjpTile - 1) / kVjpTile;
     const int tb = (int)(((long)ntile * blockIdx.y) / gridDim.y), te = (int)(((long)ntile * (blockIdx.y + 1)) / gridDim.y);
     for (int base = tb * kVjpTile; base < te * kVjpTile && base < P.n; base += kVjpTile) {
         __syncwarp();
         const int js = base + threadIdx.x;
-        if (js < P.n)
-            for (int c = 0; c < 3; c++) {
-                s_pos[c][threadIdx.x] = A.pos[3 * js + c];
-                s_l[c][threadIdx.x] = (T)lam[3 * js + c];
-            }
+        for (int c = 0; c < 3; c++) {
+            s_pos[c][threadIdx.x] = js < P.n ? A.pos[3 * js + c] : 0.0;
+            s_l[c][threadIdx.x] = js < P.n ? (T)lam[3 * js + c] : T(0);
+        }
         __syncwarp();
         if (!act) continue;
-        const int cnt = min(kVjpTile, P.n - base);
         T a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-        for (int jj = 0; jj < cnt; jj++) {
-            const int i = base + jj;
-            if (i == k) continue;
+#pragma unroll 4
+        for (int jj = 0; jj < kVjpTile; jj++) {
             // d = p_k - p_i
             const V3 d = min_image(P, {px - s_pos[0][jj], py - s_pos[1][jj], pz - s_pos[2][jj]});
-            const double r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-            if (r2 < damp_r2) {
-                fixed_vjp_visit(P, A, lam, k, i, 1.0, acc, false);
-                continue;
-            }
+            const double r2 = norm2(d);
+            const bool off = r2 < damp_r2 || base + jj == k || base + jj >= P.n;
             const T dx = (T)d.x, dy = (T)d.y, dz = (T)d.z;
-            const T ri = div_sqrt(T(1), (T)r2), ri2 = ri * ri, rr3 = ri * ri2, rr5 = T(3) * rr3 * ri2;
+            const T ri = off ? T(0) : rsq((T)r2), ri2 = ri * ri, rr3 = ri * ri2, rr5 = T(3) * rr3 * ri2;
             const T lx = s_l[0][jj], ly = s_l[1][jj], lz = s_l[2][jj];
             const T ldd = lx * dx + ly * dy + lz * dz;
             a0 -= rr3 * ldd;
@@ -299,10 +287,9 @@ __global__ void __launch_bounds__(kVjpTile) k_fixed_vjp_fast(PairParams P, AtomD
         acc[3] += (double)a3;
     }
     if (!act) return;
-    if (blockIdx.y == 0)
-        for (int e = exc_off[k]; e < exc_off[k + 1]; e++) fixed_vjp_visit(P, A, lam, k, exc_j[e], exc_m[e] - 1.0, acc);
     double* o = part + 5 * ((size_t)blockIdx.y * P.n + k);
-    for (int c = 0; c < 5; c++) o[c] = acc[c];
+    for (int c = 0; c < 4; c++) o[c] = acc[c];
+    o[4] = 0.0;
 }
 
 // out[k] = sum over splits s of part[s * m + k], in split order.
@@ -330,24 +317,33 @@ __device__ __forceinline__ bool list_overflow(const AdjPairList& L, int n, int k
     return false;
 }
 
-// out[5 k + 4] += d/dt_k of lambda . Efix over the unit-scale damped pairs.
-__global__ void k_fixed_dual_list(PairParams P, AtomData A, const double* __restrict__ lam, AdjPairList L,
-                                  double* __restrict__ out) {
+// k_fixed_vjp's damped pairs (unit scale) and covalent corrections in FP64, added
+// to out.  Listed pairs beyond the damping range (on the x axis) were
+// k_fixed_vjp_fast's.  A lane's pairs come before its corrections, so that a
+// partner of scale 0 listed in the same place cancels exactly.
+__global__ void k_fixed_list(PairParams P, AtomData A, const double* __restrict__ lam, AdjPairList L,
+                             const int* __restrict__ exc_off, const int* __restrict__ exc_j,
+                             const double* __restrict__ exc_m, double* __restrict__ out) {
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, l = threadIdx.x & 31;
     if (k >= P.n) return;   // whole warps leave together
-    double acc = 0.0;
+    double acc[5] = {0, 0, 0, 0, 0};
     if (list_overflow(L, P.n, k)) {
         for (int i = l; i < P.n; i += 32)
-            if (i != k) acc += fixed_vjp_dual(P, A, lam, k, i, 1.0);
+            if (i != k) fixed_vjp_damped(P, A, lam, k, i, acc);
     } else {
         for (int sp = 0; sp < L.nsplit; sp++) {
             const size_t sk = (size_t)sp * P.n + k;
             const int* row = L.slow + sk * L.cap;
-            for (int e = l; e < L.nslow[sk]; e += 32) acc += fixed_vjp_dual(P, A, lam, k, row[e], 1.0);
+            for (int e = l; e < L.nslow[sk]; e += 32) fixed_vjp_damped(P, A, lam, k, row[e], acc);
         }
     }
-    acc = warp_sum_fixed(acc);
-    if (l == 0) out[5 * k + 4] += acc;
+    for (int e = exc_off[k] + l; e < exc_off[k + 1]; e += 32)
+        fixed_vjp_visit(P, A, lam, k, exc_j[e], exc_m[e] - 1.0, acc);
+#pragma unroll
+    for (int c = 0; c < 5; c++) {
+        acc[c] = warp_sum_fixed(acc[c]);
+        if (l == 0) out[5 * k + c] += acc[c];
+    }
 }
 
 // k_matvec_t_vjp over the damped-partner lists.
@@ -504,21 +500,33 @@ __global__ void k_set_operand(int n, const int* __restrict__ rank, const double*
 // ---------------------------------------------------------------------------
 static inline int nb(int n) { return (n + 127) / 128; }
 
-// Scratch of the two-pass pair VJP, per (split, atom): 8 FP64 sums, the
-// slow-pair row and its count.
-// Splits of the J range of the tiled passes: about 16 warps per SM (148 SMs)
-// in total, at most kVjpSplit.
+// J splits of k_pair_vjp_fast: whole rounds of its 12 resident blocks an SM,
+// the time going with rounds / splits (12,288 atoms: 7 splits made 1.5 rounds,
+// 1666 us; 9 make 1.95, 1479).
 static int vjp_splits(int n) {
-    const int blocks = (std::max(n, 1) + adj::kVjpTile - 1) / adj::kVjpTile;
-    return std::min(adj::kVjpSplit, std::max(1, (16 * 148 + blocks - 1) / blocks));
+    const long blocks = (std::max(n, 1) + adj::kVjpTile - 1) / adj::kVjpTile, resident = 12L * 148;
+    int best = 1;
+    const auto rounds = [&](int s) { return (double)((blocks * s + resident - 1) / resident) / s; };
+    for (int s = 2; s <= adj::kVjpSplit; s++)
+        if (rounds(s) < rounds(best)) best = s;
+    return best;
 }
 
+// J splits of k_fixed_vjp_fast: one round of 32 resident blocks an SM
+// (12,288 atoms, 7 and 12 splits: 436 and 399 us).
+static int fixed_splits(int n) {
+    const int blocks = (std::max(n, 1) + adj::kVjpTile - 1) / adj::kVjpTile;
+    return std::min(adj::kFixedSplit, std::max(1, 32 * 148 / blocks));
+}
+
+// Scratch of the two-pass pair VJP, per (split, atom): 8 FP64 sums, the
+// slow-pair row and its count.
 size_t adjoint_pair_scratch(int n) {
     const size_t m = (size_t)vjp_splits(n) * (size_t)std::max(n, 1);
     return 8 * m + (m * (adj::kSlowCap + 1) * sizeof(int) + sizeof(double) - 1) / sizeof(double);
 }
 
-size_t adjoint_fixed_scratch(int n) { return 5 * (size_t)vjp_splits(n) * (size_t)std::max(n, 1); }
+size_t adjoint_fixed_scratch(int n) { return 5 * (size_t)fixed_splits(n) * (size_t)std::max(n, 1); }
 
 void launch_adjoint_pair(const Dev& d, const double* g, const double* gT, double gE, double* a8, int precision,
                          double* scratch, AdjPairList* list, cudaStream_t st) {
@@ -550,18 +558,18 @@ void launch_adjoint_fixed(const Dev& d, const double* lam, double* b5, const Adj
     if (d.n <= 0) return;
     adj::AtomData A{d.pos, d.charge, d.lab, d.mu, d.thole, d.yz};
     if (list.nsplit <= 0 || !scratch) {
-        adj::k_fixed_vjp<<<nb(d.n * adj::kLanes), 128, 0, st>>>(d.pp, A, lam, d.exc_off, d.exc_j, d.exc_m, b5, 1);
+        adj::k_fixed_vjp<<<nb(d.n * adj::kLanes), 128, 0, st>>>(d.pp, A, lam, d.exc_off, d.exc_j, d.exc_m, b5);
         return;
     }
     const int blocks = (d.n + adj::kVjpTile - 1) / adj::kVjpTile;
-    const int nsplit = vjp_splits(d.n);
+    const int nsplit = fixed_splits(d.n);
     const dim3 grid(blocks, nsplit);
     if (precision == TDP_PRECISION_MIXED)
-        adj::k_fixed_vjp_fast<float><<<grid, adj::kVjpTile, 0, st>>>(d.pp, A, lam, d.exc_off, d.exc_j, d.exc_m, scratch);
+        adj::k_fixed_vjp_fast<float><<<grid, adj::kVjpTile, 0, st>>>(d.pp, A, lam, scratch);
     else
-        adj::k_fixed_vjp_fast<double><<<grid, adj::kVjpTile, 0, st>>>(d.pp, A, lam, d.exc_off, d.exc_j, d.exc_m, scratch);
+        adj::k_fixed_vjp_fast<double><<<grid, adj::kVjpTile, 0, st>>>(d.pp, A, lam, scratch);
     adj::k_sum_splits<<<nb(5 * d.n), 128, 0, st>>>(5 * d.n, nsplit, scratch, b5);
-    adj::k_fixed_dual_list<<<nb(32 * d.n), 128, 0, st>>>(d.pp, A, lam, list, b5);
+    adj::k_fixed_list<<<nb(32 * d.n), 128, 0, st>>>(d.pp, A, lam, list, d.exc_off, d.exc_j, d.exc_m, b5);
 }
 void launch_adjoint_matvec_t(const Dev& d, const double* lam, double* ct, const AdjPairList& list, cudaStream_t st) {
     launch_adjoint_matvec_t_mu(d, lam, d.mu, ct, false, list, st);

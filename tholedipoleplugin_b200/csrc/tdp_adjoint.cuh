@@ -234,13 +234,19 @@ __device__ T pair_loss(double dx, double dy, double dz, bool yzd, T qI, const T*
 }
 
 __device__ __forceinline__ V3 min_image(const PairParams& P, V3 d) {
-    if (P.periodic) {
-        d.x = fold_d(d.x, P.box[0], P.inv_box[0]);
-        d.y = fold_d(d.y, P.box[1], P.inv_box[1]);
-        d.z = fold_d(d.z, P.box[2], P.inv_box[2]);
-    }
-    return d;
+    if (!P.periodic) return d;
+    const V3 f = {round_fold(d.x, P.box[0], P.inv_box[0]), round_fold(d.y, P.box[1], P.inv_box[1]),
+                  round_fold(d.z, P.box[2], P.inv_box[2])};
+    if (!near_tie(f.x, __double2hiint(P.half_box_tol[0])) && !near_tie(f.y, __double2hiint(P.half_box_tol[1])) &&
+        !near_tie(f.z, __double2hiint(P.half_box_tol[2])))
+        return f;
+    return {fold_d(d.x, P.box[0], P.inv_box[0]), fold_d(d.y, P.box[1], P.inv_box[1]),
+            fold_d(d.z, P.box[2], P.inv_box[2])};
 }
+
+// |d|^2 with its roundings spelled out: passes that divide the pairs between
+// them by r^2 < damp_r2 have to agree to the last bit.
+__device__ __forceinline__ double norm2(V3 d) { return fma(d.z, d.z, fma(d.y, d.y, d.x * d.x)); }
 
 struct AtomData {
     const double* pos;     // n*3
@@ -447,39 +453,34 @@ __device__ __forceinline__ double fixed_vjp_dt(const AtomData& A, V3 d, double r
 
 // Contribution of the pair (i, k) with M scale m to atom k's
 // d/d(q_k, lab_k, t_k) of lambda . Efix (k_fixed_vjp), added to acc[5].
-// dual = false leaves out the Thole-factor term (acc[4]); fixed_vjp_dual adds
-// it alone.
 __device__ __forceinline__ void fixed_vjp_visit(const PairParams& P, const AtomData& A, const double* lam, int k,
-                                                int i, double m, double* acc, bool dual = true) {
+                                                int i, double m, double* acc) {
     const double damp_r2 = (double)P.damp_r2;
     const V3 lk = ld(lam + 3 * k);
     V3 d = min_image(P, {A.pos[3 * k] - A.pos[3 * i], A.pos[3 * k + 1] - A.pos[3 * i + 1],
                          A.pos[3 * k + 2] - A.pos[3 * i + 2]});  // p_k - p_i
-    double r2 = d.x * d.x + d.y * d.y + d.z * d.z, r = sqrt(r2);
+    double r2 = norm2(d), r = sqrt(r2);
     V3 li = ld(lam + 3 * i);
     double rr3, rr5;
     field_damping<double>(r, r2, damp_r2, A.thole[i], A.thole[k], rr3, rr5);
     double ldd = li.x * d.x + li.y * d.y + li.z * d.z;
-    acc[0] += -m * rr3 * ldd;  // d(lambda_i . f_ik)/dq_k
-    acc[1] += m * (rr5 * ldd * d.x - rr3 * li.x);
-    acc[2] += m * (rr5 * ldd * d.y - rr3 * li.y);
-    acc[3] += m * (rr5 * ldd * d.z - rr3 * li.z);
+    // Each term is rounded before m, so that the pair and its correction by -1 cancel exactly.
+    const double a = rr5 * ldd;
+    acc[0] -= m * __dmul_rn(rr3, ldd);  // d(lambda_i . f_ik)/dq_k
+    acc[1] += m * __dadd_rn(a * d.x, -__dmul_rn(rr3, li.x));
+    acc[2] += m * __dadd_rn(a * d.y, -__dmul_rn(rr3, li.y));
+    acc[3] += m * __dadd_rn(a * d.z, -__dmul_rn(rr3, li.z));
     // t_k enters f_ik and f_ki (only within the damping range).
-    if (!dual || !(r2 < damp_r2)) return;
+    if (!(r2 < damp_r2)) return;
     acc[4] += fixed_vjp_dt(A, d, r, li, lk, k, i, m);
 }
 
-// The Thole-factor term of fixed_vjp_visit alone (zero beyond the damping range).
-__device__ __forceinline__ double fixed_vjp_dual(const PairParams& P, const AtomData& A, const double* lam, int k,
-                                                 int i, double m) {
-    const double damp_r2 = (double)P.damp_r2;
-    V3 d = min_image(P, {A.pos[3 * k] - A.pos[3 * i], A.pos[3 * k + 1] - A.pos[3 * i + 1],
-                         A.pos[3 * k + 2] - A.pos[3 * i + 2]});  // p_k - p_i
-    const double r2 = d.x * d.x + d.y * d.y + d.z * d.z;
-    if (!(r2 < damp_r2)) return 0.0;
-    const double r = sqrt(r2);
-    const V3 li = ld(lam + 3 * i), lk = ld(lam + 3 * k);
-    return fixed_vjp_dt(A, d, r, li, lk, k, i, m);
+// fixed_vjp_visit of a unit-scale pair within the damping range, nothing beyond.
+__device__ __forceinline__ void fixed_vjp_damped(const PairParams& P, const AtomData& A, const double* lam, int k,
+                                                 int i, double* acc) {
+    const V3 d = min_image(P, {A.pos[3 * k] - A.pos[3 * i], A.pos[3 * k + 1] - A.pos[3 * i + 1],
+                               A.pos[3 * k + 2] - A.pos[3 * i + 2]});
+    if (norm2(d) < (double)P.damp_r2) fixed_vjp_visit(P, A, lam, k, i, 1.0, acc);
 }
 
 // d/dt_k of the pair (k, j) terms of lambda^T T(t) mu with I scale s

@@ -560,7 +560,7 @@ void solve_cg(tdp_handle* h, bool fused = false, bool cold = true) {
     // iteration is queued before the host has seen the epsilon; its kernels do
     // nothing if that shows the solve has stopped.  (Not while the stages are
     // timed.)
-    const bool one = cg_cluster(d), collect = one && !h->ew && sizeof(R) == 4;
+    const bool one = cg_cluster(d), collect = cg_collects(d) && !h->ew && sizeof(R) == 4;
     const bool ahead = one && !h->ew && d.field_parts > 1 && !h->timing;
     // The residual of y in scalar slot `slot` (use_partial: of a matvec).
     const auto start = [&](bool use_partial) {
@@ -587,15 +587,16 @@ void solve_cg(tdp_handle* h, bool fused = false, bool cold = true) {
             return;
         }
         clear_eps(h, from + 1);
-        if (h->ew) {
-            matvec<R>(h);
-        } else {
+        if (collect) {
             size_t k = kernel_begin(h, 0);
-            launch_cg_matvec<R>(d, stop, h->target_eps, st);
+            launch_cg_matvec(d, stop, h->target_eps, st);
             kernel_end(h, k);
             h->launches++;
-            if (!conditional) h->matvecs++;
+            h->matvecs++;
+        } else {
+            matvec<R>(h);
         }
+        if (conditional) h->matvecs--;   // counted when the host takes the step
         launch_cg_step<R>(d, from, collect, stop, h->target_eps, eps_word(h, from + 1), st);
         h->launches++;
     };

@@ -44,6 +44,19 @@ __device__ __forceinline__ double fold_d(double d, double L, double invL) {
     return d - L * floor(d * invL + 0.5);
 }
 
+// fold_d without its rounding instruction: round to nearest by the 1.5 * 2^52
+// constant.  Only an exact tie rounds differently, so displacements that end
+// within half_box_tol of half a box (near_tie) are folded again by fold_d.
+__device__ __forceinline__ double round_fold(double d, double L, double invL) {
+    const double magic = 6755399441055744.0;
+    return __fma_rn(-__dadd_rn(__fma_rn(d, invL, magic), -magic), L, d);
+}
+__device__ __forceinline__ bool near_tie(double f, int tol_hi) { return (__double2hiint(f) & 0x7fffffff) >= tol_hi; }
+__device__ __forceinline__ double fold_magic(double d, double L, double invL, int tol_hi) {
+    const double f = round_fold(d, L, invL);
+    return near_tie(f, tol_hi) ? fold_d(d, L, invL) : f;
+}
+
 // FP32 minimum image: round-to-nearest via the 1.5*2^23 constant (valid for
 // |d/L| < 2^22), three FP32-pipe operations and no conversion instruction.
 __device__ __forceinline__ float fold_f(float d, float L, float invL) {

@@ -130,11 +130,10 @@ void launch_cg_q(const Dev& d, cudaStream_t st);
 // word that receives the new epsilon.  collect: the all-pairs matvec was
 // launch_cg_matvec.
 bool cg_cluster(const Dev& d);
+bool cg_collects(const Dev& d);
 template <class R>
 void launch_cg_start(const Dev& d, int slot, bool use_partial, double* host_eps, cudaStream_t st);
-template <class R> void launch_cg_matvec(const Dev& d, const double* stop_eps, double target, cudaStream_t st);
-template <> void launch_cg_matvec<float>(const Dev& d, const double* stop_eps, double target, cudaStream_t st);
-template <> void launch_cg_matvec<double>(const Dev& d, const double* stop_eps, double target, cudaStream_t st);
+void launch_cg_matvec(const Dev& d, const double* stop_eps, double target, cudaStream_t st);
 template <class R>
 void launch_cg_step(const Dev& d, int slot, bool collect, const double* stop_eps, double target, double* host_eps,
                     cudaStream_t st);

@@ -122,16 +122,6 @@ __device__ __forceinline__ d3 exact_delta(const PairParams& P, const double* __r
     return d;
 }
 
-// fold_d without its rounding instruction: round to nearest by the 1.5 * 2^52
-// constant.  Only an exact tie rounds differently, so displacements that end
-// within half_box_tol of half a box are folded again by fold_d.
-__device__ __forceinline__ double fold_magic(double d, double L, double invL, int tol_hi) {
-    const double magic = 6755399441055744.0;
-    const double t = __dadd_rn(__fma_rn(d, invL, magic), -magic);
-    const double f = __fma_rn(-t, L, d);
-    return (__double2hiint(f) & 0x7fffffff) >= tol_hi ? fold_d(d, L, invL) : f;
-}
-
 // p_j - p_i from j's position and i's shifted into j's image; fold: bits of the
 // dimensions that need folding.
 template <bool FOLD>
@@ -2326,8 +2316,12 @@ void launch_field<double>(const Dev& d, int kind, cudaStream_t st) {
     }
 }
 
-// The cluster form of the CG kernels holds up to four atoms a thread.
+// The cluster form of the CG kernels holds up to four atoms a thread.  With one
+// atom a thread it also collects the mixed matvec's sums; beyond, the partner
+// pairs of several atoms in a row would take longer than k_field_done (26 us
+// an iteration, cold, against 18 + 6 at 12,288 atoms).
 bool cg_cluster(const Dev& d) { return d.n <= 4 * kCgCap; }
+bool cg_collects(const Dev& d) { return d.n <= kCgCap; }
 
 namespace {
 
@@ -2350,23 +2344,6 @@ CgArrays cg_arrays(const Dev& d, int slot, double* host_eps) {
     return A;
 }
 
-template <class R, bool DONE>
-void cg_step(const Dev& d, const CgArrays& A, cudaStream_t st) {
-    typedef typename Vec4T<R>::type V4;
-    const V4* pq = (const V4*)d.posq_s;
-    V4* vec = (V4*)d.vec_s;
-    const int m = (d.n + kCgCap - 1) / kCgCap;
-    if (m <= 1)
-        k_cg_step<R, DONE, 1><<<kCgCtas, kCgThreads, 0, st>>>(d.pp, A, pq, vec, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
-                                                              d.exs_s);
-    else if (m == 2)
-        k_cg_step<R, DONE, 2><<<kCgCtas, kCgThreads, 0, st>>>(d.pp, A, pq, vec, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
-                                                              d.exs_s);
-    else
-        k_cg_step<R, DONE, 4><<<kCgCtas, kCgThreads, 0, st>>>(d.pp, A, pq, vec, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
-                                                              d.exs_s);
-}
-
 }  // namespace
 
 template <class R>
@@ -2377,18 +2354,14 @@ void launch_cg_start(const Dev& d, int slot, bool use_partial, double* host_eps,
 template void launch_cg_start<float>(const Dev&, int, bool, double*, cudaStream_t);
 template void launch_cg_start<double>(const Dev&, int, bool, double*, cudaStream_t);
 
-// All-pairs matvec without the collection of its sums, which launch_cg_step does.
-template <>
-void launch_cg_matvec<float>(const Dev& d, const double* stop_eps, double target, cudaStream_t st) {
+// Mixed all-pairs matvec without the collection of its sums, which
+// launch_cg_step does.
+void launch_cg_matvec(const Dev& d, const double* stop_eps, double target, cudaStream_t st) {
     const int L = d.field_L, B = std::max(L, kFieldNS), nb = (d.pp.n_tiles + B - 1) / B;
     const dim3 grid((unsigned)((long)nb * (nb + 1) / 2 * (B / std::min(L, kFieldNS))), d.field_parts);
     k_field_items<1, kFieldNS><<<grid, 32, 0, st>>>(d.pp, L, (const float4*)d.posq_s, (const float4*)d.vec_s, d.tctr_s,
                                                     d.text_s, d.pos_s, d.exs_off, d.exs_j, d.exs_s, d.exs_tiles,
                                                     d.n_pad, fix_of(d), CgStop{stop_eps, target});
-}
-template <>
-void launch_cg_matvec<double>(const Dev& d, const double*, double, cudaStream_t st) {
-    launch_field<double>(d, 1, st);
 }
 
 template <class R>
@@ -2396,13 +2369,23 @@ void launch_cg_step(const Dev& d, int slot, bool collect, const double* stop_eps
                     cudaStream_t st) {
     CgArrays A = cg_arrays(d, slot, host_eps);
     A.stop = CgStop{stop_eps, target};
-    if (sizeof(R) == 4 && collect) {
-        A.acc = d.fixacc;
-        A.inv_scale = 1.0 / d.fix_scale;
-        cg_step<R, true>(d, A, st);
-    } else {
-        cg_step<R, false>(d, A, st);
-    }
+    typedef typename Vec4T<R>::type V4;
+    const V4* pq = (const V4*)d.posq_s;
+    V4* vec = (V4*)d.vec_s;
+#define TDP_CG_STEP(DONE, M)                                                                                       \
+    k_cg_step<R, DONE, M><<<kCgCtas, kCgThreads, 0, st>>>(d.pp, A, pq, vec, d.pos_s, d.exs_off, d.exs_j, d.exs_m, \
+                                                          d.exs_s)
+    if constexpr (sizeof(R) == 4)
+        if (collect) {
+            A.acc = d.fixacc;
+            A.inv_scale = 1.0 / d.fix_scale;
+            TDP_CG_STEP(true, 1);
+            return;
+        }
+    if (d.n <= kCgCap) TDP_CG_STEP(false, 1);
+    else if (d.n <= 2 * kCgCap) TDP_CG_STEP(false, 2);
+    else TDP_CG_STEP(false, 4);
+#undef TDP_CG_STEP
 }
 template void launch_cg_step<float>(const Dev&, int, bool, const double*, double, double*, cudaStream_t);
 template void launch_cg_step<double>(const Dev&, int, bool, const double*, double, double*, cudaStream_t);
