@@ -275,10 +275,6 @@ __device__ __forceinline__ V3T<T> sub3v(V3T<T> a, V3T<T> b) { return {a.x - b.x,
 // perm(v) = (v_y, v_z, v_x).
 template <class T>
 __device__ __forceinline__ V3T<T> permT(V3T<T> a) { return {a.z, a.x, a.y}; }
-// a / sqrt(x): exact division in FP64, the reciprocal square root in FP32.
-__device__ __forceinline__ double div_sqrt(double a, double x) { return a / sqrt(x); }
-__device__ __forceinline__ float div_sqrt(float a, float x) { return a * rsqrtf(x); }
-
 // 1/sqrt(x): rsqrt in either arithmetic.
 __device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
 __device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }

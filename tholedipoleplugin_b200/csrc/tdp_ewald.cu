@@ -74,8 +74,6 @@ struct PmeGrid {
     double L[3], invL[3], sc[3];   // sc = K/L
 };
 
-__device__ __forceinline__ float erfc_r(float x) { return erfcf(x); }
-__device__ __forceinline__ double erfc_r(double x) { return erfc(x); }
 
 // Real-space kernels of erfc(alpha r)/r:  B0 = erfc/r,
 // B_{n+1} = ((2n+1) B_n + (2 alpha^2)^(n+1) / (alpha sqrt(pi)) e^(-alpha^2 r^2)) / r^2.
@@ -85,7 +83,7 @@ __device__ __forceinline__ void erfc_kernels(R r2, R rinv, R alpha, R ca, R a2, 
     R x = alpha * r;
     R e = exp_r(-x * x);
     R rinv2 = rinv * rinv;
-    B0 = erfc_r(x) * rinv;
+    B0 = erfc(x) * rinv;
     R t = ca * e;
     B1 = (B0 + t) * rinv2;
     t *= a2;
