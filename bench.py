@@ -877,10 +877,10 @@ def run_ours(args):
         mv_tf = pairs * FLOP_MATVEC_PAIR / (mv_avg * 1e-3) / 1e12
         en_tf = pairs * FLOP_ENERGY_PAIR / (en_avg * 1e-3) / 1e12
         if m["en_ms"] >= m["mv_ms"]:
-            kname, ach, avg, share, flop = "k_energy_sym<float>", en_tf, en_avg, m["en_ms"] / m["t_ms"], FLOP_ENERGY_PAIR
+            kname, ach, avg, share, flop = "k_energy_items<0,0>", en_tf, en_avg, m["en_ms"] / m["t_ms"], FLOP_ENERGY_PAIR
             bytes_ = n * BYTES_ENERGY_ATOM
         else:
-            kname, ach, avg, share, flop = "k_field_sym<float,1>", mv_tf, mv_avg, m["mv_ms"] / m["t_ms"], FLOP_MATVEC_PAIR
+            kname, ach, avg, share, flop = "k_field_items<1,2>", mv_tf, mv_avg, m["mv_ms"] / m["t_ms"], FLOP_MATVEC_PAIR
             bytes_ = n * BYTES_MATVEC_ATOM
         out["roofline"] = {"bound": "fp32", "kernel": kname, "achieved": _r(ach), "peak": _r(fp32), "unit": "TFLOP/s",
                            "frac": _r(ach / fp32), "traffic": profile_traffic(kname),

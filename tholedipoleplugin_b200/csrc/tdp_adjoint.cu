@@ -240,9 +240,11 @@ __global__ void k_matvec_t_vjp(PairParams P, AtomData A, const double* __restric
 // k_fixed_vjp's undamped pairs, over shared-memory J tiles, one thread per atom,
 // in the arithmetic T (FP32 in the mixed form) from an FP64 minimum-image
 // displacement.  The damped pairs are those of the pair pass's lists and left,
-// with the covalent corrections, to k_fixed_list, so that the loop has no branch and four pairs overlap (820 -> 399 us at 12,288 atoms, and 35 us more in the list kernel).  The
-// J range is split over blockIdx.y as in k_pair_vjp_fast; split s writes
-// part + s * n * 5 and k_sum_splits5 adds the splits in order.
+// with the covalent corrections, to k_fixed_list, so that the loop has no
+// branch and four pairs overlap (820 -> 399 us at 12,288 atoms, and 35 us more
+// in the list kernel).  The J range is split over blockIdx.y as in
+// k_pair_vjp_fast; split s writes part + s * n * 5 and k_sum_splits adds the
+// splits in order.
 template <class T>
 __global__ void __launch_bounds__(kVjpTile) k_fixed_vjp_fast(PairParams P, AtomData A, const double* __restrict__ lam,
                                                             double* __restrict__ part) {

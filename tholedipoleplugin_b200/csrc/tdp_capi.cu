@@ -1259,7 +1259,7 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
             d.n_eblk = 1;
         } else if (h->precision == TDP_PRECISION_MIXED && !variational) {
             // Mixed all-pairs form: the band sums go into the fixed-point
-            // accumulator and one flushed slot.  Each atom's word receives at
+            // accumulator and one slot.  Each atom's word receives at
             // most `adds` adds of magnitude < 2^23, so with 2^bits units per
             // e/nm^2 the sum stays below 2^63.
             d.nslot = 1;

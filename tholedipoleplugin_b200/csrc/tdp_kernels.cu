@@ -4,7 +4,7 @@
 // of the tile records, lab-frame rotation, the O(N) kernels of the solvers,
 // the torque gather and the queries.  The all-pairs kernels (permanent field,
 // mutual-field matvec, energy/force/torque) are in tdp_sym.cu; they leave
-// per-band partial sums that the consumers here reduce in a fixed order.
+// one sum per atom that the consumers here read.
 //
 // Mixed form: positions are FP32 offsets from FP64 32-atom tile centres, so
 // near pairs keep full FP32 precision wherever they are in the box.

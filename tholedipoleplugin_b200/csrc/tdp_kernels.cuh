@@ -69,10 +69,10 @@ struct Dev {
     double* q = nullptr;
     double* hist = nullptr;      // extrapolation orders, korder*n*3
     double* partial = nullptr;   // nslot*6*n_pad pair-kernel partial sums (scratch)
-    // Mixed all-pairs form: the field and energy kernels add their per-band
+    // Mixed all-pairs form: the field and energy kernels add their
     // sums into one 64-bit fixed-point accumulator (6*n_pad + 1, units of
     // 1/fix_scale; integer addition makes the result independent of the order)
-    // that a flush kernel converts into partial slot 0 and clears (nsplit = 1).
+    // that the kernels collecting them read and clear (nsplit = 1).
     // A sum of magnitude >= fix_limit sets *fix_err instead of wrapping.
     unsigned long long* fixacc = nullptr;
     int* fix_err = nullptr;

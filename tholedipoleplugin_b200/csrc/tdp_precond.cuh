@@ -12,7 +12,8 @@
 // of its total dipole M, the tin-foil Ewald sum none, so B carries that term.
 // Applying B^-1 costs a few real-space walks within a short cutoff plus a
 // coarse PME grid, a small fraction of one all-pairs walk (1.2 ms against
-// 8.7 ms at 98,304 atoms, mixed form), and cuts the outer iterations there
+// 8.7 ms at 98,304 atoms, mixed form, when the line below was drawn; the walk
+// takes 6.9 ms now and the application shares the Ewald kernels' gains), and cuts the outer iterations there
 // from 7 to 2 from a cold start (which also begins at y = M(b), see
 // precond_cold_start) and from 5-6 to 2 per warm-started MD step.  Below about
 // 30,000 atoms an all-pairs matvec is cheap enough that plain CG is as fast,

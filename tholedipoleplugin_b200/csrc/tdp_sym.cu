@@ -515,8 +515,9 @@ __device__ __forceinline__ void fix_add(const FixAcc& F, size_t k, float v) {
 // block, summed the J side in shared memory and flushed 2 x 3 x 512 sums; its
 // bands had to shrink with the system, which left warps with one I tile (half
 // the work per J load and shuffle) or none.  Matvec, before -> now: 19.7 ->
-// 12 us at 648 atoms (with k_field_done), 94 -> 43 at 3,993, 242 -> 175 at
-// 12,288, 8730 -> 6950 at 98,304.  NS = 4 is slower (7126 us there, 321 at
+// 12 us at 648 atoms (with k_field_done), 94 -> 41 at 3,993, 242 -> 169 at
+// 12,288, 8730 -> 6890 at 98,304 (in Hilbert order, undamped beyond exponent
+// 25; 43, 175 and 6950 before these).  NS = 4 is slower (7126 us there, 321 at
 // 12,288): the tiles of an item share the fold and damping variant of a walk.
 template <int KIND, int NS>
 __global__ void __launch_bounds__(32, 16) k_field_items(
