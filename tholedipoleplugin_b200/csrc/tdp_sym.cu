@@ -889,7 +889,7 @@ __global__ void __launch_bounds__(96)
 // launches before it were (sums, q, update, p: 4.4 + 4.2 + 5.3 + 5.1 us at 648
 // atoms, 6.1 + 4.7 + 5.3 + 4.9 at 12,288, and a gap after each).  With the
 // epsilon through pinned memory and the next iteration queued ahead, an
-// evaluation went from 436 to 295 us at 648 atoms (mixed), 555 to 474 at 1,029
+// evaluation went from 436 to 270 us at 648 atoms (mixed), 555 to 453 at 1,029
 // and 5111 to 5033 at 12,288 (FP64), 2369 to 2267 at 12,288 (mixed).
 // ---------------------------------------------------------------------------
 constexpr int kCgCtas = 8, kCgThreads = 512, kCgCap = kCgCtas * kCgThreads;
@@ -907,7 +907,7 @@ __device__ __forceinline__ void cluster_sum2(cg::cluster_group& cl, double& a, d
     __syncthreads();
     if (threadIdx.x < 2) {
         double t = 0.0;
-        for (int k = 0; k < kCgThreads / 32; k++) t += buf[threadIdx.x][k];
+        for (int k = 0; k < (int)blockDim.x / 32; k++) t += buf[threadIdx.x][k];
         buf[threadIdx.x][16] = t;
     }
     cl.sync();
@@ -940,7 +940,7 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads)
               const int* __restrict__ exc_j, const double* __restrict__ exc_m, const double* __restrict__ exc_s) {
     __shared__ double buf[2][2][17];
     cg::cluster_group cl = cg::this_cluster();
-    const int k0 = blockIdx.x * kCgThreads + threadIdx.x;
+    const int k0 = blockIdx.x * blockDim.x + threadIdx.x;
     const bool stopped = A.stop.stopped();
     d3 t[M], p[M], r[M];
     double s[M], pq = 0.0, zero = 0.0;
@@ -1025,7 +1025,7 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads)
     k_cg_start(CgArrays A, typename Vec4T<R>::type* __restrict__ vec, int use_partial) {
     __shared__ double buf[2][17];
     cg::cluster_group cl = cg::this_cluster();
-    const int k0 = blockIdx.x * kCgThreads + threadIdx.x;
+    const int k0 = blockIdx.x * blockDim.x + threadIdx.x;
     double rr = 0.0, ee = 0.0;
 #pragma unroll
     for (int m = 0; m < M; m++) {
@@ -2326,6 +2326,13 @@ bool cg_collects(const Dev& d) { return d.n <= kCgCap; }
 
 namespace {
 
+// Threads of a CTA: one atom each up to kCgThreads, the atoms spread over all
+// eight CTAs, so that the partner pairs use all eight SMs and the sums fewer
+// warps (an evaluation with CTAs of 512 threads and with these: 286 and 270 us
+// at 648 atoms, mixed, 467 and 453 at 1,029, FP64).  Beyond, a thread's further
+// atoms lie kCgCap apart.
+int cg_threads(const Dev& d) { return std::min(kCgThreads, (d.n_pad + 32 * kCgCtas - 1) / (32 * kCgCtas) * 32); }
+
 CgArrays cg_arrays(const Dev& d, int slot, double* host_eps) {
     CgArrays A{};
     A.order = d.order;
@@ -2350,7 +2357,7 @@ CgArrays cg_arrays(const Dev& d, int slot, double* host_eps) {
 template <class R>
 void launch_cg_start(const Dev& d, int slot, bool use_partial, double* host_eps, cudaStream_t st) {
     const CgArrays A = cg_arrays(d, slot, host_eps);
-    k_cg_start<R, 4><<<kCgCtas, kCgThreads, 0, st>>>(A, (typename Vec4T<R>::type*)d.vec_s, use_partial ? 1 : 0);
+    k_cg_start<R, 4><<<kCgCtas, cg_threads(d), 0, st>>>(A, (typename Vec4T<R>::type*)d.vec_s, use_partial ? 1 : 0);
 }
 template void launch_cg_start<float>(const Dev&, int, bool, double*, cudaStream_t);
 template void launch_cg_start<double>(const Dev&, int, bool, double*, cudaStream_t);
@@ -2373,8 +2380,9 @@ void launch_cg_step(const Dev& d, int slot, bool collect, const double* stop_eps
     typedef typename Vec4T<R>::type V4;
     const V4* pq = (const V4*)d.posq_s;
     V4* vec = (V4*)d.vec_s;
+    const int threads = cg_threads(d);
 #define TDP_CG_STEP(DONE, M)                                                                                       \
-    k_cg_step<R, DONE, M><<<kCgCtas, kCgThreads, 0, st>>>(d.pp, A, pq, vec, d.pos_s, d.exs_off, d.exs_j, d.exs_m, \
+    k_cg_step<R, DONE, M><<<kCgCtas, threads, 0, st>>>(d.pp, A, pq, vec, d.pos_s, d.exs_off, d.exs_j, d.exs_m, \
                                                           d.exs_s)
     if constexpr (sizeof(R) == 4)
         if (collect) {
