@@ -8,6 +8,7 @@
 #include "tholedipole_b200.h"
 #include "tdp_ewald.cuh"
 #include "tdp_precond.cuh"
+#include "tdp_hilbert.h"
 #include "tdp_host.h"
 #include "tdp_kernels.cuh"
 
@@ -293,45 +294,15 @@ void build_components(tdp_handle* h, const tdp_system_desc* desc) {
     for (int i = 0; i < n; i++) h->comp_atoms[fill[cid[root[i]]]++] = i;
 }
 
-// Position along the Hilbert curve of a 2^21-sided cube (the transform of
-// J. Skilling, AIP Conf. Proc. 707, 381 (2004): Gray-code undo from the top
-// bit down, exchanging or inverting the lower bits of the axes, then the Gray
-// encode), the axes' bits interleaved with x highest.  Consecutive points stay
-// neighbours everywhere; along a Morton curve every other block boundary is a
-// jump, which stretched the 32-atom tiles of boxes that are not a power of two
-// of molecules wide (tiles within 0.9 nm of a tile: 137 -> 111 at 6,591 atoms,
-// 176 -> 116 at 24,000, 166 -> 105 at 52,728, 113 -> 102 at 98,304; tile pairs
-// that fold at 12,288: 67 -> 63 %).
-uint64_t hilbert_key(uint32_t x, uint32_t y, uint32_t z) {
-    constexpr int kBits = 21;
-    uint32_t v[3] = {x, y, z};
-    for (uint32_t q = 1u << (kBits - 1); q > 1; q >>= 1) {
-        const uint32_t low = q - 1;
-        for (int k = 0; k < 3; k++) {
-            if (v[k] & q) {
-                v[0] ^= low;
-            } else {
-                const uint32_t d = (v[0] ^ v[k]) & low;
-                v[0] ^= d;
-                v[k] ^= d;
-            }
-        }
-    }
-    v[1] ^= v[0];
-    v[2] ^= v[1];
-    uint32_t g = 0;
-    for (uint32_t q = 1u << (kBits - 1); q > 1; q >>= 1)
-        if (v[2] & q) g ^= q - 1;
-    uint64_t key = 0;
-    for (int b = kBits - 1; b >= 0; b--)
-        for (int k = 0; k < 3; k++) key = key << 1 | (((v[k] ^ g) >> b) & 1u);
-    return key;
-}
-
 // Orders molecules along a Hilbert curve of their centroids (wrapped into the
 // box when periodic) and uploads order/rank plus the slot-indexed exception
 // tables.  Only the field kernels' memory layout changes; results are the
 // same up to summation order.
+// Consecutive points of the curve stay neighbours everywhere; along a Morton
+// curve every other block boundary is a jump, which stretched the 32-atom
+// tiles of boxes that are not a power of two of molecules wide (tiles within
+// 0.9 nm of a tile: 137 -> 111 at 6,591 atoms, 176 -> 116 at 24,000, 166 -> 105
+// at 52,728, 113 -> 102 at 98,304; tile pairs that fold at 12,288: 67 -> 63 %).
 void sort_atoms(tdp_handle* h) {
     int n = h->n;
     Dev& d = h->d;
@@ -363,7 +334,7 @@ void sort_atoms(tdp_handle* h) {
             double f = span > 0.0 ? (cen[3 * (size_t)c + k] - lo[k]) / span : 0.0;
             q[k] = (uint32_t)std::min(std::max(f, 0.0) * 2097151.0, 2097151.0);
         }
-        keys[c] = {hilbert_key(q[0], q[1], q[2]), c};
+        keys[c] = {kHilbert.key(q[0], q[1], q[2]), c};
     }
     std::stable_sort(keys.begin(), keys.end());
     std::vector<int> order(d.n_pad, -1), rank(n);
