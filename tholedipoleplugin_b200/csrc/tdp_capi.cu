@@ -907,7 +907,7 @@ void check_flags(tdp_handle* h) {
     if (h->d.fix_err && *h->h_fixerr)
         throw TdpError{TDP_ERR_NON_FINITE,
                        "a field or force sum is not finite or exceeds the fixed-point accumulator range "
-                       "(2^23 per band sum; near-coincident particles?)"};
+                       "(2^23 for the sum over a tile; near-coincident particles?)"};
 }
 
 // positions == &kStaged: the coordinates are already in d.pos.
@@ -1229,10 +1229,11 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
             d.nslot = d.nsplit = 1;
             d.n_eblk = 1;
         } else if (h->precision == TDP_PRECISION_MIXED && !variational) {
-            // Mixed all-pairs form: the band sums go into the fixed-point
-            // accumulator and one slot.  Each atom's word receives at
-            // most `adds` adds of magnitude < 2^23, so with 2^bits units per
-            // e/nm^2 the sum stays below 2^63.
+            // Mixed all-pairs form: the walks' sums go into the fixed-point
+            // accumulator and one slot.  Each atom's word receives at most
+            // `adds` of them, of magnitude < 2^23, so with 2^bits units per
+            // e/nm^2 the total stays below 2^63.  (What k_axis_pairs adds to
+            // the energy kernel's words is checked add by add.)
             d.nslot = 1;
             // Items of the field kernel: J chunks as long as seven rounds of
             // resident warps (16 an SM) allow (matvec with L = 1, 2, 4, 8, 16:

@@ -1474,77 +1474,99 @@ __device__ __forceinline__ QiPair qi_pair2(const PairParams& P, f2 DX, f2 DY, f2
 // for its tiles, so that a new spatial order moves no pair across it.
 constexpr float kNearAxis2 = 3.6e-5f, kNearAxisFar2 = 4.0e-6f, kAxisListRange2 = 2.2f;
 
-// Pairs (slots) that a walk left to k_axis_pairs.  Sized for 16 an atom; past
-// that a pair stays in its walk.
+// Pairs (slots) that the walks left to k_axis_pairs, sized for 16 an atom.  A
+// count beyond the capacity says that not all of them are here; it is not
+// raised further then, so that no number of pairs takes it past an int.
 struct AxisList {
     int2* pairs;
     int* count;
     int cap;
 };
 
-__device__ __forceinline__ bool axis_push(const AxisList& A, int i, int j) {
+__device__ __forceinline__ void axis_push(const AxisList& A, int i, int j) {
+    if (*(volatile int*)A.count > A.cap) return;
     const int k = atomicAdd(A.count, 1);
-    if (k >= A.cap) return false;
-    A.pairs[k] = make_int2(i, j);
-    return true;
+    if (k < A.cap) A.pairs[k] = make_int2(i, j);
 }
 
-// The listed pairs close to the x axis, each by itself: X's azimuth is that of
+// fix_add of a pair's 13 sums (I's six, J's six, the energy) on top of the
+// walks', which alone the scale is sized for: a word that leaves its range
+// shows by its sign.  All the adds are on their way before the first old value
+// is looked at (one after the other they took 4 us more).
+__device__ __forceinline__ void fix_add_checked(const FixAcc& F, int n_pad, int i, int j, const float (&v)[13]) {
+    bool bad = false;
+#pragma unroll
+    for (int c = 0; c < 13; c++) bad |= !(fabsf(v[c]) < (float)F.limit);
+    if (!bad) {
+        unsigned long long a[13], old[13];
+#pragma unroll
+        for (int c = 0; c < 13; c++) {
+            a[c] = (unsigned long long)__float2ll_rn(v[c] * (float)F.scale);
+            old[c] = atomicAdd(F.acc + (size_t)(c < 12 ? c % 6 : 6) * n_pad + (c < 6 ? i : c < 12 ? j : 0), a[c]);
+        }
+#pragma unroll
+        for (int c = 0; c < 13; c++) {
+            const unsigned long long now = old[c] + a[c];
+            bad |= (long long)((old[c] ^ now) & (a[c] ^ now)) < 0;
+        }
+    }
+    if (bad) atomicExch(F.err, 1);
+}
+
+// A pair close to the x axis (slots i, j) by itself: X's azimuth is that of
 // (d_y, d_z), so such a pair amplifies every rounding on the way to it by
 // r / |(d_y, d_z)|.  It takes the reference's orientation (lower index first)
 // and Gram-Schmidt sequence and the index-order displacement, so that its
 // result depends neither on the spatial sort nor on the walk that met it.
 // Both atoms' forces and torques, and the energy (word 6 n_pad), go into the
 // accumulator.
-__global__ void k_axis_pairs(PairParams P, IndexRecords R, AxisList axis, const int* __restrict__ order,
-                             const double* __restrict__ pos, FixAcc fix, int n_pad) {
-    const int count = min(*axis.count, axis.cap);
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
-        const int2 ij = axis.pairs[q];
-        const int id_i = order[ij.x], id_j = order[ij.y];
-        const int lo = id_i < id_j ? ij.x : ij.y, hi = id_i < id_j ? ij.y : ij.x;
-        float dx, dy, dz;
-        index_delta(P, R, pos, lo, hi, min(id_i, id_j), max(id_i, id_j), dx, dy, dz);
-        const float4 pl = R.posq_s[lo], dl = R.dipt_s[lo], ul = R.ind_s[lo];
-        const float4 ph = R.posq_s[hi], dh = R.dipt_s[hi], uh = R.ind_s[hi];
-        const f2 DX = bc2(dx), DY = bc2(dy), DZ = bc2(dz), R2 = dot2(DX, DY, DZ, DX, DY, DZ);
-        float r2, t;
-        un2(R2, r2, t);
-        const f2 RINV = bc2(rsqrtf(r2));
-        const f2 ZX = mul2(DX, RINV), ZY = mul2(DY, RINV), ZZ = mul2(DZ, RINV);
-        const bool yz = yz_differ_slot(dy, dz, pos, lo, hi);
-        f2 XX = add2(ZX, bc2(yz ? 1.0f : 0.0f)), XY = add2(ZY, bc2(yz ? 0.0f : 1.0f)), XZ = ZZ;
-        const f2 NDT = neg2(dot2(ZX, ZY, ZZ, XX, XY, XZ));
-        XX = fma2(ZX, NDT, XX);
-        XY = fma2(ZY, NDT, XY);
-        XZ = fma2(ZZ, NDT, XZ);
-        float xn;
-        un2(dot2(XX, XY, XZ, XX, XY, XZ), xn, t);
-        const f2 SN = bc2(xn > 0.0f ? rsqrtf(xn) : 1.0f);
-        XX = mul2(XX, SN);
-        XY = mul2(XY, SN);
-        XZ = mul2(XZ, SN);
-        const QiPair o =
-            qi_pair2(P, DX, DY, DZ, R2, RINV, r2, r2, XX, XY, XZ, bc2(pl.w), bc2(dl.x), bc2(dl.y), bc2(dl.z), bc2(ul.x),
-                     bc2(ul.y), bc2(ul.z), dl.w, 1.0f / dl.w, bc2(ph.w), bc2(dh.x), bc2(dh.y), bc2(dh.z), bc2(uh.x),
-                     bc2(uh.y), bc2(uh.z), dh.w, dh.w, 1.0f / dh.w, 1.0f / dh.w);
-        const f2 I[6] = {o.nfx, o.nfy, o.nfz, xneg2(o.tx), xneg2(o.ty), xneg2(o.tz)};
-        const f2 K[6] = {xneg2(o.nfx), xneg2(o.nfy), xneg2(o.nfz), xneg2(o.ux), xneg2(o.uy), xneg2(o.uz)};
-        for (int c = 0; c < 6; c++) {
-            float v, w;
-            un2(I[c], v, t);
-            un2(K[c], w, t);
-            fix_add(fix, (size_t)c * n_pad + lo, v);
-            fix_add(fix, (size_t)c * n_pad + hi, w);
-        }
-        float e;
-        un2(o.e2, e, t);
-        fix_add(fix, 6 * (size_t)n_pad, 0.5f * e);
+__device__ __forceinline__ void axis_pair(const PairParams& P, const IndexRecords& R, const int* __restrict__ order,
+                                          const double* __restrict__ pos, const FixAcc& fix, int n_pad, int i,
+                                          int j) {
+    const int id_i = order[i], id_j = order[j];
+    const int lo = id_i < id_j ? i : j, hi = id_i < id_j ? j : i;
+    float dx, dy, dz;
+    index_delta(P, R, pos, lo, hi, min(id_i, id_j), max(id_i, id_j), dx, dy, dz);
+    const float4 pl = R.posq_s[lo], dl = R.dipt_s[lo], ul = R.ind_s[lo];
+    const float4 ph = R.posq_s[hi], dh = R.dipt_s[hi], uh = R.ind_s[hi];
+    const f2 DX = bc2(dx), DY = bc2(dy), DZ = bc2(dz), R2 = dot2(DX, DY, DZ, DX, DY, DZ);
+    float r2, t;
+    un2(R2, r2, t);
+    const f2 RINV = bc2(rsqrtf(r2));
+    const f2 ZX = mul2(DX, RINV), ZY = mul2(DY, RINV), ZZ = mul2(DZ, RINV);
+    const bool yz = yz_differ_slot(dy, dz, pos, lo, hi);
+    f2 XX = add2(ZX, bc2(yz ? 1.0f : 0.0f)), XY = add2(ZY, bc2(yz ? 0.0f : 1.0f)), XZ = ZZ;
+    const f2 NDT = neg2(dot2(ZX, ZY, ZZ, XX, XY, XZ));
+    XX = fma2(ZX, NDT, XX);
+    XY = fma2(ZY, NDT, XY);
+    XZ = fma2(ZZ, NDT, XZ);
+    float xn;
+    un2(dot2(XX, XY, XZ, XX, XY, XZ), xn, t);
+    const f2 SN = bc2(xn > 0.0f ? rsqrtf(xn) : 1.0f);
+    XX = mul2(XX, SN);
+    XY = mul2(XY, SN);
+    XZ = mul2(XZ, SN);
+    const QiPair o =
+        qi_pair2(P, DX, DY, DZ, R2, RINV, r2, r2, XX, XY, XZ, bc2(pl.w), bc2(dl.x), bc2(dl.y), bc2(dl.z), bc2(ul.x),
+                 bc2(ul.y), bc2(ul.z), dl.w, 1.0f / dl.w, bc2(ph.w), bc2(dh.x), bc2(dh.y), bc2(dh.z), bc2(uh.x),
+                 bc2(uh.y), bc2(uh.z), dh.w, dh.w, 1.0f / dh.w, 1.0f / dh.w);
+    const f2 I[6] = {o.nfx, o.nfy, o.nfz, xneg2(o.tx), xneg2(o.ty), xneg2(o.tz)};
+    const f2 K[6] = {xneg2(o.nfx), xneg2(o.nfy), xneg2(o.nfz), xneg2(o.ux), xneg2(o.uy), xneg2(o.uz)};
+    float v[13];
+#pragma unroll
+    for (int c = 0; c < 6; c++) {
+        un2(I[c], v[c], t);
+        un2(K[c], v[6 + c], t);
     }
+    un2(o.e2, v[12], t);
+    v[12] *= 0.5f;
+    fix_add_checked(fix, n_pad, lo, hi, v);
 }
 
 // f: I side (force; sum of V, or the torque in MODE 2), g: the same for J atom
 // ((lane + s1) & 15) | (lane & 16).
+// MODE 3: only the pairs that the other modes leave to k_axis_pairs, evaluated
+// here by axis_pair.
 // OPEN: the charge-charge energy in FP64 (xi: the I atom's position, XJ: the J
 // atoms'), from the FP32 1/r by one Newton step.  The energy of an open system
 // is the small remainder of charge sums that grow with n^2 (20 e^2/nm of
@@ -1552,8 +1574,10 @@ __global__ void k_axis_pairs(PairParams P, IndexRecords R, AxisList axis, const 
 // 1e-6 to 5e-6 of it.
 template <int MODE, bool FOLD, bool MASK, bool OPEN>
 __device__ __forceinline__ void energy_item_walk(const PairParams& P, const double* __restrict__ pos,
-                                                 const IndexRecords& R, const AxisList& axis, const EItemTile& T,
-                                                 int lane, int i, int id, int jbase, float oix, float oiy, float oiz, float4 pi, float4 di, float4 ui, unsigned mk,
+                                                 const IndexRecords& R, const AxisList& axis,
+                                                 const int* __restrict__ order, const FixAcc& fix, int n_pad,
+                                                 const EItemTile& T, int lane, int i, int id, int jbase, float oix,
+                                                 float oiy, float oiz, float4 pi, float4 di, float4 ui, unsigned mk,
                                                  unsigned fm, float damp_r2, int s0, int s1, float (&f)[6],
                                                  float (&g)[6], float& en, d3 xi, const EItemPos* XJ, double& en64) {
     const int nxt = (lane + 1) & 31;
@@ -1659,10 +1683,15 @@ __device__ __forceinline__ void energy_item_walk(const PairParams& P, const doub
             for (int k = 0; k < 2; k++) {
                 const int j = k ? jb : ja;
                 float& r2 = k ? r2b : r2a;
-                const bool listed = MODE == 2 || r2 < kAxisListRange2 * P.damp_r2;
+                const bool listed = MODE == 2 || (MODE == 3 && !P.lab_energy) || r2 < kAxisListRange2 * P.damp_r2;
                 if (xr[k] > (listed ? kNearAxis2 : kNearAxisFar2)) continue;
+                if (MODE == 3) {
+                    if (listed && r2 < INFINITY) axis_pair(P, R, order, pos, fix, n_pad, i, j);
+                    continue;
+                }
                 if (listed) {
-                    if (r2 < INFINITY && axis_push(axis, i, j)) {
+                    if (r2 < INFINITY) {
+                        axis_push(axis, i, j);
                         r2 = INFINITY;
                         rv[k] = 0.0f;
                     }
@@ -1685,6 +1714,7 @@ __device__ __forceinline__ void energy_item_walk(const PairParams& P, const doub
             XY = pk2(xy[0], xy[1]);
             XZ = pk2(xz[0], xz[1]);
         }
+        if constexpr (MODE == 3) continue;
         if constexpr (MODE == 2) {
             const QiPair o = qi_pair2(P, DX, DY, DZ, R2, RINV, r2a, r2b, XX, XY, XZ, QIS, MIX, MIY, MIZ, UIX, UIY, UIZ,
                                       ti, iti, QJS, MJX, MJY, MJZ, UJX, UJY, UJZ, d.z, d.w, h.z, h.w);
@@ -1827,44 +1857,51 @@ struct EItemRaw {
     float4 p[32], d[32], u[32];
 };
 
-// Mixed-form energy kernel: warp items as in k_field_items, one I tile against
-// J tiles [c L, c L + L), in the spatial order of the field kernels (compact
-// tiles: few tile pairs fold or reach the damping range, and the FP32 offsets
-// are short).  Pairs that do not count (self, padding, the second visit on a
-// diagonal tile, listed partners) are masked out; k_energy_items_done
-// evaluates the partners.  GENERAL: MODE 2 for every tile pair.  OPEN: no
-// box, the charge energy in FP64.
-//
-// Bound by the FP32 pipe (82 FMA-pipe f32x2 instructions a step of two pairs
-// in MODE 0, about 100 in MODE 1).  The band-pair kernel before it ran in
-// index order: its tiles were as long as the input's rows (3.3 nm on a
-// lattice), so most tile pairs folded, and those within the damping range
-// took the quasi-internal frame walk (about 230).  Before -> now (the done
-// kernels included): 31 -> 27 us at 648 atoms, 210 -> 83 at 3,993, 535 -> 409
-// at 12,288, 24,200 -> 20,300 at 98,304.
-template <bool GENERAL, bool OPEN>
-__global__ void __launch_bounds__(32, 12) k_energy_items(
-    PairParams P, int L, const float4* __restrict__ posq, const float4* __restrict__ dipt,
-    const float4* __restrict__ indv, const int* __restrict__ order, const double4* __restrict__ tctr,
-    const double4* __restrict__ text, const double* __restrict__ pos, const int* __restrict__ exc_off,
-    const int* __restrict__ exc_j, const double* __restrict__ exc_m, const double* __restrict__ exc_s,
-    const int2* __restrict__ exc_tiles, IndexRecords R, AxisList axis, int n_pad,
-    double* __restrict__ energy_partial, FixAcc fix) {
-    __shared__ EItemTile T;
-    __shared__ EItemRaw raw;
-    __shared__ EItemPos XJ[1];
-    __shared__ double s_my[6][32];
-    const int lane = threadIdx.x;
+// Shared memory of an item.
+struct EItemShared {
+    EItemTile T;
+    EItemRaw raw;
+    double my[6][32];
+};
+
+// Records and tables of the energy items, by slot.
+struct EItemArrays {
+    const float4 *posq, *dipt, *indv;
+    const int* order;
+    const double4 *tctr, *text;
+    const double* pos;
+    const int *exc_off, *exc_j;
+    const double *exc_m, *exc_s;
+    const int2* exc_tiles;
+    IndexRecords R;
+    AxisList axis;
+    FixAcc fix;
+    int L, n_pad;
+};
+
+// Part `part` of `parts` of item `bx`: see k_energy_items.  SCAN: nothing but the
+// pairs that belong to k_axis_pairs (MODE 3).
+template <bool GENERAL, bool OPEN, bool SCAN>
+__device__ __forceinline__ void energy_item(const PairParams& P, const EItemArrays& A, EItemShared& S, EItemPos* XJ,
+                                            unsigned bx, unsigned part, unsigned parts,
+                                            double* __restrict__ item_energy) {
+    const int lane = threadIdx.x, L = A.L, n_pad = A.n_pad;
+    const float4 *__restrict__ posq = A.posq, *__restrict__ dipt = A.dipt, *__restrict__ indv = A.indv;
+    const int *__restrict__ order = A.order, *__restrict__ exc_j = A.exc_j;
+    const double *__restrict__ pos = A.pos, *__restrict__ exc_m = A.exc_m, *__restrict__ exc_s = A.exc_s;
+    const double4 *__restrict__ tctr = A.tctr, *__restrict__ text = A.text;
+    const FixAcc& fix = A.fix;
+    EItemTile& T = S.T;
+    EItemRaw& raw = S.raw;
     int p, q;
-    band_pair(blockIdx.x / L, p, q);
-    const int I = p * L + blockIdx.x % L, J0 = q * L, J1 = min(J0 + L, P.n_tiles);
-    const size_t item = (size_t)blockIdx.y * gridDim.x + blockIdx.x;
+    band_pair(bx / L, p, q);
+    const int I = p * L + (int)(bx % L), J0 = q * L, J1 = min(J0 + L, P.n_tiles);
     int J = max(J0, I);
     if (I >= P.n_tiles || J >= J1) {
-        if (lane == 0) energy_partial[item] = 0.0;
+        if (!SCAN && lane == 0) *item_energy = 0.0;
         return;
     }
-    const int s0 = 16 * blockIdx.y / gridDim.y, s1 = 16 * (blockIdx.y + 1) / gridDim.y;
+    const int s0 = 16 * part / parts, s1 = 16 * (part + 1) / parts;
     const float damp_r2 = kDampRange32 * P.damp_r2;
     const auto fetch = [&](int t) {
         copy16_async(&raw.p[lane], posq + t * 32 + lane);
@@ -1878,13 +1915,13 @@ __global__ void __launch_bounds__(32, 12) k_energy_items(
     const int id = order[i];
     d3 xi = {0.0, 0.0, 0.0};
     if (OPEN) xi = ld3(pos + 3 * (size_t)i);
-    const int2 et = exc_tiles[I];
+    const int2 et = A.exc_tiles[I];
     int e0 = 0, e1 = 0;
     unsigned own = 0u;
     if (i < P.n) {
         own = ~0u;
-        e0 = exc_off[i];
-        e1 = exc_off[i + 1];
+        e0 = A.exc_off[i];
+        e1 = A.exc_off[i + 1];
     }
     float gdx = 0.f, gdy = 0.f, gdz = 0.f;
     unsigned gfl = 0u;
@@ -1896,7 +1933,7 @@ __global__ void __launch_bounds__(32, 12) k_energy_items(
         gfl = g.fmask | (g.fold ? 8u : 0u) | (g.near ? 16u : 0u);
     }
 #pragma unroll
-    for (int k = 0; k < 6; k++) s_my[k][lane] = 0.0;
+    for (int k = 0; k < 6; k++) S.my[k][lane] = 0.0;
     double energy = 0.0;
     for (; J < J1; J++) {
         const int jbase = J * 32, jid = order[jbase + lane];
@@ -1936,9 +1973,12 @@ __global__ void __launch_bounds__(32, 12) k_energy_items(
         const float ox = pi.x - dx, oy = pi.y - dy, oz = pi.z - dz;
         float f[6], g[6], en;
 #define TDP_EWALK(M, F, K) \
-    energy_item_walk<M, F, K, OPEN>(P, pos, R, axis, T, lane, i, id, jbase, ox, oy, oz, pi, di, ui, mk, fl, damp_r2, \
-                                    s0, s1, f, g, en, xi, XJ, energy)
-        if constexpr (GENERAL) {
+    energy_item_walk<M, F, K, OPEN>(P, pos, A.R, A.axis, order, fix, n_pad, T, lane, i, id, jbase, ox, oy, oz, pi, di, \
+                                    ui, mk, fl, damp_r2, s0, s1, f, g, en, xi, XJ, energy)
+        if constexpr (SCAN) {
+            TDP_EWALK(3, true, true);
+            continue;
+        } else if constexpr (GENERAL) {
             TDP_EWALK(2, true, true);
         } else if (plain) {
             if (fl & 8u) TDP_EWALK(0, true, false);
@@ -1957,13 +1997,56 @@ __global__ void __launch_bounds__(32, 12) k_energy_items(
 #pragma unroll
         for (int k = 0; k < 6; k++) {
             fix_add(fix, (size_t)k * n_pad + jbase + jl, g[k]);
-            s_my[k][lane] += (double)f[k];
+            S.my[k][lane] += (double)f[k];
         }
     }
+    if constexpr (!SCAN) {
 #pragma unroll
-    for (int k = 0; k < 6; k++) fix_add(fix, (size_t)k * n_pad + i, s_my[k][lane]);
-    energy = warp_sum(energy);
-    if (lane == 0) energy_partial[item] = energy;
+        for (int k = 0; k < 6; k++) fix_add(fix, (size_t)k * n_pad + i, S.my[k][lane]);
+        energy = warp_sum(energy);
+        if (lane == 0) *item_energy = energy;
+    }
+}
+
+// Mixed-form energy kernel: warp items as in k_field_items, one I tile against
+// J tiles [c L, c L + L), in the spatial order of the field kernels (compact
+// tiles: few tile pairs fold or reach the damping range, and the FP32 offsets
+// are short).  Pairs that do not count (self, padding, the second visit on a
+// diagonal tile, listed partners) are masked out; k_energy_items_done
+// evaluates the partners.  GENERAL: MODE 2 for every tile pair.  OPEN: no
+// box, the charge energy in FP64.
+//
+// Bound by the FP32 pipe (82 FMA-pipe f32x2 instructions a step of two pairs
+// in MODE 0, about 100 in MODE 1).  The band-pair kernel before it ran in
+// index order: its tiles were as long as the input's rows (3.3 nm on a
+// lattice), so most tile pairs folded, and those within the damping range
+// took the quasi-internal frame walk (about 230).  Before -> now (the done
+// kernels included): 31 -> 27 us at 648 atoms, 210 -> 83 at 3,993, 535 -> 409
+// at 12,288, 24,200 -> 20,300 at 98,304.
+template <bool GENERAL, bool OPEN>
+__global__ void __launch_bounds__(32, 12)
+    k_energy_items(PairParams P, EItemArrays A, double* __restrict__ energy_partial) {
+    __shared__ EItemShared S;
+    __shared__ EItemPos XJ;
+    energy_item<GENERAL, OPEN, false>(P, A, S, &XJ, blockIdx.x, blockIdx.y, gridDim.y,
+                                      energy_partial + (size_t)blockIdx.y * gridDim.x + blockIdx.x);
+}
+
+// The pairs that the walks left out, each by axis_pair: from the list, or,
+// where that could not hold them, from a second pass over the items, which
+// meets the same pairs.  The sums are integers, so the two give the same bits.
+__global__ void __launch_bounds__(32) k_axis_pairs(PairParams P, EItemArrays A, int items) {
+    __shared__ EItemShared S;
+    const int count = *A.axis.count;
+    if (count <= A.axis.cap) {
+        for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
+            const int2 ij = A.axis.pairs[q];
+            axis_pair(P, A.R, A.order, A.pos, A.fix, A.n_pad, ij.x, ij.y);
+        }
+        return;
+    }
+    for (int bx = blockIdx.x; bx < items; bx += gridDim.x)
+        energy_item<false, false, true>(P, A, S, nullptr, bx, 0, 1, nullptr);
 }
 
 // Fixed-point force and torque sums -> FP64 in index order, clearing them,
@@ -2407,20 +2490,12 @@ void launch_energy<float>(const Dev& d, cudaStream_t st) {
     FixAcc fix = fix_of(d);
     fix.scale = d.fix_scale_energy;
     const IndexRecords rec{(const float4*)d.posq, d.tctr, pq, dp, u};
-    const AxisList axis{d.axis_pairs, d.axis_count, d.axis_cap};
-    if (d.pp.lab_energy && !d.pp.periodic)
-        k_energy_items<false, true><<<grid, 32, 0, st>>>(d.pp, L, pq, dp, u, d.order, d.tctr_s, d.text_s, d.pos_s,
-                                                         d.exs_off, d.exs_j, d.exs_m, d.exs_s, d.exs_tiles, rec, axis,
-                                                         d.n_pad, d.energy_partial, fix);
-    else if (d.pp.lab_energy)
-        k_energy_items<false, false><<<grid, 32, 0, st>>>(d.pp, L, pq, dp, u, d.order, d.tctr_s, d.text_s, d.pos_s, d.exs_off,
-                                                   d.exs_j, d.exs_m, d.exs_s, d.exs_tiles, rec, axis, d.n_pad,
-                                                   d.energy_partial, fix);
-    else
-        k_energy_items<true, false><<<grid, 32, 0, st>>>(d.pp, L, pq, dp, u, d.order, d.tctr_s, d.text_s, d.pos_s, d.exs_off,
-                                                  d.exs_j, d.exs_m, d.exs_s, d.exs_tiles, rec, axis, d.n_pad,
-                                                  d.energy_partial, fix);
-    k_axis_pairs<<<148, 64, 0, st>>>(d.pp, rec, axis, d.order, d.pos_s, fix, d.n_pad);
+    const EItemArrays A{pq, dp, u, d.order, d.tctr_s, d.text_s, d.pos_s, d.exs_off, d.exs_j, d.exs_m, d.exs_s,
+                        d.exs_tiles, rec, AxisList{d.axis_pairs, d.axis_count, d.axis_cap}, fix, L, d.n_pad};
+    if (d.pp.lab_energy && !d.pp.periodic) k_energy_items<false, true><<<grid, 32, 0, st>>>(d.pp, A, d.energy_partial);
+    else if (d.pp.lab_energy) k_energy_items<false, false><<<grid, 32, 0, st>>>(d.pp, A, d.energy_partial);
+    else k_energy_items<true, false><<<grid, 32, 0, st>>>(d.pp, A, d.energy_partial);
+    k_axis_pairs<<<2 * 148, 32, 0, st>>>(d.pp, A, (int)grid.x);
     k_energy_items_done<<<d.n_pad / 128, 128, 0, st>>>(d.pp, pq, dp, u, d.order, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
                                                        d.exs_s, rec, d.axis_count, d.n_pad, d.fixacc,
                                                        1.0 / fix.scale, d.n_eblk,
