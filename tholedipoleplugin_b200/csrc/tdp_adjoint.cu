@@ -504,12 +504,16 @@ static inline int nb(int n) { return (n + 127) / 128; }
 
 // J splits of k_pair_vjp_fast: whole rounds of its 12 resident blocks an SM,
 // the time going with rounds / splits (12,288 atoms: 7 splits made 1.5 rounds,
-// 1666 us; 9 make 1.95, 1479).
+// 1666 us; 9 make 1.95, 1479).  Every split has a list row for each atom, so
+// no more of them than make two rounds: the lists stay within 95 MB, or one
+// row an atom from 56,833 atoms on (98,304 atoms: 4 splits would save an
+// eighth of the rounds and take 329 MB in place of 82).
 static int vjp_splits(int n) {
     const long blocks = (std::max(n, 1) + adj::kVjpTile - 1) / adj::kVjpTile, resident = 12L * 148;
+    const long most = std::min((long)adj::kVjpSplit, 2 * resident / blocks);
     int best = 1;
     const auto rounds = [&](int s) { return (double)((blocks * s + resident - 1) / resident) / s; };
-    for (int s = 2; s <= adj::kVjpSplit; s++)
+    for (int s = 2; s <= most; s++)
         if (rounds(s) < rounds(best)) best = s;
     return best;
 }
