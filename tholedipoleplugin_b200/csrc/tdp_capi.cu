@@ -470,15 +470,16 @@ void kernel_end(tdp_handle* h, size_t k) {
     if (h->timing) TDP_CUDA(cudaEventRecord(h->kev[2 * k + 1], h->stream));
 }
 
-// One mutual-field matvec (pair kernel), timed and counted.
+// One mutual-field matvec (pair kernel), timed and counted.  stop: all-pairs
+// form only.
 template <class R>
-void matvec(tdp_handle* h) {
+void matvec(tdp_handle* h, CgStop stop = {}) {
     size_t k = kernel_begin(h, 0);
     if (h->ew) {
         ewald_matvec<R>(h->ew, h->d, h->stream);
         h->launches += ewald_last_launches(h->ew);
     } else {
-        launch_field<R>(h->d, 1, h->stream);
+        launch_field<R>(h->d, 1, h->stream, stop);
         h->launches++;
     }
     kernel_end(h, k);
@@ -529,8 +530,8 @@ void solve_cg(tdp_handle* h, bool fused = false, bool cold = true) {
     // cluster, and the epsilon reaches the host through pinned memory.  Where
     // the matvec is so short that its parts are split (field_parts), the next
     // iteration is queued before the host has seen the epsilon; its kernels do
-    // nothing if that shows the solve has stopped.  (Not while the stages are
-    // timed.)
+    // nothing if that shows the solve has stopped (CgStop).  Not while the
+    // stages are timed.
     const bool one = cg_cluster(d), collect = cg_collects(d) && !h->ew && sizeof(R) == 4;
     const bool ahead = one && !h->ew && d.field_parts > 1 && !h->timing;
     // The residual of y in scalar slot `slot` (use_partial: of a matvec).
@@ -548,7 +549,7 @@ void solve_cg(tdp_handle* h, bool fused = false, bool cold = true) {
     };
     // Queues the iteration from slot `from`; conditional: only if that has not stopped.
     const auto queue = [&](int from, bool conditional) {
-        const double* stop = conditional ? d.scal_eps + from : nullptr;
+        const CgStop stop = conditional ? CgStop{d.scal_eps + from, h->target_eps} : CgStop{};
         if (!one) {
             matvec<R>(h);
             launch_cg_q(d, st);
@@ -560,15 +561,15 @@ void solve_cg(tdp_handle* h, bool fused = false, bool cold = true) {
         clear_eps(h, from + 1);
         if (collect) {
             size_t k = kernel_begin(h, 0);
-            launch_cg_matvec(d, stop, h->target_eps, st);
+            launch_cg_matvec(d, stop, st);
             kernel_end(h, k);
             h->launches++;
             h->matvecs++;
         } else {
-            matvec<R>(h);
+            matvec<R>(h, stop);
         }
         if (conditional) h->matvecs--;   // counted when the host takes the step
-        launch_cg_step<R>(d, from, collect, stop, h->target_eps, eps_word(h, from + 1), st);
+        launch_cg_step<R>(d, from, collect, stop, eps_word(h, from + 1), st);
         h->launches++;
     };
     // Residual of the starting point (mu = alpha E, or the previous solution).

@@ -104,9 +104,22 @@ template <class R> void launch_pack(const Dev& d, cudaStream_t st);
 template <class R> void launch_rotate(const Dev& d, cudaStream_t st);
 // I tiles per item of the mixed field kernel.
 constexpr int kFieldNS = 2;
-template <class R> void launch_field(const Dev& d, int kind, cudaStream_t st);
-template <> void launch_field<float>(const Dev& d, int kind, cudaStream_t st);
-template <> void launch_field<double>(const Dev& d, int kind, cudaStream_t st);
+// Whether the solve had stopped before a launch that was queued before the
+// host knew: eps (may be null: never) at or below the target, or not finite.
+struct CgStop {
+    const double* eps = nullptr;
+    double target = 0.0;
+    __device__ __forceinline__ bool stopped() const {
+        if (!eps) return false;
+        const double e = *eps;
+        return !(e > target && e < (double)INFINITY);
+    }
+};
+// stop: the pair kernels do nothing where it says so (the mixed form's
+// k_field_done then collects sums of zero).
+template <class R> void launch_field(const Dev& d, int kind, cudaStream_t st, CgStop stop = {});
+template <> void launch_field<float>(const Dev& d, int kind, cudaStream_t st, CgStop stop);
+template <> void launch_field<double>(const Dev& d, int kind, cudaStream_t st, CgStop stop);
 // Pair forces, torques (index order) and the energy from the records of
 // launch_pack_ind.
 template <class R> void launch_energy(const Dev& d, cudaStream_t st);
@@ -125,18 +138,17 @@ template <class R> void launch_pack_total(const Dev& d, cudaStream_t st);
 template <class R> void launch_fused_done(const Dev& d, cudaStream_t st);
 void launch_cg_q(const Dev& d, cudaStream_t st);
 // One CG iteration in two launches for systems that fit a cluster (cg_cluster):
-// the matvec, and everything after it.  stop_eps (may be null): the launches do
-// nothing where *stop_eps shows that the solve has stopped.  host_eps: pinned
-// word that receives the new epsilon.  collect: the all-pairs matvec was
+// the matvec, and everything after it.  stop: the launches do nothing where the
+// solve has stopped.  host_eps: pinned word that receives the new epsilon.
+// collect: the all-pairs matvec was
 // launch_cg_matvec.
 bool cg_cluster(const Dev& d);
 bool cg_collects(const Dev& d);
 template <class R>
 void launch_cg_start(const Dev& d, int slot, bool use_partial, double* host_eps, cudaStream_t st);
-void launch_cg_matvec(const Dev& d, const double* stop_eps, double target, cudaStream_t st);
+void launch_cg_matvec(const Dev& d, CgStop stop, cudaStream_t st);
 template <class R>
-void launch_cg_step(const Dev& d, int slot, bool collect, const double* stop_eps, double target, double* host_eps,
-                    cudaStream_t st);
+void launch_cg_step(const Dev& d, int slot, bool collect, CgStop stop, double* host_eps, cudaStream_t st);
 void launch_cg_update(const Dev& d, int slot, cudaStream_t st);
 template <class R> void launch_cg_p(const Dev& d, int prev, int slot, cudaStream_t st);
 // mu0 != NULL: the packed operand is mu - mu0 (the final check of a fused start).

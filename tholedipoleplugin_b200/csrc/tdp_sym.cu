@@ -165,18 +165,6 @@ __device__ __forceinline__ unsigned partner_bits(const int* __restrict__ exc_j, 
     return b;
 }
 
-// Whether the solve had stopped before this launch, which was queued before
-// the host knew: eps (may be null) at or below the target, or not finite.
-struct CgStop {
-    const double* eps;
-    double target;
-    __device__ __forceinline__ bool stopped() const {
-        if (!eps) return false;
-        const double e = *eps;
-        return !(e > target && e < (double)INFINITY);
-    }
-};
-
 template <class R>
 __device__ __forceinline__ void store_operand(typename Vec4T<R>::type* v, int k, d3 a, double t) {
     typename Vec4T<R>::type o;
@@ -720,7 +708,8 @@ __global__ void __launch_bounds__(128, 4)
     k_field_bands(PairParams P, int BT, const double4* __restrict__ posq, const double4* __restrict__ jvec,
                   const double4* __restrict__ tctr, const double4* __restrict__ text, const int* __restrict__ exc_off,
                   const int* __restrict__ exc_j, const double* __restrict__ exc_scale,
-                  const int2* __restrict__ exc_tiles, int n_pad, double* __restrict__ partial) {
+                  const int2* __restrict__ exc_tiles, int n_pad, double* __restrict__ partial, CgStop stop) {
+    if (stop.stopped()) return;
     extern __shared__ __align__(16) unsigned char smem[];
     const int NA = BT * 32, warps = BT / 2;
     Rec64 T;
@@ -861,7 +850,8 @@ __global__ void __launch_bounds__(96)
     k_field_slots(PairParams P, int fused, const double4* __restrict__ posq, const double4* __restrict__ jvec,
                   const double4* __restrict__ lab, const double* __restrict__ pos, const int* __restrict__ exc_off,
                   const int* __restrict__ exc_j, const double* __restrict__ exc_m, const double* __restrict__ exc_s,
-                  int n_pad, int nslot, double* __restrict__ partial) {
+                  int n_pad, int nslot, double* __restrict__ partial, CgStop stop) {
+    if (stop.stopped()) return;
     __shared__ double s_part[3][3][32];
     const int lane = threadIdx.x & 31, c = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;
     double f[3] = {0.0, 0.0, 0.0};
@@ -2359,19 +2349,18 @@ void slot_sum(const Dev& d, int ncomp, cudaStream_t st) {
 // permanent field plus T mu0 in one walk (operand vec = m + mu0, see
 // field_partners).
 template <>
-void launch_field<float>(const Dev& d, int kind, cudaStream_t st) {
+void launch_field<float>(const Dev& d, int kind, cudaStream_t st, CgStop stop) {
     const int L = d.field_L, B = std::max(L, kFieldNS), nb = (d.pp.n_tiles + B - 1) / B;
     const dim3 grid((unsigned)((long)nb * (nb + 1) / 2 * (B / std::min(L, kFieldNS))), d.field_parts);
     const float4 *pq = (const float4*)d.posq_s, *op = (const float4*)(kind == 0 ? d.dipt_s : d.vec_s);
     const unsigned blocks = (unsigned)((d.n_pad + 127) / 128);
     if (kind == 1) {
-        k_field_items<1, kFieldNS><<<grid, 32, 0, st>>>(d.pp, L, pq, op, d.tctr_s, d.text_s, d.pos_s, d.exs_off,
-                                                        d.exs_j, d.exs_s, d.exs_tiles, d.n_pad, fix_of(d), CgStop{nullptr, 0.0});
+        launch_cg_matvec(d, stop, st);
         k_field_done<1><<<blocks, 128, 0, st>>>(d.pp, 0, pq, op, nullptr, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
                                                 d.exs_s, d.n_pad, d.fixacc, 1.0 / d.fix_scale, d.partial);
     } else {
         k_field_items<0, kFieldNS><<<grid, 32, 0, st>>>(d.pp, L, pq, op, d.tctr_s, d.text_s, d.pos_s, d.exs_off,
-                                                        d.exs_j, d.exs_m, d.exs_tiles, d.n_pad, fix_of(d), CgStop{nullptr, 0.0});
+                                                        d.exs_j, d.exs_m, d.exs_tiles, d.n_pad, fix_of(d), stop);
         k_field_done<0><<<blocks, 128, 0, st>>>(d.pp, kind == 2 ? 1 : 0, pq, op, (const float4*)d.dipt_s, d.pos_s,
                                                 d.exs_off, d.exs_j, d.exs_m, d.exs_s, d.n_pad, d.fixacc,
                                                 1.0 / d.fix_scale, d.partial);
@@ -2379,7 +2368,7 @@ void launch_field<float>(const Dev& d, int kind, cudaStream_t st) {
 }
 
 template <>
-void launch_field<double>(const Dev& d, int kind, cudaStream_t st) {
+void launch_field<double>(const Dev& d, int kind, cudaStream_t st, CgStop stop) {
     const int BT = d.field_L, nb = (d.pp.n_tiles + BT - 1) / BT;
     const dim3 grid((unsigned)(nb * (nb + 1) / 2), d.field_parts);
     const size_t smem = field_smem(BT);
@@ -2387,16 +2376,16 @@ void launch_field<double>(const Dev& d, int kind, cudaStream_t st) {
     if (kind == 1) {
         cudaFuncSetAttribute(k_field_bands<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         k_field_bands<1><<<grid, 16 * BT, smem, st>>>(d.pp, BT, pq, op, d.tctr_s, d.text_s, d.exs_off, d.exs_j,
-                                                      d.exs_s, d.exs_tiles, d.n_pad, d.partial);
+                                                      d.exs_s, d.exs_tiles, d.n_pad, d.partial, stop);
         k_field_slots<1><<<d.n_pad / 32, 96, 0, st>>>(d.pp, 0, pq, op, nullptr, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
-                                                      d.exs_s, d.n_pad, nb * d.field_parts, d.partial);
+                                                      d.exs_s, d.n_pad, nb * d.field_parts, d.partial, stop);
     } else {
         cudaFuncSetAttribute(k_field_bands<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         k_field_bands<0><<<grid, 16 * BT, smem, st>>>(d.pp, BT, pq, op, d.tctr_s, d.text_s, d.exs_off, d.exs_j,
-                                                      d.exs_m, d.exs_tiles, d.n_pad, d.partial);
+                                                      d.exs_m, d.exs_tiles, d.n_pad, d.partial, stop);
         k_field_slots<0><<<d.n_pad / 32, 96, 0, st>>>(d.pp, kind == 2 ? 1 : 0, pq, op, (const double4*)d.dipt_s,
                                                       d.pos_s, d.exs_off, d.exs_j, d.exs_m, d.exs_s, d.n_pad,
-                                                      nb * d.field_parts, d.partial);
+                                                      nb * d.field_parts, d.partial, stop);
     }
 }
 
@@ -2447,19 +2436,18 @@ template void launch_cg_start<double>(const Dev&, int, bool, double*, cudaStream
 
 // Mixed all-pairs matvec without the collection of its sums, which
 // launch_cg_step does.
-void launch_cg_matvec(const Dev& d, const double* stop_eps, double target, cudaStream_t st) {
+void launch_cg_matvec(const Dev& d, CgStop stop, cudaStream_t st) {
     const int L = d.field_L, B = std::max(L, kFieldNS), nb = (d.pp.n_tiles + B - 1) / B;
     const dim3 grid((unsigned)((long)nb * (nb + 1) / 2 * (B / std::min(L, kFieldNS))), d.field_parts);
     k_field_items<1, kFieldNS><<<grid, 32, 0, st>>>(d.pp, L, (const float4*)d.posq_s, (const float4*)d.vec_s, d.tctr_s,
                                                     d.text_s, d.pos_s, d.exs_off, d.exs_j, d.exs_s, d.exs_tiles,
-                                                    d.n_pad, fix_of(d), CgStop{stop_eps, target});
+                                                    d.n_pad, fix_of(d), stop);
 }
 
 template <class R>
-void launch_cg_step(const Dev& d, int slot, bool collect, const double* stop_eps, double target, double* host_eps,
-                    cudaStream_t st) {
+void launch_cg_step(const Dev& d, int slot, bool collect, CgStop stop, double* host_eps, cudaStream_t st) {
     CgArrays A = cg_arrays(d, slot, host_eps);
-    A.stop = CgStop{stop_eps, target};
+    A.stop = stop;
     typedef typename Vec4T<R>::type V4;
     const V4* pq = (const V4*)d.posq_s;
     V4* vec = (V4*)d.vec_s;
@@ -2479,8 +2467,8 @@ void launch_cg_step(const Dev& d, int slot, bool collect, const double* stop_eps
     else TDP_CG_STEP(false, 4);
 #undef TDP_CG_STEP
 }
-template void launch_cg_step<float>(const Dev&, int, bool, const double*, double, double*, cudaStream_t);
-template void launch_cg_step<double>(const Dev&, int, bool, const double*, double, double*, cudaStream_t);
+template void launch_cg_step<float>(const Dev&, int, bool, CgStop, double*, cudaStream_t);
+template void launch_cg_step<double>(const Dev&, int, bool, CgStop, double*, cudaStream_t);
 
 template <>
 void launch_energy<float>(const Dev& d, cudaStream_t st) {
