@@ -1,6 +1,6 @@
-"""The mixed form's list of pairs close to the x axis, where it is nearly full, just too short and far too
-short (65,536 pairs: a chain of 362 atoms has 65,341, one of 363 has 65,703): the same bits in every run,
-and the plain form's results.
+"""The mixed form's list of pairs close to the x axis (16 an atom), where it is just full (a chain of 33
+atoms has 528 pairs), just too short (34: 561 pairs, room for 544) and far too short: the same bits in every
+run, and the plain form's results.
 
 Tolerances are the mixed form's: forces 2e-5 relative RMS, energy 1e-6 |E| + 3e-7 sqrt(sum (q_i q_j /
 r_ij)^2)."""
@@ -35,7 +35,7 @@ def random_chain(n):
                  rng.uniform(0.3e-3, 1.5e-3, n))
 
 
-@pytest.mark.parametrize("n", [362, 363, 400, 1000])
+@pytest.mark.parametrize("n", [32, 33, 34, 362, 363, 400, 1000])
 def test_chain_beyond_the_list(n):
     s = random_chain(n)
     runs = []

@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -1338,7 +1339,7 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
         d.partial = dalloc<double>((size_t)d.nslot * 6 * d.n_pad, o);
         if (d.fix_scale > 0.0) {
             d.fixacc = dalloc<unsigned long long>(6 * (size_t)d.n_pad + 1, o);
-            d.axis_cap = std::max(1 << 16, 16 * n);
+            d.axis_cap = (int)std::min(16L * n, (long)INT_MAX / 2);
             d.axis_pairs = dalloc<int2>(d.axis_cap, o);
             d.axis_count = dalloc<int>(1, o);
             d.fix_err = dalloc<int>(1, o);
