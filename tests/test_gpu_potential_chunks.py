@@ -28,3 +28,14 @@ def test_potential_blocks_and_chunks(n_side, method, points):
     with CudaCalcTholeDipoleForceKernel(s, precision="double") as k:
         got = k.getElectrostaticPotential(grid, s.positions)
     assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("waters", [42, 43, 85, 86])   # 126, 129, 255, 258 atoms: one, two and three staged steps
+@pytest.mark.parametrize("points", [1, 300])
+def test_potential_about_one_staged_step(waters, points):
+    s = S.water_cluster(waters, np.random.default_rng(waters), polarization=S.DIRECT)
+    grid = np.random.default_rng(points).uniform(-0.5, 2.5, size=(points, 3))
+    ref = O.potential(s, grid, "port")
+    with CudaCalcTholeDipoleForceKernel(s, precision="double") as k:
+        got = k.getElectrostaticPotential(grid, s.positions)
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))

@@ -852,8 +852,9 @@ void launch_forces_out_fixed(const Dev& d, const int* atom_index, int padded, lo
     k_forces_out_fixed<<<nblk(d.n, kVecThreads), kVecThreads, 0, st>>>(d.n, d.ftotal, atom_index, padded,
                                                                         (unsigned long long*)acc);
 }
-// Chunks of atoms for ng points: enough blocks for 16 resident per SM (the
-// register limit) in whole rounds, no chunk below one staged step.
+// Chunks of atoms for ng points: about 16 blocks an SM (the register limit), no
+// more chunks than staged steps of kPotAtoms atoms (an even split of them, so
+// that a chunk holds more than half a step).
 int potential_chunks(int n, int ng) {
     const long gb = nblk(ng, kPotPoints);
     const long want = (16L * 148 + gb - 1) / gb;
