@@ -32,3 +32,19 @@ def test_tile_edges_and_partner_scales(n, method, polarization, tol):
         got = k.getInducedDipoles(s.positions)
     assert rel_rms(got, ref) < tol
 
+
+
+@pytest.mark.parametrize("n", [4, 31, 32, 33, 65, 200])
+@pytest.mark.parametrize("method", [S.NO_CUTOFF, S.PME])
+def test_mutual_dipoles_within_the_solver_target(n, method):
+    """A solve stopped at an RMS Jacobi step of eps is off by at most eps / lambda per atom, lambda the
+    smallest eigenvalue of 1 - alpha T, which is above 0.5 at these polarizabilities: a relative RMS of
+    2 eps / (sqrt(3) rms mu), and 1e-10 for the oracle's own target and the sums."""
+    s = F.small_random_system(n, seed=n, method=method, polarization=S.MUTUAL, box=3.0)
+    s = s.copy(polarizabilities=0.1 * s.polarizabilities, target_eps=1e-13, max_iter=5000)
+    ref = O.compute(s.copy(target_eps=1e-12), "port").induced
+    with CudaCalcTholeDipoleForceKernel(s, precision="double") as k:
+        got = k.getInducedDipoles(s.positions)
+        assert k.solverStats()["converged"] == 1
+    rms = float(np.sqrt(np.mean(ref ** 2)))
+    assert rel_rms(got, ref) < 2e-13 / (np.sqrt(3.0) * rms) + 1e-10
