@@ -1232,10 +1232,8 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
             d.n_eblk = 1;
         } else if (h->precision == TDP_PRECISION_MIXED && !variational) {
             // Mixed all-pairs form: the walks' sums go into the fixed-point
-            // accumulator and one slot.  Each atom's word receives at most
-            // `adds` of them, of magnitude < 2^23, so with 2^bits units per
-            // e/nm^2 the total stays below 2^63.  (What k_axis_pairs adds to
-            // the energy kernel's words is checked add by add.)
+            // accumulator and one slot.  (What k_axis_pairs adds to the energy
+            // kernel's words is checked add by add.)
             d.nslot = 1;
             // Items of the field kernel: J chunks as long as seven rounds of
             // resident warps (16 an SM) allow (matvec with L = 1, 2, 4, 8, 16:
@@ -1254,11 +1252,7 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
                 }
             d.field_parts = 1;
             while (d.field_parts < 8 && 2 * d.field_parts * visits <= 9L * 148) d.field_parts *= 2;
-            const long adds = d.field_parts * (groups + (nt + d.field_L - 1) / d.field_L);
-            int lg = 0;
-            while ((1L << lg) < adds) lg++;
-            const int bits = std::min(32, 40 - lg);
-            d.fix_scale = std::ldexp(1.0, bits);
+            d.fix_scale = std::ldexp(1.0, fix_bits(fix_adds(nt, kFieldNS, d.field_L, d.field_parts)));
             d.fix_limit = std::ldexp(1.0, 23);
             // The energy kernel's items (one I tile, 12 warps an SM).
             const long evisits = (long)nt * (nt + 1) / 2, eresident = 12L * 148;
@@ -1270,9 +1264,7 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
             while (d.energy_parts < 8 && 2 * d.energy_parts * evisits <= 9L * 148) d.energy_parts *= 2;
             const long echunks = (nt + d.energy_L - 1) / d.energy_L;
             d.n_eblk = (int)(echunks * (echunks + 1) / 2 * d.energy_L * d.energy_parts);
-            lg = 0;
-            while ((1L << lg) < d.energy_parts * (nt + echunks)) lg++;
-            d.fix_scale_energy = std::ldexp(1.0, std::min(32, 40 - lg));
+            d.fix_scale_energy = std::ldexp(1.0, fix_bits(fix_adds(nt, 1, d.energy_L, d.energy_parts)));
         }
 
         std::vector<int> eoff(n + 1, 0), ej;

@@ -45,6 +45,27 @@ inline void upload(void* dst, const void* src, size_t bytes) {
     if (bytes) TDP_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
 }
 
+// The mixed pair kernels' fixed-point accumulator.  Items are groups of `group`
+// I tiles against chunks of `chunk` J tiles, the walks split into `parts`: a
+// tile's words get one sum a part from every group that walks over the tile
+// (J side) and from every chunk that the tile's own group walks (I side).
+inline long fix_adds(long tiles, long group, long chunk, long parts) {
+    const long chunks = (tiles + chunk - 1) / chunk;
+    long most = 1;
+    for (long t = 0; t < tiles; t++) {
+        const long g = t / group;
+        most = std::max(most, parts * (g + 1 + chunks - g * group / chunk));
+    }
+    return most;
+}
+// Bits below the unit (1 e/nm^2 or e^2/nm^2), 32 at most: sums of magnitude
+// < 2^23 each, `adds` of them, stay below 2^63.
+inline int fix_bits(long adds) {
+    int lg = 0;
+    while ((1L << lg) < adds) lg++;
+    return std::min(32, 40 - lg);
+}
+
 // Validation: TholeDipoleForceImpl::initialize (openmmapi/src/TholeDipoleForceImpl.cpp:52-108)
 // plus the inputs on which the reference dereferences null or out-of-range
 // memory (rotation of an atom with Z set and no X atom, RTDF.cpp:556-568).
