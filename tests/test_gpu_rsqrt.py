@@ -39,7 +39,8 @@ def test_error(tmp_path):
     subprocess.run([B.nvcc(), "-std=c++17", "-O3", *B.ARCH, "-ftz=true", "-shared", "-Xcompiler", "-fPIC", "-I", B.CSRC,
                     "-o", str(lib), str(src)], check=True)
     rng = np.random.default_rng(3)
-    m = np.concatenate([1.0 + rng.random(20000), 1.0 + 2.0 ** -rng.integers(1, 53, 400), 2.0 - 2.0 ** -rng.integers(0, 52, 400)])
+    m = np.concatenate([1.0 + rng.random(20000), 1.0 + 2.0 ** -rng.integers(1, 53, 400),
+                        2.0 - 2.0 ** -rng.integers(0, 52, 400)])
     x = np.concatenate([np.ldexp(m, e) for e in [*range(-34, 16), -1022, -1021, -501, 500, 1022]])
     y = np.zeros_like(x)
     p = C.POINTER(C.c_double)
@@ -60,11 +61,11 @@ def test_pair_whose_yz_distance_squared_is_subnormal(offset):
     pos[0] = [0.0, 0.0, 0.0]
     axis = np.full((n, 4), -1, dtype=np.int32)
     axis[:, 0] = S.NOAXISTYPE
+    charges, dipoles = rng.permutation(np.resize([0.4, -0.4], n)), rng.normal(scale=0.01, size=(n, 3))
     forces = []
     for y in (offset, 1e-6):
         pos[40] = [5.0, y, 0.0]
-        s = S.TholeSystem(positions=pos.copy(), charges=rng.permutation(np.resize([0.4, -0.4], n)) if not forces else s.charges,
-                          dipoles=rng.normal(scale=0.01, size=(n, 3)) if not forces else s.dipoles,
+        s = S.TholeSystem(positions=pos.copy(), charges=charges, dipoles=dipoles,
                           polarizabilities=np.full(n, 1e-4), tholes=np.full(n, 0.3), axis=axis,
                           cov12=[[] for _ in range(n)], cov13=[[] for _ in range(n)], polarization=S.DIRECT)
         with CudaCalcTholeDipoleForceKernel(s, precision="double") as k:

@@ -297,7 +297,8 @@ __device__ __forceinline__ float rsq(float x) { return rsqrtf(x); }
 // (260 with damping), where evaluating the routine with the atom's multipoles
 // set to unit vectors and a dual number for the Thole factor takes about
 // 4,500 (256 clusters, FP64: reverse pass 2.5 -> 1.1 ms; 12,288-atom box:
-// k_pair_vjp_slow 896 -> 255 us, k_pair_vjp_fast 1927 -> 1561 us).  lam: 2 (Mutual) or 0.  acc[0..6] += dq, dm[3], du[3], acc[7] += dt.
+// k_pair_vjp_slow 896 -> 255 us, k_pair_vjp_fast 1927 -> 1561 us).  lam: 2
+// (Mutual) or 0.  acc[0..6] += dq, dm[3], du[3], acc[7] += dt.
 template <class T, bool DAMP>
 __device__ __forceinline__ void pair_vjp_me(V3T<T> d, T sg, T q, V3T<T> m, V3T<T> u, T t, T qo, V3T<T> mo, V3T<T> uo,
                                             T to, T mS, T iS, T damp_r2, T lam, T gE, V3T<T> gF, V3T<T> gFo,

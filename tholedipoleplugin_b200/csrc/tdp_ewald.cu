@@ -1269,13 +1269,14 @@ __global__ void k_pme_influence(PmeGrid G, double alpha, const double* __restric
 // 1), the whole field into partial slot 0; FORCE: force q E + (d.grad) E in
 // components 0..2 and E in 3..5, for k_ew_finish.
 template <class R, class GT, int KIND, bool FORCE>
-__global__ void __launch_bounds__(kPmeThreads) k_pme_gather(PairParams P, EwParams EP, const double* __restrict__ real_part, EwExceptions X,
-                             const typename Vec4T<R>::type* __restrict__ lab_s, PmeGrid G, int n, int n_pad,
-                             double selfc, const double* __restrict__ pos_s,
-                             const typename Vec4T<R>::type* __restrict__ posq_s,
-                             const typename Vec4T<R>::type* __restrict__ dipt_s,
-                             const typename Vec4T<R>::type* __restrict__ vec_s, const GT* __restrict__ phi,
-                             double* __restrict__ out) {
+__global__ void __launch_bounds__(kPmeThreads)
+    k_pme_gather(PairParams P, EwParams EP, const double* __restrict__ real_part, EwExceptions X,
+                 const typename Vec4T<R>::type* __restrict__ lab_s, PmeGrid G, int n, int n_pad,
+                 double selfc, const double* __restrict__ pos_s,
+                 const typename Vec4T<R>::type* __restrict__ posq_s,
+                 const typename Vec4T<R>::type* __restrict__ dipt_s,
+                 const typename Vec4T<R>::type* __restrict__ vec_s, const GT* __restrict__ phi,
+                 double* __restrict__ out) {
     int c;
     const int at = pme_atom(n_pad, c), k = at >= 0 && at < n ? at : 0;   // idle lanes take atom 0 and write nothing
     int base[3];
@@ -1404,8 +1405,8 @@ __global__ void k_ew_finish(int n, int n_pad, const int* __restrict__ rank, cons
                             const double* __restrict__ pol, double alpha, double selfc, int recip, PairParams PP,
                             EwParams EP, const double* __restrict__ real_part, EwExceptions X,
                             const double* __restrict__ pos_s, int n_we, const double* __restrict__ warp_energy,
-                            int n_re, const double* __restrict__ rec_energy, double* __restrict__ fpair, double* __restrict__ torque, double* __restrict__ epart,
-                            int subtract = 0) {
+                            int n_re, const double* __restrict__ rec_energy, double* __restrict__ fpair,
+                            double* __restrict__ torque, double* __restrict__ epart, int subtract = 0) {
     __shared__ double red[40];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     double e = 0.0;

@@ -211,8 +211,8 @@ struct Rec64 {
 template <int KIND, bool FOLD, bool DAMP, bool MASK>
 __device__ __forceinline__ void field_walk64(const PairParams& P, const Rec64& T, int lane, int j0,
                                              const double (&o)[2][3], const double (&v)[2][3], const double (&q)[2],
-                                             const double (&ti)[2], const double (&c3)[2], const unsigned (&m)[2], unsigned fold, int s0,
-                                             int s1, double (&f)[2][3], double (&g)[3]) {
+                                             const double (&ti)[2], const double (&c3)[2], const unsigned (&m)[2],
+                                             unsigned fold, int s0, int s1, double (&f)[2][3], double (&g)[3]) {
     const int nxt = (lane + 1) & 31;
 #pragma unroll 1
     for (int s = s0; s < s1; s++) {
@@ -266,8 +266,9 @@ __device__ __forceinline__ void field_walk64(const PairParams& P, const Rec64& T
 // J-side sums stay packed.  Lane l takes pair m = (l + s) & 15 at step s and
 // passes its packed J-side sums one lane on; lanes l and l ^ 16 hold two
 // partial copies of the same pair, added by one xor-16 exchange at the end.
-// Each lane carries one or two I atoms (slots a and b), each with the pair
-// arithmetic of pair_delta + pair_matvec2 / pair_fixed2 per half.
+// Each lane carries NS I atoms; both sides of every pair are evaluated
+// (calculateInducedDipolePairIxn and calculateFixedDipoleFieldPairIxn,
+// RTDF.cpp:766-818 and :678-713).
 // ---------------------------------------------------------------------------
 struct FPackedTile {
     float4 p0[16], p1[16];   // (x, x', y, y'), (z, z', q, q')   (' = atom m + 16)
@@ -317,8 +318,8 @@ __device__ __forceinline__ XSlot xslot(int i, float ox, float oy, float oz, floa
 // MASK: bit m of mk (bit m + 16 for the second half) says whether the pair counts.
 template <int KIND, bool FOLD, bool DAMP, bool MASK = false>
 __device__ __forceinline__ void xslot_pairs(const PairParams& P, const double* __restrict__ pos, const XSlot& x,
-                                            unsigned mk, int m, int ja, f2 PX, f2 PY, f2 PZ, f2 QJ, f2 VJX, f2 VJY, f2 VJZ, float tja,
-                                            float tjb, unsigned fm, f2 Lx, f2 Ly, f2 Lz, f2 Ix, f2 Iy, f2 Iz,
+                                            unsigned mk, int m, int ja, f2 PX, f2 PY, f2 PZ, f2 QJ, f2 VJX, f2 VJY,
+                                            f2 VJZ, float tja, float tjb, unsigned fm, f2 Lx, f2 Ly, f2 Lz, f2 Ix, f2 Iy, f2 Iz,
                                             f2 NTx, f2 NTy, f2 NTz, float damp_r2, f2& FX, f2& FY, f2& FZ,
                                             f2& GX, f2& GY, f2& GZ) {
     f2 DX = sub2(PX, x.OX), DY = sub2(PY, x.OY), DZ = sub2(PZ, x.OZ);
@@ -392,7 +393,7 @@ __device__ __forceinline__ void xslot_pairs(const PairParams& P, const double* _
         }
     }
     if (KIND == 1) {
-        // pair_matvec2 with both sums negated: -f_i += rr3 v_j - (rr5 v_j.d) d,
+        // Mutual field, both sums negated: -f_i += rr3 v_j - (rr5 v_j.d) d,
         // -f_j += rr3 v_i - (rr5 v_i.d) d.
         const f2 DDJ = mul2(NRR5, fma2(VJX, DX, fma2(VJY, DY, mul2(VJZ, DZ))));
         const f2 DDI = mul2(NRR5, fma2(x.VX, DX, fma2(x.VY, DY, mul2(x.VZ, DZ))));
@@ -403,7 +404,7 @@ __device__ __forceinline__ void xslot_pairs(const PairParams& P, const double* _
         GY = fma2(RR3, x.VY, fma2(DDI, DY, GY));
         GZ = fma2(RR3, x.VZ, fma2(DDI, DZ, GZ));
     } else {
-        // pair_fixed2: a = rr3 q_j - rr5 m_j.d, b = rr3 q_i + rr5 m_i.d;
+        // Permanent field: a = rr3 q_j - rr5 m_j.d, b = rr3 q_i + rr5 m_i.d;
         // -f_i += d a + m_j rr3;  -f_j += m_i rr3 - d b, with nb = -b.
         const f2 A = fma2(NRR5, fma2(VJX, DX, fma2(VJY, DY, mul2(VJZ, DZ))), mul2(RR3, QJ));
         const f2 NB = fma2(NRR5, fma2(x.VX, DX, fma2(x.VY, DY, mul2(x.VZ, DZ))), mul2(RR3, x.NQ));
@@ -2049,9 +2050,9 @@ __global__ void k_energy_items_done(PairParams P, const float4* __restrict__ pos
                                     const double* __restrict__ pos, const int* __restrict__ exc_off,
                                     const int* __restrict__ exc_j, const double* __restrict__ exc_m,
                                     const double* __restrict__ exc_s, IndexRecords R, int* __restrict__ axis_count,
-                                    int n_pad, unsigned long long* __restrict__ acc, double inv_scale, int n_items, const double* __restrict__ energy_item,
-                                    double* __restrict__ fpair, double* __restrict__ torque,
-                                    double* __restrict__ energy_block) {
+                                    int n_pad, unsigned long long* __restrict__ acc, double inv_scale, int n_items,
+                                    const double* __restrict__ energy_item, double* __restrict__ fpair,
+                                    double* __restrict__ torque, double* __restrict__ energy_block) {
     __shared__ double red[40];
     const int per = (n_items + gridDim.x - 1) / gridDim.x;
     const int a0 = min(n_items, blockIdx.x * per), a1 = min(n_items, a0 + per);
@@ -2347,7 +2348,7 @@ void slot_sum(const Dev& d, int ncomp, cudaStream_t st) {
 // kind 0: permanent field (operand: the lab dipoles); kind 1: mutual-field
 // matvec (operand: vec); kind 2: the start of a warm-started solve, the
 // permanent field plus T mu0 in one walk (operand vec = m + mu0, see
-// field_partners).
+// add_partner).
 template <>
 void launch_field<float>(const Dev& d, int kind, cudaStream_t st, CgStop stop) {
     const int L = d.field_L, B = std::max(L, kFieldNS), nb = (d.pp.n_tiles + B - 1) / B;
