@@ -1333,7 +1333,7 @@ int tdp_create(const tdp_system_desc* desc, tdp_handle** out) {
             d.fixacc = dalloc<unsigned long long>(6 * (size_t)d.n_pad + 1, o);
             d.axis_cap = (int)std::min(16L * n, (long)INT_MAX / 2);
             d.axis_pairs = dalloc<int2>(d.axis_cap, o);
-            d.axis_count = dalloc<int>(1, o);
+            d.axis_count = dalloc<unsigned long long>(1, o);
             d.fix_err = dalloc<int>(1, o);
         }
         d.energy_partial = dalloc<double>((size_t)d.n_eblk + d.n_pad / 128, o);

@@ -84,7 +84,7 @@ struct Dev {
     int energy_L = 1, energy_parts = 1;
     double fix_scale_energy = 0.0;
     int2* axis_pairs = nullptr;   // pairs close to the x axis, evaluated apart
-    int* axis_count = nullptr;
+    unsigned long long* axis_count = nullptr;
     int axis_cap = 0;
     double* energy_partial = nullptr;
     double* fpair = nullptr;

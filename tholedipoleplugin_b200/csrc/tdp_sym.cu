@@ -1466,17 +1466,16 @@ __device__ __forceinline__ QiPair qi_pair2(const PairParams& P, f2 DX, f2 DY, f2
 constexpr float kNearAxis2 = 3.6e-5f, kNearAxisFar2 = 4.0e-6f, kAxisListRange2 = 2.2f;
 
 // Pairs (slots) that the walks left to k_axis_pairs, sized for 16 an atom.  A
-// count beyond the capacity says that not all of them are here; it is not
-// raised further then, so that no number of pairs takes it past an int.
+// count beyond the capacity says that not all of them are here; it takes 64
+// bits because the pairs of a long chain do not fit an int.
 struct AxisList {
     int2* pairs;
-    int* count;
-    int cap;
+    unsigned long long* count;
+    unsigned long long cap;
 };
 
 __device__ __forceinline__ void axis_push(const AxisList& A, int i, int j) {
-    if (*(volatile int*)A.count > A.cap) return;
-    const int k = atomicAdd(A.count, 1);
+    const unsigned long long k = atomicAdd(A.count, 1ull);
     if (k < A.cap) A.pairs[k] = make_int2(i, j);
 }
 
@@ -2028,9 +2027,9 @@ __global__ void __launch_bounds__(32, 12)
 // meets the same pairs.  The sums are integers, so the two give the same bits.
 __global__ void __launch_bounds__(32) k_axis_pairs(PairParams P, EItemArrays A, int items) {
     __shared__ EItemShared S;
-    const int count = *A.axis.count;
+    const unsigned long long count = *A.axis.count;
     if (count <= A.axis.cap) {
-        for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < count; q += gridDim.x * blockDim.x) {
+        for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < (int)count; q += gridDim.x * blockDim.x) {
             const int2 ij = A.axis.pairs[q];
             axis_pair(P, A.R, A.order, A.pos, A.fix, A.n_pad, ij.x, ij.y);
         }
@@ -2049,7 +2048,7 @@ __global__ void k_energy_items_done(PairParams P, const float4* __restrict__ pos
                                     const float4* __restrict__ indv, const int* __restrict__ order,
                                     const double* __restrict__ pos, const int* __restrict__ exc_off,
                                     const int* __restrict__ exc_j, const double* __restrict__ exc_m,
-                                    const double* __restrict__ exc_s, IndexRecords R, int* __restrict__ axis_count,
+                                    const double* __restrict__ exc_s, IndexRecords R, unsigned long long* __restrict__ axis_count,
                                     int n_pad, unsigned long long* __restrict__ acc, double inv_scale, int n_items,
                                     const double* __restrict__ energy_item, double* __restrict__ fpair,
                                     double* __restrict__ torque, double* __restrict__ energy_block) {
@@ -2061,7 +2060,7 @@ __global__ void k_energy_items_done(PairParams P, const float4* __restrict__ pos
     if (blockIdx.x == 0 && threadIdx.x == 0) {   // the listed pairs' energy; the list is empty again
         energy += (double)(long long)acc[6 * (size_t)n_pad] * inv_scale;
         acc[6 * (size_t)n_pad] = 0ull;
-        *axis_count = 0;
+        *axis_count = 0ull;
     }
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k < n_pad) {
@@ -2480,11 +2479,11 @@ void launch_energy<float>(const Dev& d, cudaStream_t st) {
     fix.scale = d.fix_scale_energy;
     const IndexRecords rec{(const float4*)d.posq, d.tctr, pq, dp, u};
     const EItemArrays A{pq, dp, u, d.order, d.tctr_s, d.text_s, d.pos_s, d.exs_off, d.exs_j, d.exs_m, d.exs_s,
-                        d.exs_tiles, rec, AxisList{d.axis_pairs, d.axis_count, d.axis_cap}, fix, L, d.n_pad};
+                        d.exs_tiles, rec, AxisList{d.axis_pairs, d.axis_count, (unsigned long long)d.axis_cap}, fix, L, d.n_pad};
     if (d.pp.lab_energy && !d.pp.periodic) k_energy_items<false, true><<<grid, 32, 0, st>>>(d.pp, A, d.energy_partial);
     else if (d.pp.lab_energy) k_energy_items<false, false><<<grid, 32, 0, st>>>(d.pp, A, d.energy_partial);
     else k_energy_items<true, false><<<grid, 32, 0, st>>>(d.pp, A, d.energy_partial);
-    k_axis_pairs<<<2 * 148, 32, 0, st>>>(d.pp, A, (int)grid.x);
+    k_axis_pairs<<<148, 32, 0, st>>>(d.pp, A, (int)grid.x);
     k_energy_items_done<<<d.n_pad / 128, 128, 0, st>>>(d.pp, pq, dp, u, d.order, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
                                                        d.exs_s, rec, d.axis_count, d.n_pad, d.fixacc,
                                                        1.0 / fix.scale, d.n_eblk,
