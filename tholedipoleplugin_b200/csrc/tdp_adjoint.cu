@@ -29,6 +29,8 @@
 // atoms (each atom owns kLanes threads), so no atomics are needed.
 #include "tholedipole_b200.h"
 #include <algorithm>
+#include <climits>
+#include <cmath>
 #include "tdp_adjoint.cuh"
 
 namespace tdp {
@@ -73,28 +75,26 @@ __global__ void k_pair_vjp(PairParams P, AtomData A, const double* __restrict__ 
 // the mixed form, FP64 in the plain form) from a displacement formed in FP64
 // with the minimum image and rounded once; per-tile sums are added in FP64.
 // The other pairs (damped or degenerate, ~0.6 % of a box) are listed in the
-// atom's row of `slow`, in index order (beyond kSlowCap they are evaluated in
-// place).  Pass 2 (k_pair_vjp_slow): one warp per atom runs the FP64 routine
-// over the listed pairs and the covalent corrections, lane l taking entries
-// l, l + 32, ..., and adds the warp's sums, reduced by a fixed shuffle tree.
-// Small systems split the J range over blockIdx.y (at most kVjpSplit
-// splits) to fill the GPU: split s keeps its own sums and slow rows, and
-// pass 2 adds the splits in order.  Both passes are deterministic.
+// atom's row of `slow`.  Pass 2 (k_pair_vjp_slow): one warp per atom puts the
+// row into index order and runs the FP64 routine over the listed pairs (over
+// all pairs that belong there, where the row is too short) and the covalent
+// corrections, lane l taking entries l, l + 32, ..., and adds the warp's sums,
+// reduced by a fixed shuffle tree.
+// The J range is split over blockIdx.y (at most kVjpSplit splits) to fill the
+// GPU: split s keeps its own sums, which pass 2 adds in order, and all share
+// the atom's row (a row a split would take 1 KB or more of each).  Both passes
+// are deterministic.
 constexpr int kVjpTile = 32;
-constexpr int kSlowCap = 192;
-// k_pair_vjp_fast at 12 blocks per SM (168 registers, 48 B of spills):
-// 7.3 ms per 12,288-atom adjoint against 7.9 ms at 215 registers and 8.2 ms
-// at 128 (mixed form).
 constexpr int kVjpSplit = 9, kFixedSplit = 16;
-// The FP64 routine out of line, so that the rare overflow of a slow row does
-// not set the fast pass's register budget.
-__device__ __noinline__ void visit_pair_call(const PairParams& P, const AtomData& A, const double* g,
-                                             const double* gT, double gE, int me, int j, double* acc) {
-    visit_pair(P, A, g, gT, gE, me, j, 1.0, 1.0, acc);
+// Whether a pair (d = p_K - p_I, I the lower index) takes the closed form of
+// pass 1.
+__device__ __forceinline__ bool regular_pair(V3 d, double2 yz0, double2 yz1, double damp_r2) {
+    const bool yzd = (yz0.x != yz1.x) || (yz0.y != yz1.y);
+    return !(norm2(d) < damp_r2) && yzd && d.y * d.y + d.z * d.z > 0.0;
 }
 template <class T>
 __global__ void __launch_bounds__(kVjpTile, 12) k_pair_vjp_fast(PairParams P, AtomData A, const double* __restrict__ g,
-                                                           const double* __restrict__ gT, double gE,
+                                                           const double* __restrict__ gT, double gE, int cap,
                                                            int* __restrict__ slow, int* __restrict__ nslow,
                                                            double* __restrict__ part_out) {
     typedef V3T<T> W;
@@ -115,9 +115,7 @@ __global__ void __launch_bounds__(kVjpTile, 12) k_pair_vjp_fast(PairParams P, At
     const T lam = P.mutual ? T(2) : T(0), tgE = (T)gE;
     const double damp_r2 = P.damp_r2 == 0.0f ? 0.0 : (double)P.damp_r2;
     double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    int ns = 0;
     const size_t sm = (size_t)blockIdx.y * P.n + mi;   // (split, atom)
-    int* row = slow + sm * kSlowCap;
     const int ntile = (P.n + kVjpTile - 1) / kVjpTile;
     const int tb = (int)(((long)ntile * blockIdx.y) / gridDim.y), te = (int)(((long)ntile * (blockIdx.y + 1)) / gridDim.y);
     for (int base = tb * kVjpTile; base < te * kVjpTile && base < P.n; base += kVjpTile) {
@@ -138,6 +136,7 @@ __global__ void __launch_bounds__(kVjpTile, 12) k_pair_vjp_fast(PairParams P, At
         if (!act) continue;
         const int cnt = min(kVjpTile, P.n - base);
         T part[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        unsigned aside = 0u;   // the tile's pairs for the list
         for (int jj = 0; jj < cnt; jj++) {
             const int j = base + jj;
             if (j == me) continue;
@@ -145,10 +144,7 @@ __global__ void __launch_bounds__(kVjpTile, 12) k_pair_vjp_fast(PairParams P, At
             // d = p_K - p_I with I the lower index.
             V3 d = min_image(P, {s_pos[0][jj] - px, s_pos[1][jj] - py, s_pos[2][jj] - pz});
             if (!meI) d = {-d.x, -d.y, -d.z};
-            const double2 yj = s_yz[jj];
-            const bool yzd = (myz.x != yj.x) || (myz.y != yj.y);
-            const double r2 = norm2(d);
-            if (!(r2 < damp_r2) && yzd && d.y * d.y + d.z * d.z > 0.0) {
+            if (regular_pair(d, myz, s_yz[jj], damp_r2)) {
                 const T sg = meI ? T(1) : T(-1);
                 const W dj = {sg * (T)d.x, sg * (T)d.y, sg * (T)d.z};
                 const W mj = {s_v[0][jj], s_v[1][jj], s_v[2][jj]}, uj = {s_v[3][jj], s_v[4][jj], s_v[5][jj]};
@@ -156,32 +152,74 @@ __global__ void __launch_bounds__(kVjpTile, 12) k_pair_vjp_fast(PairParams P, At
                 pair_vjp_me<T, false>(dj, sg, q0, m0, u0, T(0), s_q[jj], mj, uj, T(0), T(1), T(1), T(0), lam, tgE, g0,
                                       gj, t0, tj, part);
             } else {
-                // The count goes on past the row (the list users then scan all
-                // partners of this atom).
-                if (ns < kSlowCap) row[ns] = j;
-                else visit_pair_call(P, A, g, gT, gE, me, j, acc);
-                ns++;
+                aside |= 1u << jj;
             }
         }
         for (int a = 0; a < 7; a++) acc[a] += (double)part[a];
+        if (aside) {
+            // The count goes on past the row (the list users then scan all
+            // partners of this atom).
+            int at = atomicAdd(nslow + me, __popc(aside));
+            for (; aside && at < cap; aside &= aside - 1u) slow[(size_t)me * cap + at++] = base + __ffs(aside) - 1;
+        }
     }
     if (!act) return;
-    nslow[sm] = ns;
     for (int k = 0; k < 8; k++) part_out[8 * sm + k] = acc[k];
 }
 
-__global__ void k_pair_vjp_slow(PairParams P, AtomData A, const double* __restrict__ g, const double* __restrict__ gT,
-                                double gE, int nsplit, const int* __restrict__ slow, const int* __restrict__ nslow,
-                                const double* __restrict__ part, const int* __restrict__ exc_off,
-                                const int* __restrict__ exc_j, const double* __restrict__ exc_m,
-                                const double* __restrict__ exc_s, double* __restrict__ out) {
+constexpr int kSlowWarps = 4;
+// The power of two, 32 at least, that a row of n entries is sorted in.
+__host__ __device__ __forceinline__ int sort_size(int n) {
+    int m = 32;
+    while (m < n) m <<= 1;
+    return m;
+}
+__global__ void __launch_bounds__(32 * kSlowWarps)
+    k_pair_vjp_slow(PairParams P, AtomData A, const double* __restrict__ g, const double* __restrict__ gT, double gE,
+                    int nsplit, int cap, int* slow, const int* __restrict__ nslow, const double* __restrict__ part,
+                    const int* __restrict__ exc_off, const int* __restrict__ exc_j, const double* __restrict__ exc_m,
+                    const double* __restrict__ exc_s, double* __restrict__ out) {
+    extern __shared__ int s_rows[];   // a row a warp
+    int* s_row = s_rows + (threadIdx.x >> 5) * sort_size(cap);
     const int me = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, l = threadIdx.x & 31;
     if (me >= P.n) return;   // whole warps leave together
     double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int sp = 0; sp < nsplit; sp++) {
-        const size_t sm = (size_t)sp * P.n + me;
-        const int* row = slow + sm * kSlowCap;
-        for (int e = l; e < min(nslow[sm], kSlowCap); e += 32) visit_pair(P, A, g, gT, gE, me, row[e], 1.0, 1.0, acc);
+    const int count = nslow[me];
+    int* row = slow + (size_t)me * cap;
+    if (count <= cap) {
+        // The row's entries came in the order of the splits' atomics: a bitonic
+        // sort puts them into index order.
+        const int m = sort_size(count);
+        for (int e = l; e < m; e += 32) s_row[e] = e < count ? row[e] : INT_MAX;
+        for (int k = 2; k <= m; k <<= 1)
+            for (int h = k >> 1; h > 0; h >>= 1) {
+                __syncwarp();
+                for (int t = l; t < m / 2; t += 32) {
+                    const int a = 2 * t - (t & (h - 1)), b = a + h;
+                    const int x = s_row[a], y = s_row[b];
+                    if ((x > y) == ((a & k) == 0)) {
+                        s_row[a] = y;
+                        s_row[b] = x;
+                    }
+                }
+            }
+        __syncwarp();
+        for (int e = l; e < count; e += 32) {
+            row[e] = s_row[e];
+            visit_pair(P, A, g, gT, gE, me, s_row[e], 1.0, 1.0, acc);
+        }
+    } else {
+        const V3 pm = ld(A.pos + 3 * me);
+        const double damp_r2 = P.damp_r2 == 0.0f ? 0.0 : (double)P.damp_r2;
+        const double2 myz = A.yz ? A.yz[me] : make_double2(pm.y, pm.z);
+        for (int j = l; j < P.n; j += 32) {
+            if (j == me) continue;
+            const V3 pj = ld(A.pos + 3 * j);
+            V3 d = min_image(P, {pj.x - pm.x, pj.y - pm.y, pj.z - pm.z});
+            if (j < me) d = {-d.x, -d.y, -d.z};
+            if (!regular_pair(d, myz, A.yz ? A.yz[j] : make_double2(pj.y, pj.z), damp_r2))
+                visit_pair(P, A, g, gT, gE, me, j, 1.0, 1.0, acc);
+        }
     }
     // Covalent scales: the pair function is linear in (mScale, iScale).
     for (int e = exc_off[me] + l; e < exc_off[me + 1]; e += 32)
@@ -306,17 +344,11 @@ __global__ void k_sum_splits(int m, int nsplit, const double* __restrict__ part,
 // Warp-per-atom passes over the damped-partner lists of the pair VJP (the
 // same pairs, within the damping range, are the only ones whose Thole factors
 // matter).  An atom whose list overflowed its row falls back to a scan of all
-// partners.  Lanes take entries l, l + 32, ... in split order; a fixed
+// partners.  Lanes take entries l, l + 32, ... of the row; a fixed
 // shuffle tree adds them.
 __device__ __forceinline__ double warp_sum_fixed(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
-}
-
-__device__ __forceinline__ bool list_overflow(const AdjPairList& L, int n, int k) {
-    for (int sp = 0; sp < L.nsplit; sp++)
-        if (L.nslow[(size_t)sp * n + k] > L.cap) return true;
-    return false;
 }
 
 // k_fixed_vjp's damped pairs (unit scale) and covalent corrections in FP64, added
@@ -329,15 +361,12 @@ __global__ void k_fixed_list(PairParams P, AtomData A, const double* __restrict_
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, l = threadIdx.x & 31;
     if (k >= P.n) return;   // whole warps leave together
     double acc[5] = {0, 0, 0, 0, 0};
-    if (list_overflow(L, P.n, k)) {
+    const int count = L.nslow[k];
+    if (count > L.cap) {
         for (int i = l; i < P.n; i += 32)
             if (i != k) fixed_vjp_damped(P, A, lam, k, i, acc);
     } else {
-        for (int sp = 0; sp < L.nsplit; sp++) {
-            const size_t sk = (size_t)sp * P.n + k;
-            const int* row = L.slow + sk * L.cap;
-            for (int e = l; e < L.nslow[sk]; e += 32) fixed_vjp_damped(P, A, lam, k, row[e], acc);
-        }
+        for (int e = l; e < count; e += 32) fixed_vjp_damped(P, A, lam, k, L.slow[(size_t)k * L.cap + e], acc);
     }
     for (int e = exc_off[k] + l; e < exc_off[k + 1]; e += 32)
         fixed_vjp_visit(P, A, lam, k, exc_j[e], exc_m[e] - 1.0, acc);
@@ -355,15 +384,13 @@ __global__ void k_matvec_t_list(PairParams P, AtomData A, const double* __restri
     const int k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, l = threadIdx.x & 31;
     if (k >= P.n) return;
     double acc = 0.0;
-    if (list_overflow(L, P.n, k)) {
+    const int count = L.nslow[k];
+    if (count > L.cap) {
         for (int j = l; j < P.n; j += 32)
             if (j != k) acc += matvec_t_visit(P, A, lam, k, j, 1.0);
     } else {
-        for (int sp = 0; sp < L.nsplit; sp++) {
-            const size_t sk = (size_t)sp * P.n + k;
-            const int* row = L.slow + sk * L.cap;
-            for (int e = l; e < L.nslow[sk]; e += 32) acc += matvec_t_visit(P, A, lam, k, row[e], 1.0);
-        }
+        for (int e = l; e < count; e += 32)
+            acc += matvec_t_visit(P, A, lam, k, L.slow[(size_t)k * L.cap + e], 1.0);
     }
     for (int e = exc_off[k] + l; e < exc_off[k + 1]; e += 32)
         acc += matvec_t_visit(P, A, lam, k, exc_j[e], exc_s[e] - 1.0);
@@ -502,20 +529,14 @@ __global__ void k_set_operand(int n, const int* __restrict__ rank, const double*
 // ---------------------------------------------------------------------------
 static inline int nb(int n) { return (n + 127) / 128; }
 
-// J splits of k_pair_vjp_fast: whole rounds of its 12 resident blocks an SM,
-// the time going with rounds / splits (12,288 atoms: 7 splits made 1.5 rounds,
-// 1666 us; 9 make 1.95, 1479).  Every split has a list row for each atom, so
-// no more of them than make two rounds: the lists stay within 95 MB, or one
-// row an atom from 56,833 atoms on (98,304 atoms: 4 splits would save an
-// eighth of the rounds and take 329 MB in place of 82).
+// J splits of k_pair_vjp_fast: nine, or as many as make about eight rounds of 12
+// blocks an SM (1, 4, 6, 9, 12 splits: 1142, 306, 264, 179, 178 us at 3,993
+// atoms, 3402, 1500, 1285, 1321, 1269 at 12,288, 19.7, 14.5, 14.5, 13.7,
+// 13.8 ms at 41,472; FP64 5090, 2376, 2184, 2051, 2024 us at 12,288).  More
+// would only take memory: a split's sums are 64 bytes an atom.
 static int vjp_splits(int n) {
-    const long blocks = (std::max(n, 1) + adj::kVjpTile - 1) / adj::kVjpTile, resident = 12L * 148;
-    const long most = std::min((long)adj::kVjpSplit, 2 * resident / blocks);
-    int best = 1;
-    const auto rounds = [&](int s) { return (double)((blocks * s + resident - 1) / resident) / s; };
-    for (int s = 2; s <= most; s++)
-        if (rounds(s) < rounds(best)) best = s;
-    return best;
+    const long blocks = (std::max(n, 1) + adj::kVjpTile - 1) / adj::kVjpTile;
+    return (int)std::min((long)adj::kVjpSplit, std::max(1L, 8L * 12 * 148 / blocks));
 }
 
 // J splits of k_fixed_vjp_fast: one round of 32 resident blocks an SM
@@ -525,17 +546,27 @@ static int fixed_splits(int n) {
     return std::min(adj::kFixedSplit, std::max(1, 32 * 148 / blocks));
 }
 
-// Scratch of the two-pass pair VJP, per (split, atom): 8 FP64 sums, the
-// slow-pair row and its count.
-size_t adjoint_pair_scratch(int n) {
-    const size_t m = (size_t)vjp_splits(n) * (size_t)std::max(n, 1);
-    return 8 * m + (m * (adj::kSlowCap + 1) * sizeof(int) + sizeof(double) - 1) / sizeof(double);
+// Entries of an atom's list row for `expected` damped partners: 30 % more, in
+// steps of 64 from 256 (liquid water: 190 give or take 15 within its 0.77 nm)
+// to 2048, which pass 2 can sort in shared memory.  An atom with more has all
+// its partners scanned, at several times the cost (12,288 atoms with half the
+// rows too short: passes over the lists 0.34 -> 2.7 ms).
+int adjoint_list_cap(int n, double expected) {
+    const double want = std::min(std::min(1.3 * expected, 2048.0), (double)std::max(n - 1, 1));
+    return std::max(256, 64 * (int)std::ceil(want / 64.0));
+}
+
+// Scratch of the two-pass pair VJP: 8 FP64 sums per (split, atom), the slow-pair
+// row and its count per atom.
+size_t adjoint_pair_scratch(int n, int cap) {
+    const size_t m = (size_t)std::max(n, 1);
+    return 8 * m * vjp_splits(n) + (m * (cap + 1) * sizeof(int) + sizeof(double) - 1) / sizeof(double);
 }
 
 size_t adjoint_fixed_scratch(int n) { return 5 * (size_t)fixed_splits(n) * (size_t)std::max(n, 1); }
 
 void launch_adjoint_pair(const Dev& d, const double* g, const double* gT, double gE, double* a8, int precision,
-                         double* scratch, AdjPairList* list, cudaStream_t st) {
+                         double* scratch, int cap, AdjPairList* list, cudaStream_t st) {
     if (list) *list = AdjPairList{};
     if (d.n <= 0) return;
     adj::AtomData A{d.pos, d.charge, d.lab, d.mu, d.thole, d.yz};
@@ -546,24 +577,24 @@ void launch_adjoint_pair(const Dev& d, const double* g, const double* gT, double
     }
     const int blocks = (d.n + adj::kVjpTile - 1) / adj::kVjpTile;
     const int nsplit = vjp_splits(d.n);
-    const size_t m = (size_t)nsplit * d.n;
     double* part = scratch;
-    int* slow = reinterpret_cast<int*>(scratch + 8 * m);
-    int* nslow = slow + m * adj::kSlowCap;
+    int* slow = reinterpret_cast<int*>(scratch + 8 * (size_t)nsplit * d.n);
+    int* nslow = slow + (size_t)d.n * cap;
+    cudaMemsetAsync(nslow, 0, sizeof(int) * d.n, st);
     const dim3 grid(blocks, nsplit);
     if (precision == TDP_PRECISION_MIXED)
-        adj::k_pair_vjp_fast<float><<<grid, adj::kVjpTile, 0, st>>>(d.pp, A, g, gT, gE, slow, nslow, part);
+        adj::k_pair_vjp_fast<float><<<grid, adj::kVjpTile, 0, st>>>(d.pp, A, g, gT, gE, cap, slow, nslow, part);
     else
-        adj::k_pair_vjp_fast<double><<<grid, adj::kVjpTile, 0, st>>>(d.pp, A, g, gT, gE, slow, nslow, part);
-    adj::k_pair_vjp_slow<<<nb(32 * d.n), 128, 0, st>>>(d.pp, A, g, gT, gE, nsplit, slow, nslow, part, d.exc_off,
-                                                        d.exc_j, d.exc_m, d.exc_s, a8);
-    if (list) *list = AdjPairList{nsplit, adj::kSlowCap, slow, nslow};
+        adj::k_pair_vjp_fast<double><<<grid, adj::kVjpTile, 0, st>>>(d.pp, A, g, gT, gE, cap, slow, nslow, part);
+    adj::k_pair_vjp_slow<<<nb(32 * d.n), 32 * adj::kSlowWarps, sizeof(int) * adj::kSlowWarps * adj::sort_size(cap), st>>>(
+        d.pp, A, g, gT, gE, nsplit, cap, slow, nslow, part, d.exc_off, d.exc_j, d.exc_m, d.exc_s, a8);
+    if (list) *list = AdjPairList{cap, slow, nslow};
 }
 void launch_adjoint_fixed(const Dev& d, const double* lam, double* b5, const AdjPairList& list, int precision,
                           double* scratch, cudaStream_t st) {
     if (d.n <= 0) return;
     adj::AtomData A{d.pos, d.charge, d.lab, d.mu, d.thole, d.yz};
-    if (list.nsplit <= 0 || !scratch) {
+    if (!list.slow || !scratch) {
         adj::k_fixed_vjp<<<nb(d.n * adj::kLanes), 128, 0, st>>>(d.pp, A, lam, d.exc_off, d.exc_j, d.exc_m, b5);
         return;
     }
@@ -584,7 +615,7 @@ void launch_adjoint_matvec_t_mu(const Dev& d, const double* lam, const double* m
                                 const AdjPairList& list, cudaStream_t st) {
     if (d.n <= 0) return;
     adj::AtomData A{d.pos, d.charge, d.lab, mu, d.thole, d.yz};
-    if (list.nsplit > 0)
+    if (list.slow)
         adj::k_matvec_t_list<<<nb(32 * d.n), 128, 0, st>>>(d.pp, A, lam, list, d.exc_off, d.exc_j, d.exc_s, ct,
                                                             accumulate ? 1 : 0);
     else

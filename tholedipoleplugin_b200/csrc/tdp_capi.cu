@@ -117,6 +117,7 @@ struct tdp_handle {
     double* d_pstat = nullptr;
 
     // Adjoint work buffers (allocated on first use).
+    int adj_cap = 0;   // its list entries an atom
     double* adj = nullptr;
     double adj_eps = 0.0;
     int adj_iterations = 0;
@@ -928,6 +929,25 @@ void solve_at(tdp_handle* h, const void* positions, int dtype, int on_device) {
     }
 }
 
+// Atoms within the damping range r of one, at the mean density of the box or,
+// without one, of the box around the coordinates of the last sort.  Edges below
+// 4r/3 count as that: a slab has pi r^2 of its area in range, a row 2.4 r.
+double expected_damped(const tdp_handle* h) {
+    const double r = std::sqrt((double)h->d.pp.damp_r2);
+    if (!std::isfinite(r)) return h->n;
+    double volume = 1.0;
+    for (int k = 0; k < 3; k++) {
+        double lo = INFINITY, hi = -INFINITY;
+        for (size_t i = k; i < h->hpos.size(); i += 3) {
+            lo = std::min(lo, h->hpos[i]);
+            hi = std::max(hi, h->hpos[i]);
+        }
+        volume *= std::max(h->d.pp.periodic ? h->d.pp.box[k] : hi - lo, 4.0 / 3.0 * r);
+    }
+    const double sphere = 4.18879 * r * r * r;
+    return sphere < volume ? h->n * (sphere / volume) : h->n;
+}
+
 // Reverse mode of one evaluation (tdp_adjoint.cu has the kernels and the
 // derivation).  Needs the state of the last evaluation (positions, lab-frame
 // and induced dipoles, permanent field); leaves it as it was.
@@ -937,9 +957,12 @@ void run_adjoint(tdp_handle* h, const double* g_in, double gE, double* out_dst, 
     cudaStream_t st = h->stream;
     const int n = h->n;
     const size_t n3 = 3 * (size_t)n;
-    if (!h->adj) h->adj = dalloc<double>(n3 * 11 + 8 * (size_t)n + 5 * (size_t)n + 2 * (size_t)n + 6 * (size_t)n +
-                                             adjoint_pair_scratch(n) + adjoint_fixed_scratch(n),
-                                         h->owned);
+    if (!h->adj) {
+        h->adj_cap = adjoint_list_cap(n, expected_damped(h));
+        h->adj = dalloc<double>(n3 * 11 + 8 * (size_t)n + 5 * (size_t)n + 2 * (size_t)n + 6 * (size_t)n +
+                                    adjoint_pair_scratch(n, h->adj_cap) + adjoint_fixed_scratch(n),
+                                h->owned);
+    }
     double* g = h->adj;
     double* gt = g + n3;
     double* amu = gt + n3;
@@ -957,7 +980,7 @@ void run_adjoint(tdp_handle* h, const double* g_in, double gE, double* out_dst, 
     double* ext_v = out + 6 * (size_t)n;   // Extrapolated: E + T mu_(k-1)
     double* galpha = ext_v + n3;           // Extrapolated: polarizability gradient
     double* pair_scratch = galpha + n;     // split sums and damped-partner lists of the pair VJP
-    double* fixed_scratch = pair_scratch + adjoint_pair_scratch(n);   // split sums of the fixed-field VJP
+    double* fixed_scratch = pair_scratch + adjoint_pair_scratch(n, h->adj_cap);   // split sums of the fixed-field VJP
     if (g_in)
         TDP_CUDA(cudaMemcpyAsync(g, g_in, n3 * 8, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, st));
     else
@@ -966,7 +989,7 @@ void run_adjoint(tdp_handle* h, const double* g_in, double gE, double* out_dst, 
     TDP_CUDA(cudaMemcpyAsync(E_fwd, d.E, n3 * 8, cudaMemcpyDeviceToDevice, st));
     launch_torque_vjp(d, g, gt, st);
     AdjPairList plist;
-    launch_adjoint_pair(d, g, gt, gE, a8, h->precision, pair_scratch, &plist, st);
+    launch_adjoint_pair(d, g, gt, gE, a8, h->precision, pair_scratch, h->adj_cap, &plist, st);
     launch_adjoint_split(d, a8, nullptr, amu, nullptr, st);
     if (h->polarization == TDP_MUTUAL) {
         // One solve of the same symmetric system: A lambda = a_mu.  Target:

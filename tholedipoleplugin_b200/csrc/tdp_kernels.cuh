@@ -172,23 +172,24 @@ void launch_moments(const Dev& d, const double* mass, double* scratch, double* o
 
 // Adjoint (tdp_adjoint.cu).
 void launch_torque_vjp(const Dev& d, const double* g, double* gt, cudaStream_t st);
-// Damped (and degenerate) partners of every atom, listed by the pair VJP per
-// (split, atom) in rows of `cap` entries (a count above cap means the row
-// overflowed), reused by the fixed-field and matvec Thole VJPs; nsplit = 0:
-// no list (those passes scan all pairs).  Valid while the scratch of
+// Damped (and degenerate) partners of every atom, listed by the pair VJP in
+// rows of `cap` entries in index order (a count above cap means the row
+// overflowed), reused by the fixed-field and matvec Thole VJPs; slow NULL: no
+// list (those passes scan all pairs).  Valid while the scratch of
 // launch_adjoint_pair is untouched.
 struct AdjPairList {
-    int nsplit = 0, cap = 0;
+    int cap = 0;
     const int* slow = nullptr;
     const int* nslow = nullptr;
 };
 // precision: the arithmetic of the closed-form pairs (FP32 in the mixed form);
-// scratch: adjoint_pair_scratch(n) doubles; list (may be NULL) receives the
-// damped-partner lists.
-size_t adjoint_pair_scratch(int n);
+// scratch: adjoint_pair_scratch(n, cap) doubles, cap list entries an atom
+// (adjoint_list_cap); list (may be NULL) receives the damped-partner lists.
+int adjoint_list_cap(int n, double expected);
+size_t adjoint_pair_scratch(int n, int cap);
 size_t adjoint_fixed_scratch(int n);
 void launch_adjoint_pair(const Dev& d, const double* g, const double* gT, double gE, double* a8, int precision,
-                         double* scratch, AdjPairList* list, cudaStream_t st);
+                         double* scratch, int cap, AdjPairList* list, cudaStream_t st);
 // scratch: adjoint_fixed_scratch(n) doubles (the split sums of the tiled pass), or NULL.
 void launch_adjoint_fixed(const Dev& d, const double* lam, double* b5, const AdjPairList& list, int precision,
                           double* scratch, cudaStream_t st);
