@@ -95,3 +95,23 @@ def test_same_bits_in_every_run(n_side, precision):
             runs += [k.adjoint(g, 0.3) for _ in range(3)]
     for r in runs[1:]:
         assert np.array_equal(r, runs[0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["mixed", "double"])
+def test_rows_follow_the_thole_factors(precision):
+    """After an adjoint at factors that damp next to nothing, one at factors that damp every pair is the one
+    of a new handle: its rows hold the 299 partners (shorter ones are scanned, in another order)."""
+    s = dense_system(300)
+    g = np.random.default_rng(1).normal(size=(s.n, 3))
+    out = []
+    for first in (0.05, None):
+        with CudaCalcTholeDipoleForceKernel(s, precision=precision) as k:
+            if first is not None:
+                k.copyParametersToContext(s.copy(tholes=first * s.tholes, polarizabilities=0.1 * s.polarizabilities))
+                k.execute(s.positions)
+                k.adjoint(g, 0.7)
+                k.copyParametersToContext(s)
+            k.execute(s.positions)
+            out.append(k.adjoint(g, 0.7))
+    assert np.array_equal(*out)

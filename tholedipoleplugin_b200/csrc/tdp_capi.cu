@@ -117,7 +117,8 @@ struct tdp_handle {
     double* d_pstat = nullptr;
 
     // Adjoint work buffers (allocated on first use).
-    int adj_cap = 0;   // its list entries an atom
+    int adj_cap = 0;       // their list entries an atom
+    float adj_r2 = 0.0f;   // the largest squared damping range these were chosen for
     double* adj = nullptr;
     double adj_eps = 0.0;
     int adj_iterations = 0;
@@ -957,8 +958,17 @@ void run_adjoint(tdp_handle* h, const double* g_in, double gE, double* out_dst, 
     cudaStream_t st = h->stream;
     const int n = h->n;
     const size_t n3 = 3 * (size_t)n;
-    if (!h->adj) {
-        h->adj_cap = adjoint_list_cap(n, expected_damped(h));
+    // New Thole factors may ask for longer list rows.
+    const int cap = !h->adj || d.pp.damp_r2 > h->adj_r2 ? adjoint_list_cap(n, expected_damped(h)) : h->adj_cap;
+    h->adj_r2 = std::max(h->adj_r2, d.pp.damp_r2);
+    if (!h->adj || cap > h->adj_cap) {
+        if (h->adj) {
+            TDP_CUDA(cudaStreamSynchronize(st));
+            h->owned.erase(std::find(h->owned.begin(), h->owned.end(), (void*)h->adj));
+            TDP_CUDA(cudaFree(h->adj));
+            h->adj = nullptr;
+        }
+        h->adj_cap = cap;
         h->adj = dalloc<double>(n3 * 11 + 8 * (size_t)n + 5 * (size_t)n + 2 * (size_t)n + 6 * (size_t)n +
                                     adjoint_pair_scratch(n, h->adj_cap) + adjoint_fixed_scratch(n),
                                 h->owned);
