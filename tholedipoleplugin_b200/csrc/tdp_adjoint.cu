@@ -586,7 +586,8 @@ void launch_adjoint_pair(const Dev& d, const double* g, const double* gT, double
         adj::k_pair_vjp_fast<float><<<grid, adj::kVjpTile, 0, st>>>(d.pp, A, g, gT, gE, cap, slow, nslow, part);
     else
         adj::k_pair_vjp_fast<double><<<grid, adj::kVjpTile, 0, st>>>(d.pp, A, g, gT, gE, cap, slow, nslow, part);
-    adj::k_pair_vjp_slow<<<nb(32 * d.n), 32 * adj::kSlowWarps, sizeof(int) * adj::kSlowWarps * adj::sort_size(cap), st>>>(
+    const size_t rows = sizeof(int) * adj::kSlowWarps * adj::sort_size(cap);
+    adj::k_pair_vjp_slow<<<nb(32 * d.n), 32 * adj::kSlowWarps, rows, st>>>(
         d.pp, A, g, gT, gE, nsplit, cap, slow, nslow, part, d.exc_off, d.exc_j, d.exc_m, d.exc_s, a8);
     if (list) *list = AdjPairList{cap, slow, nslow};
 }

@@ -319,7 +319,8 @@ __device__ __forceinline__ XSlot xslot(int i, float ox, float oy, float oz, floa
 template <int KIND, bool FOLD, bool DAMP, bool MASK = false>
 __device__ __forceinline__ void xslot_pairs(const PairParams& P, const double* __restrict__ pos, const XSlot& x,
                                             unsigned mk, int m, int ja, f2 PX, f2 PY, f2 PZ, f2 QJ, f2 VJX, f2 VJY,
-                                            f2 VJZ, float tja, float tjb, unsigned fm, f2 Lx, f2 Ly, f2 Lz, f2 Ix, f2 Iy, f2 Iz,
+                                            f2 VJZ, float tja, float tjb, unsigned fm, f2 Lx, f2 Ly, f2 Lz, f2 Ix,
+                                            f2 Iy, f2 Iz,
                                             f2 NTx, f2 NTy, f2 NTz, float damp_r2, f2& FX, f2& FY, f2& FZ,
                                             f2& GX, f2& GY, f2& GZ) {
     f2 DX = sub2(PX, x.OX), DY = sub2(PY, x.OY), DZ = sub2(PZ, x.OZ);
@@ -2048,7 +2049,8 @@ __global__ void k_energy_items_done(PairParams P, const float4* __restrict__ pos
                                     const float4* __restrict__ indv, const int* __restrict__ order,
                                     const double* __restrict__ pos, const int* __restrict__ exc_off,
                                     const int* __restrict__ exc_j, const double* __restrict__ exc_m,
-                                    const double* __restrict__ exc_s, IndexRecords R, unsigned long long* __restrict__ axis_count,
+                                    const double* __restrict__ exc_s, IndexRecords R,
+                                    unsigned long long* __restrict__ axis_count,
                                     int n_pad, unsigned long long* __restrict__ acc, double inv_scale, int n_items,
                                     const double* __restrict__ energy_item, double* __restrict__ fpair,
                                     double* __restrict__ torque, double* __restrict__ energy_block) {
@@ -2479,7 +2481,8 @@ void launch_energy<float>(const Dev& d, cudaStream_t st) {
     fix.scale = d.fix_scale_energy;
     const IndexRecords rec{(const float4*)d.posq, d.tctr, pq, dp, u};
     const EItemArrays A{pq, dp, u, d.order, d.tctr_s, d.text_s, d.pos_s, d.exs_off, d.exs_j, d.exs_m, d.exs_s,
-                        d.exs_tiles, rec, AxisList{d.axis_pairs, d.axis_count, (unsigned long long)d.axis_cap}, fix, L, d.n_pad};
+                        d.exs_tiles, rec, AxisList{d.axis_pairs, d.axis_count, (unsigned long long)d.axis_cap}, fix, L,
+                        d.n_pad};
     if (d.pp.lab_energy && !d.pp.periodic) k_energy_items<false, true><<<grid, 32, 0, st>>>(d.pp, A, d.energy_partial);
     else if (d.pp.lab_energy) k_energy_items<false, false><<<grid, 32, 0, st>>>(d.pp, A, d.energy_partial);
     else k_energy_items<true, false><<<grid, 32, 0, st>>>(d.pp, A, d.energy_partial);
