@@ -2486,7 +2486,7 @@ void launch_energy<float>(const Dev& d, cudaStream_t st) {
     if (d.pp.lab_energy && !d.pp.periodic) k_energy_items<false, true><<<grid, 32, 0, st>>>(d.pp, A, d.energy_partial);
     else if (d.pp.lab_energy) k_energy_items<false, false><<<grid, 32, 0, st>>>(d.pp, A, d.energy_partial);
     else k_energy_items<true, false><<<grid, 32, 0, st>>>(d.pp, A, d.energy_partial);
-    k_axis_pairs<<<148, 32, 0, st>>>(d.pp, A, (int)grid.x);
+    k_axis_pairs<<<std::min(8 * 148, std::max(148, d.pp.n_tiles)), 32, 0, st>>>(d.pp, A, (int)grid.x);
     k_energy_items_done<<<d.n_pad / 128, 128, 0, st>>>(d.pp, pq, dp, u, d.order, d.pos_s, d.exs_off, d.exs_j, d.exs_m,
                                                        d.exs_s, rec, d.axis_count, d.n_pad, d.fixacc,
                                                        1.0 / fix.scale, d.n_eblk,
