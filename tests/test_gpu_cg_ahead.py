@@ -22,6 +22,8 @@ def test_matvec_after_the_last_iteration(precision, kernel):
             torch.cuda.synchronize()
         steps = k.solverStats()["iterations"]
     us = [e.device_time for e in p.events() if kernel in e.name.replace("(int)", "")]
+    if not us:
+        pytest.skip("the profiler records no kernels here")
     # one walk a step, one queued ahead of the stop, perhaps one for the true residual
     assert steps + 1 <= len(us) <= steps + 3
     assert sum(t > 0.5 * np.median(us) for t in us) <= len(us) - 1
